@@ -467,13 +467,15 @@ def main() -> None:
             dist.barrier()
         torch.cuda.synchronize(dev)
 
-    # launches per layer: fused router (linear + top-k + plan), gate/up, down, combine (+3 for a shared expert);
-    # expert parallel adds the local plan kernel (the NCCL and torch kernels are not counted)
-    launches_per_layer = 4 + (3 if cfg.n_shared else 0) + (1 if use_ep else 0)
+    # launches per layer: fused router (linear + top-k + plan), gate/up, down, combine (+2 for a shared expert); above
+    # eight rows the router is three launches and each matmul has its row preparation in front.  Expert parallel adds the
+    # local plan kernel (the NCCL and torch kernels are not counted)
+    launches_per_layer = (4 if T * (world if use_ep else 1) <= 8 else 8) + (1 if use_ep else 0)
+    launches_per_layer += (2 if T <= 8 else 4) if cfg.n_shared else 0
     one_launch = ep_peer or ((not use_ep) and layers[0].fused and layers[0].fused_workspace_bytes(T) > 0)
     if one_launch:
         launches_per_layer = 1  # zmoe_layer_decode: the whole block, shared expert included
-    elif (not use_ep) and layers[0].fused and getattr(layers[0], "_chunked_ok", lambda t: False)(T):
+    elif (not use_ep) and layers[0].fused and layers[0]._passes_win(T) and layers[0]._chunked_ok(T):
         one_launch = True  # consecutive one-launch passes over eight rows each
         launches_per_layer = len(layers[0]._chunks(T))
 

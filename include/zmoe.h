@@ -173,6 +173,23 @@ int zmoe_gather_qmm(const void* x, int x_rows, int ldx, const uint32_t* w, const
                     int E, int N, int K, int group_size, int qmode, const void* plan, int rows, int rows_hint,
                     int x_by_output_row, void* out, void* stream);
 
+/*
+ * The same two calls for a caller that brings a workspace, where one helps: zmoe_qmm_workspace_bytes says how large
+ * (0: this call gains nothing from one).  rows, E, K and rows_hint as in the call.  The workspace (256-byte aligned
+ * device memory, contents irrelevant) then holds the token rows in expert order in the tensor cores' own format while
+ * the call runs; a call whose workspace is NULL or too small, or whose pointers the tensor maps cannot take (packed
+ * weights 16-byte aligned), is served by the kernels of the calls above.  One workspace serves one stream at a time.
+ */
+size_t zmoe_qmm_workspace_bytes(int rows, int E, int K, int rows_hint, int qmode);
+int zmoe_gather_qmm_swiglu_ws(const void* x, int x_rows, int ldx, const uint32_t* gate_w, const void* gate_scales,
+                              const void* gate_biases, const uint32_t* up_w, const void* up_scales,
+                              const void* up_biases, int E, int N, int K, int group_size, int qmode,
+                              const void* plan, int rows, int rows_hint, void* out, int swiglu_mode, void* workspace,
+                              size_t workspace_bytes, void* stream);
+int zmoe_gather_qmm_ws(const void* x, int x_rows, int ldx, const uint32_t* w, const void* scales, const void* biases,
+                       int E, int N, int K, int group_size, int qmode, const void* plan, int rows, int rows_hint,
+                       int x_by_output_row, void* out, void* workspace, size_t workspace_bytes, void* stream);
+
 /* ------------------------------------------------------------------- combine */
 
 /*

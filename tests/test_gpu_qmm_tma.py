@@ -1,0 +1,122 @@
+"""GPU: the grouped matmul that is fed through tensor memory (csrc/qmm_tma.cu) against float64, and against the register-fed
+kernels that serve the same call without a workspace.
+
+Sizes sit at the edges of its tiles: one to several token blocks per expert with ragged ends, output rows that do not
+fill a tile of 128 (64 for gate and up), the smallest K, one expert and many, experts without rows.
+"""
+
+import pytest
+import torch
+
+from zmlx_b200 import _lib, ops, quant
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _bank(g, E, N, K, mode, spread):
+    w = torch.randn((E, N, K), generator=g, device=DEV) * 0.02
+    if spread:  # scales over 12 binades inside a row
+        s = torch.exp2(torch.randint(-6, 7, (E, N, K // 64, 1), generator=g, device=DEV).float())
+        w = (w.view(E, N, K // 64, 64) * s).view(E, N, K)
+    if mode == "affine":
+        p, s, b = quant.quantize_affine(w, 64)
+        return (p, s, b), quant.dequantize_affine(p, s, b, 64).double()
+    p, s = quant.quantize_mxfp4(w)
+    return (p, s, None), quant.dequantize_mxfp4(p, s).double()
+
+
+def _call(x, T, K, banks, E, N, mode, plan, rows, hint, by_dst, ws):
+    lib, p, st = _lib.load(), ops._ptr, ops._stream()
+    gs, qm = (64 if mode == "affine" else 32), ops.qmode_code(mode)
+    out = torch.full((rows, N), float("nan"), dtype=torch.bfloat16, device=DEV)
+    w = ops._ws_args(ws)
+    if len(banks) == 1:
+        (a,) = banks
+        _lib.check(lib.zmoe_gather_qmm_ws(p(x), T, K, p(a[0]), p(a[1]), p(a[2]), E, N, K, gs, qm, p(plan), rows, hint,
+                                          by_dst, p(out), *w, st))
+    else:
+        a, u = banks
+        _lib.check(lib.zmoe_gather_qmm_swiglu_ws(p(x), T, K, p(a[0]), p(a[1]), p(a[2]), p(u[0]), p(u[1]), p(u[2]), E, N,
+                                                 K, gs, qm, p(plan), rows, hint, p(out), _lib.SWIGLU_CPU, *w, st))
+    torch.cuda.synchronize()
+    assert int(plan[2]) == 0
+    return out
+
+
+def _within(got, ref, mass, K):
+    """The result's bfloat16 rounding (half an ulp: 2^-8 relative) plus fp32 sums: a chunk adds 272 products, then the
+    chunks are added, each step within 2^-23 of the partial sums, which the sum of magnitudes `mass` bounds."""
+    bound = 2.0 ** -8 * ref.abs() + (272 + K // 256) * 2.0 ** -23 * mass
+    bad = (got.double() - ref).abs() > bound
+    assert not bool(bad.any()), f"{int(bad.sum())} of {bad.numel()} outside"
+
+
+CASES = [
+    # E, N, K, rows of each expert
+    (1, 64, 256, [9]), (1, 200, 768, [16]), (2, 128, 512, [17, 15]), (3, 72, 1024, [96, 97, 0]),
+    (4, 136, 2048, [1, 193, 33, 64]), (8, 256, 256, [12, 0, 3, 48, 49, 1, 0, 25]), (2, 192, 7168, [95, 289]),
+    (40, 128, 768, [i % 5 for i in range(40)]), (300, 64, 256, [2] * 300),
+]
+
+
+@pytest.mark.parametrize("mode", ["affine", "mxfp4"])
+@pytest.mark.parametrize("spread", [False, True])
+@pytest.mark.parametrize("case", range(len(CASES)))
+def test_matches_float64_and_the_register_fed_kernels(case, spread, mode):
+    E, N, K, counts = CASES[case]
+    g = torch.Generator(device=DEV).manual_seed(100 + case)
+    rows = sum(counts)
+    ids = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))
+    ids = ids[torch.randperm(rows, generator=torch.Generator().manual_seed(case))].to(DEV)
+    plan = ops.build_plan(ids, E)
+    x = torch.randn((rows, K), generator=g, device=DEV)
+    x *= torch.exp2(torch.randint(-20, 12, (rows, 1), generator=g, device=DEV).float())  # rows of very different size
+    x = x.to(torch.bfloat16)
+    a, A = _bank(g, E, N, K, mode, spread)
+    u, U = _bank(g, E, N, K, mode, spread)
+    ws = ops.qmm_workspace(rows, E, K, rows_hint=rows, mode=mode, device=DEV)
+    assert ws is not None
+    ref = torch.empty((rows, N), dtype=torch.float64, device=DEV)
+    up, mass, up_mass = torch.empty_like(ref), torch.empty_like(ref), torch.empty_like(ref)
+    for e in range(E):
+        m = ids == e
+        xe = x[m].double()
+        ref[m], up[m], mass[m], up_mass[m] = xe @ A[e].T, xe @ U[e].T, xe.abs() @ A[e].abs().T, xe.abs() @ U[e].abs().T
+    got = _call(x, rows, K, [a], E, N, mode, plan, rows, rows, case & 1, ws)
+    _within(got, ref, mass, K)
+    assert torch.equal(got, _call(x, rows, K, [a], E, N, mode, plan, rows, rows, case & 1, ws))
+    h = _call(x, rows, K, [a, u], E, N, mode, plan, rows, rows, 0, ws)
+    old = _call(x, rows, K, [a, u], E, N, mode, plan, rows, rows, 0, None)
+    assert torch.equal(h, _call(x, rows, K, [a, u], E, N, mode, plan, rows, rows, 0, ws))
+    if not spread:  # gate and up round to bfloat16 first: at most a few of them fall to the other side of a boundary
+        differ = (h != old) & ~(h.isnan() & old.isnan())
+        # rows far below 2^-14 lose bits in the fp16 staging of the older kernels: compare the ordinary ones
+        ordinary = (x.float().abs().amax(1) > 2.0 ** -6)[:, None]
+        assert float((differ & ordinary).float().mean()) < 0.01
+        gv, uv = ref.to(torch.bfloat16).double(), up.to(torch.bfloat16).double()
+        want = gv * torch.sigmoid(gv) * uv
+        err = (h.double() - want).abs()
+        # gate and up may round to the neighbour (2^-7 of them; |silu'| <= 1.1), their fp32 sums are off as in _within,
+        # and the result rounds once (2^-8)
+        sums = (272 + K // 256) * 2.0 ** -23
+        bound = 1.1 * (2.0 ** -7 * gv.abs() + sums * mass) * uv.abs() + (2.0 ** -7 + 2.0 ** -8) * want.abs() + \
+            (gv * torch.sigmoid(gv)).abs() * sums * up_mass + 1e-30
+        assert bool((err <= 1.01 * bound).all())
+
+
+@pytest.mark.parametrize("tokens", [96 * 3 + 5, 1400])
+def test_repeated_calls_give_the_same_bits_under_load(tokens):
+    """Many items per CTA, full token tiles: a hand-over between the kernel's roles that is not ordered shows as a
+    rare difference between runs."""
+    E, N, K, top = 16, 768, 2048, 4
+    g = torch.Generator(device=DEV).manual_seed(7)
+    a, _ = _bank(g, E, N, K, "affine", False)
+    u, _ = _bank(g, E, N, K, "affine", False)
+    x = torch.randn((tokens, K), generator=g, device=DEV).to(torch.bfloat16)
+    ids = torch.rand((tokens, E), generator=g, device=DEV).topk(top, dim=-1).indices.to(torch.int32)
+    plan = ops.build_plan(ids.reshape(-1), E, lhs_div=top)
+    ws = ops.qmm_workspace(tokens * top, E, K, rows_hint=tokens, mode="affine", device=DEV)
+    first = _call(x, tokens, K, [a, u], E, N, "affine", plan, tokens * top, tokens, 0, ws)
+    for _ in range(20):
+        assert torch.equal(first, _call(x, tokens, K, [a, u], E, N, "affine", plan, tokens * top, tokens, 0, ws))

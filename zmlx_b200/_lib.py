@@ -74,6 +74,12 @@ SIGNATURES = {
                                        c_int, c_void_p]),
     "zmoe_gather_qmm": (c_int, [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                                 c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p]),
+    "zmoe_qmm_workspace_bytes": (c_size_t, [c_int, c_int, c_int, c_int, c_int]),
+    "zmoe_gather_qmm_swiglu_ws": (c_int, [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                                          c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int,
+                                          c_void_p, c_int, c_void_p, c_size_t, c_void_p]),
+    "zmoe_gather_qmm_ws": (c_int, [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
+                                   c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_size_t, c_void_p]),
     "zmoe_moe_combine": (c_int, [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int,
                                  c_void_p, c_void_p]),
     "zmoe_swiglu": (c_int, [c_void_p, c_void_p, ctypes.c_longlong, c_int, c_void_p, c_void_p]),

@@ -8,7 +8,8 @@ namespace zmoe {
 
 int qmm_launch(int nmat, const void* x, int x_rows, int ldx, const uint32_t* const* w, const void* const* s,
                const void* const* b, int E, int N, int K, int group_size, int qmode, const void* plan, int rows,
-               int rows_hint, void* out, int epilogue, int x_by_dst, void* stream, const char* who);
+               int rows_hint, void* out, int epilogue, int x_by_dst, void* ws, size_t ws_bytes, void* stream,
+               const char* who);
 
 __device__ __forceinline__ float load_as_float(const void* p, int dtype, size_t i) {
   if (dtype == ZMOE_F32) return reinterpret_cast<const float*>(p)[i];
@@ -207,7 +208,7 @@ int zmoe_gather_qmm_combine(const void* act, int ldx, const uint32_t* w_, const 
     cudaError_t e = cudaMemsetAsync(scratch, 0, (size_t)T * K * N * sizeof(__nv_bfloat16), (cudaStream_t)stream);
     if (e != cudaSuccess) return fail(ZMOE_ERR_CUDA, "zmoe_gather_qmm_combine: clearing the scratch: %s", cudaGetErrorString(e));
   }
-  int rc = qmm_launch(1, act, T * K, ldx, w, s, b, E, N, Kin, group_size, qmode, plan, T * K, T, scratch, 0, 1, stream,
+  int rc = qmm_launch(1, act, T * K, ldx, w, s, b, E, N, Kin, group_size, qmode, plan, T * K, T, scratch, 0, 1, nullptr, 0, stream,
                       "zmoe_gather_qmm_combine");
   if (rc != ZMOE_OK) return rc;
   return combine_launch(scratch, ZMOE_BF16, gate, gate_dtype, T, K, N, mode, out, out_t, nullptr, stream,

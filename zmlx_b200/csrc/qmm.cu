@@ -485,9 +485,14 @@ static int launch_nmat(const QmmParams& p, const QmmChoice& c, int max_groups, c
   return fail(ZMOE_ERR_UNSUPPORTED, "qmm: no kernel for wk=%d wm=%d", c.wk, c.wm);
 }
 
+bool qmm_tma_covers(const QmmParams& q, int nmat, bool mx, int rows_hint, const void* ws, size_t ws_bytes);
+int qmm_tma_launch(const QmmParams& q, int nmat, bool mx, int rows_hint, int max_groups, void* ws, cudaStream_t st,
+                   const char* who);
+
 int qmm_launch(int nmat, const void* x, int x_rows, int ldx, const uint32_t* const* w, const void* const* s,
                const void* const* b, int E, int N, int K, int group_size, int qmode, const void* plan, int rows,
-               int rows_hint, void* out, int epilogue, int x_by_dst, void* stream, const char* who) {
+               int rows_hint, void* out, int epilogue, int x_by_dst, void* ws, size_t ws_bytes, void* stream,
+               const char* who) {
   ZMOE_REQUIRE(x && plan && out, ZMOE_ERR_SHAPE, "%s: null pointer", who);
   for (int m = 0; m < nmat; ++m)
     ZMOE_REQUIRE(w[m] && s[m], ZMOE_ERR_SHAPE, "%s: null weight or scale pointer", who);
@@ -529,6 +534,8 @@ int qmm_launch(int nmat, const void* x, int x_rows, int ldx, const uint32_t* con
   p.x_by_dst = x_by_dst & 1;
   p.late_wait = (x_by_dst & 2) ? 1 : 0;
 
+  if (qmm_tma_covers(p, nmat, mx, rows_hint, ws, ws_bytes))
+    return qmm_tma_launch(p, nmat, mx, rows_hint, rows < E ? rows : E, ws, (cudaStream_t)stream, who);
   if (mx) {
     int mg = rows < E ? rows : E;
     if (mg > 65535) mg = 65535;
@@ -576,10 +583,11 @@ using namespace zmoe;
 
 extern "C" {
 
-int zmoe_gather_qmm_swiglu(const void* x, int x_rows, int ldx, const uint32_t* gate_w, const void* gate_scales,
-                           const void* gate_biases, const uint32_t* up_w, const void* up_scales,
-                           const void* up_biases, int E, int N, int K, int group_size, int qmode,
-                           const void* plan, int rows, int rows_hint, void* out, int swiglu_mode, void* stream) {
+int zmoe_gather_qmm_swiglu_ws(const void* x, int x_rows, int ldx, const uint32_t* gate_w, const void* gate_scales,
+                              const void* gate_biases, const uint32_t* up_w, const void* up_scales,
+                              const void* up_biases, int E, int N, int K, int group_size, int qmode,
+                              const void* plan, int rows, int rows_hint, void* out, int swiglu_mode, void* workspace,
+                              size_t workspace_bytes, void* stream) {
   ZMOE_REQUIRE(swiglu_mode == ZMOE_SWIGLU_CPU || swiglu_mode == ZMOE_SWIGLU_PER_OP ||
                    (swiglu_mode == ZMOE_SWIGLU_FP32 && qmode == ZMOE_Q_AFFINE4),
                ZMOE_ERR_UNSUPPORTED,
@@ -588,18 +596,33 @@ int zmoe_gather_qmm_swiglu(const void* x, int x_rows, int ldx, const uint32_t* g
   const void* s[2] = {gate_scales, up_scales};
   const void* b[2] = {gate_biases, up_biases};
   return qmm_launch(2, x, x_rows, ldx, w, s, b, E, N, K, group_size, qmode, plan, rows, rows_hint, out,
-                    swiglu_mode == ZMOE_SWIGLU_CPU ? 1 : (swiglu_mode == ZMOE_SWIGLU_PER_OP ? 2 : 3), 0, stream,
-                    "zmoe_gather_qmm_swiglu");
+                    swiglu_mode == ZMOE_SWIGLU_CPU ? 1 : (swiglu_mode == ZMOE_SWIGLU_PER_OP ? 2 : 3), 0, workspace,
+                    workspace_bytes, stream, "zmoe_gather_qmm_swiglu");
+}
+
+int zmoe_gather_qmm_swiglu(const void* x, int x_rows, int ldx, const uint32_t* gate_w, const void* gate_scales,
+                           const void* gate_biases, const uint32_t* up_w, const void* up_scales,
+                           const void* up_biases, int E, int N, int K, int group_size, int qmode,
+                           const void* plan, int rows, int rows_hint, void* out, int swiglu_mode, void* stream) {
+  return zmoe_gather_qmm_swiglu_ws(x, x_rows, ldx, gate_w, gate_scales, gate_biases, up_w, up_scales, up_biases, E, N, K,
+                                   group_size, qmode, plan, rows, rows_hint, out, swiglu_mode, nullptr, 0, stream);
+}
+
+int zmoe_gather_qmm_ws(const void* x, int x_rows, int ldx, const uint32_t* w_, const void* scales, const void* biases,
+                       int E, int N, int K, int group_size, int qmode, const void* plan, int rows, int rows_hint,
+                       int x_by_output_row, void* out, void* workspace, size_t workspace_bytes, void* stream) {
+  const uint32_t* w[2] = {w_, nullptr};
+  const void* s[2] = {scales, nullptr};
+  const void* b[2] = {biases, nullptr};
+  return qmm_launch(1, x, x_rows, ldx, w, s, b, E, N, K, group_size, qmode, plan, rows, rows_hint, out, 0,
+                    x_by_output_row, workspace, workspace_bytes, stream, "zmoe_gather_qmm");
 }
 
 int zmoe_gather_qmm(const void* x, int x_rows, int ldx, const uint32_t* w_, const void* scales, const void* biases,
                     int E, int N, int K, int group_size, int qmode, const void* plan, int rows, int rows_hint,
                     int x_by_output_row, void* out, void* stream) {
-  const uint32_t* w[2] = {w_, nullptr};
-  const void* s[2] = {scales, nullptr};
-  const void* b[2] = {biases, nullptr};
-  return qmm_launch(1, x, x_rows, ldx, w, s, b, E, N, K, group_size, qmode, plan, rows, rows_hint, out, 0,
-                    x_by_output_row, stream, "zmoe_gather_qmm");
+  return zmoe_gather_qmm_ws(x, x_rows, ldx, w_, scales, biases, E, N, K, group_size, qmode, plan, rows, rows_hint,
+                            x_by_output_row, out, nullptr, 0, stream);
 }
 
 }  // extern "C"

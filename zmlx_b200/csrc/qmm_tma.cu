@@ -1,0 +1,780 @@
+// Token-grouped 4-bit expert matmul on the 5th-generation tensor cores, fed through tensor memory: the path of every
+// call that brings a workspace and more than a few token rows (serving batches and prompts, affine and mxfp4 banks).
+//
+// What bounds it: at a few rows per expert the packed weights' way from HBM, at many rows the token tiles' way from
+// L2 (one SM reads 128 weight rows x 256 codes = 18 KB against 544 B per token row for them).  So the packed codes
+// must be expanded at the rate at which they arrive, and the token side must cost nothing but the copy:
+//
+//   prep_rows_kernel  writes, once per call, every token row in expert-sorted order as fp16 under a per-row power of
+//              two, and beside it the row's group sums as two fp16 pieces.  A token tile is then a plain TMA box
+//              with the 128-byte swizzle the tensor core reads, whatever the gather was.
+//   qmm_tma_kernel    one persistent CTA per SM walks items (expert, 128 weight rows, a block of token rows) as one
+//              unbroken stream of chunks of 256 codes:
+//     weights   one thread keeps kTmRaw boxes of 128 rows x 128 packed bytes in flight;
+//     tokens    one thread keeps the ring of token tiles full;
+//     expanders two sets of 128 threads (one per weight row) turn every other chunk's codes into the fp16 A operand
+//               and store it straight into the set's stage in TENSOR MEMORY (tcgen05.st): no shared-memory round trip,
+//               no swizzle arithmetic; one set's waits and latencies lie under the other set's arithmetic;
+//     issuer    one thread issues tcgen05.mma (M 128 x N 16..96 x K 16, A in tensor memory, B in shared memory);
+//     finishers 256 threads fold the chunk's accumulator into fp32 registers and, at the end of an item, apply the
+//               SwiGLU contract and store bf16 rows through the plan.
+//
+// Arithmetic.  Affine: w = q s + b = (q - 8) s + (b + 8 s).  q - 8 has three bits and a sign, s eight: their product
+// is EXACT in fp16's eleven, so the scale goes into the operand and the accumulator runs over a whole chunk of four
+// groups.  The second term is one more K = 16 step against the group sums X = X1 + X2 (22 bits): per group the
+// columns (b, b, -8s, -8s) x (X1, X2, -X1, -X2).  The chunk's scales are first multiplied by a power of two per (row,
+// chunk) that puts max(8|s|, |b|) near 2^13, undone in fp32 by the finishers, so the range of fp16 is no limit on the
+// checkpoint's.  mxfp4: e2m1 value x 2^(e - emax + 11), exact in fp16 over 35 binades, same row factor.  Token rows
+// carry |x|max in [2^7, 2^8): a bfloat16 of that row is exact down to 2^-25 of its largest.  Chunks are summed in
+// fp32 registers rather than in the accumulator over all of K, so that no sum is longer than 272 products.
+//
+// gate and up share one accumulator: lanes 0-15 of each warp's 32 tensor-memory lanes hold gate rows, lanes 16-31 the
+// up rows of the same outputs, and the epilogue pairs them with one shuffle.
+//
+// Every wait is bounded by a second; one that runs out sets the plan's status word, everybody else leaves at the next
+// wait, copies and MMAs in flight are waited for, and the tensor memory is given back.
+#include <cuda.h>
+#include <cuda_fp16.h>
+
+#include "qmm_common.cuh"
+
+namespace zmoe {
+
+constexpr int kTmExp = 256, kTmFin = 256;
+constexpr int kTmThreads = kTmExp + kTmFin + 96;  // + one warp each: issuer, weight copies, token copies
+constexpr int kTmRows = 128;                      // tensor-memory lanes = weight rows of an item
+constexpr int kTmChunk = 256;                     // codes per chunk
+constexpr int kTmRaw = 5;                         // chunks of packed bytes in flight
+constexpr int kTmRawBytes = kTmRows * kTmChunk / 2;
+constexpr int kTmScRing = 4, kTmScAhead = 3;      // scales: a thread's chunks in the ring, copy distance
+constexpr int kTmMaxTok = 96;                     // token rows per item, at most
+constexpr int kTmMaxX = 8;                        // token stages, at most
+constexpr int kTmMaxTasks = 1024;
+constexpr int kTmCols = 512;
+constexpr int kTmColD = 128;                      // columns between the two accumulators
+constexpr int kTmColA = 224, kTmAStage = 136;     // two A stages: 128 columns of codes, 8 of scales and biases
+
+struct TmArgs {
+  CUtensorMap w[2];  // packed bytes (E*N, K/2): box 128 bytes x 128 (gate and up: 64) rows
+  CUtensorMap x;     // prepared rows (rows, K) fp16: box 64 x 16
+  CUtensorMap xb;    // their group sums (rows, K/16) fp16: box 16 x 16
+  QmmParams q;
+  const float* xinv;  // (rows): 1 / the row's power of two
+  int nch;            // K / 256
+  int tn;             // token rows per item, at most (a multiple of 16)
+  int rx;             // token stages
+  int xstage;         // bytes of one
+};
+
+__device__ __forceinline__ uint32_t tm_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void tm_bar_init(uint32_t bar, int count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
+}
+__device__ __forceinline__ void tm_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void tm_expect(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+// One look at a phase; the hardware may suspend the thread in it for up to `ns`, and wakes it when the phase completes.
+__device__ __forceinline__ bool tm_try(uint32_t bar, uint32_t parity, uint32_t ns) {
+  uint32_t ok;
+  asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3; selp.u32 %0, 1, 0, p; }"
+               : "=r"(ok)
+               : "r"(bar), "r"(parity), "r"(ns)
+               : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ unsigned long long tm_now() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+// Waits for the phase; false when a second passed or, unless `drain`, another thread of the CTA gave up.  Suspended
+// looks rather than a spin: polling warps would take the issue slots that the expanders live on.
+__device__ __forceinline__ bool tm_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, bool drain = false) {
+  for (int i = 0; i < 8; ++i)
+    if (tm_try(bar, parity, 20000u)) return true;
+  const unsigned long long t0 = tm_now();
+  while (true) {
+    if (tm_try(bar, parity, 20000u)) return true;
+    if (!drain && *abort_flag) return false;
+    if (tm_now() - t0 > 1000000000ull) {
+      *abort_flag = 1;
+      return false;
+    }
+  }
+}
+// The same for a whole warp: all lanes leave together, as the tcgen05.ld and .st that follow need them to.
+__device__ __forceinline__ bool tm_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, tm_wait(bar, parity, abort_flag));
+}
+__device__ __forceinline__ void tm_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+          dst),
+      "l"(map), "r"(x), "r"(y), "r"(bar)
+      : "memory");
+}
+// Shared-memory descriptors of K-major tiles: rows of 128 (32) bytes under the 128-byte (32-byte) swizzle, eight rows
+// per atom.
+__device__ __forceinline__ uint64_t tm_desc128(uint32_t addr) {
+  return (uint64_t)((addr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
+}
+__device__ __forceinline__ uint64_t tm_desc32(uint32_t addr) {
+  return (uint64_t)((addr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)(256 >> 4) << 32) | (1ull << 46) | (6ull << 61);
+}
+// D fp32, A and B fp16, both K-major, M = 128, N = n.
+__device__ __forceinline__ uint32_t tm_idesc(int n) {
+  return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kTmRows >> 4) << 24);
+}
+__device__ __forceinline__ void tm_mma(uint32_t d, uint32_t a, uint64_t bdesc, uint32_t idesc, bool accumulate) {
+  asm volatile("{ .reg .pred p; setp.ne.b32 p, %4, 0; tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p; }" ::"r"(d),
+               "r"(a), "l"(bdesc), "r"(idesc), "r"((uint32_t)accumulate)
+               : "memory");
+}
+__device__ __forceinline__ void tm_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void tm_ld16(uint32_t taddr, float (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7]), "=f"(r[8]),
+        "=f"(r[9]), "=f"(r[10]), "=f"(r[11]), "=f"(r[12]), "=f"(r[13]), "=f"(r[14]), "=f"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tm_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(
+          taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+__device__ __forceinline__ void tm_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]),
+               "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+// One lane of a converged warp.  The compiler knows an elected thread to be alone; behind `lane == 0` it would wrap
+// every tcgen05.mma and TMA instruction in a loop over the lanes that might be active (measured: 190 cycles per MMA
+// whatever its shape, 17 of them per chunk).
+__device__ __forceinline__ bool tm_elect() {
+  uint32_t one;
+  asm volatile("{ .reg .pred p; elect.sync _|p, 0xffffffff; selp.u32 %0, 1, 0, p; }" : "=r"(one));
+  return one != 0;
+}
+__device__ __forceinline__ uint32_t tm_bits(__half2 h) { return *reinterpret_cast<const uint32_t*>(&h); }
+__device__ __forceinline__ __half2 tm_half2(uint32_t u) { return *reinterpret_cast<const __half2*>(&u); }
+
+// Eight codes of a packed word times the group's scale, as four half2 in the order (0,4) (1,5) (2,6) (3,7) that the
+// token rows are written in.  A nibble at bits 4-7 of a half IS the fp16 number q 2^-20 (subnormal or not), so one
+// fused multiply-add gives q 2^-20 (s 2^20) - 8 s = (q - 8) s, exact: three shifts, four masks, four half2 operations
+// per eight codes.
+__device__ __forceinline__ void tm_expand_affine(uint32_t w, __half2 s20, __half2 m8s, uint32_t* out) {
+  const uint32_t m = 0x00F000F0u;
+  out[0] = tm_bits(__hfma2(tm_half2((w << 4) & m), s20, m8s));
+  out[1] = tm_bits(__hfma2(tm_half2(w & m), s20, m8s));
+  out[2] = tm_bits(__hfma2(tm_half2((w >> 4) & m), s20, m8s));
+  out[3] = tm_bits(__hfma2(tm_half2((w >> 8) & m), s20, m8s));
+}
+// Eight e2m1 codes in their own order, times the block's power of two.
+__device__ __forceinline__ void tm_expand_mx(uint32_t w, __half2 s, uint32_t* out) {
+  uint32_t a, b, c, d;
+  asm("{ .reg .b8 t0, t1, t2, t3;\n"
+      "mov.b32 {t0, t1, t2, t3}, %4;\n"
+      "cvt.rn.f16x2.e2m1x2 %0, t0;\n"
+      "cvt.rn.f16x2.e2m1x2 %1, t1;\n"
+      "cvt.rn.f16x2.e2m1x2 %2, t2;\n"
+      "cvt.rn.f16x2.e2m1x2 %3, t3; }"
+      : "=r"(a), "=r"(b), "=r"(c), "=r"(d)
+      : "r"(w));
+  out[0] = tm_bits(__hmul2(tm_half2(a), s));
+  out[1] = tm_bits(__hmul2(tm_half2(b), s));
+  out[2] = tm_bits(__hmul2(tm_half2(c), s));
+  out[3] = tm_bits(__hmul2(tm_half2(d), s));
+}
+
+// One item of the work list: token rows [p0, p0 + nt) of the sorted order against rows n0.. of expert e.
+struct TmItem {
+  int e, p0, nt, n0;
+};
+// Items are numbered task-major; inside a task the token blocks of one row tile are neighbours, so that they run at
+// the same time on different SMs and share the weights through L2.  prefix[a] = token blocks of the tasks before a.
+__device__ __forceinline__ TmItem tm_item(const PlanView& pv, const int* prefix, int ntasks, int ntiles, int tile_rows,
+                                          int w) {
+  int lo = 0, hi = ntasks - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (ntiles * prefix[mid] <= w) lo = mid; else hi = mid - 1;
+  }
+  const int local = w - ntiles * prefix[lo];
+  const int nblk = prefix[lo + 1] - prefix[lo];
+  const int tile = local / nblk, blk = local - tile * nblk;
+  const int4 task = __ldg(reinterpret_cast<const int4*>(pv.tasks) + lo);  // {expert, offset, count, -}
+  const int per = ((task.z + nblk - 1) / nblk + 15) & ~15;                // equal blocks, whole 16s
+  TmItem it;
+  it.e = task.x;
+  it.p0 = task.y + blk * per;
+  it.nt = min(per, task.z - blk * per);
+  it.n0 = tile * tile_rows;
+  return it;
+}
+
+template <bool MX, int NMAT>
+__global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_constant__ TmArgs a) {
+  extern __shared__ __align__(1024) unsigned char tm_dyn[];
+  __shared__ uint32_t tmem_base_s;
+  // raw full / empty, token full / empty, A full, MMAs done, accumulator free
+  __shared__ __align__(8) unsigned long long bars_s[2 * kTmRaw + 2 * kTmMaxX + 6];
+  __shared__ float inv_s[4][kTmRows];
+  __shared__ volatile int abort_s;
+  __shared__ int prefix_s[kTmMaxTasks + 1];
+
+  constexpr int kTile = kTmRows / NMAT;  // output rows of an item
+  const QmmParams& p = a.q;
+  const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
+  const int N = p.N, nch = a.nch, tn = a.tn, rx = a.rx;
+  const PlanView pv = plan_view(const_cast<int*>(p.plan), p.rows, p.E);
+  unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tm_dyn) + 1023) & ~(uintptr_t)1023);
+  unsigned char* raw = base;
+  unsigned char* tok = raw + kTmRaw * kTmRawBytes;
+  unsigned char* scr = tok + rx * a.xstage;  // [slot][expander thread][16 bytes]
+  const uint32_t bars = tm_smem(bars_s);
+  const uint32_t b_rawf = bars, b_rawe = bars + 8 * kTmRaw, b_tokf = bars + 16 * kTmRaw;
+  const uint32_t b_toke = b_tokf + 8 * kTmMaxX, b_af = b_toke + 8 * kTmMaxX, b_done = b_af + 16, b_dfree = b_done + 16;
+
+  pdl_wait();
+  pdl_trigger();
+  const int ntasks = min(pv.hdr[0], kTmMaxTasks);
+  if (wid == 0) {  // token blocks per task, prefix-summed (lane = a contiguous run of tasks)
+    const int per = (ntasks + 31) >> 5;
+    int sum = 0;
+    for (int i = lane * per; i < min(ntasks, (lane + 1) * per); ++i) sum += (__ldg(pv.tasks + 4 * i + 2) + tn - 1) / tn;
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    int run = incl - sum;
+    for (int i = lane * per; i < min(ntasks, (lane + 1) * per); ++i) {
+      prefix_s[i] = run;
+      run += (__ldg(pv.tasks + 4 * i + 2) + tn - 1) / tn;
+    }
+    if (lane == 31) prefix_s[ntasks] = incl;
+  }
+  __syncthreads();
+  const int ntiles = (N + kTile - 1) / kTile;
+  const int total = ntiles * prefix_s[ntasks];
+  if ((int)blockIdx.x >= total) return;  // before any tensor memory is taken
+  const int n_items = (total - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int n_chunks = n_items * nch;
+
+  if (tid == 0) {
+    for (int i = 0; i < kTmRaw; ++i) {
+      tm_bar_init(b_rawf + 8 * i, 1);
+      tm_bar_init(b_rawe + 8 * i, kTmExp / 64);
+    }
+    for (int i = 0; i < kTmMaxX; ++i) {
+      tm_bar_init(b_tokf + 8 * i, 1);
+      tm_bar_init(b_toke + 8 * i, 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      tm_bar_init(b_af + 8 * i, kTmExp / 64);
+      tm_bar_init(b_done + 8 * i, 1);
+      tm_bar_init(b_dfree + 8 * i, kTmFin / 32);
+    }
+    abort_s = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (wid == 0) {
+    __syncwarp();
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tm_smem(&tmem_base_s)),
+                 "r"(kTmCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_base_s;
+  volatile int* ab = &abort_s;
+  bool ok = true;
+
+  if (wid < kTmExp / 32) {
+    // ================================================================== expanders: a weight row of every other chunk
+    const int q4 = wid & 3, set = wid >> 2;
+    const int r = q4 * 32 + lane;  // tensor-memory lane
+    const int mat = NMAT == 2 ? (lane >> 4) : 0;
+    const int rb = NMAT == 2 ? q4 * 16 + (lane & 15) : r;  // row inside the matrix's box
+    const uint32_t at = tmem + ((uint32_t)(q4 * 32) << 16) + kTmColA + set * kTmAStage;
+    const unsigned char* my_raw = raw + mat * (kTile * 128) + rb * 128;
+    unsigned char* my_sc = scr + tid * 16;
+    // the cursor of the scale copies runs kTmScAhead of the thread's chunks ahead
+    int f_item = 0, f_c = set, f_slot = 0;
+    bool f_new = true;
+    const unsigned char *f_s = nullptr, *f_b = nullptr;
+    auto fetch = [&] {
+      while (f_c >= nch) {
+        f_c -= nch;
+        ++f_item;
+        f_new = true;
+      }
+      if (f_item < n_items) {
+        if (f_new) {
+          f_new = false;
+          const TmItem it = tm_item(pv, prefix_s, ntasks, ntiles, kTile, (int)blockIdx.x + f_item * (int)gridDim.x);
+          const size_t row = (size_t)it.e * N + min(it.n0 + rb, N - 1);  // clamped rows are computed, not stored
+          // 8 bytes per chunk: four bfloat16 scales (biases) or eight e8m0 bytes
+          f_s = reinterpret_cast<const unsigned char*>(p.s[mat]) + row * nch * 8;
+          if (!MX) f_b = reinterpret_cast<const unsigned char*>(p.b[mat]) + row * nch * 8;
+        }
+        unsigned char* dst = my_sc + f_slot * (kTmExp * 16);
+        cp_async_8(dst, f_s + f_c * 8);
+        if (!MX) cp_async_8(dst + 8, f_b + f_c * 8);
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      f_c += 2;
+      f_slot = (f_slot + 1) % kTmScRing;
+    };
+#pragma unroll 1
+    for (int i = 0; i < kTmScAhead; ++i) fetch();
+    int rs = set, rph = 0, slot = 0;  // raw slot and its phase, scale slot
+#pragma unroll 1
+    for (int c = set; c < n_chunks; c += 2) {
+      fetch();
+      asm volatile("cp.async.wait_group %0;" ::"n"(kTmScAhead) : "memory");
+      const uint4 sc = *reinterpret_cast<const uint4*>(my_sc + slot * (kTmExp * 16));
+      slot = (slot + 1) % kTmScRing;
+      // ---- the chunk's power of two and its scales in fp16
+      __half2 s_op[MX ? 8 : 4], s_off[MX ? 1 : 4], b_op[MX ? 1 : 4];
+      float inv;
+      if (MX) {
+        uint32_t v = __vmaxu4(sc.x, sc.y);
+        v = __vmaxu4(v, v >> 16);
+        const int emax = (int)max(v & 0xffu, (v >> 8) & 0xffu);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {  // fp16 2^(e - emax + 11) in both halves; 0 from 26 binades below emax
+          const int e = (int)(((i < 4 ? sc.x : sc.y) >> (8 * (i & 3))) & 0xffu);
+          s_op[i] = tm_half2((uint32_t)max(e - emax + 26, 0) * 0x04000400u);
+        }
+        inv = emax >= 255 ? __uint_as_float(0x7f800000u) : exp2f((float)(emax - 127 - 11));
+      } else {
+        // largest |s| and |b| (bits order like magnitudes), as bfloat16 bits
+        uint32_t ms = __vmaxu2(sc.x & 0x7fff7fffu, sc.y & 0x7fff7fffu);
+        uint32_t mb = __vmaxu2(sc.z & 0x7fff7fffu, sc.w & 0x7fff7fffu);
+        ms = max(ms & 0xffffu, ms >> 16);
+        mb = max(mb & 0xffffu, mb >> 16);
+        // 2^(140 - e) brings |s| below 2^-4 (so that s 2^20 stays below 2^16) and |b| below 2^14
+        const int e = min(max(max((int)(ms >> 7) + 18, (int)(mb >> 7)), 34), 253);
+        const float P = __uint_as_float((uint32_t)(267 - e) << 23), P20 = __uint_as_float((uint32_t)(287 - e) << 23);
+        inv = __uint_as_float((uint32_t)(e - 13) << 23);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const uint32_t sw = i < 2 ? sc.x : sc.y, bw = i < 2 ? sc.z : sc.w;
+          const float s = __uint_as_float((i & 1) ? (sw & 0xffff0000u) : (sw << 16));
+          const float b = __uint_as_float((i & 1) ? (bw & 0xffff0000u) : (bw << 16));
+          s_op[i] = __float2half2_rn(s * P20);
+          s_off[i] = __float2half2_rn(s * (-8.0f * P));
+          b_op[i] = __float2half2_rn(b * P);
+        }
+      }
+      // ---- the stage is free once the MMAs of the thread's previous chunk are done
+      ok = tm_wait_warp(b_rawf + 8 * rs, rph, ab);
+      if (ok && c >= 2) ok = tm_wait_warp(b_done + 8 * set, ((c >> 1) - 1) & 1, ab);
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const unsigned char* src = my_raw + rs * kTmRawBytes;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {  // 32 codes each: half a group, or one mxfp4 block
+        const uint4 w4 = *reinterpret_cast<const uint4*>(src + ((i ^ (rb & 7)) << 4));
+        const uint32_t ws[4] = {w4.x, w4.y, w4.z, w4.w};
+        uint32_t o[16];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (MX)
+            tm_expand_mx(ws[k], s_op[i], o + 4 * k);
+          else
+            tm_expand_affine(ws[k], s_op[i >> 1], s_off[i >> 1], o + 4 * k);
+        }
+        tm_st16(at + i * 16, o);
+      }
+      if (!MX) {
+        uint32_t o[8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          o[2 * i] = tm_bits(b_op[i]);
+          o[2 * i + 1] = tm_bits(s_off[i]);
+        }
+        tm_st8(at + 128, o);
+      }
+      inv_s[c & 3][r] = inv;
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) {
+        tm_arrive(b_af + 8 * set);
+        tm_arrive(b_rawe + 8 * rs);
+      }
+      __syncwarp();
+      rs += 2;
+      if (rs >= kTmRaw) {
+        rs -= kTmRaw;
+        rph ^= 1;
+      }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  } else if (wid < (kTmExp + kTmFin) / 32) {
+    // ================================================================== finishers: weight row x every other 16 tokens
+    const int q4 = wid & 3, ch = (wid - kTmExp / 32) >> 2;
+    const int r = q4 * 32 + lane;
+    const uint32_t lane_base = tmem + ((uint32_t)(q4 * 32) << 16);
+    float acc[3][16];
+    int c = 0;
+#pragma unroll 1
+    for (int item = 0; item < n_items && ok; ++item) {
+      const TmItem it = tm_item(pv, prefix_s, ntasks, ntiles, kTile, (int)blockIdx.x + item * (int)gridDim.x);
+      int dst[3];     // output row and row factor of token 16 (ch + 2 j) + lane % 16
+      float xin[3];
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        const int t = 16 * (ch + 2 * j) + (lane & 15);
+        dst[j] = t < it.nt ? __ldg(pv.row_dst + it.p0 + t) : 0;
+        xin[j] = t < it.nt ? __ldg(a.xinv + it.p0 + t) : 0.0f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc[j][i] = 0.0f;
+      }
+#pragma unroll 1
+      for (int cc = 0; cc < nch; ++cc, ++c) {
+        const int buf = c & 1;
+        ok = tm_wait_warp(b_done + 8 * buf, (c >> 1) & 1, ab);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const float inv = inv_s[c & 3][r];
+        const uint32_t at = lane_base + buf * kTmColD;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          if (16 * (ch + 2 * j) < it.nt) {
+            float d[16];
+            tm_ld16(at + 16 * (ch + 2 * j), d);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int i = 0; i < 16; ++i) acc[j][i] = fmaf(d[i], inv, acc[j][i]);
+          }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) tm_arrive(b_dfree + 8 * buf);
+      }
+      if (!ok) break;
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        const int t0 = 16 * (ch + 2 * j);
+        if (t0 >= it.nt) break;
+        if (NMAT == 2) {
+          const int n = it.n0 + q4 * 16 + (lane & 15);
+          const bool hi = lane >= 16;  // the lower lanes finish the even tokens, the upper lanes the odd ones
+#pragma unroll
+          for (int i = 0; i < 16; i += 2) {
+            const float other = __shfl_xor_sync(0xffffffffu, hi ? acc[j][i] : acc[j][i + 1], 16);
+            const int k = hi ? i + 1 : i;
+            const float xs = __shfl_sync(0xffffffffu, xin[j], k);
+            const int row = __shfl_sync(0xffffffffu, dst[j], k);
+            if (t0 + k < it.nt && n < N) {
+              const float g = (hi ? other : acc[j][i]) * xs;
+              const float u = (hi ? acc[j][i + 1] : other) * xs;
+              p.out[(size_t)row * p.ldo + n] = __float2bfloat16_rn(swiglu_epilogue(p.epilogue, g, u));
+            }
+          }
+        } else {
+          const int n = it.n0 + r;
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const float xs = __shfl_sync(0xffffffffu, xin[j], i);
+            const int row = __shfl_sync(0xffffffffu, dst[j], i);
+            if (t0 + i < it.nt && n < N) p.out[(size_t)row * p.ldo + n] = __float2bfloat16_rn(acc[j][i] * xs);
+          }
+        }
+      }
+    }
+  } else if (wid == (kTmExp + kTmFin) / 32) {
+    // ================================================================== the warp that issues the MMAs (one lane does)
+    int c = 0;
+#pragma unroll 1
+    for (int item = 0; item < n_items && ok; ++item) {
+      const TmItem it = tm_item(pv, prefix_s, ntasks, ntiles, kTile, (int)blockIdx.x + item * (int)gridDim.x);
+      const uint32_t idesc = tm_idesc((it.nt + 15) & ~15);
+#pragma unroll 1
+      for (int cc = 0; cc < nch; ++cc, ++c) {
+        const int buf = c & 1, xs = c % rx;
+        ok = tm_wait_warp(b_tokf + 8 * xs, (c / rx) & 1, ab);
+        if (ok && c >= 2) ok = tm_wait_warp(b_dfree + 8 * buf, ((c >> 1) - 1) & 1, ab);
+        if (ok) ok = tm_wait_warp(b_af + 8 * buf, (c >> 1) & 1, ab);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t d = tmem + buf * kTmColD, at = tmem + kTmColA + buf * kTmAStage;
+        const uint32_t bt = tm_smem(tok + xs * a.xstage);
+        if (tm_elect()) {
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {
+            const uint64_t bd = tm_desc128(bt + g * tn * 128);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) tm_mma(d, at + g * 32 + k * 8, bd + 2 * k, idesc, (g | k) != 0);
+          }
+          if (!MX) tm_mma(d, at + 128, tm_desc32(bt + tn * 512), idesc, true);
+          tm_commit(b_done + 8 * buf);
+          tm_commit(b_toke + 8 * xs);
+        }
+        __syncwarp();
+      }
+    }
+    // MMAs in flight, and the arrivals they still owe
+    for (int i = max(c - 2, 0); i < c; ++i) tm_wait(b_done + 8 * (i & 1), (i >> 1) & 1, ab, true);
+    for (int i = max(c - rx, 0); i < c; ++i) tm_wait(b_toke + 8 * (i % rx), (i / rx) & 1, ab, true);
+  } else if (wid == (kTmExp + kTmFin) / 32 + 1) {
+    // ================================================================== the warp that copies packed weights
+    int c = 0;
+#pragma unroll 1
+    for (int item = 0; item < n_items && ok; ++item) {
+      const TmItem it = tm_item(pv, prefix_s, ntasks, ntiles, kTile, (int)blockIdx.x + item * (int)gridDim.x);
+      const int y = it.e * N + it.n0;  // a tile's rows beyond N are the next expert's: computed, not stored
+#pragma unroll 1
+      for (int cc = 0; cc < nch; ++cc, ++c) {
+        const int rs = c % kTmRaw;
+        if (c >= kTmRaw) ok = tm_wait_warp(b_rawe + 8 * rs, (c / kTmRaw - 1) & 1, ab);
+        if (!ok) break;
+        const uint32_t bar = b_rawf + 8 * rs, dst = tm_smem(raw + rs * kTmRawBytes);
+        if (tm_elect()) {
+          tm_expect(bar, kTmRawBytes);
+#pragma unroll
+          for (int m = 0; m < NMAT; ++m) tm_load_2d(dst + m * (kTile * 128), &a.w[m], cc * 128, y, bar);
+        }
+        __syncwarp();
+      }
+    }
+    for (int i = max(c - kTmRaw, 0); i < c; ++i) tm_wait(b_rawf + 8 * (i % kTmRaw), (i / kTmRaw) & 1, ab, true);
+  } else {
+    // ================================================================== the warp that copies token tiles
+    int c = 0;
+#pragma unroll 1
+    for (int item = 0; item < n_items && ok; ++item) {
+      const TmItem it = tm_item(pv, prefix_s, ntasks, ntiles, kTile, (int)blockIdx.x + item * (int)gridDim.x);
+      const int nb = (it.nt + 15) >> 4;
+#pragma unroll 1
+      for (int cc = 0; cc < nch; ++cc, ++c) {
+        const int xs = c % rx;
+        if (c >= rx) ok = tm_wait_warp(b_toke + 8 * xs, (c / rx - 1) & 1, ab);
+        if (!ok) break;
+        const uint32_t bar = b_tokf + 8 * xs, dst = tm_smem(tok + xs * a.xstage);
+        if (tm_elect()) {
+          tm_expect(bar, nb * (MX ? 8192 : 8192 + 512));
+          for (int b = 0; b < nb; ++b) {
+#pragma unroll
+            for (int g = 0; g < 4; ++g)
+              tm_load_2d(dst + g * tn * 128 + b * 2048, &a.x, cc * kTmChunk + g * 64, it.p0 + 16 * b, bar);
+            if (!MX) tm_load_2d(dst + tn * 512 + b * 512, &a.xb, cc * 16, it.p0 + 16 * b, bar);
+          }
+        }
+        __syncwarp();
+      }
+    }
+    for (int i = max(c - rx, 0); i < c; ++i) tm_wait(b_tokf + 8 * (i % rx), (i / rx) & 1, ab, true);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  if (abort_s && tid == 0) atomicExch(pv.hdr + 2, 2);  // the plan's status word: a bounded wait ran out
+  if (wid == 0) {
+    __syncwarp();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmCols) : "memory");
+  }
+}
+
+// ------------------------------------------------------------------ token rows in sorted order
+// One CTA per sorted row: |x|max, then fp16 values under 2^k with |x|max 2^k in [2^7, 2^8) and, for affine banks, the
+// sums of its groups of 64 as (X1, X2, -X1, -X2).  Affine rows take the order in which tm_expand_affine leaves codes.
+constexpr int kPrepThreads = 128;
+
+template <bool MX>
+__global__ void __launch_bounds__(kPrepThreads) prep_rows_kernel(const __nv_bfloat16* __restrict__ x, int ldx,
+                                                                 const int* plan, int rows, int E, int x_by_dst, int K,
+                                                                 __half* __restrict__ xs, float* __restrict__ xinv) {
+  __shared__ uint32_t warp_max[kPrepThreads / 32];
+  pdl_wait();
+  pdl_trigger();
+  const PlanView pv = plan_view(const_cast<int*>(plan), rows, E);
+  const int pos = blockIdx.x, tid = threadIdx.x;
+  if (pos >= pv.offset[E]) return;
+  const int src = x_by_dst ? pv.row_dst[pos] : pv.row_src[pos];
+  const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)src * ldx);
+  const int nv = K >> 3;
+  uint32_t mx = 0;
+  for (int i = tid; i < nv; i += kPrepThreads) {
+    const uint4 v = __ldg(xr + i);
+    const uint32_t q[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) mx = max(mx, max(q[k] & 0x7fffu, (q[k] >> 16) & 0x7fffu));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if ((tid & 31) == 0) warp_max[tid >> 5] = mx;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kPrepThreads / 32; ++i) mx = max(mx, warp_max[i]);
+  int ef = 261 - (int)(mx >> 7);
+  ef = (mx == 0) ? 127 : min(max(ef, 2), 252);
+  const float scale = __uint_as_float((uint32_t)ef << 23);
+  if (tid == 0) xinv[pos] = __uint_as_float((uint32_t)(254 - ef) << 23);
+  const size_t stride = MX ? (size_t)K : (size_t)K + K / 16;
+  __half* row = xs + (size_t)pos * stride;
+  for (int i = tid; i < nv; i += kPrepThreads) {  // nv is a multiple of 32: a warp is whole or absent
+    const uint4 v = __ldg(xr + i);
+    const uint32_t q[4] = {v.x, v.y, v.z, v.w};
+    float f[8];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      f[2 * k] = __uint_as_float(q[k] << 16) * scale;
+      f[2 * k + 1] = __uint_as_float(q[k] & 0xffff0000u) * scale;
+    }
+    uint4 o;
+    if (MX)
+      o = make_uint4(tm_bits(__floats2half2_rn(f[0], f[1])), tm_bits(__floats2half2_rn(f[2], f[3])),
+                     tm_bits(__floats2half2_rn(f[4], f[5])), tm_bits(__floats2half2_rn(f[6], f[7])));
+    else
+      o = make_uint4(tm_bits(__floats2half2_rn(f[0], f[4])), tm_bits(__floats2half2_rn(f[1], f[5])),
+                     tm_bits(__floats2half2_rn(f[2], f[6])), tm_bits(__floats2half2_rn(f[3], f[7])));
+    *reinterpret_cast<uint4*>(row + (size_t)i * 8) = o;
+    if (!MX) {
+      float s = ((f[0] + f[1]) + (f[2] + f[3])) + ((f[4] + f[5]) + (f[6] + f[7]));
+      s += __shfl_xor_sync(0xffffffffu, s, 1);
+      s += __shfl_xor_sync(0xffffffffu, s, 2);
+      s += __shfl_xor_sync(0xffffffffu, s, 4);
+      if ((tid & 7) == 0) {
+        const __half x1 = __float2half_rn(s);
+        const uint32_t pr = tm_bits(__halves2half2(x1, __float2half_rn(s - __half2float(x1))));
+        *reinterpret_cast<uint2*>(row + K + (size_t)(i >> 3) * 4) = make_uint2(pr, pr ^ 0x80008000u);
+      }
+    }
+  }
+}
+
+// ------------------------------------------------------------------ host side
+
+size_t qmm_tma_workspace(int rows, int K, bool mx) {
+  const size_t row = mx ? (size_t)K * 2 : (size_t)K * 2 + K / 8;
+  return (((size_t)rows * row + 255) & ~(size_t)255) + (size_t)rows * sizeof(float);
+}
+
+// Which calls gain from the path: whole chunks along K, and more than eight rows on some expert (by the caller's
+// bound).  A block of up to eight token rows is taken by the one-launch kernel or the register-fed ones, whose cost per
+// expert is the same for one row as for eight (whole block, c2, T = 8: 78 us in one launch, 136 here; T = 16: 151 us in
+// two launches, 138 here).
+bool qmm_tma_wants(int E, int K, int rows_hint) {
+  return K % kTmChunk == 0 && E <= kTmMaxTasks && rows_hint > 8;
+}
+
+// Whether this call takes it: wanted, a workspace is there, and the encoder takes the tensor maps.
+bool qmm_tma_covers(const QmmParams& q, int nmat, bool mx, int rows_hint, const void* ws, size_t ws_bytes) {
+  if (!ws || ((uintptr_t)ws & 255) || ws_bytes < qmm_tma_workspace(q.rows, q.K, mx)) return false;
+  if (!qmm_tma_wants(q.E, q.K, rows_hint) || (long long)q.E * q.N > (1ll << 31) - kTmRows) return false;
+  for (int m = 0; m < nmat; ++m)
+    if ((uintptr_t)q.w[m] & 15) return false;
+  return true;
+}
+
+typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+static EncodeTiled encoder() {
+  static const EncodeTiled fn = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult res;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &res) != cudaSuccess ||
+        res != cudaDriverEntryPointSuccess)
+      f = nullptr;
+    return (EncodeTiled)f;
+  }();
+  return fn;
+}
+
+static bool map_2d(CUtensorMap* m, CUtensorMapDataType dt, const void* ptr, size_t cols, size_t nrows, size_t stride,
+                   int box_cols, int box_rows, CUtensorMapSwizzle sw, CUtensorMapL2promotion prom) {
+  const cuuint64_t dims[2] = {cols, nrows}, strides[1] = {stride};
+  const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows}, es[2] = {1, 1};
+  return encoder()(m, dt, 2, const_cast<void*>(ptr), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, sw, prom,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <bool MX, int NMAT>
+static int launch_tma(const TmArgs& a, int grid, size_t smem, cudaStream_t st, const char* who) {
+  cudaError_t e = cudaFuncSetAttribute(qmm_tma_kernel<MX, NMAT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) e = launch_pdl(qmm_tma_kernel<MX, NMAT>, dim3(grid), dim3(kTmThreads), smem, st, a);
+  if (e != cudaSuccess) return fail(ZMOE_ERR_CUDA, "%s: launch failed: %s", who, cudaGetErrorString(e));
+  return check_launch("qmm_tma_kernel");
+}
+
+int qmm_tma_launch(const QmmParams& q, int nmat, bool mx, int rows_hint, int max_groups, void* ws, cudaStream_t st,
+                   const char* who) {
+  if (!encoder()) return fail(ZMOE_ERR_CUDA, "%s: cuTensorMapEncodeTiled is not available", who);
+  const size_t row = mx ? (size_t)q.K * 2 : (size_t)q.K * 2 + q.K / 8;  // bytes of a prepared row
+  unsigned char* xs = reinterpret_cast<unsigned char*>(ws);
+  float* xinv = reinterpret_cast<float*>(xs + (((size_t)q.rows * row + 255) & ~(size_t)255));
+  TmArgs a;
+  a.q = q;
+  a.xinv = xinv;
+  a.nch = q.K / kTmChunk;
+  bool fine = true;
+  for (int m = 0; m < 2; ++m)
+    fine = fine && map_2d(&a.w[m], CU_TENSOR_MAP_DATA_TYPE_UINT8, q.w[m], (size_t)q.K / 2, (size_t)q.E * q.N,
+                          (size_t)q.K / 2, 128, kTmRows / nmat, CU_TENSOR_MAP_SWIZZLE_128B,
+                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+  fine = fine && map_2d(&a.x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, xs, q.K, q.rows, row, 64, 16, CU_TENSOR_MAP_SWIZZLE_128B,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+  if (mx)
+    a.xb = a.x;
+  else
+    fine = fine && map_2d(&a.xb, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, xs + (size_t)q.K * 2, q.K / 16, q.rows, row, 16, 16,
+                          CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_NONE);
+  if (!fine) return fail(ZMOE_ERR_CUDA, "%s: a tensor map was refused", who);
+  // Token rows per item: up to twice the average task in whole 16s (a larger task takes several equal blocks); the
+  // fewer rows a stage must hold, the more stages are in flight.
+  long long tn = 2ll * q.rows / max_groups + 8;
+  if (tn > rows_hint) tn = rows_hint;
+  tn = (tn + 15) / 16 * 16;
+  a.tn = tn > kTmMaxTok ? kTmMaxTok : (int)tn;
+  a.xstage = (a.tn * (mx ? 512 : 544) + 1023) & ~1023;
+  const int fixed = 1024 + kTmRaw * kTmRawBytes + kTmScRing * kTmExp * 16;
+  const int room = 227 * 1024 - 8 * 1024 - fixed;  // 8 KB: the static part (prefix sums, barriers, row factors)
+  a.rx = room / a.xstage > kTmMaxX ? kTmMaxX : room / a.xstage;
+  const size_t smem = (size_t)fixed + (size_t)a.rx * a.xstage;
+  int sms = 0, dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
+    return fail(ZMOE_ERR_CUDA, "%s: SM count query failed", who);
+  cudaError_t e =
+      mx ? launch_pdl(prep_rows_kernel<true>, dim3(q.rows), dim3(kPrepThreads), 0, st, q.x, q.ldx, q.plan, q.rows, q.E,
+                      q.x_by_dst, q.K, (__half*)xs, xinv)
+         : launch_pdl(prep_rows_kernel<false>, dim3(q.rows), dim3(kPrepThreads), 0, st, q.x, q.ldx, q.plan, q.rows, q.E,
+                      q.x_by_dst, q.K, (__half*)xs, xinv);
+  if (e != cudaSuccess) return fail(ZMOE_ERR_CUDA, "%s: launch failed: %s", who, cudaGetErrorString(e));
+  // one CTA per SM, fewer when the work list is shorter
+  const long long ntiles = (q.N * (long long)nmat + kTmRows - 1) / kTmRows;
+  const long long items = ntiles * ((long long)q.rows / a.tn + max_groups);
+  const int grid = (int)(items < sms ? items : sms);
+  if (mx) return nmat == 2 ? launch_tma<true, 2>(a, grid, smem, st, who) : launch_tma<true, 1>(a, grid, smem, st, who);
+  return nmat == 2 ? launch_tma<false, 2>(a, grid, smem, st, who) : launch_tma<false, 1>(a, grid, smem, st, who);
+}
+
+}  // namespace zmoe
+
+using namespace zmoe;
+
+extern "C" size_t zmoe_qmm_workspace_bytes(int rows, int E, int K, int rows_hint, int qmode) {
+  if (rows <= 0 || E <= 0 || K <= 0) return 0;
+  if (rows_hint <= 0 || rows_hint > rows) rows_hint = rows;
+  return qmm_tma_wants(E, K, rows_hint) ? qmm_tma_workspace(rows, K, qmode == ZMOE_Q_MXFP4) : 0;
+}

@@ -134,17 +134,9 @@ class EPMoELayer:
         st = ops._stream()
         _lib.check(lib.zmoe_build_plan(None, K, p(li), TA * K, 1, self.n_local, p(self.local_plan),
                                        self.local_plan.numel() * 4, st))
-        qm = ops.qmode_code(cfg.mode)
-        W = inner.p
         y = inner.y[:TA * K]
         y.zero_()
-        _lib.check(lib.zmoe_gather_qmm_swiglu(p(x_all), TA, x_all.stride(0), p(W["gate_w"]), p(W["gate_s"]),
-                                              p(W["gate_b"]), p(W["up_w"]), p(W["up_s"]), p(W["up_b"]),
-                                              self.n_local, cfg.d_ff, cfg.d_model, inner.gs, qm,
-                                              p(self.local_plan), TA * K, TA, p(inner.h), inner.swiglu, st))
-        _lib.check(lib.zmoe_gather_qmm(p(inner.h), TA * K, cfg.d_ff, p(W["down_w"]), p(W["down_s"]),
-                                       p(W["down_b"]), self.n_local, cfg.d_model, cfg.d_ff, inner.gs, qm,
-                                       p(self.local_plan), TA * K, TA, 1, p(y), st))
+        inner._mlp(x_all, inner.p, self.n_local, cfg.d_ff, self.local_plan, TA * K, TA, inner.h, y, inner.swiglu, 1)
 
     def _run_segment(self, TA: int) -> None:
         if not self.segment_graphs:

@@ -110,17 +110,18 @@ class MoELayer:
         return [(r, min(M, T - r)) for r in range(0, T, M)]
 
     def _chunked_ok(self, T: int) -> bool:
-        """More rows than one launch takes, but still fewer than two per expert on average: the block runs as
-        consecutive one-launch passes over eight rows each.  Every pass streams only its own rows' experts, and
-        measured against the separate kernels it wins up to about that density (c2 T=16: 79 vs 121 us, c5 T=64:
-        2.3 vs 3.5 ms per layer); beyond it the experts are shared by enough rows for the grouped matmuls."""
+        """Whether more rows than one launch takes can run as consecutive one-launch passes over eight rows each."""
         cfg = self.cfg
-        # blocks so wide that the register-fed matmul cannot stage eight token rows (its 96 KB budget) keep the
-        # passes up to four rows per expert: measured c5 T=128, 4.6 ms in 16 passes against 5.7 ms
         dense = 4 if cfg.d_model * 2 * 8 > 96 * 1024 else 2
         if self.ep is not None or T <= self.FUSED_MAX_TOKENS or T * cfg.top_k > dense * cfg.n_experts:
             return False
         return all(self.fused_workspace_bytes(n) > 0 for n in {n for _, n in self._chunks(T)})
+
+    def _passes_win(self, T: int) -> bool:
+        """Every pass streams its own rows' experts again, the grouped matmuls stream each expert once but cost some
+        launches: two passes win for wide blocks (c5, T = 16: 893 against 1003 us; T = 24: 1357 against 1334), and where
+        the second one is nearly empty (c2, T = 9: 100 against 108 us; T = 12: 127 against 125)."""
+        return T <= (16 if self.cfg.d_model * 2 * 8 > 96 * 1024 else 11)
 
     def forward_fused(self, x: torch.Tensor, out: torch.Tensor | None = None, *, row0: int = 0,
                       key=None) -> torch.Tensor:
@@ -266,29 +267,31 @@ class MoELayer:
         cfg = self.cfg
         T = x.shape[0]
         K = cfg.top_k
+        self._mlp(x, self.p, cfg.n_experts, cfg.d_ff, self.plan, T * K, T, self.h, self.y, self.swiglu, 3)
+
+    def _mlp(self, x, bank: dict, E: int, f: int, plan, rows: int, rows_hint: int, h, y, swiglu: int, down_flags: int):
+        """gate/up + SwiGLU of `rows` planned rows into h, and their down projection into y."""
+        cfg = self.cfg
         lib = _lib.load()
         st = ops._stream()
         p = ops._ptr
         qm = ops.qmode_code(cfg.mode)
-        W = self.p
-        _lib.check(lib.zmoe_gather_qmm_swiglu(p(x), T, x.stride(0), p(W["gate_w"]), p(W["gate_s"]), p(W["gate_b"]),
-                                              p(W["up_w"]), p(W["up_s"]), p(W["up_b"]), cfg.n_experts, cfg.d_ff,
-                                              cfg.d_model, self.gs, qm, p(self.plan), T * K, T, p(self.h),
-                                              self.swiglu, st))
-        _lib.check(lib.zmoe_gather_qmm(p(self.h), T * K, cfg.d_ff, p(W["down_w"]), p(W["down_s"]), p(W["down_b"]),
-                                       cfg.n_experts, cfg.d_model, cfg.d_ff, self.gs, qm, p(self.plan), T * K, T, 3,
-                                       p(self.y), st))
+        # one workspace serves both calls: the second prepares its rows after the first has read its own
+        ws = ops._ws_args(ops.qmm_workspace(rows, E, max(cfg.d_model, f), rows_hint=rows_hint, mode=cfg.mode,
+                                            device=self.device))
+        _lib.check(lib.zmoe_gather_qmm_swiglu_ws(p(x), x.shape[0], x.stride(0), p(bank["gate_w"]), p(bank["gate_s"]),
+                                                 p(bank["gate_b"]), p(bank["up_w"]), p(bank["up_s"]), p(bank["up_b"]),
+                                                 E, f, cfg.d_model, self.gs, qm, p(plan), rows, rows_hint, p(h),
+                                                 swiglu, *ws, st))
+        _lib.check(lib.zmoe_gather_qmm_ws(p(h), rows, f, p(bank["down_w"]), p(bank["down_s"]), p(bank["down_b"]), E,
+                                          cfg.d_model, f, self.gs, qm, p(plan), rows, rows_hint, down_flags, p(y), *ws,
+                                          st))
 
     def shared(self, x: torch.Tensor):
         """The always-on shared expert: the same kernels with a one-expert bank."""
         cfg = self.cfg
         T = x.shape[0]
-        lib = _lib.load()
-        st = ops._stream()
         p = ops._ptr
-        qm = ops.qmode_code(cfg.mode)
-        S = self.p["shared"]
-        f = cfg.d_ff * cfg.n_shared
         # the shared expert's plan depends on the token count only (row t -> expert 0): built once per count and
         # kept, unless this call is being captured in a CUDA graph (a captured launch does not run now)
         plan = self._shared_plans.get(T)
@@ -296,14 +299,11 @@ class MoELayer:
             capturing = torch.cuda.is_current_stream_capturing()
             plan = self.shared_plan if capturing else torch.empty(ops.plan_bytes(T, 1) // 4, dtype=torch.int32,
                                                                   device=self.device)
-            _lib.check(lib.zmoe_build_plan(None, 1, p(self.zero_idx), T, 1, 1, p(plan), plan.numel() * 4, st))
+            _lib.check(_lib.load().zmoe_build_plan(None, 1, p(self.zero_idx), T, 1, 1, p(plan), plan.numel() * 4,
+                                                   ops._stream()))
             if not capturing:
                 self._shared_plans[T] = plan
-        _lib.check(lib.zmoe_gather_qmm_swiglu(p(x), T, x.stride(0), p(S["gate_w"]), p(S["gate_s"]), p(S["gate_b"]),
-                                              p(S["up_w"]), p(S["up_s"]), p(S["up_b"]), 1, f, cfg.d_model, self.gs,
-                                              qm, p(plan), T, T, p(self.sh_h), _lib.SWIGLU_PER_OP, st))
-        _lib.check(lib.zmoe_gather_qmm(p(self.sh_h), T, f, p(S["down_w"]), p(S["down_s"]), p(S["down_b"]), 1,
-                                       cfg.d_model, f, self.gs, qm, p(plan), T, T, 1, p(self.sh_y), st))
+        self._mlp(x, self.p["shared"], 1, cfg.d_ff * cfg.n_shared, plan, T, T, self.sh_h, self.sh_y, _lib.SWIGLU_PER_OP, 1)
 
     def forward(self, x: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
         """x (T, d_model) bfloat16 on this layer's device -> (T, d_model) bfloat16: ``out`` when given (contiguous,
@@ -324,7 +324,8 @@ class MoELayer:
             if self.fused:
                 ok = self._fused_ok.get(T)
                 if ok is None:
-                    ok = self.fused_workspace_bytes(T) > 0 or ("chunks" if self._chunked_ok(T) else False)
+                    passes = self._passes_win(T) and self._chunked_ok(T)
+                    ok = self.fused_workspace_bytes(T) > 0 or ("chunks" if passes else False)
                     self._fused_ok[T] = ok
                 if ok == "chunks":
                     dst = self.out if out is None else out

@@ -80,6 +80,17 @@ def build_plan(rhs: torch.Tensor, E: int, *, M: int = 1, lhs: torch.Tensor | Non
     return out
 
 
+def qmm_workspace(rows: int, E: int, K: int, *, rows_hint: int, mode: str, device) -> torch.Tensor | None:
+    """Workspace of one grouped matmul call, from torch's allocator (so it belongs to the current stream and goes back
+    to the pool when the call's reference is dropped), or None where the call gains nothing from one."""
+    n = int(_lib.load().zmoe_qmm_workspace_bytes(int(rows), int(E), int(K), int(rows_hint), qmode_code(mode)))
+    return torch.empty(n, dtype=torch.uint8, device=device) if n else None
+
+
+def _ws_args(ws: torch.Tensor | None):
+    return (None, 0) if ws is None else (_ptr(ws), ws.numel())
+
+
 def _check_packed(w: torch.Tensor, name: str) -> None:
     if w.dtype not in _U32_LIKE:
         raise TypeError(f"{name} must be uint32-packed (torch.uint32 or torch.int32), got {w.dtype}")
@@ -102,10 +113,11 @@ def gather_qmm_swiglu_rows(x2: torch.Tensor, gate_w, gate_s, gate_b, up_w, up_s,
     if out is None:
         out = torch.empty((rows, N), dtype=torch.bfloat16, device=dev)
     with torch.cuda.device(dev):
-        _lib.check(_lib.load().zmoe_gather_qmm_swiglu(
+        ws = qmm_workspace(rows, E, K, rows_hint=rows_hint, mode=mode, device=dev)
+        _lib.check(_lib.load().zmoe_gather_qmm_swiglu_ws(
             _ptr(x2), x2.shape[0], x2.stride(0), _ptr(gate_w), _ptr(gate_s), _ptr(gate_b), _ptr(up_w), _ptr(up_s),
             _ptr(up_b), E, N, K, int(group_size), qmode_code(mode), _ptr(plan), int(rows), int(rows_hint), _ptr(out),
-            int(swiglu), _stream()))
+            int(swiglu), *_ws_args(ws), _stream()))
     return out
 
 
@@ -123,10 +135,11 @@ def gather_qmm_rows(x2: torch.Tensor, w, s, b, plan: torch.Tensor, rows: int, *,
     if out is None:
         out = torch.empty((rows, N), dtype=torch.bfloat16, device=dev)
     with torch.cuda.device(dev):
-        _lib.check(_lib.load().zmoe_gather_qmm(
+        ws = qmm_workspace(rows, E, K, rows_hint=rows_hint, mode=mode, device=dev)
+        _lib.check(_lib.load().zmoe_gather_qmm_ws(
             _ptr(x2), x2.shape[0], x2.stride(0), _ptr(w), _ptr(s), _ptr(b), E, N, K, int(group_size),
             qmode_code(mode), _ptr(plan), int(rows), int(rows_hint), int(bool(x_by_output_row)), _ptr(out),
-            _stream()))
+            *_ws_args(ws), _stream()))
     return out
 
 
