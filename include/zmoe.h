@@ -329,6 +329,12 @@ size_t zmoe_layer_decode_workspace_bytes(const zmoe_layer_desc* L, int T);
 int zmoe_layer_decode(const zmoe_layer_desc* L, const void* x, int ldx, int T, void* workspace,
                       size_t workspace_bytes, float* weights, uint32_t* indices, void* out, void* stream);
 
+/* The same block for mxfp4 banks (qmode ZMOE_Q_MXFP4, group_size 32, biases ignored) on one GPU: everything else as
+   above, with its own pair of entries because the ones above refuse these banks. */
+size_t zmoe_layer_decode_mxfp4_workspace_bytes(const zmoe_layer_desc* L, int T);
+int zmoe_layer_decode_mxfp4(const zmoe_layer_desc* L, const void* x, int ldx, int T, void* workspace,
+                            size_t workspace_bytes, float* weights, uint32_t* indices, void* out, void* stream);
+
 /*
  * Expert parallel form of zmoe_layer_decode (no reference counterpart: the reference runs on one device and
  * only disables its MoE pattern under tensor parallelism, src/zmlx/exo.py:141-151; the exchange sits where its

@@ -92,6 +92,9 @@ SIGNATURES = {
     "zmoe_layer_decode_workspace_bytes": (c_size_t, [ctypes.POINTER(LayerDesc), c_int]),
     "zmoe_layer_decode": (c_int, [ctypes.POINTER(LayerDesc), c_void_p, c_int, c_int, c_void_p, c_size_t, c_void_p,
                                   c_void_p, c_void_p, c_void_p]),
+    "zmoe_layer_decode_mxfp4_workspace_bytes": (c_size_t, [ctypes.POINTER(LayerDesc), c_int]),
+    "zmoe_layer_decode_mxfp4": (c_int, [ctypes.POINTER(LayerDesc), c_void_p, c_int, c_int, c_void_p, c_size_t, c_void_p,
+                                        c_void_p, c_void_p, c_void_p]),
     "zmoe_layer_decode_status": (c_int, [c_void_p, c_int, c_void_p]),
     "zmoe_layer_decode_inbox_bytes": (c_size_t, [ctypes.POINTER(LayerDesc), c_int]),
     "zmoe_ep_alloc": (c_int, [c_size_t, ctypes.POINTER(c_void_p)]),

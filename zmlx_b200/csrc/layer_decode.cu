@@ -35,6 +35,8 @@
 // Spare mma columns carry other groups (column multiplexing, see qmm.cu).  Scales and biases are read straight
 // from L1/L2 into registers one block of groups ahead.
 //
+// mxfp4 banks are an instance of their own (ld_item_mx): the blocks' powers of two go into the fp16 operand.
+//
 // Every wait on another warp, CTA or copy is bounded: when the limit is hit the warp records it in the status
 // word and leaves; the producer then waits (bounded) for its copies in flight before the CTA ends.
 #include <cuda_fp16.h>
@@ -361,7 +363,9 @@ __device__ __forceinline__ void ld_stage_pass1(unsigned char* xs, int xs_stride,
   ld_csync();
 }
 
-// Pass 2: scale by the row's power of two, convert, permute in place; group sums.
+// Pass 2: scale by the row's power of two, convert, permute in place; group sums.  MX: the values keep their order and
+// need no sums.
+template <bool MX>
 __device__ __forceinline__ void ld_stage_pass2(unsigned char* xs, int xs_stride, float2* xsum, int rs, float* isig,
                                                const int* rowmax, int nrows, int K8) {
   const int tid = threadIdx.x, lane = tid & 31;
@@ -387,7 +391,7 @@ __device__ __forceinline__ void ld_stage_pass2(unsigned char* xs, int xs_stride,
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const float lo = bf16_bits_to_float(q[k] & 0xffffu) * sigma;            // element 2k (even position)
-        const float hi = bf16_bits_to_float(q[k] >> 16) * sigma * 0.0625f;      // element 2k+1 (odd position)
+        const float hi = bf16_bits_to_float(q[k] >> 16) * sigma * (MX ? 1.0f : 0.0625f);  // element 2k+1 (odd position)
         hv[2 * k] = __float2half_rn(lo);
         hv[2 * k + 1] = __float2half_rn(hi);
         se += __half2float(hv[2 * k]);
@@ -397,13 +401,14 @@ __device__ __forceinline__ void ld_stage_pass2(unsigned char* xs, int xs_stride,
         return (uint32_t)__half_as_ushort(hv[a]) | ((uint32_t)__half_as_ushort(hv[b]) << 16);
       };
       uint4 o;
-      o.x = pack(0, 4);
-      o.y = pack(1, 5);
-      o.z = pack(2, 6);
-      o.w = pack(3, 7);
+      o.x = MX ? pack(0, 1) : pack(0, 4);
+      o.y = MX ? pack(2, 3) : pack(1, 5);
+      o.z = MX ? pack(4, 5) : pack(2, 6);
+      o.w = MX ? pack(6, 7) : pack(3, 7);
       *slot = o;
       if (blk == 0) isig[t] = __uint_as_float((uint32_t)(127 - sexp) << 23);
     }
+    if (MX) continue;
     se += __shfl_xor_sync(0xffffffffu, se, 1);
     so += __shfl_xor_sync(0xffffffffu, so, 1);
     se += __shfl_xor_sync(0xffffffffu, se, 2);
@@ -415,12 +420,12 @@ __device__ __forceinline__ void ld_stage_pass2(unsigned char* xs, int xs_stride,
   ld_csync();
 }
 
-template <bool TAGGED, bool SYS = false>
+template <bool TAGGED, bool MX>
 __device__ __forceinline__ void ld_stage_rows(unsigned char* xs, int xs_stride, float2* xsum, int rs, float* isig,
                                               int* rowmax, const void* src, int ld, const unsigned char* rowlist,
                                               int nrows, int K8, uint32_t tag, volatile int* flags, int* status) {
-  ld_stage_pass1<TAGGED, SYS>(xs, xs_stride, rowmax, src, ld, rowlist, nrows, K8, tag, flags, status);
-  ld_stage_pass2(xs, xs_stride, xsum, rs, isig, rowmax, nrows, K8);
+  ld_stage_pass1<TAGGED>(xs, xs_stride, rowmax, src, ld, rowlist, nrows, K8, tag, flags, status);
+  ld_stage_pass2<MX>(xs, xs_stride, xsum, rs, isig, rowmax, nrows, K8);
 }
 
 // ------------------------------------------------------------------ what a consumer warp carries around
@@ -492,6 +497,67 @@ __device__ __forceinline__ void ld_fixup(float (&acc)[2][4], const float (&dg)[2
         const float dsum = dg[m][0][h * 2 + c] + dg[m][1][h * 2 + c];
         acc[m][h * 2 + c] = fmaf(sv, dsum - xc.y, fmaf(bv, xc.x, acc[m][h * 2 + c]));
       }
+  }
+}
+
+// K-split: the partial sums of a team's warps 1..3 go to its first warp, which adds them in warp order; FOLD: then the
+// multiplexed columns are folded back onto their tokens.
+template <int TT, bool FOLD = true>
+__device__ __forceinline__ void ld_join(LdCtx& c, float (&acc)[2][4]) {
+  const int wk = c.wk;
+  const int it = c.itn++;
+  if (c.alive) {
+    if (wk != 0) {
+      // the first warp must have read the previous item's sums before they are overwritten
+      if (it > 0 && !ld_flag_wait(c.flags + 1 + c.team, it, c.flags)) {
+        c.alive = false;
+        c.flags[0] = 1;
+      }
+      float* mine = c.red + ((c.team * 3 + wk - 1) * 32 + c.lane) * 8;
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) mine[m * 4 + j] = acc[m][j];
+      __threadfence_block();
+      __syncwarp();
+      if (c.lane == 0) c.flags[8 + c.team * 3 + wk - 1] = it + 1;
+    } else {
+#pragma unroll 1
+      for (int o = 1; o < 4; ++o) {
+        if (c.alive && !ld_flag_wait(c.flags + 8 + c.team * 3 + o - 1, it + 1, c.flags)) {
+          c.alive = false;
+          c.flags[0] = 1;
+        }
+        __threadfence_block();
+        const float* other = c.red + ((c.team * 3 + o - 1) * 32 + c.lane) * 8;
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[m][j] += other[m * 4 + j];
+      }
+      __threadfence_block();
+      __syncwarp();
+      if (c.lane == 0) c.flags[1 + c.team] = it + 1;
+      // fold the multiplexed columns back onto their tokens: afterwards column col < TT holds token col
+      if (FOLD && TT < 8) {
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            if (TT == 1) {
+              acc[m][h * 2] += acc[m][h * 2 + 1];
+              acc[m][h * 2 + 1] = 0.0f;
+            }
+#pragma unroll
+            for (int cc = 0; cc < 2; ++cc) {
+              float v = acc[m][h * 2 + cc];
+              if (TT <= 2) v += __shfl_xor_sync(0xffffffffu, v, 1);
+              v += __shfl_xor_sync(0xffffffffu, v, 2);
+              acc[m][h * 2 + cc] = v;
+            }
+          }
+      }
+    }
   }
 }
 
@@ -596,67 +662,124 @@ __device__ __forceinline__ void ld_item(LdCtx& c, float (&acc)[2][4], int K8, ui
   // a last chunk that holds groups of the team's first warps only) still owes that block its fix-up
   if (open_p0 >= 0 && c.alive) ld_fixup<TT>(acc, dg, sb, xsum, rs, srow_c, ng, open_p0, wk, tig);
 
-  // ---- K-split: the partial sums of warps 1..3 go to the team's first warp in warp order
-  const int it = c.itn++;
-  if (c.alive) {
-    if (wk != 0) {
-      // the first warp must have read the previous item's sums before they are overwritten
-      if (it > 0 && !ld_flag_wait(c.flags + 1 + c.team, it, c.flags)) {
-        c.alive = false;
-        c.flags[0] = 1;
-      }
-      float* mine = c.red + ((c.team * 3 + wk - 1) * 32 + c.lane) * 8;
+  ld_join<TT>(c, acc);
+}
+
+// ------------------------------------------------------------------ mxfp4 items
+// Eight e2m1 codes of a word -> four half2 in their own order.
+__device__ __forceinline__ void ld_e2m1x8(uint32_t w, __half2 s, uint32_t (&o)[4]) {
+  asm("{ .reg .b8 t0, t1, t2, t3;\n"
+      "mov.b32 {t0, t1, t2, t3}, %4;\n"
+      "cvt.rn.f16x2.e2m1x2 %0, t0;\n"
+      "cvt.rn.f16x2.e2m1x2 %1, t1;\n"
+      "cvt.rn.f16x2.e2m1x2 %2, t2;\n"
+      "cvt.rn.f16x2.e2m1x2 %3, t3; }"
+      : "=r"(o[0]), "=r"(o[1]), "=r"(o[2]), "=r"(o[3])
+      : "r"(w));
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const __half2 v = __hmul2(*reinterpret_cast<const __half2*>(&o[k]), s);
+    o[k] = *reinterpret_cast<const uint32_t*>(&v);
+  }
+}
+
+// The same item for mxfp4 banks.  An e2m1 value times a power of two has one mantissa bit, so the blocks' scales go
+// into the fp16 operand, relative to the largest of the warp's eight blocks of a row in the stage (exact over 23
+// binades below it); that largest one is applied to the stage's sum in fp32.  With the scales inside the operand
+// nothing has to be kept apart per group: column t of the accumulator is token t, and no columns are multiplexed.
+// Bound like the affine block by the chain router -> gate/up -> down -> combine at these sizes.  Measured (c3, us per
+// block in a graph, separate kernels -> one launch): T = 1 46.0 -> 21.4, T = 4 76.5 -> 43.6, T = 8 111.7 -> 61.7; called
+// from Python, where thirteen launches on two streams cost more than they compute, T = 1 104.6 -> 23.0.
+template <int TT>
+__device__ __forceinline__ void ld_item_mx(LdCtx& c, float (&acc)[2][4], int K8, uint32_t xaddr, bool tok_ok) {
+  const int rb = K8 << 2;
+  const int nch = (rb + kLdSegBytes - 1) / kLdSegBytes;
+  const int wk = c.wk, g = c.g, tig = c.tig;
+  static_assert(kLdGW == 4, "a warp takes four groups of a stage");
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[m][j] = 0.0f;
+#pragma unroll 1
+  for (int ch = 0; ch < nch; ++ch) {
+    const uint32_t full = ld_full_bar(c.bars, c.team, c.slot);
+    if (c.alive && !ld_mbar_wait(full, c.use & 1, c.flags)) {
+      c.alive = false;
+      c.flags[0] = 1;
+    }
+    if (c.alive && ((ch * kLdSegGroups + wk * kLdGW) * 32 < rb)) {
+      const uint32_t stage = c.ring + (uint32_t)(c.slot0 + c.slot) * kLdSlotBytes;
+      const uint32_t wbase = stage + g * kLdSegStride + wk * (kLdGW * 32) + tig * 8;
+      const uint32_t xchunk = xaddr + (uint32_t)(ch * kLdSegGroups + wk * kLdGW) * 128;
+      uint2 eb[2][2];   // the eight block exponents of row g + 8h of matrix m
+      int eref[2][2];   // the largest
+      float dg[2][2][4];
 #pragma unroll
       for (int m = 0; m < 2; ++m)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) mine[m * 4 + j] = acc[m][j];
-      __threadfence_block();
-      __syncwarp();
-      if (c.lane == 0) c.flags[8 + c.team * 3 + wk - 1] = it + 1;
-    } else {
-#pragma unroll 1
-      for (int o = 1; o < 4; ++o) {
-        if (c.alive && !ld_flag_wait(c.flags + 8 + c.team * 3 + o - 1, it + 1, c.flags)) {
-          c.alive = false;
-          c.flags[0] = 1;
+        for (int h = 0; h < 2; ++h) {
+          eb[m][h] = ld_lds64<0>(stage + kLdScOff + (uint32_t)((m * 16 + g + 8 * h) * kLdScRow + wk * 8));
+          uint32_t v = __vmaxu4(eb[m][h].x, eb[m][h].y);
+          v = __vmaxu4(v, v >> 16);
+          eref[m][h] = (int)max(v & 0xffu, (v >> 8) & 0xffu);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) dg[m][h][j] = 0.0f;
         }
-        __threadfence_block();
-        const float* other = c.red + ((c.team * 3 + o - 1) * 32 + c.lane) * 8;
+      auto group = [&](auto jc) {
+        constexpr int j = decltype(jc)::value;
+        const bool mine = tok_ok && (TT == 8 || g < TT);
+        const uint32_t xa = xchunk + j * 128;
+        const uint4 xb0 = ld_lds128_if<0>(xa, mine);
+        const uint4 xb1 = ld_lds128_if<16>(xa, mine);
+        const int sh = (j & 1) * 16 + (tig >> 1) * 8;  // a lane's 16 codes lie in one of the group's two blocks
 #pragma unroll
-        for (int m = 0; m < 2; ++m)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) acc[m][j] += other[m * 4 + j];
-      }
-      __threadfence_block();
-      __syncwarp();
-      if (c.lane == 0) c.flags[1 + c.team] = it + 1;
-      // fold the multiplexed columns back onto their tokens: afterwards column col < TT holds token col
-      if (TT < 8) {
-#pragma unroll
-        for (int m = 0; m < 2; ++m)
+        for (int m = 0; m < 2; ++m) {
+          const uint2 wa = (m == 0) ? ld_lds64<j * 32>(wbase) : ld_lds64<16 * kLdSegStride + j * 32>(wbase);
+          const uint2 wb = (m == 0) ? ld_lds64<8 * kLdSegStride + j * 32>(wbase)
+                                    : ld_lds64<24 * kLdSegStride + j * 32>(wbase);
+          __half2 s[2];
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            if (TT == 1) {
-              acc[m][h * 2] += acc[m][h * 2 + 1];
-              acc[m][h * 2 + 1] = 0.0f;
-            }
-#pragma unroll
-            for (int cc = 0; cc < 2; ++cc) {
-              float v = acc[m][h * 2 + cc];
-              if (TT <= 2) v += __shfl_xor_sync(0xffffffffu, v, 1);
-              v += __shfl_xor_sync(0xffffffffu, v, 2);
-              acc[m][h * 2 + cc] = v;
-            }
+            const int e = (int)(((j < 2 ? eb[m][h].x : eb[m][h].y) >> sh) & 0xffu);
+            s[h] = __float2half2_rn(__uint_as_float((uint32_t)max(127 + e - eref[m][h], 0) << 23));
           }
-      }
+          uint32_t a0[4], a1[4];
+          ld_e2m1x8(wa.x, s[0], a0);
+          ld_e2m1x8(wb.x, s[1], a1);
+          mma_f16_m16n8k16(dg[m][0], a0[0], a1[0], a0[1], a1[1], xb0.x, xb0.y);
+          mma_f16_m16n8k16(dg[m][1], a0[2], a1[2], a0[3], a1[3], xb0.z, xb0.w);
+          ld_e2m1x8(wa.y, s[0], a0);
+          ld_e2m1x8(wb.y, s[1], a1);
+          mma_f16_m16n8k16(dg[m][0], a0[0], a1[0], a0[1], a1[1], xb1.x, xb1.y);
+          mma_f16_m16n8k16(dg[m][1], a0[2], a1[2], a0[3], a1[3], xb1.z, xb1.w);
+        }
+      };
+      group(std::integral_constant<int, 0>{});
+      group(std::integral_constant<int, 1>{});
+      group(std::integral_constant<int, 2>{});
+      group(std::integral_constant<int, 3>{});
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float sv = __uint_as_float((uint32_t)eref[m][j >> 1] << 23);  // 2^(e - 127)
+          acc[m][j] = fmaf(sv, dg[m][0][j] + dg[m][1][j], acc[m][j]);
+        }
+    }
+    __syncwarp();
+    if (c.alive && c.lane == 0) ld_mbar_arrive(ld_empty_bar(c.bars, c.team, c.slot));
+    if (++c.slot == c.depth) {
+      c.slot = 0;
+      ++c.use;
     }
   }
+  ld_join<TT, false>(c, acc);
 }
 
 // ------------------------------------------------------------------ the kernel
 // EP: the token rows come from, and the projected rows go to, the ranks' inboxes (expert parallel, or the one-GPU
 // test of that data path).  The plain instance carries none of that code: the kernel is sensitive to its size.
-template <int TT, bool EP>
+template <int TT, bool EP, bool MX>
 __global__ void __launch_bounds__(kLdThreads, 1) layer_decode_kernel(const LdParams p) {
   extern __shared__ __align__(128) unsigned char smem[];
   const int tid = threadIdx.x;
@@ -800,7 +923,21 @@ __global__ void __launch_bounds__(kLdThreads, 1) layer_decode_kernel(const LdPar
           for (int r = 0; r < 16; r += SPI) ld_cp16(dst + (16 + r) * kLdSegStride, src1 + (size_t)r * rb, pol);
         }
       }
-      {
+      if (MX) {
+        // block exponents: two per group of 64 codes, [matrix][row 0..15][blocks of the stage]; 8 bytes per lane
+        constexpr int PPP = kLdScRow / 8, RPI = 32 / PPP;
+        const int part = lane % PPP, srow = lane / PPP;
+        if (part * 8 < (bytes >> 4)) {
+          const uint32_t dst = stage + kLdScOff + srow * kLdScRow + part * 8;
+          const size_t off = (row0 + srow) * (2 * ng) + ch * kLdScRow + part * 8;
+#pragma unroll
+          for (int it = 0; it < 32 / RPI; ++it) {
+            const int m = (it * RPI) >> 4, r0 = (it * RPI) & 15;
+            const unsigned char* base = reinterpret_cast<const unsigned char*>(bank.s[dn ? 0 : m]);
+            ld_cp8(dst + (m * 16 + r0) * kLdScRow, base + off + (size_t)((dn ? m * 16 : 0) + r0) * (2 * ng));
+          }
+        }
+      } else {
         // scales and biases: 8 bytes per lane; kLdScRow / 8 lanes cover the groups of one row of one tensor
         constexpr int PPP = kLdScRow / 8, RPI = 32 / PPP;  // parts per piece, rows per instruction
         const int part = lane % PPP, srow = lane / PPP;
@@ -946,7 +1083,7 @@ __global__ void __launch_bounds__(kLdThreads, 1) layer_decode_kernel(const LdPar
   }
 
   // ---- the staged rows become fp16 in fragment order with their group sums (pass 2), while the logits travel
-  ld_stage_pass2(xs, qmm_xs_stride(d), xsum, T, isig, rowmax, T, d >> 3);
+  ld_stage_pass2<MX>(xs, qmm_xs_stride(d), xsum, T, isig, rowmax, T, d >> 3);
   LD_STAMP(2);
   // ---- routing of every row, repeated by every CTA (one warp per row); the logits arrive as hand-over words,
   // so this is also where the CTA waits for the router threads of the other CTAs
@@ -1098,8 +1235,11 @@ __global__ void __launch_bounds__(kLdThreads, 1) layer_decode_kernel(const LdPar
         }
       }
       float acc[2][4];
-      ld_item<TT, false>(c, acc, d >> 3, smem_base + lay.xs + trow * xs_stride + tig * 32, smem_base + lay.zero, tok_ok, slot_g, xsum, T,
-                         srow_c);
+      const uint32_t xaddr = smem_base + lay.xs + trow * xs_stride + tig * 32;
+      if constexpr (MX)
+        ld_item_mx<TT>(c, acc, d >> 3, xaddr, tok_ok);
+      else
+        ld_item<TT, false>(c, acc, d >> 3, xaddr, smem_base + lay.zero, tok_ok, slot_g, xsum, T, srow_c);
       if (c.alive && c.wk == 0) {
         const int epi = is_sh ? p.sepi : p.epi;
 #pragma unroll
@@ -1147,7 +1287,7 @@ __global__ void __launch_bounds__(kLdThreads, 1) layer_decode_kernel(const LdPar
   }
   ld_csync();
   const int n_h = meta->n_h;
-  ld_stage_rows<true>(xs, qmm_xs_stride(f), xsum, p.hrows, isig, rowmax, p.h, f, meta->hlist, n_h, f >> 3, tag, flags,
+  ld_stage_rows<true, MX>(xs, qmm_xs_stride(f), xsum, p.hrows, isig, rowmax, p.h, f, meta->hlist, n_h, f >> 3, tag, flags,
                       p.sync + 3);
   LD_STAMP(7);
   if (flags[0]) c.alive = false;
@@ -1169,8 +1309,11 @@ __global__ void __launch_bounds__(kLdThreads, 1) layer_decode_kernel(const LdPar
         srow_c[cc] = (sl < cnt) ? (int)meta->hloc[meta->task_rows[a][sl]] : -1;
       }
       float acc[2][4];
-      ld_item<TT, true>(c, acc, f >> 3, smem_base + lay.xs + srow * xs_stride + tig * 32, smem_base + lay.zero, tok_ok, slot_g, xsum, p.hrows,
-                        srow_c);
+      const uint32_t xaddr = smem_base + lay.xs + srow * xs_stride + tig * 32;
+      if constexpr (MX)
+        ld_item_mx<TT>(c, acc, f >> 3, xaddr, tok_ok);
+      else
+        ld_item<TT, true>(c, acc, f >> 3, xaddr, smem_base + lay.zero, tok_ok, slot_g, xsum, p.hrows, srow_c);
       if (c.alive && c.wk == 0) {
 #pragma unroll
         for (int m = 0; m < 2; ++m)
@@ -1299,12 +1442,16 @@ struct LdPlan {
 static int ld_world(const zmoe_layer_desc* L) { return L->ep_world > 1 ? L->ep_world : 1; }
 
 // T = the rank's own tokens; the kernel routes T * ep_world of them.
-static const char* ld_plan(const zmoe_layer_desc* L, int T_own, int sms, LdPlan* out) {
+static const char* ld_plan(const zmoe_layer_desc* L, int T_own, int sms, bool want_mx, LdPlan* out) {
   const int world = ld_world(L);
   if (world > kLdMaxRanks || L->ep_rank < 0 || L->ep_rank >= world) return "takes at most 8 ranks";
   if (L->E % world != 0) return "needs the expert count to be a multiple of the rank count";
   const int T = T_own * world;
-  if (L->qmode != ZMOE_Q_AFFINE4 || L->group_size != 64) return "needs 4-bit affine weights with group size 64";
+  const bool mx = L->qmode == ZMOE_Q_MXFP4;
+  if (!mx && L->qmode != ZMOE_Q_AFFINE4) return "needs 4-bit affine or mxfp4 weights";
+  if (L->group_size != (mx ? 32 : 64)) return "needs groups of 64 (affine) or 32 (mxfp4)";
+  if (mx && (world > 1 || (L->debug_flags & ZMOE_DEBUG_FORCE_INBOX))) return "takes mxfp4 weights on one GPU only";
+  if (mx != want_mx) return mx ? "of this entry needs 4-bit affine weights" : "of this entry needs mxfp4 weights";
   if (T_own < 1 || T > kLdMaxT) return "takes 1..8 tokens (over all ranks)";
   if (L->top_k < 1 || L->top_k > kLdMaxK) return "takes top_k <= 8";
   if (L->E < L->top_k || L->E > 256) return "takes at most 256 experts";
@@ -1341,9 +1488,9 @@ static size_t ld_ws_y_off(const zmoe_layer_desc* L, int T_own) {
   return (ld_ws_h_off(L, T_own) + rows * L->d_ff * 4 + 255) & ~(size_t)255;
 }
 
-template <int TT, bool EP>
+template <int TT, bool EP, bool MX = false>
 static int ld_launch(const LdParams& p, int grid, size_t smem_bytes, cudaStream_t st) {
-  auto kern = layer_decode_kernel<TT, EP>;
+  auto kern = layer_decode_kernel<TT, EP, MX>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
   if (e != cudaSuccess)
     return fail(ZMOE_ERR_CUDA, "zmoe_layer_decode: shared memory of %zu bytes refused: %s", smem_bytes,
@@ -1369,21 +1516,28 @@ static int ld_launch(const LdParams& p, int grid, size_t smem_bytes, cudaStream_
   return check_launch("layer_decode_kernel");
 }
 
+static size_t ld_workspace(const zmoe_layer_desc* L, int T, bool want_mx) {
+  if (!L) return 0;
+  int sms = 0;
+  if (ld_sm_count(&sms) != ZMOE_OK) return 0;
+  LdPlan plan;
+  if (ld_plan(L, T, sms, want_mx, &plan)) return 0;
+  const size_t rows = (size_t)T * L->top_k + (L->n_shared ? T : 0);  // the rank's own projected rows
+  return ld_ws_y_off(L, T) + rows * L->d_model * 4;
+}
+
+static int ld_decode(const zmoe_layer_desc* L, const void* x, int ldx, int T, void* workspace, size_t workspace_bytes,
+                     float* weights, uint32_t* indices, void* out, void* stream, bool want_mx);
+
 }  // namespace zmoe
 
 using namespace zmoe;
 
 extern "C" {
 
-size_t zmoe_layer_decode_workspace_bytes(const zmoe_layer_desc* L, int T) {
-  if (!L) return 0;
-  int sms = 0;
-  if (ld_sm_count(&sms) != ZMOE_OK) return 0;
-  LdPlan plan;
-  if (ld_plan(L, T, sms, &plan)) return 0;
-  const size_t rows = (size_t)T * L->top_k + (L->n_shared ? T : 0);  // the rank's own projected rows
-  return ld_ws_y_off(L, T) + rows * L->d_model * 4;
-}
+size_t zmoe_layer_decode_workspace_bytes(const zmoe_layer_desc* L, int T) { return ld_workspace(L, T, false); }
+
+size_t zmoe_layer_decode_mxfp4_workspace_bytes(const zmoe_layer_desc* L, int T) { return ld_workspace(L, T, true); }
 
 size_t zmoe_layer_decode_inbox_bytes(const zmoe_layer_desc* L, int T) {
   if (!L || T < 1) return 0;
@@ -1412,22 +1566,34 @@ int zmoe_layer_decode_status(const void* workspace, int clear, void* stream) {
 
 int zmoe_layer_decode(const zmoe_layer_desc* L, const void* x, int ldx, int T, void* workspace,
                       size_t workspace_bytes, float* weights, uint32_t* indices, void* out, void* stream) {
+  return ld_decode(L, x, ldx, T, workspace, workspace_bytes, weights, indices, out, stream, false);
+}
+
+int zmoe_layer_decode_mxfp4(const zmoe_layer_desc* L, const void* x, int ldx, int T, void* workspace,
+                            size_t workspace_bytes, float* weights, uint32_t* indices, void* out, void* stream) {
+  return ld_decode(L, x, ldx, T, workspace, workspace_bytes, weights, indices, out, stream, true);
+}
+
+}  // extern "C"
+
+namespace zmoe {
+
+static int ld_decode(const zmoe_layer_desc* L, const void* x, int ldx, int T, void* workspace, size_t workspace_bytes,
+                     float* weights, uint32_t* indices, void* out, void* stream, bool want_mx) {
   ZMOE_REQUIRE(L && x && workspace && out, ZMOE_ERR_SHAPE, "zmoe_layer_decode: null pointer");
   int sms = 0;
   int rc = ld_sm_count(&sms);
   if (rc != ZMOE_OK) return rc;
   LdPlan plan;
-  const char* why = ld_plan(L, T, sms, &plan);
+  const char* why = ld_plan(L, T, sms, want_mx, &plan);
   ZMOE_REQUIRE(why == nullptr, ZMOE_ERR_UNSUPPORTED, "zmoe_layer_decode: the one-launch path %s", why);
-  ZMOE_REQUIRE(L->router_w && L->routed.gate_w && L->routed.gate_scales && L->routed.gate_biases && L->routed.up_w &&
-                   L->routed.up_scales && L->routed.up_biases && L->routed.down_w && L->routed.down_scales &&
-                   L->routed.down_biases,
-               ZMOE_ERR_SHAPE, "zmoe_layer_decode: null router or expert tensor");
-  if (L->n_shared)
-    ZMOE_REQUIRE(L->shared.gate_w && L->shared.gate_scales && L->shared.gate_biases && L->shared.up_w &&
-                     L->shared.up_scales && L->shared.up_biases && L->shared.down_w && L->shared.down_scales &&
-                     L->shared.down_biases,
-                 ZMOE_ERR_SHAPE, "zmoe_layer_decode: null shared-expert tensor");
+  const bool mx = L->qmode == ZMOE_Q_MXFP4;
+  auto whole = [mx](const zmoe_expert_bank& b) {
+    return b.gate_w && b.gate_scales && b.up_w && b.up_scales && b.down_w && b.down_scales &&
+           (mx || (b.gate_biases && b.up_biases && b.down_biases));
+  };
+  ZMOE_REQUIRE(L->router_w && whole(L->routed), ZMOE_ERR_SHAPE, "zmoe_layer_decode: null router or expert tensor");
+  if (L->n_shared) ZMOE_REQUIRE(whole(L->shared), ZMOE_ERR_SHAPE, "zmoe_layer_decode: null shared-expert tensor");
   ZMOE_REQUIRE(L->router_family >= 0 && L->router_family <= 2, ZMOE_ERR_UNSUPPORTED,
                "zmoe_layer_decode: router family %d", L->router_family);
   if (L->router_family == 2) {
@@ -1465,7 +1631,7 @@ int zmoe_layer_decode(const zmoe_layer_desc* L, const void* x, int ldx, int T, v
       ZMOE_REQUIRE(((uintptr_t)sptr[j] % 8) == 0, ZMOE_ERR_ALIGN,
                    "zmoe_layer_decode: scales and biases must be 8-byte aligned");
   }
-  const size_t need = zmoe_layer_decode_workspace_bytes(L, T);
+  const size_t need = ld_workspace(L, T, want_mx);
   ZMOE_REQUIRE(workspace_bytes >= need, ZMOE_ERR_WORKSPACE, "zmoe_layer_decode: workspace of %zu bytes, need %zu",
                workspace_bytes, need);
   ZMOE_REQUIRE(L->launch_mode == 0 || L->launch_mode == 1, ZMOE_ERR_UNSUPPORTED,
@@ -1539,10 +1705,16 @@ int zmoe_layer_decode(const zmoe_layer_desc* L, const void* x, int ldx, int T, v
     if (Tt <= 4) return ld_launch<4, true>(p, sms, smem_bytes, st);
     return ld_launch<8, true>(p, sms, smem_bytes, st);
   }
+  if (mx) {
+    if (Tt == 1) return ld_launch<1, false, true>(p, sms, smem_bytes, st);
+    if (Tt <= 2) return ld_launch<2, false, true>(p, sms, smem_bytes, st);
+    if (Tt <= 4) return ld_launch<4, false, true>(p, sms, smem_bytes, st);
+    return ld_launch<8, false, true>(p, sms, smem_bytes, st);
+  }
   if (Tt == 1) return ld_launch<1, false>(p, sms, smem_bytes, st);
   if (Tt <= 2) return ld_launch<2, false>(p, sms, smem_bytes, st);
   if (Tt <= 4) return ld_launch<4, false>(p, sms, smem_bytes, st);
   return ld_launch<8, false>(p, sms, smem_bytes, st);
 }
 
-}  // extern "C"
+}  // namespace zmoe

@@ -99,10 +99,19 @@ class MoELayer:
         return d
 
     def fused_workspace_bytes(self, T: int) -> int:
-        """Bytes of workspace the one-launch path needs for T tokens; 0 when the block's shape is outside it."""
+        """Bytes of workspace ``zmoe_layer_decode`` needs for T tokens; 0 when the block is outside it (mxfp4 banks
+        have their own one-launch entry)."""
         if T < 1 or T > self.FUSED_MAX_TOKENS:
             return 0
         return int(_lib.load().zmoe_layer_decode_workspace_bytes(ctypes.byref(self._desc), T))
+
+    def _one_launch_bytes(self, T: int) -> int:
+        """The same for whichever one-launch entry takes this block's banks."""
+        if self.cfg.mode != "mxfp4":
+            return self.fused_workspace_bytes(T)
+        if T < 1 or T > self.FUSED_MAX_TOKENS:
+            return 0
+        return int(_lib.load().zmoe_layer_decode_mxfp4_workspace_bytes(ctypes.byref(self._desc), T))
 
     def _chunks(self, T: int) -> list[tuple[int, int]]:
         """(first row, rows) of the one-launch passes that cover T rows."""
@@ -137,7 +146,7 @@ class MoELayer:
                 # a workspace zeroed inside the graph would be zeroed again at every replay, and with it the launch
                 # count that tells this launch's hand-over words from the previous one's
                 raise RuntimeError(f"run the block once with {T} token(s) before capturing it in a CUDA graph")
-            need = self.fused_workspace_bytes(T)
+            need = self._one_launch_bytes(T)
             if need == 0:
                 raise _lib.ZmoeError(_lib.ERR_UNSUPPORTED, f"no one-launch path for this block at T={T}")
             ws = torch.zeros(need, dtype=torch.uint8, device=self.device)  # the sync words start at zero
@@ -147,9 +156,10 @@ class MoELayer:
                 self._inbox = torch.zeros(nb, dtype=torch.uint8, device=self.device)
                 self._desc = self._describe()
         p = ops._ptr
-        _lib.check(_lib.load().zmoe_layer_decode(ctypes.byref(self._desc), p(x), x.stride(0), T, p(ws), ws.numel(),
-                                                 p(self.weights[row0:]), p(self.indices[row0:]), p(dst[row0:]),
-                                                 ops._stream()))
+        lib = _lib.load()
+        decode = lib.zmoe_layer_decode_mxfp4 if self.cfg.mode == "mxfp4" else lib.zmoe_layer_decode
+        _lib.check(decode(ctypes.byref(self._desc), p(x), x.stride(0), T, p(ws), ws.numel(), p(self.weights[row0:]),
+                          p(self.indices[row0:]), p(dst[row0:]), ops._stream()))
         return dst[row0:row0 + T]
 
     def launch_count(self, T: int) -> int:
@@ -325,14 +335,15 @@ class MoELayer:
                 ok = self._fused_ok.get(T)
                 if ok is None:
                     passes = self._passes_win(T) and self._chunked_ok(T)
-                    ok = self.fused_workspace_bytes(T) > 0 or ("chunks" if passes else False)
+                    ok = self._one_launch_bytes(T) > 0 or ("chunks" if passes else False)
                     self._fused_ok[T] = ok
                 if ok == "chunks":
                     dst = self.out if out is None else out
                     for ci, (r, n) in enumerate(self._chunks(T)):
                         self.forward_fused(x[r:r + n], dst, row0=r, key=(T, ci))
                     return dst[:T]
-                if ok:
+                # mxfp4 blocks may also be captured without a warm-up pass: on the separate kernels
+                if ok and (cfg.mode != "mxfp4" or T in self._fused_ws or not torch.cuda.is_current_stream_capturing()):
                     return self.forward_fused(x, out)
             residual = None
             if cfg.n_shared:
