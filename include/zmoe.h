@@ -245,6 +245,30 @@ int zmoe_gather_qmm_combine_noalloc(const void* act, int ldx, const uint32_t* w,
                                     const void* plan, int T, int K, const void* gate, int gate_dtype, int mode,
                                     void* out, int out_t, void* stream);
 
+/* ------------------------------------------------------- attention side of the stacked decoder */
+
+/* h (rows, d) T += delta (rows, d) T in place when delta is not NULL; x = T(h * rsqrt(mean(h^2) + eps) * w) with float
+   statistics.  d % 8 == 0, d <= 16384, everything 16-byte aligned.  No reference counterpart (mlx_lm's decoder). */
+int zmoe_add_rms_norm(void* h, const void* delta, const void* w, float eps, int rows, int d, void* x, void* stream);
+
+/* q (B*S, hq*hd), k, v (B*S, hk*hd) T as projected: q and k heads are RMS-normed (q_norm, k_norm (hd) T), rounded to T
+   and rotated (rotate-half; cos_t, sin_t (>= positions, hd/2) float); q goes to q_out (B, hq, S, hd), k and v into the
+   caches (B, hk, max_seq, hd) at positions pos .. pos + S - 1, where pos is *pos_dev (device memory) or, with pos_dev
+   NULL, pos0. */
+int zmoe_qkv_post(const void* q, const void* k, const void* v, const void* q_norm, const void* k_norm,
+                  const float* cos_t, const float* sin_t, float eps, int B, int S, int hq, int hk, int hd,
+                  const int64_t* pos_dev, int pos0, int max_seq, void* q_out, void* k_cache, void* v_cache,
+                  void* stream);
+
+/* Grouped-query attention of one token per sequence over the cache, float arithmetic: q (B, hq, hd) T, caches
+   (B, hk, max_seq, hd) T, out (B, hq, hd) T; the first npos positions, or with pos_dev up to and including *pos_dev.
+   hd 64 or 128, hq / hk in {1, 2, 4, 8}; other shapes have a workspace of 0 bytes and are refused.  max_pos: npos, or
+   max_seq with pos_dev. */
+size_t zmoe_decode_attention_workspace_bytes(int B, int hq, int hk, int hd, int max_pos);
+int zmoe_decode_attention(const void* q, const void* k_cache, const void* v_cache, int B, int hq, int hk, int hd,
+                          const int64_t* pos_dev, int npos, int max_seq, float scale, void* workspace,
+                          size_t workspace_bytes, void* out, void* stream);
+
 /* --------------------------------------------------------- one-launch decode block */
 
 /* Packed tensors of one expert bank: (E, N, K/8) uint32 weights, (E, N, K/64) T scales and biases. */

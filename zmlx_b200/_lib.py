@@ -97,6 +97,13 @@ SIGNATURES = {
                                         c_void_p, c_void_p, c_void_p]),
     "zmoe_layer_decode_status": (c_int, [c_void_p, c_int, c_void_p]),
     "zmoe_layer_decode_inbox_bytes": (c_size_t, [ctypes.POINTER(LayerDesc), c_int]),
+    "zmoe_add_rms_norm": (c_int, [c_void_p, c_void_p, c_void_p, c_float, c_int, c_int, c_void_p, c_void_p]),
+    "zmoe_qkv_post": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_int,
+                              c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p,
+                              c_void_p]),
+    "zmoe_decode_attention_workspace_bytes": (c_size_t, [c_int, c_int, c_int, c_int, c_int]),
+    "zmoe_decode_attention": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int,
+                                      c_float, c_void_p, c_size_t, c_void_p, c_void_p]),
     "zmoe_ep_alloc": (c_int, [c_size_t, ctypes.POINTER(c_void_p)]),
     "zmoe_ep_free": (c_int, [c_void_p]),
     "zmoe_ep_export": (c_int, [c_void_p, c_void_p]),

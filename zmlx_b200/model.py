@@ -4,8 +4,10 @@
 q/k RMSNorm, RoPE base 1e6, KV cache) -> residual -> RMSNorm -> MoE block -> residual; greedy
 sampling.  The reference drives its patched MoE blocks with mlx_lm's decoder and validates
 token fidelity with greedy decoding (src/zmlx/validate.py:68-125, 211-225); here the attention side
-is plain torch ops -- float32 score/softmax arithmetic, so that a CPU restatement can reproduce it
--- and every MoE block is a :class:`zmlx_b200.layer.MoELayer` (or its expert-parallel form), i.e.
+runs float32 score/softmax arithmetic, so that a CPU restatement can reproduce it: libzmoe kernels for
+the norms, the q/k post-processing and the one-token attention (head dimension 64 or 128, 1, 2, 4 or 8
+query heads per KV head), torch for the projections, for prompts and for other head shapes.  Every MoE
+block is a :class:`zmlx_b200.layer.MoELayer` (or its expert-parallel form), i.e.
 the libzmoe kernels.  Weights are random-init: no checkpoint is involved.
 
 Command line: ``python -m zmlx_b200.model --layers 48 --prompt 4096 --new 256 --batch 1`` prints
@@ -22,7 +24,7 @@ from dataclasses import dataclass, field
 
 import torch
 
-from . import synthetic
+from . import ops, synthetic
 from .layer import MoELayer
 from .synthetic import MoEConfig
 
@@ -235,6 +237,12 @@ class StackedDecoder:
         self.k_cache = torch.zeros((L, max_batch, hk, max_seq, hd), dtype=torch.bfloat16, device=dev)
         self.v_cache = torch.zeros_like(self.k_cache)
         self.pos = 0
+        # the norm kernels take bfloat16 weights, as checkpoints of this layout hold them; others go through torch
+        norms = [params["final_norm"]] + [lp[n] for lp in params["layers"]
+                                          for n in ("attn_norm", "ffn_norm", "q_norm", "k_norm")]
+        self._kernels = (cfg.d_model <= 16384 and cfg.head_dim % 2 == 0 and params["embed"].dtype == torch.bfloat16
+                         and all(w.dtype == torch.bfloat16 and w.is_contiguous() and w.data_ptr() % 16 == 0
+                                 for w in norms))
         self.peer, self.peer_tokens = None, 0
         if moe_impl == "torch":  # the dequantised torch reference in place of the kernels (fidelity check)
             self.chunk = 1 << 30
@@ -261,6 +269,29 @@ class StackedDecoder:
     def reset(self) -> None:
         self.pos = 0
 
+    def _norm(self, h: torch.Tensor, delta: torch.Tensor | None, w: torch.Tensor) -> torch.Tensor:
+        """h (R, d) += delta in place, then its RMS norm."""
+        if self._kernels:
+            return ops.add_rms_norm(h, delta, w, self.cfg.rms_eps)
+        if delta is not None:
+            h += delta
+        return rms_norm(h, w, self.cfg.rms_eps)
+
+    def _qkv(self, i: int, lp: dict, x: torch.Tensor, B: int, S: int, pos) -> torch.Tensor:
+        """Project, normalise and rotate; k and v go to layer i's cache from position ``pos`` (an int, or an int64
+        device scalar with S == 1).  Returns q (B, Hq, S, hd)."""
+        cfg = self.cfg
+        q, k, v = x @ lp["q_w"].T, x @ lp["k_w"].T, x @ lp["v_w"].T
+        if self._kernels:
+            return ops.qkv_post(q, k, v, lp["q_norm"], lp["k_norm"], self.cos, self.sin, cfg.rms_eps, B, S, pos,
+                                self.k_cache[i], self.v_cache[i])
+        at = pos if isinstance(pos, torch.Tensor) else torch.arange(pos, pos + S, device=self.device)
+        cos, sin = self.cos.index_select(0, at), self.sin.index_select(0, at)
+        q, k, v = (t.view(B, S, -1, cfg.head_dim).transpose(1, 2) for t in (q, k, v))
+        self.k_cache[i, :B].index_copy_(2, at, apply_rope(rms_norm(k, lp["k_norm"], cfg.rms_eps), cos, sin))
+        self.v_cache[i, :B].index_copy_(2, at, v)
+        return apply_rope(rms_norm(q, lp["q_norm"], cfg.rms_eps), cos, sin)
+
     def _moe(self, i: int, x: torch.Tensor) -> torch.Tensor:
         """x (N, d) bfloat16 -> (N, d); long prefills go through in chunks."""
         if self.peer is not None and x.shape[0] == self.peer_tokens:
@@ -279,25 +310,24 @@ class StackedDecoder:
             raise ValueError(f"batch {B} / positions {self.pos + S} exceed the cache ({self.max_batch}, {self.max_seq})")
         hq, hk, hd = cfg.n_heads, cfg.n_kv_heads, cfg.head_dim
         p0, p1 = self.pos, self.pos + S
-        cos, sin = self.cos[p0:p1], self.sin[p0:p1]
-        h = self.p["embed"][ids]  # (B, S, d) bfloat16
+        h = self.p["embed"][ids].reshape(B * S, cfg.d_model)  # bfloat16, this call's own
+        m = None  # the previous block's output, not yet added to h
         for i, lp in enumerate(self.p["layers"]):
-            x = rms_norm(h, lp["attn_norm"], cfg.rms_eps)
-            q = (x @ lp["q_w"].T).view(B, S, hq, hd).transpose(1, 2)
-            k = (x @ lp["k_w"].T).view(B, S, hk, hd).transpose(1, 2)
-            v = (x @ lp["v_w"].T).view(B, S, hk, hd).transpose(1, 2)
-            q = apply_rope(rms_norm(q, lp["q_norm"], cfg.rms_eps), cos, sin)
-            k = apply_rope(rms_norm(k, lp["k_norm"], cfg.rms_eps), cos, sin)
-            self.k_cache[i, :B, :, p0:p1] = k
-            self.v_cache[i, :B, :, p0:p1] = v
-            a = attention(q, self.k_cache[i, :B, :, :p1], self.v_cache[i, :B, :, :p1], p0)
-            a = a.transpose(1, 2).reshape(B, S, hq * hd)
-            h = h + (a @ lp["o_w"].T)
-            x = rms_norm(h, lp["ffn_norm"], cfg.rms_eps)
-            m = self._moe(i, x.reshape(B * S, cfg.d_model))
-            h = h + m.view(B, S, cfg.d_model)
+            x = self._norm(h, m, lp["attn_norm"])
+            q = self._qkv(i, lp, x, B, S, p0)
+            a = None
+            if S == 1:
+                a = ops.decode_attention(q, self.k_cache[i], self.v_cache[i], npos=p1)
+            if a is None:
+                a = attention(q, self.k_cache[i, :B, :, :p1], self.v_cache[i, :B, :, :p1], p0)
+                a = a.transpose(1, 2).reshape(B * S, hq * hd)
+            x = self._norm(h, a @ lp["o_w"].T, lp["ffn_norm"])
+            m = self._moe(i, x)
         self.pos = p1
-        last = rms_norm(h[:, -1], self.p["final_norm"], cfg.rms_eps)
+        last = h.view(B, S, -1)[:, -1].contiguous()
+        if m is not None:
+            m = m.view(B, S, -1)[:, -1].contiguous()
+        last = self._norm(last, m, self.p["final_norm"])
         return (last @ self.p["lm_head"].T).float()
 
     # -- decode step with static shapes (for CUDA-graph replay) ------------------------------------------
@@ -310,27 +340,21 @@ class StackedDecoder:
         ids, pos = st["ids"], st["pos"]
         B = ids.shape[0]
         hq, hk, hd = cfg.n_heads, cfg.n_kv_heads, cfg.head_dim
-        rep = hq // hk
-        cos, sin = self.cos.index_select(0, pos), self.sin.index_select(0, pos)
-        dead = (st["kpos"] > pos)[None, None, None, None, :]  # cache slots after the current position
-        scale = 1.0 / math.sqrt(hd)
-        h = self.p["embed"].index_select(0, ids).unsqueeze(1)  # (B, 1, d)
+        h = self.p["embed"].index_select(0, ids)  # (B, d)
+        m = None
         for i, lp in enumerate(self.p["layers"]):
-            x = rms_norm(h, lp["attn_norm"], cfg.rms_eps)
-            q = (x @ lp["q_w"].T).view(B, 1, hq, hd).transpose(1, 2)
-            k = (x @ lp["k_w"].T).view(B, 1, hk, hd).transpose(1, 2)
-            v = (x @ lp["v_w"].T).view(B, 1, hk, hd).transpose(1, 2)
-            q = apply_rope(rms_norm(q, lp["q_norm"], cfg.rms_eps), cos, sin)
-            k = apply_rope(rms_norm(k, lp["k_norm"], cfg.rms_eps), cos, sin)
-            self.k_cache[i, :B].index_copy_(2, pos, k)
-            self.v_cache[i, :B].index_copy_(2, pos, v)
-            sc = torch.einsum("bgrsd,bgpd->bgrsp", q.float().view(B, hk, rep, 1, hd), self.k_cache[i, :B].float())
-            pr = torch.softmax((sc * scale).masked_fill(dead, float("-inf")), dim=-1)
-            a = torch.einsum("bgrsp,bgpd->bgrsd", pr, self.v_cache[i, :B].float()).to(torch.bfloat16)
-            h = h + (a.reshape(B, 1, hq * hd) @ lp["o_w"].T)
-            x = rms_norm(h, lp["ffn_norm"], cfg.rms_eps)
-            h = h + self._moe(i, x.reshape(B, cfg.d_model)).view(B, 1, cfg.d_model)
-        last = rms_norm(h[:, -1], self.p["final_norm"], cfg.rms_eps)
+            x = self._norm(h, m, lp["attn_norm"])
+            q = self._qkv(i, lp, x, B, 1, pos)
+            a = ops.decode_attention(q, self.k_cache[i], self.v_cache[i], pos=pos)
+            if a is None:  # head shapes outside the kernel: the whole cache, positions after the current one masked
+                dead = (st["kpos"] > pos)[None, None, None, None, :]
+                sc = torch.einsum("bgrsd,bgpd->bgrsp", q.float().view(B, hk, hq // hk, 1, hd), self.k_cache[i, :B].float())
+                pr = torch.softmax((sc * (1.0 / math.sqrt(hd))).masked_fill(dead, float("-inf")), dim=-1)
+                a = torch.einsum("bgrsp,bgpd->bgrsd", pr, self.v_cache[i, :B].float()).to(torch.bfloat16)
+                a = a.reshape(B, hq * hd)
+            x = self._norm(h, a @ lp["o_w"].T, lp["ffn_norm"])
+            m = self._moe(i, x)
+        last = self._norm(h, m, self.p["final_norm"])
         nxt = (last @ self.p["lm_head"].T).float().argmax(-1)
         st["log"].index_copy_(1, st["n"], nxt[:, None])
         ids.copy_(nxt)

@@ -8,6 +8,7 @@ there is no CPU path.
 from __future__ import annotations
 
 import ctypes
+import math
 
 import torch
 
@@ -235,3 +236,52 @@ def router_logits(x: torch.Tensor, wr: torch.Tensor, *, out_dtype: torch.dtype =
             _lib.check(_lib.load().zmoe_router_logits(_ptr(x2), _ptr(wr), T, E, d, _ptr(out), _dtype_code(out),
                                                       _stream()))
     return out.reshape(x.shape[:-1] + (E,))
+
+
+# ------------------------------------------------------------------ the attention side of the decoder
+
+
+def add_rms_norm(h: torch.Tensor, delta: torch.Tensor | None, w: torch.Tensor, eps: float) -> torch.Tensor:
+    """``h += delta`` in place (when given), then the RMS norm of the rows of h (R, d) with weight w (d)."""
+    dev = _need_cuda(h, delta, w)
+    x = torch.empty_like(h)
+    with torch.cuda.device(dev):
+        _lib.check(_lib.load().zmoe_add_rms_norm(_ptr(h), _ptr(delta), _ptr(w), ctypes.c_float(eps), h.shape[0],
+                                                 h.shape[1], _ptr(x), _stream()))
+    return x
+
+
+def qkv_post(q, k, v, q_norm, k_norm, cos, sin, eps: float, B: int, S: int, pos, k_cache, v_cache) -> torch.Tensor:
+    """Normalise and rotate the q and k heads of B*S projected tokens, append k and v to one layer's caches
+    (>= B, Hk, max_seq, hd); returns q (B, Hq, S, hd).  ``pos``: position of the first token, or an int64 device scalar."""
+    dev = _need_cuda(q, k, v, k_cache, v_cache)
+    hk, max_seq, hd = k_cache.shape[-3:]
+    hq = q.shape[-1] // hd
+    out = torch.empty((B, hq, S, hd), dtype=torch.bfloat16, device=dev)
+    on_dev = isinstance(pos, torch.Tensor)
+    with torch.cuda.device(dev):
+        _lib.check(_lib.load().zmoe_qkv_post(
+            _ptr(q), _ptr(k), _ptr(v), _ptr(q_norm), _ptr(k_norm), _ptr(cos), _ptr(sin), ctypes.c_float(eps), B, S, hq,
+            hk, hd, _ptr(pos) if on_dev else None, 0 if on_dev else int(pos), max_seq, _ptr(out), _ptr(k_cache),
+            _ptr(v_cache), _stream()))
+    return out
+
+
+def decode_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, *, npos: int | None = None,
+                     pos: torch.Tensor | None = None) -> torch.Tensor | None:
+    """Attention of one token per sequence, q (B, Hq, 1, hd), over the first ``npos`` positions of the caches (or up to
+    and including the int64 device scalar ``pos``): (B, Hq * hd) bfloat16, or None for head shapes without a kernel."""
+    dev = _need_cuda(q, k_cache, v_cache, pos)
+    B, hq, _, hd = q.shape
+    hk, max_seq = k_cache.shape[-3], k_cache.shape[-2]
+    lib = _lib.load()
+    n = int(lib.zmoe_decode_attention_workspace_bytes(B, hq, hk, hd, max_seq if npos is None else npos))
+    if n == 0:
+        return None
+    ws = torch.empty(n, dtype=torch.uint8, device=dev)
+    out = torch.empty((B, hq * hd), dtype=torch.bfloat16, device=dev)
+    with torch.cuda.device(dev):
+        _lib.check(lib.zmoe_decode_attention(_ptr(q), _ptr(k_cache), _ptr(v_cache), B, hq, hk, hd, _ptr(pos),
+                                             0 if npos is None else int(npos), max_seq,
+                                             ctypes.c_float(1.0 / math.sqrt(hd)), _ptr(ws), n, _ptr(out), _stream()))
+    return out
