@@ -50,6 +50,7 @@ constexpr int kTmScRing = 4, kTmScAhead = 3;      // scales: a thread's chunks i
 constexpr int kTmMaxTok = 96;                     // token rows per item, at most
 constexpr int kTmMaxX = 8;                        // token stages, at most
 constexpr int kTmMaxTasks = 1024;
+constexpr int kTmItems = 256;                     // work items of a CTA kept in shared memory
 constexpr int kTmCols = 512;
 constexpr int kTmColD = 128;                      // columns between the two accumulators
 constexpr int kTmColA = 224, kTmAStage = 136;     // two A stages: 128 columns of codes, 8 of scales and biases
@@ -91,10 +92,9 @@ __device__ __forceinline__ unsigned long long tm_now() {
   return t;
 }
 // Waits for the phase; false when a second passed or, unless `drain`, another thread of the CTA gave up.  Suspended
-// looks rather than a spin: polling warps would take the issue slots that the expanders live on.
-__device__ __forceinline__ bool tm_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, bool drain = false) {
-  for (int i = 0; i < 8; ++i)
-    if (tm_try(bar, parity, 20000u)) return true;
+// looks rather than a spin: polling warps would take the issue slots that the expanders live on.  The patient part is
+// out of line: the roles' loops share one instruction cache.
+__device__ __noinline__ bool tm_wait_long(uint32_t bar, uint32_t parity, volatile int* abort_flag, bool drain) {
   const unsigned long long t0 = tm_now();
   while (true) {
     if (tm_try(bar, parity, 20000u)) return true;
@@ -104,6 +104,12 @@ __device__ __forceinline__ bool tm_wait(uint32_t bar, uint32_t parity, volatile 
       return false;
     }
   }
+}
+__device__ __forceinline__ bool tm_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, bool drain = false) {
+#pragma unroll 1
+  for (int i = 0; i < 8; ++i)
+    if (tm_try(bar, parity, 20000u)) return true;
+  return tm_wait_long(bar, parity, abort_flag, drain);
 }
 // The same for a whole warp: all lanes leave together, as the tcgen05.ld and .st that follow need them to.
 __device__ __forceinline__ bool tm_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
@@ -152,10 +158,8 @@ __device__ __forceinline__ void tm_st16(uint32_t taddr, const uint32_t (&r)[16])
       "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
 }
-__device__ __forceinline__ void tm_st8(uint32_t taddr, const uint32_t (&r)[8]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]),
-               "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-               : "memory");
+__device__ __forceinline__ void tm_st2(uint32_t taddr, uint32_t r0, uint32_t r1) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1,%2};" ::"r"(taddr), "r"(r0), "r"(r1) : "memory");
 }
 // One lane of a converged warp.  The compiler knows an elected thread to be alone; behind `lane == 0` it would wrap
 // every tcgen05.mma and TMA instruction in a loop over the lanes that might be active (measured: 190 cycles per MMA
@@ -202,7 +206,7 @@ struct TmItem {
 };
 // Items are numbered task-major; inside a task the token blocks of one row tile are neighbours, so that they run at
 // the same time on different SMs and share the weights through L2.  prefix[a] = token blocks of the tasks before a.
-__device__ __forceinline__ TmItem tm_item(const PlanView& pv, const int* prefix, int ntasks, int ntiles, int tile_rows,
+__device__ __noinline__ TmItem tm_item(const PlanView& pv, const int* prefix, int ntasks, int ntiles, int tile_rows,
                                           int w) {
   int lo = 0, hi = ntasks - 1;
   while (lo < hi) {
@@ -222,6 +226,8 @@ __device__ __forceinline__ TmItem tm_item(const PlanView& pv, const int* prefix,
   return it;
 }
 
+__device__ __noinline__ float tm_swiglu(int epilogue, float g, float u) { return swiglu_epilogue(epilogue, g, u); }
+
 template <bool MX, int NMAT>
 __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_constant__ TmArgs a) {
   extern __shared__ __align__(1024) unsigned char tm_dyn[];
@@ -231,6 +237,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
   __shared__ float inv_s[4][kTmRows];
   __shared__ volatile int abort_s;
   __shared__ int prefix_s[kTmMaxTasks + 1];
+  __shared__ int4 items_s[kTmItems];
 
   constexpr int kTile = kTmRows / NMAT;  // output rows of an item
   const QmmParams& p = a.q;
@@ -271,6 +278,17 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
   if ((int)blockIdx.x >= total) return;  // before any tensor memory is taken
   const int n_items = (total - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
   const int n_chunks = n_items * nch;
+  // Every role walks the CTA's items: they are looked up once, by all threads (a search, two divisions and a load of
+  // the task record took each role some 1500 cycles per item); a CTA with more of them looks the rest up as it goes.
+  for (int i = tid; i < min(n_items, kTmItems); i += kTmThreads) {
+    const TmItem it = tm_item(pv, prefix_s, ntasks, ntiles, kTile, (int)blockIdx.x + i * (int)gridDim.x);
+    items_s[i] = make_int4(it.e, it.p0, it.nt, it.n0);
+  }
+  auto item_at = [&](int i) -> TmItem {
+    if (i >= kTmItems) return tm_item(pv, prefix_s, ntasks, ntiles, kTile, (int)blockIdx.x + i * (int)gridDim.x);
+    const int4 v = items_s[i];
+    return TmItem{v.x, v.y, v.z, v.w};
+  };
 
   if (tid == 0) {
     for (int i = 0; i < kTmRaw; ++i) {
@@ -326,7 +344,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
       if (f_item < n_items) {
         if (f_new) {
           f_new = false;
-          const TmItem it = tm_item(pv, prefix_s, ntasks, ntiles, kTile, (int)blockIdx.x + f_item * (int)gridDim.x);
+          const TmItem it = item_at(f_item);
           const size_t row = (size_t)it.e * N + min(it.n0 + rb, N - 1);  // clamped rows are computed, not stored
           // 8 bytes per chunk: four bfloat16 scales (biases) or eight e8m0 bytes
           f_s = reinterpret_cast<const unsigned char*>(p.s[mat]) + row * nch * 8;
@@ -349,18 +367,14 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
       asm volatile("cp.async.wait_group %0;" ::"n"(kTmScAhead) : "memory");
       const uint4 sc = *reinterpret_cast<const uint4*>(my_sc + slot * (kTmExp * 16));
       slot = (slot + 1) % kTmScRing;
-      // ---- the chunk's power of two and its scales in fp16
-      __half2 s_op[MX ? 8 : 4], s_off[MX ? 1 : 4], b_op[MX ? 1 : 4];
-      float inv;
+      // ---- the chunk's power of two
+      uint32_t s_lo = sc.x, s_hi = sc.y, b_lo = sc.z, b_hi = sc.w;  // shifted through, one group at a time
+      float inv, P = 0.0f;
+      int emax = 0;
       if (MX) {
         uint32_t v = __vmaxu4(sc.x, sc.y);
         v = __vmaxu4(v, v >> 16);
-        const int emax = (int)max(v & 0xffu, (v >> 8) & 0xffu);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {  // fp16 2^(e - emax + 11) in both halves; 0 from 26 binades below emax
-          const int e = (int)(((i < 4 ? sc.x : sc.y) >> (8 * (i & 3))) & 0xffu);
-          s_op[i] = tm_half2((uint32_t)max(e - emax + 26, 0) * 0x04000400u);
-        }
+        emax = (int)max(v & 0xffu, (v >> 8) & 0xffu);
         inv = emax >= 255 ? __uint_as_float(0x7f800000u) : exp2f((float)(emax - 127 - 11));
       } else {
         // largest |s| and |b| (bits order like magnitudes), as bfloat16 bits
@@ -370,17 +384,8 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
         mb = max(mb & 0xffffu, mb >> 16);
         // 2^(140 - e) brings |s| below 2^-4 (so that s 2^20 stays below 2^16) and |b| below 2^14
         const int e = min(max(max((int)(ms >> 7) + 18, (int)(mb >> 7)), 34), 253);
-        const float P = __uint_as_float((uint32_t)(267 - e) << 23), P20 = __uint_as_float((uint32_t)(287 - e) << 23);
+        P = __uint_as_float((uint32_t)(267 - e) << 23);
         inv = __uint_as_float((uint32_t)(e - 13) << 23);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const uint32_t sw = i < 2 ? sc.x : sc.y, bw = i < 2 ? sc.z : sc.w;
-          const float s = __uint_as_float((i & 1) ? (sw & 0xffff0000u) : (sw << 16));
-          const float b = __uint_as_float((i & 1) ? (bw & 0xffff0000u) : (bw << 16));
-          s_op[i] = __float2half2_rn(s * P20);
-          s_off[i] = __float2half2_rn(s * (-8.0f * P));
-          b_op[i] = __float2half2_rn(b * P);
-        }
       }
       // ---- the stage is free once the MMAs of the thread's previous chunk are done
       ok = tm_wait_warp(b_rawf + 8 * rs, rph, ab);
@@ -388,28 +393,37 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const unsigned char* src = my_raw + rs * kTmRawBytes;
+      uint4 wa = *reinterpret_cast<const uint4*>(src + ((rb & 7) << 4));
+      uint4 wb = *reinterpret_cast<const uint4*>(src + ((1 ^ (rb & 7)) << 4));
+#pragma unroll 1
+      for (int i = 0; i < 4; ++i) {  // 64 codes each: a group, or two mxfp4 blocks.  Rolled: see tm_wait_long
+        const int nx = 2 * min(i + 1, 3);
+        const uint4 na = *reinterpret_cast<const uint4*>(src + ((nx ^ (rb & 7)) << 4));
+        const uint4 nb = *reinterpret_cast<const uint4*>(src + (((nx + 1) ^ (rb & 7)) << 4));
+        const uint32_t ws[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+        uint32_t o[2][16];
+        if (MX) {
+          // fp16 2^(e - emax + 11) in both halves; 0 from 26 binades below emax
+          const __half2 s0 = tm_half2((uint32_t)max((int)(s_lo & 0xffu) - emax + 26, 0) * 0x04000400u);
+          const __half2 s1 = tm_half2((uint32_t)max((int)((s_lo >> 8) & 0xffu) - emax + 26, 0) * 0x04000400u);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {  // 32 codes each: half a group, or one mxfp4 block
-        const uint4 w4 = *reinterpret_cast<const uint4*>(src + ((i ^ (rb & 7)) << 4));
-        const uint32_t ws[4] = {w4.x, w4.y, w4.z, w4.w};
-        uint32_t o[16];
+          for (int k = 0; k < 8; ++k) tm_expand_mx(ws[k], k < 4 ? s0 : s1, o[k >> 2] + 4 * (k & 3));
+        } else {
+          const float s = __uint_as_float(s_lo << 16);
+          const __half2 s_op = __float2half2_rn(s * (P * 1048576.0f)), s_off = __float2half2_rn(s * (-8.0f * P));
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          if (MX)
-            tm_expand_mx(ws[k], s_op[i], o + 4 * k);
-          else
-            tm_expand_affine(ws[k], s_op[i >> 1], s_off[i >> 1], o + 4 * k);
+          for (int k = 0; k < 8; ++k) tm_expand_affine(ws[k], s_op, s_off, o[k >> 2] + 4 * (k & 3));
+          const __half2 b_op = __float2half2_rn(__uint_as_float(b_lo << 16) * P);
+          tm_st2(at + 128 + 2 * i, tm_bits(b_op), tm_bits(s_off));
+          b_lo = __funnelshift_r(b_lo, b_hi, 16);
+          b_hi >>= 16;
         }
-        tm_st16(at + i * 16, o);
-      }
-      if (!MX) {
-        uint32_t o[8];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          o[2 * i] = tm_bits(b_op[i]);
-          o[2 * i + 1] = tm_bits(s_off[i]);
-        }
-        tm_st8(at + 128, o);
+        tm_st16(at + i * 32, o[0]);
+        tm_st16(at + i * 32 + 16, o[1]);
+        s_lo = __funnelshift_r(s_lo, s_hi, 16);
+        s_hi >>= 16;
+        wa = na;
+        wb = nb;
       }
       inv_s[c & 3][r] = inv;
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -436,7 +450,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
     int c = 0;
 #pragma unroll 1
     for (int item = 0; item < n_items && ok; ++item) {
-      const TmItem it = tm_item(pv, prefix_s, ntasks, ntiles, kTile, (int)blockIdx.x + item * (int)gridDim.x);
+      const TmItem it = item_at(item);
       int dst[3];     // output row and row factor of token 16 (ch + 2 j) + lane % 16
       float xin[3];
 #pragma unroll
@@ -486,7 +500,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
             if (t0 + k < it.nt && n < N) {
               const float g = (hi ? other : acc[j][i]) * xs;
               const float u = (hi ? acc[j][i + 1] : other) * xs;
-              p.out[(size_t)row * p.ldo + n] = __float2bfloat16_rn(swiglu_epilogue(p.epilogue, g, u));
+              p.out[(size_t)row * p.ldo + n] = __float2bfloat16_rn(tm_swiglu(p.epilogue, g, u));
             }
           }
         } else {
@@ -505,7 +519,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
     int c = 0;
 #pragma unroll 1
     for (int item = 0; item < n_items && ok; ++item) {
-      const TmItem it = tm_item(pv, prefix_s, ntasks, ntiles, kTile, (int)blockIdx.x + item * (int)gridDim.x);
+      const TmItem it = item_at(item);
       const uint32_t idesc = tm_idesc((it.nt + 15) & ~15);
 #pragma unroll 1
       for (int cc = 0; cc < nch; ++cc, ++c) {
@@ -539,7 +553,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
     int c = 0;
 #pragma unroll 1
     for (int item = 0; item < n_items && ok; ++item) {
-      const TmItem it = tm_item(pv, prefix_s, ntasks, ntiles, kTile, (int)blockIdx.x + item * (int)gridDim.x);
+      const TmItem it = item_at(item);
       const int y = it.e * N + it.n0;  // a tile's rows beyond N are the next expert's: computed, not stored
 #pragma unroll 1
       for (int cc = 0; cc < nch; ++cc, ++c) {
@@ -561,7 +575,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
     int c = 0;
 #pragma unroll 1
     for (int item = 0; item < n_items && ok; ++item) {
-      const TmItem it = tm_item(pv, prefix_s, ntasks, ntiles, kTile, (int)blockIdx.x + item * (int)gridDim.x);
+      const TmItem it = item_at(item);
       const int nb = (it.nt + 15) >> 4;
 #pragma unroll 1
       for (int cc = 0; cc < nch; ++cc, ++c) {
@@ -748,7 +762,7 @@ int qmm_tma_launch(const QmmParams& q, int nmat, bool mx, int rows_hint, int max
   a.tn = tn > kTmMaxTok ? kTmMaxTok : (int)tn;
   a.xstage = (a.tn * (mx ? 512 : 544) + 1023) & ~1023;
   const int fixed = 1024 + kTmRaw * kTmRawBytes + kTmScRing * kTmExp * 16;
-  const int room = 227 * 1024 - 8 * 1024 - fixed;  // 8 KB: the static part (prefix sums, barriers, row factors)
+  const int room = 227 * 1024 - 12 * 1024 - fixed;  // 12 KB: the static part (prefix sums, items, barriers, row factors)
   a.rx = room / a.xstage > kTmMaxX ? kTmMaxX : room / a.xstage;
   const size_t smem = (size_t)fixed + (size_t)a.rx * a.xstage;
   int sms = 0, dev = 0;
