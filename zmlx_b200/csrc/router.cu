@@ -7,6 +7,7 @@
 #include "common.cuh"
 #include "layer_route.cuh"
 #include "plan.cuh"
+#include "qmm_common.cuh"
 #include "router_rows.cuh"
 
 namespace zmoe {
@@ -73,6 +74,67 @@ __global__ void __launch_bounds__(128) router_logits_kernel(const __nv_bfloat16*
       reinterpret_cast<float*>(logits)[o] = mine;
     else
       reinterpret_cast<__nv_bfloat16*>(logits)[o] = __float2bfloat16_rn(mine);
+  }
+}
+
+// Router linear for many rows, on the tensor cores: a CTA owns 16 tokens x 32 experts, its eight warps take every
+// eighth block of 32 along d and their fp32 sums are added in warp order.  Both operands are read straight into
+// mma fragments, 16 bytes per lane: a lane's eight consecutive values serve as the K pairs of two mma steps, the
+// same permutation of K on both sides.  Products of bfloat16 are exact in fp32, so this is the same sum as the warp
+// form above in another order.  The warp form spends three instructions per product on widening and adding, and one
+// warp walks all of d: bound by latency at tens of rows and by issue from hundreds on (c2, cold: 16 us for 16 rows, 31
+// us for 300).  Up to eight rows keep it: the one-launch block has the same order, and both give the same bits.
+constexpr int kRtTok = 16, kRtExp = 32, kRtWarps = 8;
+
+__global__ void __launch_bounds__(32 * kRtWarps) router_logits_mma_kernel(const __nv_bfloat16* __restrict__ x,
+                                                                          const __nv_bfloat16* __restrict__ wr, int T,
+                                                                          int E, int d, void* __restrict__ logits,
+                                                                          int out_dtype) {
+  __shared__ float part[kRtWarps][kRtTok][kRtExp + 1];
+  pdl_wait();
+  pdl_trigger();
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, g = lane >> 2, tig = lane & 3;
+  const int t0 = blockIdx.y * kRtTok, e0 = blockIdx.x * kRtExp;
+  const uint4* xa = reinterpret_cast<const uint4*>(x + (size_t)min(t0 + g, T - 1) * d) + tig;
+  const uint4* xb = reinterpret_cast<const uint4*>(x + (size_t)min(t0 + g + 8, T - 1) * d) + tig;
+  const uint4* wp[4];
+#pragma unroll
+  for (int n = 0; n < 4; ++n) wp[n] = reinterpret_cast<const uint4*>(wr + (size_t)min(e0 + 8 * n + g, E - 1) * d) + tig;
+  float acc[4][4];
+#pragma unroll
+  for (int n = 0; n < 4; ++n)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[n][j] = 0.0f;
+  const int nblk = d >> 5;
+#pragma unroll 2
+  for (int b = wid; b < nblk; b += kRtWarps) {
+    const uint4 va = __ldg(xa + b * 4), vb = __ldg(xb + b * 4);
+    uint4 vw[4];
+#pragma unroll
+    for (int n = 0; n < 4; ++n) vw[n] = __ldg(wp[n] + b * 4);
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      mma_bf16_m16n8k16(acc[n], va.x, vb.x, va.y, vb.y, vw[n].x, vw[n].y);
+      mma_bf16_m16n8k16(acc[n], va.z, vb.z, va.w, vb.w, vw[n].z, vw[n].w);
+    }
+  }
+#pragma unroll
+  for (int n = 0; n < 4; ++n)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) part[wid][g + 8 * (j >> 1)][8 * n + 2 * tig + (j & 1)] = acc[n][j];
+  __syncthreads();
+  for (int i = threadIdx.x; i < kRtTok * kRtExp; i += 32 * kRtWarps) {
+    const int t = i / kRtExp, e = i - t * kRtExp;
+    if (t0 + t < T && e0 + e < E) {
+      float v = part[0][t][e];
+#pragma unroll
+      for (int w = 1; w < kRtWarps; ++w) v += part[w][t][e];
+      const size_t o = (size_t)(t0 + t) * E + e0 + e;
+      if (out_dtype == ZMOE_F32)
+        reinterpret_cast<float*>(logits)[o] = v;
+      else
+        reinterpret_cast<__nv_bfloat16*>(logits)[o] = __float2bfloat16_rn(v);
+    }
   }
 }
 
@@ -216,6 +278,12 @@ int zmoe_router_logits(const void* x, const void* wr, int T, int E, int d, void*
   ZMOE_REQUIRE(out_dtype == ZMOE_F32 || out_dtype == ZMOE_BF16, ZMOE_ERR_DTYPE, "zmoe_router_logits: out dtype %d",
                out_dtype);
   if (T == 0) return ZMOE_OK;
+  if (T > 8 && d % 32 == 0 && (T + kRtTok - 1) / kRtTok <= 65535) {
+    launch_pdl(router_logits_mma_kernel, dim3((E + kRtExp - 1) / kRtExp, (T + kRtTok - 1) / kRtTok),
+               dim3(32 * kRtWarps), 0, (cudaStream_t)stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)wr, T, E, d,
+               logits, out_dtype);
+    return check_launch("zmoe_router_logits");
+  }
   dim3 grid((E + 3) / 4, (T + 7) / 8), block(128);
   launch_pdl(router_logits_kernel, grid, block, 0, (cudaStream_t)stream, (const __nv_bfloat16*)x,
              (const __nv_bfloat16*)wr, T, E, d, logits, out_dtype);
