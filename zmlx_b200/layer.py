@@ -155,12 +155,15 @@ class MoELayer:
                 nb = int(_lib.load().zmoe_layer_decode_inbox_bytes(ctypes.byref(self._desc), self.FUSED_MAX_TOKENS))
                 self._inbox = torch.zeros(nb, dtype=torch.uint8, device=self.device)
                 self._desc = self._describe()
-        p = ops._ptr
         lib = _lib.load()
         decode = lib.zmoe_layer_decode_mxfp4 if self.cfg.mode == "mxfp4" else lib.zmoe_layer_decode
-        _lib.check(decode(ctypes.byref(self._desc), p(x), x.stride(0), T, p(ws), ws.numel(), p(self.weights[row0:]),
-                          p(self.indices[row0:]), p(dst[row0:]), ops._stream()))
-        return dst[row0:row0 + T]
+        K4 = 4 * self.cfg.top_k  # bytes of a row of weights, of indices
+        rc = decode(ctypes.byref(self._desc), x.data_ptr(), x.stride(0), T, ws.data_ptr(), ws.numel(),
+                    self.weights.data_ptr() + row0 * K4, self.indices.data_ptr() + row0 * K4,
+                    dst.data_ptr() + row0 * dst.stride(0) * dst.element_size(), ops._stream())
+        if rc:
+            _lib.check(rc)
+        return dst if row0 == 0 and dst.shape[0] == T else dst[row0:row0 + T]
 
     def launch_count(self, T: int) -> int:
         """How many one-launch passes the T-token workspace has seen (the kernel's own launch counter)."""
@@ -330,41 +333,47 @@ class MoELayer:
             return self.out[:0]
         if x.stride(1) != 1 or x.stride(0) % 8 != 0 or x.data_ptr() % 16 != 0:
             x = x.contiguous()
+        if torch.cuda.current_device() == self.device.index:
+            return self._forward(x, T, out)
         with torch.cuda.device(self.device):
-            if self.fused:
-                ok = self._fused_ok.get(T)
-                if ok is None:
-                    passes = self._passes_win(T) and self._chunked_ok(T)
-                    ok = self._one_launch_bytes(T) > 0 or ("chunks" if passes else False)
-                    self._fused_ok[T] = ok
-                if ok == "chunks":
-                    dst = self.out if out is None else out
-                    for ci, (r, n) in enumerate(self._chunks(T)):
-                        self.forward_fused(x[r:r + n], dst, row0=r, key=(T, ci))
-                    return dst[:T]
-                # mxfp4 blocks may also be captured without a warm-up pass: on the separate kernels
-                if ok and (cfg.mode != "mxfp4" or T in self._fused_ws or not torch.cuda.is_current_stream_capturing()):
-                    return self.forward_fused(x, out)
-            residual = None
-            if cfg.n_shared:
-                # the shared expert depends on x only: it runs on a side stream beside the router and the routed
-                # experts and joins before the combine (fork and join are events, so a CUDA graph captures them)
-                cur = torch.cuda.current_stream(self.device)
-                if self._side is None:
-                    self._side = torch.cuda.Stream(device=self.device)
-                self._side.wait_stream(cur)
-                with torch.cuda.stream(self._side):
-                    self.shared(x)
-                residual = self.sh_y
-            self.route(x)
-            self.experts(x)
-            if cfg.n_shared:
-                cur.wait_stream(self._side)
-            dst = self.out if out is None else out
-            _lib.check(_lib.load().zmoe_moe_combine(
-                ops._ptr(self.y), _lib.BF16, ops._ptr(self.weights), _lib.F32, T, cfg.top_k, cfg.d_model,
-                self.combine_mode, ops._ptr(dst), 3 if cfg.family == "generic" else 1, ops._ptr(residual),
-                ops._stream()))
+            return self._forward(x, T, out)
+
+    def _forward(self, x: torch.Tensor, T: int, out: torch.Tensor | None) -> torch.Tensor:
+        cfg = self.cfg
+        if self.fused:
+            ok = self._fused_ok.get(T)
+            if ok is None:
+                passes = self._passes_win(T) and self._chunked_ok(T)
+                ok = self._one_launch_bytes(T) > 0 or ("chunks" if passes else False)
+                self._fused_ok[T] = ok
+            if ok == "chunks":
+                dst = self.out if out is None else out
+                for ci, (r, n) in enumerate(self._chunks(T)):
+                    self.forward_fused(x[r:r + n], dst, row0=r, key=(T, ci))
+                return dst[:T]
+            # mxfp4 blocks may also be captured without a warm-up pass: on the separate kernels
+            if ok and (cfg.mode != "mxfp4" or T in self._fused_ws or not torch.cuda.is_current_stream_capturing()):
+                return self.forward_fused(x, out)
+        residual = None
+        if cfg.n_shared:
+            # the shared expert depends on x only: it runs on a side stream beside the router and the routed
+            # experts and joins before the combine (fork and join are events, so a CUDA graph captures them)
+            cur = torch.cuda.current_stream(self.device)
+            if self._side is None:
+                self._side = torch.cuda.Stream(device=self.device)
+            self._side.wait_stream(cur)
+            with torch.cuda.stream(self._side):
+                self.shared(x)
+            residual = self.sh_y
+        self.route(x)
+        self.experts(x)
+        if cfg.n_shared:
+            cur.wait_stream(self._side)
+        dst = self.out if out is None else out
+        _lib.check(_lib.load().zmoe_moe_combine(
+            ops._ptr(self.y), _lib.BF16, ops._ptr(self.weights), _lib.F32, T, cfg.top_k, cfg.d_model,
+            self.combine_mode, ops._ptr(dst), 3 if cfg.family == "generic" else 1, ops._ptr(residual),
+            ops._stream()))
         return dst[:T]
 
     __call__ = forward

@@ -18,11 +18,16 @@ _U32_LIKE = (torch.int32, torch.uint32)
 
 
 def _ptr(t: torch.Tensor | None):
-    return None if t is None else ctypes.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
+
+
+# handle of the current stream of a device, without building a Stream object on every call
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
+    lambda index: torch.cuda.current_stream(index).cuda_stream)
 
 
 def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return _raw_stream(torch.cuda.current_device())
 
 
 def _need_cuda(*tensors: torch.Tensor | None) -> torch.device:

@@ -312,10 +312,10 @@ class _MoEMLPPattern:
             if fast is not None and x.dtype == torch.bfloat16 and x.is_cuda:
                 tokens = x.numel() // x.shape[-1]
                 if _should_fuse_swiglu_tokens(tokens, max_tokens):
-                    x2 = x.reshape(tokens, x.shape[-1])
+                    x2 = x if x.ndim == 2 else x.reshape(tokens, x.shape[-1])
                     out = torch.empty_like(x2)  # a fresh result, as every operator of the reference returns
                     fast.forward(x2, out=out)
-                    return out.reshape(x.shape)
+                    return out if x.ndim == 2 else out.reshape(x.shape)
             shared = getattr(self_mod, "shared_experts", None)
             indices, gate_weights = _gating(self_mod, x, gate_attr, num_experts_per_tok, is_qwen3=is_qwen3,
                                             is_gpt_oss=is_gpt_oss)
