@@ -12,10 +12,9 @@ namespace zmoe {
 constexpr int kNormThreads = 256;
 constexpr int kNormMaxVec = 8;  // 16-byte pieces a thread keeps: d up to 16384
 
-__global__ void __launch_bounds__(kNormThreads) add_rms_norm_kernel(__nv_bfloat16* __restrict__ h,
-                                                                    const __nv_bfloat16* __restrict__ delta,
-                                                                    const __nv_bfloat16* __restrict__ w, float eps,
-                                                                    int d, __nv_bfloat16* __restrict__ x) {
+__global__ void __launch_bounds__(kNormThreads) add_rms_norm_kernel(__nv_bfloat16* h, const __nv_bfloat16* delta,
+                                                                    const __nv_bfloat16* w, float eps, int d,
+                                                                    __nv_bfloat16* x) {
   __shared__ float part[kNormThreads / 32];
   pdl_wait();
   pdl_trigger();
@@ -154,7 +153,7 @@ __global__ void __launch_bounds__(kAttThreads) decode_attn_kernel(const AttParam
   __shared__ float sc[kAttBlock][REP];   // scores, then probabilities
   __shared__ float red[GRP][REP][HD];
   __shared__ float run_m[REP], run_s[REP], fac[REP];
-  pdl_wait();
+  pdl_wait();  // from here on plain loads: the non-coherent path must not run ahead of the wait
   pdl_trigger();
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int pair = blockIdx.y, b = pair / p.hk, kh = pair - b * p.hk;
@@ -167,7 +166,7 @@ __global__ void __launch_bounds__(kAttThreads) decode_attn_kernel(const AttParam
   float q[REP][8];
 #pragma unroll
   for (int r = 0; r < REP; ++r) {
-    const uint4 v = __ldg(reinterpret_cast<const uint4*>(p.q + (((size_t)b * p.hk + kh) * REP + r) * HD) + lane % LPR);
+    const uint4 v = *(reinterpret_cast<const uint4*>(p.q + (((size_t)b * p.hk + kh) * REP + r) * HD) + lane % LPR);
     const uint32_t u[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -191,7 +190,7 @@ __global__ void __launch_bounds__(kAttThreads) decode_attn_kernel(const AttParam
 #pragma unroll
     for (int j = 0; j < kAttBlock / GRP; ++j) {
       const int i = grp + j * GRP;
-      vv[j] = i < n ? __ldg(reinterpret_cast<const uint32_t*>(vc + (size_t)(p0 + i) * HD) + dp) : 0u;
+      vv[j] = i < n ? *(reinterpret_cast<const uint32_t*>(vc + (size_t)(p0 + i) * HD) + dp) : 0u;
     }
     __syncthreads();  // the previous block's probabilities are used up
 #pragma unroll
@@ -201,7 +200,7 @@ __global__ void __launch_bounds__(kAttThreads) decode_attn_kernel(const AttParam
 #pragma unroll
       for (int r = 0; r < REP; ++r) s[r] = 0.0f;
       if (i < n) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(kc + (size_t)(p0 + i) * HD) + lane % LPR);
+        const uint4 v = *(reinterpret_cast<const uint4*>(kc + (size_t)(p0 + i) * HD) + lane % LPR);
         const uint32_t u[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -280,8 +279,7 @@ __global__ void __launch_bounds__(kAttThreads) decode_attn_kernel(const AttParam
 }
 
 // One CTA of hd threads per query head: the slices' partial results under their common maximum.
-__global__ void decode_attn_join_kernel(const float* __restrict__ part, int nsplit, int rep, int hd,
-                                        __nv_bfloat16* __restrict__ out) {
+__global__ void decode_attn_join_kernel(const float* part, int nsplit, int rep, int hd, __nv_bfloat16* out) {
   pdl_wait();
   pdl_trigger();
   const int head = blockIdx.x, c = threadIdx.x;

@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(128) router_logits_kernel(const __nv_bfloat16*
 // us for 300).  Up to eight rows keep it: the one-launch block has the same order, and both give the same bits.
 constexpr int kRtTok = 16, kRtExp = 32, kRtWarps = 8;
 
-__global__ void __launch_bounds__(32 * kRtWarps) router_logits_mma_kernel(const __nv_bfloat16* __restrict__ x,
+__global__ void __launch_bounds__(32 * kRtWarps) router_logits_mma_kernel(const __nv_bfloat16* x,
                                                                           const __nv_bfloat16* __restrict__ wr, int T,
                                                                           int E, int d, void* __restrict__ logits,
                                                                           int out_dtype) {
@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(32 * kRtWarps) router_logits_mma_kernel(const 
   const int nblk = d >> 5;
 #pragma unroll 2
   for (int b = wid; b < nblk; b += kRtWarps) {
-    const uint4 va = __ldg(xa + b * 4), vb = __ldg(xb + b * 4);
+    const uint4 va = xa[b * 4], vb = xb[b * 4];
     uint4 vw[4];
 #pragma unroll
     for (int n = 0; n < 4; ++n) vw[n] = __ldg(wp[n] + b * 4);

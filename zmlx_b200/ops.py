@@ -90,7 +90,12 @@ def qmm_workspace(rows: int, E: int, K: int, *, rows_hint: int, mode: str, devic
     """Workspace of one grouped matmul call, from torch's allocator (so it belongs to the current stream and goes back
     to the pool when the call's reference is dropped), or None where the call gains nothing from one."""
     n = int(_lib.load().zmoe_qmm_workspace_bytes(int(rows), int(E), int(K), int(rows_hint), qmode_code(mode)))
-    return torch.empty(n, dtype=torch.uint8, device=device) if n else None
+    if n == 0:
+        return None
+    try:
+        return torch.empty(n, dtype=torch.uint8, device=device)
+    except torch.OutOfMemoryError:
+        return None  # the kernels that need none still serve the call
 
 
 def _ws_args(ws: torch.Tensor | None):
