@@ -77,6 +77,66 @@ __global__ void __launch_bounds__(256) combine_kernel(const void* __restrict__ y
   if (two) ob[oo + 1] = __float2bfloat16_rn(a1);
 }
 
+// The same for bfloat16 rows that can be read 16 bytes at a time (rows of 8 values, aligned): a thread owns eight adjacent
+// columns and asks for eight slots at once.  Bound by the projected rows' way from L2 or HBM (T*K*D*2 bytes): c2 with 4096
+// rows 69 -> 24 us, with 32 rows 7.1 -> 4.0 (two columns a thread, four bytes a load, one slot after the other).
+template <int MODE>
+__global__ void __launch_bounds__(128) combine8_kernel(const uint4* y, const void* w, int w_dtype, int K, int D8,
+                                                       void* out, int out_t, const uint4* residual) {
+  pdl_wait();
+  pdl_trigger();
+  const int t = blockIdx.y, d = blockIdx.x * blockDim.x + threadIdx.x;
+  if (d >= D8) return;
+  float a[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) a[j] = 0.0f;
+  for (int i0 = 0; i0 < K; i0 += 8) {
+    uint4 v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (i0 + i < K) v[i] = y[((size_t)t * K + i0 + i) * D8 + d];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if (i0 + i < K) {
+        float wi = load_as_float(w, w_dtype, (size_t)t * K + i0 + i);
+        if ((out_t & 2) || MODE == ZMOE_COMBINE_EXACT) wi = round_bf16(wi);
+        const uint32_t q[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float x = bf16_bits_to_float((j & 1) ? (q[j >> 1] >> 16) : (q[j >> 1] & 0xffffu));
+          if (MODE == ZMOE_COMBINE_FP32 || MODE == ZMOE_COMBINE_T)
+            a[j] = fmaf(wi, x, a[j]);
+          else if (MODE == ZMOE_COMBINE_FP32_NO_FMA || MODE == ZMOE_COMBINE_NO_FMA)
+            a[j] = __fadd_rn(a[j], __fmul_rn(wi, x));
+          else if (MODE == ZMOE_COMBINE_EXACT)
+            a[j] = round_bf16(__fadd_rn(a[j], round_bf16(__fmul_rn(wi, x))));
+          else
+            a[j] = round_bf16(__fadd_rn(a[j], __fmul_rn(wi, x)));
+        }
+      }
+    }
+  }
+  const size_t o = (size_t)t * D8 + d;
+  if ((MODE == ZMOE_COMBINE_FP32 || MODE == ZMOE_COMBINE_FP32_NO_FMA) && !(out_t & 1)) {
+    float4* of = reinterpret_cast<float4*>(out) + 2 * o;
+    of[0] = make_float4(a[0], a[1], a[2], a[3]);
+    of[1] = make_float4(a[4], a[5], a[6], a[7]);
+    return;
+  }
+  uint32_t r[4] = {0u, 0u, 0u, 0u}, res[4] = {0u, 0u, 0u, 0u};
+  if (residual != nullptr) {
+    const uint4 rv = residual[o];
+    res[0] = rv.x, res[1] = rv.y, res[2] = rv.z, res[3] = rv.w;
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    float v = round_bf16(a[j]);
+    if (residual != nullptr) v = __fadd_rn(v, bf16_bits_to_float((j & 1) ? (res[j >> 1] >> 16) : (res[j >> 1] & 0xffffu)));
+    r[j >> 1] |= (uint32_t)float_to_bf16_bits(v) << (16 * (j & 1));
+  }
+  reinterpret_cast<uint4*>(out)[o] = make_uint4(r[0], r[1], r[2], r[3]);
+}
+
 int combine_launch(const void* y, int y_dtype, const void* w, int w_dtype, int T, int K, int D, int mode, void* out,
                    int out_t, const void* residual, void* stream, const char* who) {
   ZMOE_REQUIRE(y && w && out, ZMOE_ERR_SHAPE, "%s: null pointer", who);
@@ -95,8 +155,16 @@ int combine_launch(const void* y, int y_dtype, const void* w, int w_dtype, int T
   dim3 block(256), grid(((D + 1) / 2 + 255) / 256, T);
   cudaStream_t st = (cudaStream_t)stream;
   const __nv_bfloat16* res = (const __nv_bfloat16*)residual;
-#define ZMOE_LAUNCH(M) \
-  launch_pdl(combine_kernel<M>, grid, block, 0, st, y, y_dtype, w, w_dtype, T, K, D, out, out_t, res)
+  const bool wide = y_dtype == ZMOE_BF16 && D % 8 == 0 && (((uintptr_t)y | (uintptr_t)out | (uintptr_t)residual) & 15) == 0;
+  const dim3 grid8((D / 8 + 127) / 128, T);
+#define ZMOE_LAUNCH(M)                                                                                              \
+  do {                                                                                                              \
+    if (wide)                                                                                                       \
+      launch_pdl(combine8_kernel<M>, grid8, dim3(128), 0, st, (const uint4*)y, w, w_dtype, K, D / 8, out, out_t,    \
+                 (const uint4*)residual);                                                                           \
+    else                                                                                                            \
+      launch_pdl(combine_kernel<M>, grid, block, 0, st, y, y_dtype, w, w_dtype, T, K, D, out, out_t, res);          \
+  } while (0)
   switch (mode) {
     case ZMOE_COMBINE_FP32: ZMOE_LAUNCH(ZMOE_COMBINE_FP32); break;
     case ZMOE_COMBINE_FP32_NO_FMA: ZMOE_LAUNCH(ZMOE_COMBINE_FP32_NO_FMA); break;
