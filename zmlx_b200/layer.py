@@ -128,9 +128,9 @@ class MoELayer:
 
     def _passes_win(self, T: int) -> bool:
         """Every pass streams its own rows' experts again, the grouped matmuls stream each expert once but cost some
-        launches: two passes win for wide blocks (c5, T = 16: 893 against 1003 us; T = 24: 1357 against 1334), and where
-        the second one is nearly empty (c2, T = 9: 100 against 108 us; T = 12: 127 against 125)."""
-        return T <= (16 if self.cfg.d_model * 2 * 8 > 96 * 1024 else 11)
+        launches: a second, half-filled pass wins for wide blocks only (c5, T = 12: 702 against 748 us; T = 16: 891
+        against 867; c2, T = 9: 100 against 102, T = 12: 127 against 113)."""
+        return T <= 12 and self.cfg.d_model * 2 * 8 > 96 * 1024
 
     def forward_fused(self, x: torch.Tensor, out: torch.Tensor | None = None, *, row0: int = 0,
                       key=None) -> torch.Tensor:
