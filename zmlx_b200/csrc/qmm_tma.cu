@@ -53,6 +53,7 @@ constexpr int kTmMaxTasks = 1024;
 constexpr int kTmItems = 256;                     // work items of a CTA kept in shared memory
 constexpr int kTmCols = 512;
 constexpr int kTmColD = 128;                      // columns between the two accumulators
+constexpr int kTmSplitTok = 48;                   // up to so many token rows an accumulator is two, one per half chunk
 constexpr int kTmColA = 224, kTmAStage = 136;     // two A stages: 128 columns of codes, 8 of scales and biases
 
 struct TmArgs {
@@ -318,6 +319,9 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_base_s;
+  // The tensor core's running sums lose a little at every step; where there is room for a second accumulator a chunk is
+  // summed as two halves, and folded as such (the finishers have the time).
+  const bool split = tn <= kTmSplitTok;
   volatile int* ab = &abort_s;
   bool ok = true;
 
@@ -476,6 +480,12 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
             for (int i = 0; i < 16; ++i) acc[j][i] = fmaf(d[i], inv, acc[j][i]);
+            if (split) {
+              tm_ld16(at + kTmSplitTok + 16 * (ch + 2 * j), d);
+              asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+              for (int i = 0; i < 16; ++i) acc[j][i] = fmaf(d[i], inv, acc[j][i]);
+            }
           }
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -535,15 +545,17 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t d = tmem + buf * kTmColD, at = tmem + kTmColA + buf * kTmAStage;
+        const uint32_t d2 = split ? d + kTmSplitTok : d;  // the second half of the chunk
         const uint32_t bt = tm_smem(tok + xs * a.xstage);
         if (tm_elect()) {
 #pragma unroll
           for (int g = 0; g < 4; ++g) {
             const uint64_t bd = tm_desc128(bt + g * tn * 128);
 #pragma unroll
-            for (int k = 0; k < 4; ++k) tm_mma(d, at + g * 32 + k * 8, bd + 2 * k, idesc, (g | k) != 0);
+            for (int k = 0; k < 4; ++k)
+              tm_mma(g < 2 ? d : d2, at + g * 32 + k * 8, bd + 2 * k, idesc, k != 0 || (g != 0 && !(split && g == 2)));
           }
-          if (!MX) tm_mma(d, at + 128, tm_desc32(bt + tn * 512), idesc, true);
+          if (!MX) tm_mma(d2, at + 128, tm_desc32(bt + tn * 512), idesc, true);
           tm_commit(b_done + 8 * buf);
           tm_commit(b_toke + 8 * xs);
         }
@@ -693,8 +705,8 @@ size_t qmm_tma_workspace(int rows, int K, bool mx) {
 
 // Which calls gain from the path: whole chunks along K, and more than eight rows on some expert (by the caller's
 // bound).  A block of up to eight token rows is taken by the one-launch kernel or the register-fed ones, whose cost per
-// expert is the same for one row as for eight (whole block, c2, T = 8: 78 us in one launch, 136 here; T = 16: 151 us in
-// two launches, 138 here).
+// expert is the same for one row as for eight (whole block, c2, T = 8: 76 us in one launch, 105 here; T = 16: 151 us in
+// two launches, 121 here).
 bool qmm_tma_wants(int E, int K, int rows_hint) {
   return K % kTmChunk == 0 && E <= kTmMaxTasks && rows_hint > 8;
 }
