@@ -4,7 +4,8 @@ This is the order of the reference's patched block
 (src/zmlx/patch/patterns/moe_mlp.py:883-1063) with every step running in a
 libzmoe kernel.  ``MoELayer`` owns the packed tensors of one layer and
 preallocated work buffers for a fixed maximum token count, so that a forward
-pass allocates nothing and can be captured in a CUDA graph.
+pass can be captured in a CUDA graph; above eight rows the grouped matmuls take a
+workspace from torch's allocator for the length of the call.
 """
 
 from __future__ import annotations
@@ -282,16 +283,21 @@ class MoELayer:
         K = cfg.top_k
         self._mlp(x, self.p, cfg.n_experts, cfg.d_ff, self.plan, T * K, T, self.h, self.y, self.swiglu, 3)
 
-    def _mlp(self, x, bank: dict, E: int, f: int, plan, rows: int, rows_hint: int, h, y, swiglu: int, down_flags: int):
-        """gate/up + SwiGLU of `rows` planned rows into h, and their down projection into y."""
+    def _workspace(self, rows: int, E: int, f: int, rows_hint: int) -> torch.Tensor | None:
+        # one workspace serves both matmuls: the second prepares its rows after the first has read its own
+        return ops.qmm_workspace(rows, E, max(self.cfg.d_model, f), rows_hint=rows_hint, mode=self.cfg.mode,
+                                 device=self.device)
+
+    def _mlp(self, x, bank: dict, E: int, f: int, plan, rows: int, rows_hint: int, h, y, swiglu: int, down_flags: int,
+             ws: torch.Tensor | None = None):
+        """gate/up + SwiGLU of `rows` planned rows into h, and their down projection into y; ``ws``: their workspace, by
+        default one of this call's own."""
         cfg = self.cfg
         lib = _lib.load()
         st = ops._stream()
         p = ops._ptr
         qm = ops.qmode_code(cfg.mode)
-        # one workspace serves both calls: the second prepares its rows after the first has read its own
-        ws = ops._ws_args(ops.qmm_workspace(rows, E, max(cfg.d_model, f), rows_hint=rows_hint, mode=cfg.mode,
-                                            device=self.device))
+        ws = ops._ws_args(self._workspace(rows, E, f, rows_hint) if ws is None else ws)
         _lib.check(lib.zmoe_gather_qmm_swiglu_ws(p(x), x.shape[0], x.stride(0), p(bank["gate_w"]), p(bank["gate_s"]),
                                                  p(bank["gate_b"]), p(bank["up_w"]), p(bank["up_s"]), p(bank["up_b"]),
                                                  E, f, cfg.d_model, self.gs, qm, p(plan), rows, rows_hint, p(h),
@@ -300,7 +306,7 @@ class MoELayer:
                                           cfg.d_model, f, self.gs, qm, p(plan), rows, rows_hint, down_flags, p(y), *ws,
                                           st))
 
-    def shared(self, x: torch.Tensor):
+    def shared(self, x: torch.Tensor, ws: torch.Tensor | None = None):
         """The always-on shared expert: the same kernels with a one-expert bank."""
         cfg = self.cfg
         T = x.shape[0]
@@ -316,7 +322,8 @@ class MoELayer:
                                                    ops._stream()))
             if not capturing:
                 self._shared_plans[T] = plan
-        self._mlp(x, self.p["shared"], 1, cfg.d_ff * cfg.n_shared, plan, T, T, self.sh_h, self.sh_y, _lib.SWIGLU_PER_OP, 1)
+        self._mlp(x, self.p["shared"], 1, cfg.d_ff * cfg.n_shared, plan, T, T, self.sh_h, self.sh_y, _lib.SWIGLU_PER_OP, 1,
+                  ws)
 
     def forward(self, x: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
         """x (T, d_model) bfloat16 on this layer's device -> (T, d_model) bfloat16: ``out`` when given (contiguous,
@@ -361,14 +368,18 @@ class MoELayer:
             cur = torch.cuda.current_stream(self.device)
             if self._side is None:
                 self._side = torch.cuda.Stream(device=self.device)
+            # its workspace is the current stream's (a side stream's pool starts empty, and memory taken there stays
+            # there): held until that stream has joined the side stream below
+            shared_ws = self._workspace(T, 1, cfg.d_ff * cfg.n_shared, T)
             self._side.wait_stream(cur)
             with torch.cuda.stream(self._side):
-                self.shared(x)
+                self.shared(x, shared_ws)
             residual = self.sh_y
         self.route(x)
         self.experts(x)
         if cfg.n_shared:
             cur.wait_stream(self._side)
+            del shared_ws
         dst = self.out if out is None else out
         _lib.check(_lib.load().zmoe_moe_combine(
             ops._ptr(self.y), _lib.BF16, ops._ptr(self.weights), _lib.F32, T, cfg.top_k, cfg.d_model,
