@@ -306,7 +306,10 @@ class MoELayer:
                                           cfg.d_model, f, self.gs, qm, p(plan), rows, rows_hint, down_flags, p(y), *ws,
                                           st))
 
-    def shared(self, x: torch.Tensor, ws: torch.Tensor | None = None):
+    def _new_shared_plan(self, T: int) -> torch.Tensor:
+        return torch.empty(ops.plan_bytes(T, 1) // 4, dtype=torch.int32, device=self.device)
+
+    def shared(self, x: torch.Tensor, ws: torch.Tensor | None = None, plan_buf: torch.Tensor | None = None):
         """The always-on shared expert: the same kernels with a one-expert bank."""
         cfg = self.cfg
         T = x.shape[0]
@@ -316,8 +319,7 @@ class MoELayer:
         plan = self._shared_plans.get(T)
         if plan is None:
             capturing = torch.cuda.is_current_stream_capturing()
-            plan = self.shared_plan if capturing else torch.empty(ops.plan_bytes(T, 1) // 4, dtype=torch.int32,
-                                                                  device=self.device)
+            plan = self.shared_plan if capturing else (self._new_shared_plan(T) if plan_buf is None else plan_buf)
             _lib.check(_lib.load().zmoe_build_plan(None, 1, p(self.zero_idx), T, 1, 1, p(plan), plan.numel() * 4,
                                                    ops._stream()))
             if not capturing:
@@ -368,12 +370,14 @@ class MoELayer:
             cur = torch.cuda.current_stream(self.device)
             if self._side is None:
                 self._side = torch.cuda.Stream(device=self.device)
-            # its workspace is the current stream's (a side stream's pool starts empty, and memory taken there stays
-            # there): held until that stream has joined the side stream below
+            # its workspace and plan are the current stream's memory (a side stream's pool starts empty, and what is
+            # taken there stays there); the workspace is held until that stream has joined the side stream below
             shared_ws = self._workspace(T, 1, cfg.d_ff * cfg.n_shared, T)
+            first = T not in self._shared_plans and not torch.cuda.is_current_stream_capturing()
+            plan_buf = self._new_shared_plan(T) if first else None
             self._side.wait_stream(cur)
             with torch.cuda.stream(self._side):
-                self.shared(x, shared_ws)
+                self.shared(x, shared_ws, plan_buf)
             residual = self.sh_y
         self.route(x)
         self.experts(x)
