@@ -244,9 +244,20 @@ class MoELayer:
             return 1, None, (2 if cfg.norm_topk_prob else 0)
         return 2, bias, 0
 
+    def _dense_rows(self, x: torch.Tensor) -> torch.Tensor:
+        """x with its rows one after the other, as the router entries read them (the matmuls and the one-launch block
+        take a row stride): a copy for views such as ``h[:, -1]``.  Rows that overlap stay refused."""
+        step = x.stride(0)
+        if x.shape[0] == 1 or step == self.cfg.d_model:
+            return x
+        if step < self.cfg.d_model:
+            raise _lib.ZmoeError(_lib.ERR_ALIGN, f"token rows of {self.cfg.d_model} values overlap (row stride {step})")
+        return x.contiguous()
+
     def route(self, x: torch.Tensor):
         """Router linear (bf16 logits), the family's top-k and the expert plan, in one launch."""
         cfg = self.cfg
+        x = self._dense_rows(x)
         T = x.shape[0]
         p = ops._ptr
         family, bias, renorm = self._route_args()
@@ -363,6 +374,7 @@ class MoELayer:
             # mxfp4 blocks may also be captured without a warm-up pass: on the separate kernels
             if ok and (cfg.mode != "mxfp4" or T in self._fused_ws or not torch.cuda.is_current_stream_capturing()):
                 return self.forward_fused(x, out)
+        x = self._dense_rows(x)
         residual = None
         if cfg.n_shared:
             # the shared expert depends on x only: it runs on a side stream beside the router and the routed
