@@ -53,3 +53,15 @@ def test_overlapping_rows_stay_refused(T):
     row = synthetic.make_tokens(cfg, 1, device=DEV)
     with pytest.raises(_lib.ZmoeError):
         layer(row.expand(T, -1))
+
+
+@pytest.mark.parametrize("T", [4, 16])
+def test_patched_block_on_a_transposed_input(T):
+    """The columns of a (d, T) matrix: the result has rows of its own, not the strides of its input."""
+    cfg, params = _params("c1")
+    block = znn.block_from_params(cfg, params)
+    patch(torch.nn.ModuleList([block]), patterns=["moe_mlp"])
+    dense = synthetic.make_tokens(cfg, T, device=DEV)
+    across = dense.T.contiguous().T
+    assert across.stride() == (1, T)
+    assert torch.equal(block(across), block(dense))

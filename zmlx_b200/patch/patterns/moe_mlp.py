@@ -313,7 +313,9 @@ class _MoEMLPPattern:
                 tokens = x.numel() // x.shape[-1]
                 if _should_fuse_swiglu_tokens(tokens, max_tokens):
                     x2 = x if x.ndim == 2 else x.reshape(tokens, x.shape[-1])
-                    out = torch.empty_like(x2)  # a fresh result, as every operator of the reference returns
+                    # a fresh result, as every operator of the reference returns; its rows are written one after the
+                    # other, so it never takes over the strides of a transposed input
+                    out = torch.empty(x2.shape, dtype=x2.dtype, device=x2.device)
                     fast.forward(x2, out=out)
                     return out if x.ndim == 2 else out.reshape(x.shape)
             shared = getattr(self_mod, "shared_experts", None)
