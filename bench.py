@@ -372,8 +372,8 @@ def main() -> None:
 
             indices = property(lambda self: self.fast.indices)
 
-            def fused_workspace_bytes(self, t):
-                return self.fast.fused_workspace_bytes(t)
+            def passes(self, t):
+                return self.fast.passes(t)
 
             def check_status(self):
                 self.fast.check_status()
@@ -472,12 +472,11 @@ def main() -> None:
     # local plan kernel (the NCCL and torch kernels are not counted)
     launches_per_layer = (4 if T * (world if use_ep else 1) <= 8 else 8) + (1 if use_ep else 0)
     launches_per_layer += (2 if T <= 8 else 4) if cfg.n_shared else 0
-    one_launch = ep_peer or ((not use_ep) and layers[0].fused and layers[0].fused_workspace_bytes(T) > 0)
+    # zmoe_layer_decode: the whole block, shared expert included, in one launch per pass of up to eight rows
+    passes = 1 if ep_peer else (0 if use_ep else len(layers[0].passes(T)))
+    one_launch = passes > 0
     if one_launch:
-        launches_per_layer = 1  # zmoe_layer_decode: the whole block, shared expert included
-    elif (not use_ep) and layers[0].fused and layers[0]._passes_win(T) and layers[0]._chunked_ok(T):
-        one_launch = True  # consecutive one-launch passes over eight rows each
-        launches_per_layer = len(layers[0]._chunks(T))
+        launches_per_layer = passes
 
     with torch.cuda.stream(stream):
         for _ in range(max(args.warmup, 3)):

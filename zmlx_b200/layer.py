@@ -121,17 +121,25 @@ class MoELayer:
 
     def _chunked_ok(self, T: int) -> bool:
         """Whether more rows than one launch takes can run as consecutive one-launch passes over eight rows each."""
-        cfg = self.cfg
-        dense = 4 if cfg.d_model * 2 * 8 > 96 * 1024 else 2
-        if self.ep is not None or T <= self.FUSED_MAX_TOKENS or T * cfg.top_k > dense * cfg.n_experts:
+        if self.ep is not None or T <= self.FUSED_MAX_TOKENS:
             return False
         return all(self.fused_workspace_bytes(n) > 0 for n in {n for _, n in self._chunks(T)})
 
     def _passes_win(self, T: int) -> bool:
         """Every pass streams its own rows' experts again, the grouped matmuls stream each expert once but cost some
-        launches: a second, half-filled pass wins for wide blocks only (c5, T = 12: 702 against 748 us; T = 16: 891
-        against 867; c2, T = 9: 100 against 102, T = 12: 127 against 113)."""
-        return T <= 12 and self.cfg.d_model * 2 * 8 > 96 * 1024
+        launches: a second, half-filled pass wins for wide blocks only, while the passes share few experts (c5, T = 12: 702
+        against 748 us; T = 16: 891 against 867; c2, T = 9: 100 against 102, T = 12: 127 against 113)."""
+        cfg = self.cfg
+        return T <= 12 and cfg.d_model * 2 * 8 > 96 * 1024 and T * cfg.top_k <= 4 * cfg.n_experts
+
+    def passes(self, T: int) -> list[tuple[int, int]]:
+        """(first row, rows) of the one-launch passes that a forward of T rows runs as; empty where the separate kernels
+        take it."""
+        if not self.fused or T < 1:
+            return []
+        if self._one_launch_bytes(T) > 0:
+            return [(0, T)]
+        return self._chunks(T) if self._passes_win(T) and self._chunked_ok(T) else []
 
     def forward_fused(self, x: torch.Tensor, out: torch.Tensor | None = None, *, row0: int = 0,
                       key=None) -> torch.Tensor:
@@ -363,9 +371,8 @@ class MoELayer:
         if self.fused:
             ok = self._fused_ok.get(T)
             if ok is None:
-                passes = self._passes_win(T) and self._chunked_ok(T)
-                ok = self._one_launch_bytes(T) > 0 or ("chunks" if passes else False)
-                self._fused_ok[T] = ok
+                n = len(self.passes(T))
+                ok = self._fused_ok[T] = "chunks" if n > 1 else n == 1
             if ok == "chunks":
                 dst = self.out if out is None else out
                 for ci, (r, n) in enumerate(self._chunks(T)):
