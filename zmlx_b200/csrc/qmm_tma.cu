@@ -217,7 +217,7 @@ __device__ __noinline__ TmItem tm_item(const PlanView& pv, const int* prefix, in
   const int local = w - ntiles * prefix[lo];
   const int nblk = prefix[lo + 1] - prefix[lo];
   const int tile = local / nblk, blk = local - tile * nblk;
-  const int4 task = __ldg(reinterpret_cast<const int4*>(pv.tasks) + lo);  // {expert, offset, count, -}
+  const int4 task = reinterpret_cast<const int4*>(pv.tasks)[lo];  // {expert, offset, count, -}
   const int per = ((task.z + nblk - 1) / nblk + 15) & ~15;                // equal blocks, whole 16s
   TmItem it;
   it.e = task.x;
@@ -252,13 +252,15 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
   const uint32_t b_rawf = bars, b_rawe = bars + 8 * kTmRaw, b_tokf = bars + 16 * kTmRaw;
   const uint32_t b_toke = b_tokf + 8 * kTmMaxX, b_af = b_toke + 8 * kTmMaxX, b_done = b_af + 16, b_dfree = b_done + 16;
 
+  // The plan, the prepared rows and their factors may be the work of the kernel before, still running when this one
+  // starts: they are read with plain loads after the wait, never through the read-only path.
   pdl_wait();
   pdl_trigger();
   const int ntasks = min(pv.hdr[0], kTmMaxTasks);
   if (wid == 0) {  // token blocks per task, prefix-summed (lane = a contiguous run of tasks)
     const int per = (ntasks + 31) >> 5;
     int sum = 0;
-    for (int i = lane * per; i < min(ntasks, (lane + 1) * per); ++i) sum += (__ldg(pv.tasks + 4 * i + 2) + tn - 1) / tn;
+    for (int i = lane * per; i < min(ntasks, (lane + 1) * per); ++i) sum += (pv.tasks[4 * i + 2] + tn - 1) / tn;
     int incl = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -268,7 +270,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
     int run = incl - sum;
     for (int i = lane * per; i < min(ntasks, (lane + 1) * per); ++i) {
       prefix_s[i] = run;
-      run += (__ldg(pv.tasks + 4 * i + 2) + tn - 1) / tn;
+      run += (pv.tasks[4 * i + 2] + tn - 1) / tn;
     }
     if (lane == 31) prefix_s[ntasks] = incl;
   }
@@ -459,8 +461,8 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
 #pragma unroll
       for (int j = 0; j < 3; ++j) {
         const int t = 16 * (ch + 2 * j) + (lane & 15);
-        dst[j] = t < it.nt ? __ldg(pv.row_dst + it.p0 + t) : 0;
-        xin[j] = t < it.nt ? __ldg(a.xinv + it.p0 + t) : 0.0f;
+        dst[j] = t < it.nt ? pv.row_dst[it.p0 + t] : 0;
+        xin[j] = t < it.nt ? a.xinv[it.p0 + t] : 0.0f;
 #pragma unroll
         for (int i = 0; i < 16; ++i) acc[j][i] = 0.0f;
       }
@@ -634,9 +636,9 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
 constexpr int kPrepThreads = 128;
 
 template <bool MX>
-__global__ void __launch_bounds__(kPrepThreads) prep_rows_kernel(const __nv_bfloat16* __restrict__ x, int ldx,
-                                                                 const int* plan, int rows, int E, int x_by_dst, int K,
-                                                                 __half* __restrict__ xs, float* __restrict__ xinv) {
+__global__ void __launch_bounds__(kPrepThreads) prep_rows_kernel(const __nv_bfloat16* x, int ldx, const int* plan,
+                                                                 int rows, int E, int x_by_dst, int K, __half* xs,
+                                                                 float* xinv) {
   __shared__ uint32_t warp_max[kPrepThreads / 32];
   pdl_wait();
   pdl_trigger();
@@ -648,7 +650,7 @@ __global__ void __launch_bounds__(kPrepThreads) prep_rows_kernel(const __nv_bflo
   const int nv = K >> 3;
   uint32_t mx = 0;
   for (int i = tid; i < nv; i += kPrepThreads) {
-    const uint4 v = __ldg(xr + i);
+    const uint4 v = xr[i];
     const uint32_t q[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
     for (int k = 0; k < 4; ++k) mx = max(mx, max(q[k] & 0x7fffu, (q[k] >> 16) & 0x7fffu));
@@ -666,7 +668,7 @@ __global__ void __launch_bounds__(kPrepThreads) prep_rows_kernel(const __nv_bflo
   const size_t stride = MX ? (size_t)K : (size_t)K + K / 16;
   __half* row = xs + (size_t)pos * stride;
   for (int i = tid; i < nv; i += kPrepThreads) {  // nv is a multiple of 32: a warp is whole or absent
-    const uint4 v = __ldg(xr + i);
+    const uint4 v = xr[i];
     const uint32_t q[4] = {v.x, v.y, v.z, v.w};
     float f[8];
 #pragma unroll
