@@ -144,6 +144,14 @@ size_t zmoe_plan_bytes(int rows, int E);
 int zmoe_build_plan(const int32_t* lhs, int lhs_div, const int32_t* rhs, int P, int M, int E, void* plan,
                     size_t plan_bytes, void* stream);
 
+/*
+ * Status of the grouped matmuls that ran on `plan`: copies its status word to the host on `stream` and WAITS for the
+ * stream.  ZMOE_OK, or ZMOE_ERR_TIMEOUT when a bounded wait ran out in one of them since the word was last cleared (the
+ * word outlives later zmoe_build_plan calls of the same sizes); with clear != 0 it is zeroed again on `stream`.  A plan
+ * buffer must not be asked before its first zmoe_build_plan unless it was zeroed.
+ */
+int zmoe_plan_status(const void* plan, int clear, void* stream);
+
 /* ------------------------------------------------------------ expert matmuls */
 
 /*
@@ -167,8 +175,10 @@ int zmoe_gather_qmm_swiglu(const void* x, int x_rows, int ldx, const uint32_t* g
  * reads x row r (the down projection after gather_qmm_swiglu, whose output rows are
  * already one per pair) instead of the plan's lhs row (bit 0).  Bit 1 of x_by_output_row
  * declares that the plan was written before the kernel that produced x started; the call
- * may then stream its first weights while that kernel is still running.
+ * may then stream its first weights while that kernel is still running.  ZMOE_DEBUG_WITHHOLD_TOKENS is a test hook of
+ * the workspace form below: the kernel's bounded waits run out (zmoe_plan_status), after about a second.
  */
+#define ZMOE_DEBUG_WITHHOLD_TOKENS 0x40000000
 int zmoe_gather_qmm(const void* x, int x_rows, int ldx, const uint32_t* w, const void* scales, const void* biases,
                     int E, int N, int K, int group_size, int qmode, const void* plan, int rows, int rows_hint,
                     int x_by_output_row, void* out, void* stream);

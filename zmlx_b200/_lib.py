@@ -16,6 +16,7 @@ LIB_PATH = os.environ.get("ZMOE_LIB") or os.path.join(_HERE, "libzmoe.so")
 
 OK = 0
 ABI_VERSION = 2
+DEBUG_WITHHOLD_TOKENS = 0x40000000
 DEBUG_WITHHOLD_LOGIT = 1
 DEBUG_FORCE_INBOX = 2
 ERR_SHAPE, ERR_DTYPE, ERR_ALIGN, ERR_UNSUPPORTED, ERR_CUDA, ERR_TIMEOUT, ERR_WORKSPACE = -1, -2, -3, -4, -5, -6, -7
@@ -95,6 +96,7 @@ SIGNATURES = {
     "zmoe_layer_decode_mxfp4_workspace_bytes": (c_size_t, [ctypes.POINTER(LayerDesc), c_int]),
     "zmoe_layer_decode_mxfp4": (c_int, [ctypes.POINTER(LayerDesc), c_void_p, c_int, c_int, c_void_p, c_size_t, c_void_p,
                                         c_void_p, c_void_p, c_void_p]),
+    "zmoe_plan_status": (c_int, [c_void_p, c_int, c_void_p]),
     "zmoe_layer_decode_status": (c_int, [c_void_p, c_int, c_void_p]),
     "zmoe_layer_decode_inbox_bytes": (c_size_t, [ctypes.POINTER(LayerDesc), c_int]),
     "zmoe_add_rms_norm": (c_int, [c_void_p, c_void_p, c_void_p, c_float, c_int, c_int, c_void_p, c_void_p]),

@@ -108,4 +108,17 @@ int zmoe_build_plan(const int32_t* lhs, int lhs_div, const int32_t* rhs, int P, 
   return check_launch("zmoe_build_plan");
 }
 
+int zmoe_plan_status(const void* plan, int clear, void* stream) {
+  ZMOE_REQUIRE(plan != nullptr, ZMOE_ERR_SHAPE, "zmoe_plan_status: null plan");
+  cudaStream_t st = (cudaStream_t)stream;
+  int word = 0;
+  int* dev = (int*)plan + 2;
+  cudaError_t e = cudaMemcpyAsync(&word, dev, sizeof(int), cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e == cudaSuccess && word == kPlanTimeout && clear) e = cudaMemsetAsync(dev, 0, sizeof(int), st);
+  if (e != cudaSuccess) return fail(ZMOE_ERR_CUDA, "zmoe_plan_status: %s", cudaGetErrorString(e));
+  if (word != kPlanTimeout) return ZMOE_OK;
+  return fail(ZMOE_ERR_TIMEOUT, "zmoe_plan_status: a bounded wait of a grouped matmul ran out; its output is NaN or void");
+}
+
 }  // extern "C"

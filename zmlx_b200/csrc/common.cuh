@@ -36,6 +36,11 @@ struct PlanView {
   int* row_dst;
 };
 
+// The header's third word: 0, 1 (pairs with an expert id outside 0..E-1 were dropped), or this, set by a matmul whose
+// bounded wait ran out.  It outlives the plan builds that follow, until zmoe_plan_status clears it; a value that fresh
+// memory does not hold by chance.
+constexpr int kPlanTimeout = 0x5a4d5457;
+
 __host__ __device__ inline PlanView plan_view(void* base, int rows, int E) {
   PlanView v;
   int* p = reinterpret_cast<int*>(base);

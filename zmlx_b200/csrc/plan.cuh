@@ -21,7 +21,11 @@ __device__ __forceinline__ void build_plan_block(const int* lhs, int lhs_div, co
   PlanView pv = plan_view(plan_base, rows, E);
   const int tid = threadIdx.x;
   __shared__ int bad;
-  if (tid == 0) bad = 0;
+  bool timed_out = false;  // of this plan's previous build: kept
+  if (tid == 0) {
+    bad = 0;
+    timed_out = pv.hdr[2] == kPlanTimeout && pv.hdr[1] == rows && pv.hdr[3] == E;
+  }
   for (int e = tid; e < E; e += NTHREADS) count[e] = 0;
   __syncthreads();
   for (int p = tid; p < P; p += NTHREADS) {
@@ -82,7 +86,7 @@ __device__ __forceinline__ void build_plan_block(const int* lhs, int lhs_div, co
     }
   }
   __syncthreads();
-  if (tid == 0) pv.hdr[2] = bad;
+  if (tid == 0) pv.hdr[2] = timed_out ? kPlanTimeout : bad;
 }
 
 }  // namespace zmoe

@@ -533,6 +533,7 @@ int qmm_launch(int nmat, const void* x, int x_rows, int ldx, const uint32_t* con
   p.epilogue = epilogue;
   p.x_by_dst = x_by_dst & 1;
   p.late_wait = (x_by_dst & 2) ? 1 : 0;
+  p.withhold = (x_by_dst & ZMOE_DEBUG_WITHHOLD_TOKENS) ? 1 : 0;
 
   if (qmm_tma_covers(p, nmat, mx, rows_hint, ws, ws_bytes))
     return qmm_tma_launch(p, nmat, mx, rows_hint, rows < E ? rows : E, ws, (cudaStream_t)stream, who);

@@ -19,6 +19,7 @@ struct QmmParams {
   int rs;        // token rows staged per pass (<= TT*NT)
   int epilogue;  // 0: store T; 1: SwiGLU CPU contract; 2: SwiGLU per-op contract
   int x_by_dst;  // token row r of the output reads x row r instead of the plan's source row
+  int withhold;   // test hook: no token tile ever arrives (ZMOE_DEBUG_WITHHOLD_TOKENS)
   int late_wait;  // the plan predates the previous kernel: stream the first weights before the dependency wait
 };
 

@@ -449,7 +449,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const TcParams tp
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  if (abort_s && tid == 0) atomicExch(pv.hdr + 2, 2);  // the plan's status word: a bounded wait ran out
+  if (abort_s && tid == 0) atomicExch(pv.hdr + 2, kPlanTimeout);  // the plan's status word: a bounded wait ran out
   if (wid == 0) {
     __syncwarp();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTcCols) : "memory");

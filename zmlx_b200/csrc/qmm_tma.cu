@@ -31,8 +31,9 @@
 // gate and up share one accumulator: lanes 0-15 of each warp's 32 tensor-memory lanes hold gate rows, lanes 16-31 the
 // up rows of the same outputs, and the epilogue pairs them with one shuffle.
 //
-// Every wait is bounded by a second; one that runs out sets the plan's status word, everybody else leaves at the next
-// wait, copies and MMAs in flight are waited for, and the tensor memory is given back.
+// Every wait is bounded by a second; one that runs out sets the plan's status word (zmoe_plan_status), everybody else
+// leaves at the next wait, copies and MMAs in flight are waited for, the tensor memory is given back and the CTA's results
+// become NaN.
 #include <cuda.h>
 #include <cuda_fp16.h>
 
@@ -597,7 +598,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
     // ================================================================== the warp that copies token tiles
     int c = 0;
 #pragma unroll 1
-    for (int item = 0; item < n_items && ok; ++item) {
+    for (int item = 0; item < n_items && ok && !p.withhold; ++item) {
       const TmItem it = item_at(item);
       const int nb = (it.nt + 15) >> 4;
 #pragma unroll 1
@@ -623,7 +624,16 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  if (abort_s && tid == 0) atomicExch(pv.hdr + 2, 2);  // the plan's status word: a bounded wait ran out
+  if (abort_s) {  // a bounded wait ran out: the plan says so, and the CTA's results are NaN rather than whatever was there
+    if (tid == 0) atomicExch(pv.hdr + 2, kPlanTimeout);
+    for (int i = 0; i < n_items; ++i) {
+      const TmItem it = item_at(i);
+      for (int j = tid; j < it.nt * kTile; j += kTmThreads) {
+        const int n = it.n0 + j % kTile;
+        if (n < N) p.out[(size_t)pv.row_dst[it.p0 + j / kTile] * p.ldo + n] = __float2bfloat16_rn(__int_as_float(0x7fc00000));
+      }
+    }
+  }
   if (wid == 0) {
     __syncwarp();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmCols) : "memory");

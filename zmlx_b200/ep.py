@@ -109,7 +109,7 @@ class EPMoELayer:
         dev = self.inner.device
         TK = max_tokens * world * cfg.top_k
         self.local_idx = torch.empty((TK,), dtype=torch.int32, device=dev)
-        self.local_plan = torch.empty(ops.plan_bytes(TK, self.n_local) // 4, dtype=torch.int32, device=dev)
+        self.local_plan = torch.zeros(ops.plan_bytes(TK, self.n_local) // 4, dtype=torch.int32, device=dev)
         self.out = torch.empty((max_tokens, cfg.d_model), dtype=torch.bfloat16, device=dev)
         self.x_all = torch.empty((max_tokens * world, cfg.d_model), dtype=torch.bfloat16, device=dev)
         self.y_mine = torch.empty((max_tokens * cfg.top_k, cfg.d_model), dtype=torch.bfloat16, device=dev)
@@ -191,6 +191,11 @@ class EPMoELayer:
         return self.out[:T]
 
     __call__ = forward
+
+    def check_status(self) -> None:
+        """As ``MoELayer.check_status``, for this rank's kernels."""
+        self.inner.check_status()
+        ops.check_plan(self.local_plan)
 
 
 # ------------------------------------------------------------------ one launch per rank, peer stores

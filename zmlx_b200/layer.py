@@ -206,13 +206,18 @@ class MoELayer:
         return 0 if ws is None else int(ws[:16].view(torch.int32)[3].item())
 
     def check_status(self) -> None:
-        """Raise ``ZmoeError(ERR_TIMEOUT)`` if a bounded wait ran out in any one-launch pass since the last check
-        (the output of that pass is void).  Synchronises the current stream: call it where the caller waits for
-        results anyway (end of a decode step, end of a timed region)."""
+        """Raise ``ZmoeError(ERR_TIMEOUT)`` if a bounded wait ran out in any one-launch pass or grouped matmul since the
+        last check (the output of that pass is void).  Synchronises the current stream: call it where the caller waits
+        for results anyway (end of a decode step, end of a timed region)."""
         lib = _lib.load()
         with torch.cuda.device(self.device):
             for ws in self._fused_ws.values():
                 _lib.check(lib.zmoe_layer_decode_status(ops._ptr(ws), 1, ops._stream()))
+            for plan in self._plans():
+                ops.check_plan(plan)
+
+    def _plans(self) -> list[torch.Tensor]:
+        return [self.plan, *([self.shared_plan] if self.cfg.n_shared else []), *self._shared_plans.values()]
 
     def enable_stamps(self) -> torch.Tensor:
         """Debug: make CTA 0 of the one-launch block record its cycle counter at the phase boundaries; returns the
@@ -229,14 +234,14 @@ class MoELayer:
         self.logits = torch.empty((T, cfg.n_experts), dtype=bf, device=dev)
         self.weights = torch.empty((T, K), dtype=f32, device=dev)
         self.indices = torch.empty((T, K), dtype=i32, device=dev)
-        self.plan = torch.empty(ops.plan_bytes(T * K, cfg.n_experts) // 4, dtype=i32, device=dev)
+        self.plan = torch.zeros(ops.plan_bytes(T * K, cfg.n_experts) // 4, dtype=i32, device=dev)  # no status yet
         self.counter = torch.zeros(1, dtype=i32, device=dev)
         self.h = torch.empty((T * K, cfg.d_ff), dtype=bf, device=dev)
         self.y = torch.empty((T * K, cfg.d_model), dtype=bf, device=dev)
         self.out = torch.empty((T, cfg.d_model), dtype=bf, device=dev)
         if cfg.n_shared:
             self.zero_idx = torch.zeros((T,), dtype=i32, device=dev)
-            self.shared_plan = torch.empty(ops.plan_bytes(T, 1) // 4, dtype=i32, device=dev)
+            self.shared_plan = torch.zeros(ops.plan_bytes(T, 1) // 4, dtype=i32, device=dev)
             self.sh_h = torch.empty((T, cfg.d_ff * cfg.n_shared), dtype=bf, device=dev)
             self.sh_y = torch.empty((T, cfg.d_model), dtype=bf, device=dev)
 
@@ -326,7 +331,7 @@ class MoELayer:
                                           st))
 
     def _new_shared_plan(self, T: int) -> torch.Tensor:
-        return torch.empty(ops.plan_bytes(T, 1) // 4, dtype=torch.int32, device=self.device)
+        return torch.zeros(ops.plan_bytes(T, 1) // 4, dtype=torch.int32, device=self.device)
 
     def shared(self, x: torch.Tensor, ws: torch.Tensor | None = None, plan_buf: torch.Tensor | None = None):
         """The always-on shared expert: the same kernels with a one-expert bank."""

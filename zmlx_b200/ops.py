@@ -86,6 +86,13 @@ def build_plan(rhs: torch.Tensor, E: int, *, M: int = 1, lhs: torch.Tensor | Non
     return out
 
 
+def check_plan(plan: torch.Tensor) -> None:
+    """Raise ``ZmoeError(ERR_TIMEOUT)`` if a bounded wait ran out in a grouped matmul on this plan since the last check.
+    Synchronises the current stream."""
+    with torch.cuda.device(plan.device):
+        _lib.check(_lib.load().zmoe_plan_status(_ptr(plan), 1, _stream()))
+
+
 def qmm_workspace(rows: int, E: int, K: int, *, rows_hint: int, mode: str, device) -> torch.Tensor | None:
     """Workspace of one grouped matmul call, from torch's allocator (so it belongs to the current stream and goes back
     to the pool when the call's reference is dropped), or None where the call gains nothing from one."""
