@@ -120,3 +120,21 @@ def test_repeated_calls_give_the_same_bits_under_load(tokens):
     first = _call(x, tokens, K, [a, u], E, N, "affine", plan, tokens * top, tokens, 0, ws)
     for _ in range(20):
         assert torch.equal(first, _call(x, tokens, K, [a, u], E, N, "affine", plan, tokens * top, tokens, 0, ws))
+
+
+@pytest.mark.parametrize("K", [768, 2048])
+@pytest.mark.parametrize("per", [40, 256])
+def test_long_sums_keep_their_precision(K, per):
+    """How often the result is not the float64 result's rounding.  A relative error of e before the rounding moves about
+    2^8 e of the results over a boundary, so 1.4e-4 of them says e = 9 x 2^-24: the few float32 roundings of chunk sums and
+    folds that the path states.  Sums over whole chunks of 256 codes in the tensor core give 1.7e-4 at 49 and more rows."""
+    N, E = 4096, 1024 // per
+    g = torch.Generator(device=DEV).manual_seed(3)
+    a, A = _bank(g, E, N, K, "affine", False)
+    rows = E * per
+    x = torch.randn((rows, K), generator=g, device=DEV).to(torch.bfloat16)
+    ids = torch.arange(rows, device=DEV) // per
+    ws = ops.qmm_workspace(rows, E, K, rows_hint=rows, mode="affine", device=DEV)
+    got = _call(x, rows, K, [a], E, N, "affine", ops.build_plan(ids, E), rows, rows, 1, ws)
+    ref = torch.cat([x[e * per:(e + 1) * per].double() @ A[e].T for e in range(E)])
+    assert float((got != ref.to(torch.bfloat16)).float().mean()) < 1.4e-4

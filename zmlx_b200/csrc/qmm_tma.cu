@@ -55,6 +55,13 @@ constexpr int kTmItems = 256;                     // work items of a CTA kept in
 constexpr int kTmCols = 512;
 constexpr int kTmColD = 128;                      // columns between the two accumulators
 constexpr int kTmSplitTok = 48;                   // up to so many token rows an accumulator is two, one per half chunk
+// How a chunk is summed.  The tensor core cuts products and sums off at a fixed distance below the largest of them, so
+// long sums lose.  Share of bfloat16 results that are not the float64 result's rounding, affine, K = 768 and 2048: whole
+// chunks 1.7e-4, halves 1.1e-4 and 1.2e-4 (float32 sums over groups of 64 unscaled codes: 0.6e-4 and 1.0e-4).  Up to
+// kTmSplitTok token rows the two halves lie side by side and are handed over together; wider items hand them over one
+// after the other, which costs 6 % (c2 with 4096 rows: 828 -> 879 us a block; quarters: 1090).  Products of e2m1 codes and
+// powers of two hardly lose any bits: whole chunks, 0.1e-4 to 0.6e-4.
+enum TmSum { kTmWhole, kTmSplit, kTmTurns };
 constexpr int kTmColA = 224, kTmAStage = 136;     // two A stages: 128 columns of codes, 8 of scales and biases
 
 struct TmArgs {
@@ -229,12 +236,12 @@ __device__ __noinline__ TmItem tm_item(const PlanView& pv, const int* prefix, in
 }
 
 // EPI: the SwiGLU contract of gate and up (QmmParams::epilogue).
-template <bool MX, int NMAT, int EPI>
+template <bool MX, int NMAT, int EPI, TmSum SUM>
 __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_constant__ TmArgs a) {
   extern __shared__ __align__(1024) unsigned char tm_dyn[];
   __shared__ uint32_t tmem_base_s;
-  // raw full / empty, token full / empty, A full, MMAs done, accumulator free
-  __shared__ __align__(8) unsigned long long bars_s[2 * kTmRaw + 2 * kTmMaxX + 6];
+  // raw full / empty, token full / empty, A full, MMAs done, accumulator free, accumulator full (kTmTurns)
+  __shared__ __align__(8) unsigned long long bars_s[2 * kTmRaw + 2 * kTmMaxX + 8];
   __shared__ float inv_s[4][kTmRows];
   __shared__ volatile int abort_s;
   __shared__ int prefix_s[kTmMaxTasks + 1];
@@ -252,6 +259,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
   const uint32_t bars = tm_smem(bars_s);
   const uint32_t b_rawf = bars, b_rawe = bars + 8 * kTmRaw, b_tokf = bars + 16 * kTmRaw;
   const uint32_t b_toke = b_tokf + 8 * kTmMaxX, b_af = b_toke + 8 * kTmMaxX, b_done = b_af + 16, b_dfree = b_done + 16;
+  const uint32_t b_acc = b_dfree + 16;
 
   // The plan, the prepared rows and their factors may be the work of the kernel before, still running when this one
   // starts: they are read with plain loads after the wait, never through the read-only path.
@@ -306,6 +314,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
       tm_bar_init(b_af + 8 * i, kTmExp / 64);
       tm_bar_init(b_done + 8 * i, 1);
       tm_bar_init(b_dfree + 8 * i, kTmFin / 32);
+      tm_bar_init(b_acc + 8 * i, 1);
     }
     abort_s = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -322,9 +331,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_base_s;
-  // The tensor core's running sums lose a little at every step; where there is room for a second accumulator a chunk is
-  // summed as two halves, and folded as such (the finishers have the time).
-  const bool split = tn <= kTmSplitTok;
+  constexpr int kParts = SUM == kTmTurns ? 2 : 1;  // hand-overs per chunk
   volatile int* ab = &abort_s;
   bool ok = true;
 
@@ -468,12 +475,12 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
         for (int i = 0; i < 16; ++i) acc[j][i] = 0.0f;
       }
 #pragma unroll 1
-      for (int cc = 0; cc < nch; ++cc, ++c) {
+      for (int cc = 0; cc < nch * kParts; ++cc, ++c) {
         const int buf = c & 1;
-        ok = tm_wait_warp(b_done + 8 * buf, (c >> 1) & 1, ab);
+        ok = tm_wait_warp((SUM == kTmTurns ? b_acc : b_done) + 8 * buf, (c >> 1) & 1, ab);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const float inv = inv_s[c & 3][r];
+        const float inv = inv_s[(c / kParts) & 3][r];
         const uint32_t at = lane_base + buf * kTmColD;
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
@@ -483,7 +490,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
             for (int i = 0; i < 16; ++i) acc[j][i] = fmaf(d[i], inv, acc[j][i]);
-            if (split) {
+            if (SUM == kTmSplit) {
               tm_ld16(at + kTmSplitTok + 16 * (ch + 2 * j), d);
               asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
@@ -534,7 +541,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
     }
   } else if (wid == (kTmExp + kTmFin) / 32) {
     // ================================================================== the warp that issues the MMAs (one lane does)
-    int c = 0, xs = 0, xph = 0;
+    int c = 0, xs = 0, xph = 0, n_first = 0;  // n_first: first halves committed (kTmTurns)
 #pragma unroll 1
     for (int item = 0; item < n_items && ok; ++item) {
       const TmItem it = item_at(item);
@@ -543,22 +550,39 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
       for (int cc = 0; cc < nch; ++cc, ++c) {
         const int buf = c & 1;
         ok = tm_wait_warp(b_tokf + 8 * xs, xph, ab);
-        if (ok && c >= 2) ok = tm_wait_warp(b_dfree + 8 * buf, ((c >> 1) - 1) & 1, ab);
+        if (ok && SUM != kTmTurns && c >= 2) ok = tm_wait_warp(b_dfree + 8 * buf, ((c >> 1) - 1) & 1, ab);
         if (ok) ok = tm_wait_warp(b_af + 8 * buf, (c >> 1) & 1, ab);
+        if (ok && SUM == kTmTurns && c >= 1) ok = tm_wait_warp(b_dfree, (c - 1) & 1, ab);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t d = tmem + buf * kTmColD, at = tmem + kTmColA + buf * kTmAStage;
-        const uint32_t d2 = split ? d + kTmSplitTok : d;  // the second half of the chunk
+        const uint32_t d = tmem + (SUM == kTmTurns ? 0 : buf * kTmColD), at = tmem + kTmColA + buf * kTmAStage;
+        const uint32_t d2 = SUM == kTmWhole ? d : d + (SUM == kTmSplit ? kTmSplitTok : kTmColD);  // the chunk's second half
         const uint32_t bt = tm_smem(tok + xs * a.xstage);
-        if (tm_elect()) {
+        auto half = [&](int h) {
 #pragma unroll
-          for (int g = 0; g < 4; ++g) {
+          for (int g = 2 * h; g < 2 * h + 2; ++g) {
             const uint64_t bd = tm_desc128(bt + g * tn * 128);
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-              tm_mma(g < 2 ? d : d2, at + g * 32 + k * 8, bd + 2 * k, idesc, k != 0 || (g != 0 && !(split && g == 2)));
+              tm_mma(h ? d2 : d, at + g * 32 + k * 8, bd + 2 * k, idesc, k != 0 || (g & 1) != 0 || (h == 1 && SUM == kTmWhole));
           }
+        };
+        if (SUM == kTmTurns) {
+          if (tm_elect()) {
+            half(0);
+            tm_commit(b_acc);
+          }
+          __syncwarp();
+          ++n_first;
+          if (c >= 1) ok = tm_wait_warp(b_dfree + 8, (c - 1) & 1, ab);
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        }
+        if (tm_elect()) {
+          if (SUM != kTmTurns) half(0);
+          half(1);
           if (!MX) tm_mma(d2, at + 128, tm_desc32(bt + tn * 512), idesc, true);
+          if (SUM == kTmTurns) tm_commit(b_acc + 8);
           tm_commit(b_done + 8 * buf);
           tm_commit(b_toke + 8 * xs);
         }
@@ -570,6 +594,10 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
       }
     }
     // MMAs in flight, and the arrivals they still owe
+    if (SUM == kTmTurns) {
+      if (n_first > 0) tm_wait(b_acc, (n_first - 1) & 1, ab, true);
+      if (c > 0) tm_wait(b_acc + 8, (c - 1) & 1, ab, true);
+    }
     for (int i = max(c - 2, 0); i < c; ++i) tm_wait(b_done + 8 * (i & 1), (i >> 1) & 1, ab, true);
     for (int i = max(c - rx, 0); i < c; ++i) tm_wait(b_toke + 8 * (i % rx), (i / rx) & 1, ab, true);
   } else if (wid == (kTmExp + kTmFin) / 32 + 1) {
@@ -758,8 +786,10 @@ static bool map_2d(CUtensorMap* m, CUtensorMapDataType dt, const void* ptr, size
 
 template <bool MX, int NMAT, int EPI>
 static int launch_tma(const TmArgs& a, int grid, size_t smem, cudaStream_t st, const char* who) {
-  cudaError_t e = cudaFuncSetAttribute(qmm_tma_kernel<MX, NMAT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess) e = launch_pdl(qmm_tma_kernel<MX, NMAT, EPI>, dim3(grid), dim3(kTmThreads), smem, st, a);
+  auto kern = a.tn <= kTmSplitTok ? qmm_tma_kernel<MX, NMAT, EPI, kTmSplit>
+                                  : qmm_tma_kernel<MX, NMAT, EPI, MX ? kTmWhole : kTmTurns>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) e = launch_pdl(kern, dim3(grid), dim3(kTmThreads), smem, st, a);
   if (e != cudaSuccess) return fail(ZMOE_ERR_CUDA, "%s: launch failed: %s", who, cudaGetErrorString(e));
   return check_launch("qmm_tma_kernel");
 }
