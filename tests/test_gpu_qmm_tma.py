@@ -138,3 +138,37 @@ def test_long_sums_keep_their_precision(K, per):
     got = _call(x, rows, K, [a], E, N, "affine", ops.build_plan(ids, E), rows, rows, 1, ws)
     ref = torch.cat([x[e * per:(e + 1) * per].double() @ A[e].T for e in range(E)])
     assert float((got != ref.to(torch.bfloat16)).float().mean()) < 1.4e-4
+
+
+def _one_row(codes, scales, biases, x, rows):
+    """`rows` equal token rows against an expert whose 64 weight rows hold the same codes: the results, all equal."""
+    K, N = x.numel(), 64
+    c = codes.to(torch.int64).view(K // 8, 8)
+    word = (c << (4 * torch.arange(8))).sum(1)
+    word = torch.where(word >= 2 ** 31, word - 2 ** 32, word).to(torch.int32)
+    a = tuple(t.expand(1, N, -1).contiguous().to(DEV)
+              for t in (word, scales.to(torch.bfloat16), biases.to(torch.bfloat16)))
+    X = x.to(torch.bfloat16).expand(rows, K).contiguous().to(DEV)
+    plan = ops.build_plan(torch.zeros(rows, dtype=torch.int32, device=DEV), 1)
+    ws = ops.qmm_workspace(rows, 1, K, rows_hint=rows, mode="affine", device=DEV)
+    got = _call(X, rows, K, [a], 1, N, "affine", plan, rows, rows, 1, ws)
+    assert bool((got == got[0, 0]).all())
+    return float(got[0, 0])
+
+
+@pytest.mark.parametrize("rows", [9, 96])
+def test_group_sums_and_offsets_keep_24_bits(rows):
+    """Results that only the last bits of a group's sum, or of b + 8 s, decide; everything else is exact."""
+    K = 256
+    # w = q - 7 = 0 everywhere, formed as -x + X; the sum 64 + 2^-5 + 2^-17 has 24 bits
+    x = torch.zeros(K)
+    x[:64] = 1.0
+    x[0], x[1], x[2] = 3.0, 2.0 ** -5, 2.0 ** -17
+    assert _one_row(torch.full((K,), 7), torch.ones(K // 64), torch.full((K // 64,), -7.0), x, rows) == 0.0
+    # codes of 8: the groups' results are their offsets, 1 + 2^-7 + 8 s and -(1 + 2^-7); what is left is 8 s, 2^-16 of it
+    x = torch.zeros(K)
+    x[5] = x[64 + 9] = 1.0
+    s8 = 2.0 ** -16 * (1 + 2.0 ** -7)
+    got = _one_row(torch.full((K,), 8), torch.tensor([s8 / 8, 0, 0, 0]), torch.tensor([1 + 2.0 ** -7, -(1 + 2.0 ** -7), 0, 0]),
+                   x, rows)
+    assert got == s8

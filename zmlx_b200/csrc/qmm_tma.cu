@@ -2,11 +2,11 @@
 // call that brings a workspace and more than a few token rows (serving batches and prompts, affine and mxfp4 banks).
 //
 // What bounds it: at a few rows per expert the packed weights' way from HBM, at many rows the token tiles' way from
-// L2 (one SM reads 128 weight rows x 256 codes = 18 KB against 544 B per token row for them).  So the packed codes
+// L2 (one SM reads 128 weight rows x 256 codes = 18 KB against 576 B per token row for them).  So the packed codes
 // must be expanded at the rate at which they arrive, and the token side must cost nothing but the copy:
 //
 //   prep_rows_kernel  writes, once per call, every token row in expert-sorted order as fp16 under a per-row power of
-//              two, and beside it the row's group sums as two fp16 pieces.  A token tile is then a plain TMA box
+//              two, and beside it the row's group sums as three fp16 pieces.  A token tile is then a plain TMA box
 //              with the 128-byte swizzle the tensor core reads, whatever the gather was.
 //   qmm_tma_kernel    one persistent CTA per SM walks items (expert, 128 weight rows, a block of token rows) as one
 //              unbroken stream of chunks of 256 codes:
@@ -21,12 +21,13 @@
 //
 // Arithmetic.  Affine: w = q s + b = (q - 8) s + (b + 8 s).  q - 8 has three bits and a sign, s eight: their product
 // is EXACT in fp16's eleven, so the scale goes into the operand and the accumulator runs over a whole chunk of four
-// groups.  The second term is one more K = 16 step against the group sums X = X1 + X2 (22 bits): per group the
-// columns (b, b, -8s, -8s) x (X1, X2, -X1, -X2).  The chunk's scales are first multiplied by a power of two per (row,
+// groups.  The second term is two more K = 16 steps: c = b + 8 s and the group's sum X, both float32, as three fp16 pieces
+// each (33 bits), per group the products of (c1, c1, c1, c2, c2, c2, c3, c3) and (X1, X2, X3, X1, X2, X3, X1, X2).  The
+// chunk's scales are first multiplied by a power of two per (row,
 // chunk) that puts max(8|s|, |b|) near 2^13, undone in fp32 by the finishers, so the range of fp16 is no limit on the
 // checkpoint's.  mxfp4: e2m1 value x 2^(e - emax + 11), exact in fp16 over 35 binades, same row factor.  Token rows
 // carry |x|max in [2^7, 2^8): a bfloat16 of that row is exact down to 2^-25 of its largest.  Chunks are summed in
-// fp32 registers rather than in the accumulator over all of K, so that no sum is longer than 272 products.
+// fp32 registers rather than in the accumulator over all of K, so that no sum is longer than 160 products (mxfp4: 256).
 //
 // gate and up share one accumulator: lanes 0-15 of each warp's 32 tensor-memory lanes hold gate rows, lanes 16-31 the
 // up rows of the same outputs, and the epilogue pairs them with one shuffle.
@@ -62,12 +63,12 @@ constexpr int kTmSplitTok = 48;                   // up to so many token rows an
 // after the other, which costs 6 % (c2 with 4096 rows: 828 -> 879 us a block; quarters: 1090).  Products of e2m1 codes and
 // powers of two hardly lose any bits: whole chunks, 0.1e-4 to 0.6e-4.
 enum TmSum { kTmWhole, kTmSplit, kTmTurns };
-constexpr int kTmColA = 224, kTmAStage = 136;     // two A stages: 128 columns of codes, 8 of scales and biases
+constexpr int kTmColA = 224, kTmAStage = 144;     // two A stages: 128 columns of codes, 16 of scales and biases
 
 struct TmArgs {
   CUtensorMap w[2];  // packed bytes (E*N, K/2): box 128 bytes x 128 (gate and up: 64) rows
   CUtensorMap x;     // prepared rows (rows, K) fp16: box 64 x 16
-  CUtensorMap xb;    // their group sums (rows, K/16) fp16: box 16 x 16
+  CUtensorMap xb;    // their group sums (rows, K/8) fp16: box 32 x 16
   QmmParams q;
   const float* xinv;  // (rows): 1 / the row's power of two
   int nch;            // K / 256
@@ -131,13 +132,13 @@ __device__ __forceinline__ void tm_load_2d(uint32_t dst, const CUtensorMap* map,
       "l"(map), "r"(x), "r"(y), "r"(bar)
       : "memory");
 }
-// Shared-memory descriptors of K-major tiles: rows of 128 (32) bytes under the 128-byte (32-byte) swizzle, eight rows
+// Shared-memory descriptors of K-major tiles: rows of 128 (64) bytes under the 128-byte (64-byte) swizzle, eight rows
 // per atom.
 __device__ __forceinline__ uint64_t tm_desc128(uint32_t addr) {
   return (uint64_t)((addr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
-__device__ __forceinline__ uint64_t tm_desc32(uint32_t addr) {
-  return (uint64_t)((addr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)(256 >> 4) << 32) | (1ull << 46) | (6ull << 61);
+__device__ __forceinline__ uint64_t tm_desc64(uint32_t addr) {
+  return (uint64_t)((addr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)(512 >> 4) << 32) | (1ull << 46) | (4ull << 61);
 }
 // D fp32, A and B fp16, both K-major, M = 128, N = n.
 __device__ __forceinline__ uint32_t tm_idesc(int n) {
@@ -167,8 +168,9 @@ __device__ __forceinline__ void tm_st16(uint32_t taddr, const uint32_t (&r)[16])
       "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
 }
-__device__ __forceinline__ void tm_st2(uint32_t taddr, uint32_t r0, uint32_t r1) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1,%2};" ::"r"(taddr), "r"(r0), "r"(r1) : "memory");
+__device__ __forceinline__ void tm_st4(uint32_t taddr, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(r0), "r"(r1), "r"(r2), "r"(r3)
+               : "memory");
 }
 // One lane of a converged warp.  The compiler knows an elected thread to be alone; behind `lane == 0` it would wrap
 // every tcgen05.mma and TMA instruction in a loop over the lanes that might be active (measured: 190 cycles per MMA
@@ -426,8 +428,14 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
           const __half2 s_op = __float2half2_rn(s * (P * 1048576.0f)), s_off = __float2half2_rn(s * (-8.0f * P));
 #pragma unroll
           for (int k = 0; k < 8; ++k) tm_expand_affine(ws[k], s_op, s_off, o[k >> 2] + 4 * (k & 3));
-          const __half2 b_op = __float2half2_rn(__uint_as_float(b_lo << 16) * P);
-          tm_st2(at + 128 + 2 * i, tm_bits(b_op), tm_bits(s_off));
+          // b + 8 s as three fp16 pieces against the three of the group's sum
+          const float co = fmaf(s, 8.0f, __uint_as_float(b_lo << 16)) * P;
+          const __half c1 = __float2half_rn(co);
+          const float co2 = co - __half2float(c1);
+          const __half c2 = __float2half_rn(co2);
+          const __half c3 = __float2half_rn(co2 - __half2float(c2));
+          tm_st4(at + 128 + 4 * i, tm_bits(__halves2half2(c1, c1)), tm_bits(__halves2half2(c1, c2)),
+                 tm_bits(__halves2half2(c2, c2)), tm_bits(__halves2half2(c3, c3)));
           b_lo = __funnelshift_r(b_lo, b_hi, 16);
           b_hi >>= 16;
         }
@@ -559,12 +567,16 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
         const uint32_t d2 = SUM == kTmWhole ? d : d + (SUM == kTmSplit ? kTmSplitTok : kTmColD);  // the chunk's second half
         const uint32_t bt = tm_smem(tok + xs * a.xstage);
         auto half = [&](int h) {
+          if (!MX && h == 1) {  // first, while the sum is short
+            tm_mma(d2, at + 128, tm_desc64(bt + tn * 512), idesc, false);
+            tm_mma(d2, at + 136, tm_desc64(bt + tn * 512) + 2, idesc, true);
+          }
 #pragma unroll
           for (int g = 2 * h; g < 2 * h + 2; ++g) {
             const uint64_t bd = tm_desc128(bt + g * tn * 128);
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-              tm_mma(h ? d2 : d, at + g * 32 + k * 8, bd + 2 * k, idesc, k != 0 || (g & 1) != 0 || (h == 1 && SUM == kTmWhole));
+              tm_mma(h ? d2 : d, at + g * 32 + k * 8, bd + 2 * k, idesc, k != 0 || (g & 1) != 0 || (h == 1 && (!MX || SUM == kTmWhole)));
           }
         };
         if (SUM == kTmTurns) {
@@ -581,7 +593,6 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
         if (tm_elect()) {
           if (SUM != kTmTurns) half(0);
           half(1);
-          if (!MX) tm_mma(d2, at + 128, tm_desc32(bt + tn * 512), idesc, true);
           if (SUM == kTmTurns) tm_commit(b_acc + 8);
           tm_commit(b_done + 8 * buf);
           tm_commit(b_toke + 8 * xs);
@@ -636,12 +647,12 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
         if (!ok) break;
         const uint32_t bar = b_tokf + 8 * xs, dst = tm_smem(tok + xs * a.xstage);
         if (tm_elect()) {
-          tm_expect(bar, nb * (MX ? 8192 : 8192 + 512));
+          tm_expect(bar, nb * (MX ? 8192 : 8192 + 1024));
           for (int b = 0; b < nb; ++b) {
 #pragma unroll
             for (int g = 0; g < 4; ++g)
               tm_load_2d(dst + g * tn * 128 + b * 2048, &a.x, cc * kTmChunk + g * 64, it.p0 + 16 * b, bar);
-            if (!MX) tm_load_2d(dst + tn * 512 + b * 512, &a.xb, cc * 16, it.p0 + 16 * b, bar);
+            if (!MX) tm_load_2d(dst + tn * 512 + b * 1024, &a.xb, cc * 32, it.p0 + 16 * b, bar);
           }
         }
         __syncwarp();
@@ -670,7 +681,8 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
 
 // ------------------------------------------------------------------ token rows in sorted order
 // One CTA per sorted row: |x|max, then fp16 values under 2^k with |x|max 2^k in [2^7, 2^8) and, for affine banks, the
-// sums of its groups of 64 as (X1, X2, -X1, -X2).  Affine rows take the order in which tm_expand_affine leaves codes.
+// sums of its groups of 64 as (X1, X2, X3, X1, X2, X3, X1, X2).  Affine rows take the order in which tm_expand_affine
+// leaves codes.
 constexpr int kPrepThreads = 128;
 
 template <bool MX>
@@ -703,7 +715,7 @@ __global__ void __launch_bounds__(kPrepThreads) prep_rows_kernel(const __nv_bflo
   ef = (mx == 0) ? 127 : min(max(ef, 2), 252);
   const float scale = __uint_as_float((uint32_t)ef << 23);
   if (tid == 0) xinv[pos] = __uint_as_float((uint32_t)(254 - ef) << 23);
-  const size_t stride = MX ? (size_t)K : (size_t)K + K / 16;
+  const size_t stride = MX ? (size_t)K : (size_t)K + K / 8;
   __half* row = xs + (size_t)pos * stride;
   for (int i = tid; i < nv; i += kPrepThreads) {  // nv is a multiple of 32: a warp is whole or absent
     const uint4 v = xr[i];
@@ -729,8 +741,12 @@ __global__ void __launch_bounds__(kPrepThreads) prep_rows_kernel(const __nv_bflo
       s += __shfl_xor_sync(0xffffffffu, s, 4);
       if ((tid & 7) == 0) {
         const __half x1 = __float2half_rn(s);
-        const uint32_t pr = tm_bits(__halves2half2(x1, __float2half_rn(s - __half2float(x1))));
-        *reinterpret_cast<uint2*>(row + K + (size_t)(i >> 3) * 4) = make_uint2(pr, pr ^ 0x80008000u);
+        const float s2 = s - __half2float(x1);
+        const __half x2 = __float2half_rn(s2);
+        const __half x3 = __float2half_rn(s2 - __half2float(x2));
+        const uint32_t x12 = tm_bits(__halves2half2(x1, x2));
+        *reinterpret_cast<uint4*>(row + K + (size_t)(i >> 3) * 8) =
+            make_uint4(x12, tm_bits(__halves2half2(x3, x1)), tm_bits(__halves2half2(x2, x3)), x12);
       }
     }
   }
@@ -739,7 +755,7 @@ __global__ void __launch_bounds__(kPrepThreads) prep_rows_kernel(const __nv_bflo
 // ------------------------------------------------------------------ host side
 
 size_t qmm_tma_workspace(int rows, int K, bool mx) {
-  const size_t row = mx ? (size_t)K * 2 : (size_t)K * 2 + K / 8;
+  const size_t row = mx ? (size_t)K * 2 : (size_t)K * 2 + K / 4;
   return (((size_t)rows * row + 255) & ~(size_t)255) + (size_t)rows * sizeof(float);
 }
 
@@ -797,7 +813,7 @@ static int launch_tma(const TmArgs& a, int grid, size_t smem, cudaStream_t st, c
 int qmm_tma_launch(const QmmParams& q, int nmat, bool mx, int rows_hint, int max_groups, void* ws, cudaStream_t st,
                    const char* who) {
   if (!encoder()) return fail(ZMOE_ERR_CUDA, "%s: cuTensorMapEncodeTiled is not available", who);
-  const size_t row = mx ? (size_t)q.K * 2 : (size_t)q.K * 2 + q.K / 8;  // bytes of a prepared row
+  const size_t row = mx ? (size_t)q.K * 2 : (size_t)q.K * 2 + q.K / 4;  // bytes of a prepared row
   unsigned char* xs = reinterpret_cast<unsigned char*>(ws);
   float* xinv = reinterpret_cast<float*>(xs + (((size_t)q.rows * row + 255) & ~(size_t)255));
   TmArgs a;
@@ -814,8 +830,8 @@ int qmm_tma_launch(const QmmParams& q, int nmat, bool mx, int rows_hint, int max
   if (mx)
     a.xb = a.x;
   else
-    fine = fine && map_2d(&a.xb, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, xs + (size_t)q.K * 2, q.K / 16, q.rows, row, 16, 16,
-                          CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_NONE);
+    fine = fine && map_2d(&a.xb, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, xs + (size_t)q.K * 2, q.K / 8, q.rows, row, 32, 16,
+                          CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE);
   if (!fine) return fail(ZMOE_ERR_CUDA, "%s: a tensor map was refused", who);
   // Token rows per item: up to twice the average task in whole 16s (a larger task takes several equal blocks); the
   // fewer rows a stage must hold, the more stages are in flight.
@@ -823,7 +839,7 @@ int qmm_tma_launch(const QmmParams& q, int nmat, bool mx, int rows_hint, int max
   if (tn > rows_hint) tn = rows_hint;
   tn = (tn + 15) / 16 * 16;
   a.tn = tn > kTmMaxTok ? kTmMaxTok : (int)tn;
-  a.xstage = (a.tn * (mx ? 512 : 544) + 1023) & ~1023;
+  a.xstage = (a.tn * (mx ? 512 : 576) + 1023) & ~1023;
   const int fixed = 1024 + kTmRaw * kTmRawBytes + kTmScRing * kTmExp * 16;
   const int room = 227 * 1024 - 12 * 1024 - fixed;  // 12 KB: the static part (prefix sums, items, barriers, row factors)
   a.rx = room / a.xstage > kTmMaxX ? kTmMaxX : room / a.xstage;
