@@ -172,3 +172,32 @@ def test_group_sums_and_offsets_keep_24_bits(rows):
     got = _one_row(torch.full((K,), 8), torch.tensor([s8 / 8, 0, 0, 0]), torch.tensor([1 + 2.0 ** -7, -(1 + 2.0 ** -7), 0, 0]),
                    x, rows)
     assert got == s8
+
+
+@pytest.mark.parametrize("rows", [9, 100])
+@pytest.mark.parametrize("steps", [(0, 7, 14, 20), (20, 0, 1, 13)])
+def test_scales_far_apart_in_one_chunk(steps, rows):
+    """A group's scale is 2^-d of the largest and its activations 2^d larger: every group weighs the same in the result,
+    and none of the small scales' bits may go."""
+    E, N, K = 2, 100, 512
+    g = torch.Generator(device=DEV).manual_seed(rows)
+    d = torch.tensor(steps, device=DEV).repeat(K // 256)
+    s = (torch.rand((E, N, K // 64), generator=g, device=DEV) + 1.0) * torch.exp2(-d.float())
+    b = -s * (4.0 + 8.0 * torch.rand((E, N, K // 64), generator=g, device=DEV))
+    s, b = s.to(torch.bfloat16), b.to(torch.bfloat16)
+    word = torch.randint(-2 ** 31, 2 ** 31, (E, N, K // 8), generator=g, device=DEV).to(torch.int32)
+    A = _weights(word, s, b)
+    x = torch.randn((2 * rows, K), generator=g, device=DEV).view(2 * rows, K // 64, 64) * torch.exp2(d.float())[None, :, None]
+    x = x.reshape(2 * rows, K).to(torch.bfloat16)
+    ids = torch.arange(2 * rows, device=DEV) % E
+    ws = ops.qmm_workspace(2 * rows, E, K, rows_hint=2 * rows, mode="affine", device=DEV)
+    got = _call(x, 2 * rows, K, [(word, s, b)], E, N, "affine", ops.build_plan(ids, E), 2 * rows, 2 * rows, 1, ws)
+    ref = torch.stack([x[r].double() @ A[ids[r]].T for r in range(2 * rows)])
+    mass = torch.stack([x[r].double().abs() @ A[ids[r]].abs().T for r in range(2 * rows)])
+    _within(got, ref, mass, K)
+
+
+def _weights(word, s, b):
+    code = (word.unsqueeze(-1) >> torch.arange(0, 32, 4, device=word.device, dtype=torch.int32)) & 15
+    code = code.reshape(*word.shape[:-1], -1).double()
+    return (code.view(*s.shape, 64) * s.double()[..., None] + b.double()[..., None]).reshape(code.shape)

@@ -19,15 +19,17 @@
 //     finishers 256 threads fold the chunk's accumulator into fp32 registers and, at the end of an item, apply the
 //               SwiGLU contract and store bf16 rows through the plan.
 //
-// Arithmetic.  Affine: w = q s + b = (q - 8) s + (b + 8 s).  q - 8 has three bits and a sign, s eight: their product
-// is EXACT in fp16's eleven, so the scale goes into the operand and the accumulator runs over a whole chunk of four
-// groups.  The second term is two more K = 16 steps: c = b + 8 s and the group's sum X, both float32, as three fp16 pieces
-// each (33 bits), per group the products of (c1, c1, c1, c2, c2, c2, c3, c3) and (X1, X2, X3, X1, X2, X3, X1, X2).  The
-// chunk's scales are first multiplied by a power of two per (row,
-// chunk) that puts max(8|s|, |b|) near 2^13, undone in fp32 by the finishers, so the range of fp16 is no limit on the
-// checkpoint's.  mxfp4: e2m1 value x 2^(e - emax + 11), exact in fp16 over 35 binades, same row factor.  Token rows
-// carry |x|max in [2^7, 2^8): a bfloat16 of that row is exact down to 2^-25 of its largest.  Chunks are summed in
-// fp32 registers rather than in the accumulator over all of K, so that no sum is longer than 160 products (mxfp4: 256).
+// Arithmetic.  Affine: w = q s + b = (q - 8) s + (b + 8 s).  q - 8 has three bits and a sign, s eight: their product fits
+// fp16's eleven, so the scale goes into the operand and the accumulator runs over several groups.  The second term is two
+// more K = 16 steps on one operand, per group (b, b, -8 s, -8 s), against the group's float32 sum X as three fp16 pieces (33
+// bits): (X1, X2, -X1, -X2) and (X3, 0, -X3, 0).  The scales are first multiplied by a
+// power of two per (row, chunk), undone in fp32 by the finishers, so the range of fp16 is no limit on the checkpoint's.
+// (q - 8) s is exact while the four scales of a row's chunk lie within 12 binades of the largest; chunks with scales
+// further apart are expanded another way (tm_expand_far), exact over 28; below, a weight is off by at most 2^-39 of the
+// largest of its row's chunk.  mxfp4: e2m1 value x 2^(e - emax + 11), exact in fp16 over 35 binades, same row factor.
+// Token rows carry |x|max in [2^7, 2^8): a bfloat16 of that row is exact down to 2^-25 of its largest.  Chunks are
+// summed in fp32 registers rather than in the accumulator over all of K, so that no sum is longer than 160 products (mxfp4:
+// 256).
 //
 // gate and up share one accumulator: lanes 0-15 of each warp's 32 tensor-memory lanes hold gate rows, lanes 16-31 the
 // up rows of the same outputs, and the epilogue pairs them with one shuffle.
@@ -63,7 +65,7 @@ constexpr int kTmSplitTok = 48;                   // up to so many token rows an
 // after the other, which costs 6 % (c2 with 4096 rows: 828 -> 879 us a block; quarters: 1090).  Products of e2m1 codes and
 // powers of two hardly lose any bits: whole chunks, 0.1e-4 to 0.6e-4.
 enum TmSum { kTmWhole, kTmSplit, kTmTurns };
-constexpr int kTmColA = 224, kTmAStage = 144;     // two A stages: 128 columns of codes, 16 of scales and biases
+constexpr int kTmColA = 224, kTmAStage = 136;     // two A stages: 128 columns of codes, 8 of scales and biases
 
 struct TmArgs {
   CUtensorMap w[2];  // packed bytes (E*N, K/2): box 128 bytes x 128 (gate and up: 64) rows
@@ -168,9 +170,8 @@ __device__ __forceinline__ void tm_st16(uint32_t taddr, const uint32_t (&r)[16])
       "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
 }
-__device__ __forceinline__ void tm_st4(uint32_t taddr, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(r0), "r"(r1), "r"(r2), "r"(r3)
-               : "memory");
+__device__ __forceinline__ void tm_st2(uint32_t taddr, uint32_t r0, uint32_t r1) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1,%2};" ::"r"(taddr), "r"(r0), "r"(r1) : "memory");
 }
 // One lane of a converged warp.  The compiler knows an elected thread to be alone; behind `lane == 0` it would wrap
 // every tcgen05.mma and TMA instruction in a loop over the lanes that might be active (measured: 190 cycles per MMA
@@ -193,6 +194,37 @@ __device__ __forceinline__ void tm_expand_affine(uint32_t w, __half2 s20, __half
   out[1] = tm_bits(__hfma2(tm_half2(w & m), s20, m8s));
   out[2] = tm_bits(__hfma2(tm_half2((w >> 4) & m), s20, m8s));
   out[3] = tm_bits(__hfma2(tm_half2((w >> 8) & m), s20, m8s));
+}
+// A chunk whose scales lie further apart than tm_expand_affine takes: a nibble at bits 6-9 of a half under the exponent of
+// 16 is 16 + q, and (16 + q) s - 24 s = (q - 8) s is exact for s from 2^-17 to 2^11 (24 s has ten bits).  One more shift and
+// four more masks per word: every chunk done this way cost 9 to 13 % (c2 with 32 rows 600 -> 657 us, c5 with 64 rows 1790
+// -> 2038), so it is a call for the warps that meet such a chunk.
+__device__ __noinline__ void tm_expand_far(const unsigned char* src, uint32_t swz, uint4 sc, float P, uint32_t taddr) {
+  const uint32_t m = 0x03C003C0u, sixteen = 0x4C004C00u;
+#pragma unroll 1
+  for (int i = 0; i < 8; ++i) {  // 16 bytes: half a group
+    const uint4 w4 = *reinterpret_cast<const uint4*>(src + ((i ^ swz) << 4));
+    const uint32_t ws[4] = {w4.x, w4.y, w4.z, w4.w};
+    const float s = __uint_as_float(sc.x << 16) * P;
+    const __half2 s_op = __float2half2_rn(s), off = __float2half2_rn(-24.0f * s);
+    uint32_t o[16];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      o[4 * k] = tm_bits(__hfma2(tm_half2(((ws[k] << 6) & m) | sixteen), s_op, off));
+      o[4 * k + 1] = tm_bits(__hfma2(tm_half2(((ws[k] << 2) & m) | sixteen), s_op, off));
+      o[4 * k + 2] = tm_bits(__hfma2(tm_half2(((ws[k] >> 2) & m) | sixteen), s_op, off));
+      o[4 * k + 3] = tm_bits(__hfma2(tm_half2(((ws[k] >> 6) & m) | sixteen), s_op, off));
+    }
+    tm_st16(taddr + i * 16, o);
+    if (i & 1) {
+      const __half2 b_op = __float2half2_rn(__uint_as_float(sc.z << 16) * P);
+      tm_st2(taddr + 127 + i, tm_bits(b_op), tm_bits(__float2half2_rn(-8.0f * s)));
+      sc.x = __funnelshift_r(sc.x, sc.y, 16);
+      sc.y >>= 16;
+      sc.z = __funnelshift_r(sc.z, sc.w, 16);
+      sc.w >>= 16;
+    }
+  }
 }
 // Eight e2m1 codes in their own order, times the block's power of two.
 __device__ __forceinline__ void tm_expand_mx(uint32_t w, __half2 s, uint32_t* out) {
@@ -386,6 +418,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
       uint32_t s_lo = sc.x, s_hi = sc.y, b_lo = sc.z, b_hi = sc.w;  // shifted through, one group at a time
       float inv, P = 0.0f;
       int emax = 0;
+      bool far = false;
       if (MX) {
         uint32_t v = __vmaxu4(sc.x, sc.y);
         v = __vmaxu4(v, v >> 16);
@@ -397,8 +430,14 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
         uint32_t mb = __vmaxu2(sc.z & 0x7fff7fffu, sc.w & 0x7fff7fffu);
         ms = max(ms & 0xffffu, ms >> 16);
         mb = max(mb & 0xffffu, mb >> 16);
-        // 2^(140 - e) brings |s| below 2^-4 (so that s 2^20 stays below 2^16) and |b| below 2^14
-        const int e = min(max(max((int)(ms >> 7) + 18, (int)(mb >> 7)), 34), 253);
+        // 2^(140 - e) brings |s| below 2^-4 (so that s 2^20 stays below 2^16) and |b| below 2^14; a scale that this
+        // leaves below 2^-17 asks for the wider form, where |s| may reach 2^11
+        const int es = (int)(ms >> 7), eb = (int)(mb >> 7);
+        int e = max(es + 18, eb);
+        const uint32_t least = __vminu2(sc.x & 0x7fff7fffu, sc.y & 0x7fff7fffu);
+        far = __any_sync(0xffffffffu, (int)(min(least & 0xffffu, least >> 16) >> 7) + 30 < e);
+        if (far) e = max(es + 3, eb);
+        e = min(max(e, far ? 14 : 34), 253);
         P = __uint_as_float((uint32_t)(267 - e) << 23);
         inv = __uint_as_float((uint32_t)(e - 13) << 23);
       }
@@ -410,8 +449,9 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
       const unsigned char* src = my_raw + rs * kTmRawBytes;
       uint4 wa = *reinterpret_cast<const uint4*>(src + ((rb & 7) << 4));
       uint4 wb = *reinterpret_cast<const uint4*>(src + ((1 ^ (rb & 7)) << 4));
+      if (!MX && far) tm_expand_far(src, rb & 7, sc, P, at);
 #pragma unroll 1
-      for (int i = 0; i < 4; ++i) {  // 64 codes each: a group, or two mxfp4 blocks.  Rolled: see tm_wait_long
+      for (int i = !MX && far ? 4 : 0; i < 4; ++i) {  // 64 codes each: a group, or two mxfp4 blocks.  Rolled: see tm_wait_long
         const int nx = 2 * min(i + 1, 3);
         const uint4 na = *reinterpret_cast<const uint4*>(src + ((nx ^ (rb & 7)) << 4));
         const uint4 nb = *reinterpret_cast<const uint4*>(src + (((nx + 1) ^ (rb & 7)) << 4));
@@ -428,14 +468,8 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
           const __half2 s_op = __float2half2_rn(s * (P * 1048576.0f)), s_off = __float2half2_rn(s * (-8.0f * P));
 #pragma unroll
           for (int k = 0; k < 8; ++k) tm_expand_affine(ws[k], s_op, s_off, o[k >> 2] + 4 * (k & 3));
-          // b + 8 s as three fp16 pieces against the three of the group's sum
-          const float co = fmaf(s, 8.0f, __uint_as_float(b_lo << 16)) * P;
-          const __half c1 = __float2half_rn(co);
-          const float co2 = co - __half2float(c1);
-          const __half c2 = __float2half_rn(co2);
-          const __half c3 = __float2half_rn(co2 - __half2float(c2));
-          tm_st4(at + 128 + 4 * i, tm_bits(__halves2half2(c1, c1)), tm_bits(__halves2half2(c1, c2)),
-                 tm_bits(__halves2half2(c2, c2)), tm_bits(__halves2half2(c3, c3)));
+          const __half2 b_op = __float2half2_rn(__uint_as_float(b_lo << 16) * P);
+          tm_st2(at + 128 + 2 * i, tm_bits(b_op), tm_bits(s_off));
           b_lo = __funnelshift_r(b_lo, b_hi, 16);
           b_hi >>= 16;
         }
@@ -567,16 +601,12 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
         const uint32_t d2 = SUM == kTmWhole ? d : d + (SUM == kTmSplit ? kTmSplitTok : kTmColD);  // the chunk's second half
         const uint32_t bt = tm_smem(tok + xs * a.xstage);
         auto half = [&](int h) {
-          if (!MX && h == 1) {  // first, while the sum is short
-            tm_mma(d2, at + 128, tm_desc64(bt + tn * 512), idesc, false);
-            tm_mma(d2, at + 136, tm_desc64(bt + tn * 512) + 2, idesc, true);
-          }
 #pragma unroll
           for (int g = 2 * h; g < 2 * h + 2; ++g) {
             const uint64_t bd = tm_desc128(bt + g * tn * 128);
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-              tm_mma(h ? d2 : d, at + g * 32 + k * 8, bd + 2 * k, idesc, k != 0 || (g & 1) != 0 || (h == 1 && (!MX || SUM == kTmWhole)));
+              tm_mma(h ? d2 : d, at + g * 32 + k * 8, bd + 2 * k, idesc, k != 0 || (g & 1) != 0 || (h == 1 && SUM == kTmWhole));
           }
         };
         if (SUM == kTmTurns) {
@@ -593,6 +623,10 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
         if (tm_elect()) {
           if (SUM != kTmTurns) half(0);
           half(1);
+          if (!MX) {  // the sums' first two pieces, and their third
+            tm_mma(d2, at + 128, tm_desc64(bt + tn * 512), idesc, true);
+            tm_mma(d2, at + 128, tm_desc64(bt + tn * 512) + 2, idesc, true);
+          }
           if (SUM == kTmTurns) tm_commit(b_acc + 8);
           tm_commit(b_done + 8 * buf);
           tm_commit(b_toke + 8 * xs);
@@ -681,7 +715,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
 
 // ------------------------------------------------------------------ token rows in sorted order
 // One CTA per sorted row: |x|max, then fp16 values under 2^k with |x|max 2^k in [2^7, 2^8) and, for affine banks, the
-// sums of its groups of 64 as (X1, X2, X3, X1, X2, X3, X1, X2).  Affine rows take the order in which tm_expand_affine
+// sums of its groups of 64 as (X1, X2, -X1, -X2) and (X3, 0, -X3, 0).  Affine rows take the order in which tm_expand_affine
 // leaves codes.
 constexpr int kPrepThreads = 128;
 
@@ -743,10 +777,12 @@ __global__ void __launch_bounds__(kPrepThreads) prep_rows_kernel(const __nv_bflo
         const __half x1 = __float2half_rn(s);
         const float s2 = s - __half2float(x1);
         const __half x2 = __float2half_rn(s2);
-        const __half x3 = __float2half_rn(s2 - __half2float(x2));
         const uint32_t x12 = tm_bits(__halves2half2(x1, x2));
-        *reinterpret_cast<uint4*>(row + K + (size_t)(i >> 3) * 8) =
-            make_uint4(x12, tm_bits(__halves2half2(x3, x1)), tm_bits(__halves2half2(x2, x3)), x12);
+        const uint32_t x3 = tm_bits(__floats2half2_rn(s2 - __half2float(x2), 0.0f));
+        const int g = i >> 3;
+        uint2* to = reinterpret_cast<uint2*>(row + K + (g >> 2) * 32 + (g & 3) * 4);  // 32 values per chunk: two K steps
+        to[0] = make_uint2(x12, x12 ^ 0x80008000u);
+        to[4] = make_uint2(x3, x3 ^ 0x80008000u);
       }
     }
   }
