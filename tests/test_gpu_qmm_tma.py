@@ -201,3 +201,31 @@ def _weights(word, s, b):
     code = (word.unsqueeze(-1) >> torch.arange(0, 32, 4, device=word.device, dtype=torch.int32)) & 15
     code = code.reshape(*word.shape[:-1], -1).double()
     return (code.view(*s.shape, 64) * s.double()[..., None] + b.double()[..., None]).reshape(code.shape)
+
+
+@pytest.mark.parametrize("rows", [9, 100])
+@pytest.mark.parametrize("mode,depth", [("affine", 24), ("mxfp4", 29)])
+def test_token_values_far_below_the_rows_largest(mode, depth, rows):
+    """The row's largest value meets a weight of zero; values of 2^-depth of it decide the result, with all their bits."""
+    E, N, K = 1, 100, 256
+    g = torch.Generator(device=DEV).manual_seed(depth)
+    word = torch.randint(-2 ** 31, 2 ** 31, (E, N, K // 8), generator=g, device=DEV).to(torch.int32)
+    if mode == "affine":
+        s = (torch.rand((E, N, K // 64), generator=g, device=DEV) + 1.0).to(torch.bfloat16)
+        s[..., 0] = 0.0
+        a = (word, s, -8.0 * s)
+        A = _weights(*a)
+    else:
+        word[..., :8] = 0
+        s = torch.full((E, N, K // 32), 120, dtype=torch.uint8, device=DEV)
+        a, A = (word, s, None), quant.dequantize_mxfp4(word, s).double()
+    # two binades of values that need all eight bits of a bfloat16
+    x = (torch.rand((rows, K), generator=g, device=DEV) + 1.0) * torch.exp2(-torch.rand((rows, K), generator=g, device=DEV))
+    x = x.to(torch.bfloat16).float() * 2.0 ** -depth
+    x[:, :64] = 0.0
+    x[:, 3] = 1.0
+    x = x.to(torch.bfloat16)
+    plan = ops.build_plan(torch.zeros(rows, dtype=torch.int32, device=DEV), E)
+    ws = ops.qmm_workspace(rows, E, K, rows_hint=rows, mode=mode, device=DEV)
+    got = _call(x, rows, K, [a], E, N, mode, plan, rows, rows, 1, ws)
+    _within(got, x.double() @ A[0].T, x.double().abs() @ A[0].abs().T, K)

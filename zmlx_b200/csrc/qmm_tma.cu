@@ -27,7 +27,8 @@
 // (q - 8) s is exact while the four scales of a row's chunk lie within 12 binades of the largest; chunks with scales
 // further apart are expanded another way (tm_expand_far), exact over 28; below, a weight is off by at most 2^-39 of the
 // largest of its row's chunk.  mxfp4: e2m1 value x 2^(e - emax + 11), exact in fp16 over 35 binades, same row factor.
-// Token rows carry |x|max in [2^7, 2^8): a bfloat16 of that row is exact down to 2^-25 of its largest.  Chunks are
+// Token rows carry a power of two per row: a bfloat16 of the row is exact down to 2^-26 (mxfp4: 2^-31) of its largest,
+// and off by at most 2^-34 (2^-39) of it below.  Chunks are
 // summed in fp32 registers rather than in the accumulator over all of K, so that no sum is longer than 160 products (mxfp4:
 // 256).
 //
@@ -714,8 +715,8 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
 }
 
 // ------------------------------------------------------------------ token rows in sorted order
-// One CTA per sorted row: |x|max, then fp16 values under 2^k with |x|max 2^k in [2^7, 2^8) and, for affine banks, the
-// sums of its groups of 64 as (X1, X2, -X1, -X2) and (X3, 0, -X3, 0).  Affine rows take the order in which tm_expand_affine
+// One CTA per sorted row: |x|max, then fp16 values under 2^k with |x|max 2^k in [2^14, 2^15), or for affine banks in [2^9,
+// 2^10), whose group sums just fit fp16 (64 x 1020 = 65280), and the sums of its groups of 64 as (X1, X2, -X1, -X2) and (X3, 0, -X3, 0).  Affine rows take the order in which tm_expand_affine
 // leaves codes.
 constexpr int kPrepThreads = 128;
 
@@ -745,7 +746,7 @@ __global__ void __launch_bounds__(kPrepThreads) prep_rows_kernel(const __nv_bflo
   __syncthreads();
 #pragma unroll
   for (int i = 0; i < kPrepThreads / 32; ++i) mx = max(mx, warp_max[i]);
-  int ef = 261 - (int)(mx >> 7);
+  int ef = (MX ? 268 : 263) - (int)(mx >> 7);
   ef = (mx == 0) ? 127 : min(max(ef, 2), 252);
   const float scale = __uint_as_float((uint32_t)ef << 23);
   if (tid == 0) xinv[pos] = __uint_as_float((uint32_t)(254 - ef) << 23);
