@@ -66,3 +66,25 @@ def test_capture_without_a_warm_up_pass():
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("T", [1, 8])
+def test_blocks_far_below_their_neighbours_keep_their_bits(T):
+    """Half of gate's and up's blocks are 2^-30 of the others, which the token rows meet with zeros: the result is the one of
+    the same blocks without neighbours, times a power of two, and follows the oracle."""
+    cfg = synthetic.CONFIGS["c3"].scaled(**SHAPES["narrow"], n_shared=0)
+    params = synthetic.make_layer(cfg, device=DEV)
+    x = synthetic.make_tokens(cfg, T, device=DEV)
+    x.view(T, -1, 32)[:, ::2] = 0
+    low = {}
+    for k in ("gate_s", "up_s"):
+        s = params[k].clone()
+        s[..., 1::2] = 120
+        low[k] = s.clone()
+        s[..., ::2] = 150  # met by zeros only
+        params[k] = s
+    layer = MoELayer(cfg, params, max_tokens=8)
+    out = layer(x).clone()
+    layer.check_status()
+    alone = MoELayer(cfg, dict(params, **low), max_tokens=8)
+    assert layer.passes(T) and torch.equal(out, alone(x))

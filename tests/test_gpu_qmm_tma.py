@@ -229,3 +229,27 @@ def test_token_values_far_below_the_rows_largest(mode, depth, rows):
     ws = ops.qmm_workspace(rows, E, K, rows_hint=rows, mode=mode, device=DEV)
     got = _call(x, rows, K, [a], E, N, mode, plan, rows, rows, 1, ws)
     _within(got, x.double() @ A[0].T, x.double().abs() @ A[0].abs().T, K)
+
+
+@pytest.mark.parametrize("rows", [9, 100])
+def test_block_exponents_far_apart_in_one_chunk(rows):
+    """mxfp4: the blocks far down carry the row's largest activations, the others small enough ones not to drown them: what
+    a block 30 binades down adds is far above the result's float32 error, and must be there."""
+    E, N, K = 2, 100, 512
+    g = torch.Generator(device=DEV).manual_seed(rows)
+    d = torch.tensor([0, 14, 27, 6, 34, 30, 21, 3], device=DEV).repeat(K // 256)
+    s = (150 - d).expand(E, N, K // 32).to(torch.uint8).contiguous()
+    word = torch.randint(-2 ** 31, 2 ** 31, (E, N, K // 8), generator=g, device=DEV).to(torch.int32)
+    A = quant.dequantize_mxfp4(word, s).double()
+    lift = torch.where(d >= 27, 0, -28)
+    x = torch.randn((2 * rows, K), generator=g, device=DEV).view(2 * rows, K // 32, 32) * torch.exp2(lift.float())[None, :, None]
+    x = x.reshape(2 * rows, K).to(torch.bfloat16)
+    ids = torch.arange(2 * rows, device=DEV) % E
+    ws = ops.qmm_workspace(2 * rows, E, K, rows_hint=2 * rows, mode="mxfp4", device=DEV)
+    got = _call(x, 2 * rows, K, [(word, s, None)], E, N, "mxfp4", ops.build_plan(ids, E), 2 * rows, 2 * rows, 1, ws)
+    ref = torch.stack([x[r].double() @ A[ids[r]].T for r in range(2 * rows)])
+    mass = torch.stack([x[r].double().abs() @ A[ids[r]].abs().T for r in range(2 * rows)])
+    # what is not exact is stated: a token value below 2^-31 of its row's largest is off by at most 2^-39 of that
+    slack = 2.0 ** -39 * x.double().abs().amax(1)[:, None] * torch.stack([A[ids[r]].abs().sum(1) for r in range(2 * rows)])
+    bound = 2.0 ** -8 * ref.abs() + (256 + K // 256) * 2.0 ** -23 * mass + slack
+    assert bool(((got.double() - ref).abs() <= bound).all())

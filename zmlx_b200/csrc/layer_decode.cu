@@ -684,8 +684,8 @@ __device__ __forceinline__ void ld_e2m1x8(uint32_t w, __half2 s, uint32_t (&o)[4
 }
 
 // The same item for mxfp4 banks.  An e2m1 value times a power of two has one mantissa bit, so the blocks' scales go
-// into the fp16 operand, relative to the largest of the warp's eight blocks of a row in the stage (exact over 23
-// binades below it); that largest one is applied to the stage's sum in fp32.  With the scales inside the operand
+// into the fp16 operand, relative to the largest of the warp's eight blocks of a row in the stage (times 2^13: exact over
+// 36 binades); that largest one is applied to the stage's sum in fp32.  With the scales inside the operand
 // nothing has to be kept apart per group: column t of the accumulator is token t, and no columns are multiplexed.
 // Bound like the affine block by the chain router -> gate/up -> down -> combine at these sizes.  Measured (c3, us per
 // block in a graph, separate kernels -> one launch): T = 1 46.0 -> 21.4, T = 4 76.5 -> 43.6, T = 8 111.7 -> 61.7; called
@@ -741,7 +741,7 @@ __device__ __forceinline__ void ld_item_mx(LdCtx& c, float (&acc)[2][4], int K8,
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             const int e = (int)(((j < 2 ? eb[m][h].x : eb[m][h].y) >> sh) & 0xffu);
-            s[h] = __float2half2_rn(__uint_as_float((uint32_t)max(127 + e - eref[m][h], 0) << 23));
+            s[h] = __float2half2_rn(__uint_as_float((uint32_t)max(140 + e - eref[m][h], 0) << 23));
           }
           uint32_t a0[4], a1[4];
           ld_e2m1x8(wa.x, s[0], a0);
@@ -762,7 +762,7 @@ __device__ __forceinline__ void ld_item_mx(LdCtx& c, float (&acc)[2][4], int K8,
       for (int m = 0; m < 2; ++m)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const float sv = __uint_as_float((uint32_t)eref[m][j >> 1] << 23);  // 2^(e - 127)
+          const float sv = __uint_as_float((uint32_t)eref[m][j >> 1] << 23) * 0x1p-13f;  // 2^(e - 127 - 13)
           acc[m][j] = fmaf(sv, dg[m][0][j] + dg[m][1][j], acc[m][j]);
         }
     }

@@ -26,7 +26,7 @@
 // power of two per (row, chunk), undone in fp32 by the finishers, so the range of fp16 is no limit on the checkpoint's.
 // (q - 8) s is exact while the four scales of a row's chunk lie within 12 binades of the largest; chunks with scales
 // further apart are expanded another way (tm_expand_far), exact over 28; below, a weight is off by at most 2^-39 of the
-// largest of its row's chunk.  mxfp4: e2m1 value x 2^(e - emax + 11), exact in fp16 over 35 binades, same row factor.
+// largest of its row's chunk.  mxfp4: e2m1 value x 2^(e - emax + 13), exact in fp16 over 36 binades, same row factor.
 // Token rows carry a power of two per row: a bfloat16 of the row is exact down to 2^-26 (mxfp4: 2^-31) of its largest,
 // and off by at most 2^-34 (2^-39) of it below.  Chunks are
 // summed in fp32 registers rather than in the accumulator over all of K, so that no sum is longer than 160 products (mxfp4:
@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
         uint32_t v = __vmaxu4(sc.x, sc.y);
         v = __vmaxu4(v, v >> 16);
         emax = (int)max(v & 0xffu, (v >> 8) & 0xffu);
-        inv = emax >= 255 ? __uint_as_float(0x7f800000u) : exp2f((float)(emax - 127 - 11));
+        inv = emax >= 255 ? __uint_as_float(0x7f800000u) : exp2f((float)(emax - 127 - 13));
       } else {
         // largest |s| and |b| (bits order like magnitudes), as bfloat16 bits
         uint32_t ms = __vmaxu2(sc.x & 0x7fff7fffu, sc.y & 0x7fff7fffu);
@@ -459,9 +459,9 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
         const uint32_t ws[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
         uint32_t o[2][16];
         if (MX) {
-          // fp16 2^(e - emax + 11) in both halves; 0 from 26 binades below emax
-          const __half2 s0 = tm_half2((uint32_t)max((int)(s_lo & 0xffu) - emax + 26, 0) * 0x04000400u);
-          const __half2 s1 = tm_half2((uint32_t)max((int)((s_lo >> 8) & 0xffu) - emax + 26, 0) * 0x04000400u);
+          // fp16 2^(e - emax + 13) in both halves, subnormal ones included
+          const __half2 s0 = __float2half2_rn(__uint_as_float((uint32_t)max((int)(s_lo & 0xffu) - emax + 140, 0) << 23));
+          const __half2 s1 = __float2half2_rn(__uint_as_float((uint32_t)max((int)((s_lo >> 8) & 0xffu) - emax + 140, 0) << 23));
 #pragma unroll
           for (int k = 0; k < 8; ++k) tm_expand_mx(ws[k], k < 4 ? s0 : s1, o[k >> 2] + 4 * (k & 3));
         } else {
