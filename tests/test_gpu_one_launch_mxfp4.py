@@ -88,3 +88,24 @@ def test_blocks_far_below_their_neighbours_keep_their_bits(T):
     layer.check_status()
     alone = MoELayer(cfg, dict(params, **low), max_tokens=8)
     assert layer.passes(T) and torch.equal(out, alone(x))
+
+
+@pytest.mark.parametrize("T", [1, 8, 12])
+def test_weights_on_eight_byte_boundaries_take_the_separate_kernels(T):
+    """A tensor that starts eight bytes into its storage, as slices of a mapped file do, was always served."""
+    cfg = synthetic.CONFIGS["c3"].scaled(**SHAPES["narrow"])
+    params = synthetic.make_layer(cfg, device=DEV)
+    x = synthetic.make_tokens(cfg, T, device=DEV)
+    want = MoELayer(cfg, params, max_tokens=16, fused=False)(x).clone()
+
+    def shifted(w):
+        buf = torch.empty(w.numel() + 2, dtype=torch.int32, device=DEV)
+        buf[2:] = w.view(torch.int32).reshape(-1)
+        return buf[2:].view(w.shape).view(w.dtype)
+
+    moved = dict(params, **{f"{k}_w": shifted(params[f"{k}_w"]) for k in ("gate", "up", "down")},
+                 gate_b=torch.zeros(3, dtype=torch.uint8, device=DEV)[1:])
+    assert moved["gate_w"].data_ptr() % 16 == 8
+    layer = MoELayer(cfg, moved, max_tokens=16)
+    assert_close_rel(t2n(layer(x)), t2n(want), 2e-2, f"T={T}")
+    assert not layer.passes(T)

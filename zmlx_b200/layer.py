@@ -91,7 +91,7 @@ class MoELayer:
             for proj in ("gate", "up", "down"):
                 setattr(dst, f"{proj}_w", src[f"{proj}_w"].data_ptr())
                 setattr(dst, f"{proj}_scales", src[f"{proj}_s"].data_ptr())
-                b = src.get(f"{proj}_b")
+                b = src.get(f"{proj}_b") if cfg.mode != "mxfp4" else None  # mxfp4 has none: what is there is ignored
                 setattr(dst, f"{proj}_biases", b.data_ptr() if b is not None else None)
 
         bank(d.routed, W)
@@ -110,7 +110,10 @@ class MoELayer:
         """The same for whichever one-launch entry takes this block's banks."""
         if self.cfg.mode != "mxfp4":
             return self.fused_workspace_bytes(T)
-        if T < 1 or T > self.FUSED_MAX_TOKENS:
+        # the separate kernels take packed weights on 8-byte boundaries, the one launch fetches 16 bytes at a time
+        banks = [self.p, self.p["shared"]] if self.cfg.n_shared else [self.p]
+        if T < 1 or T > self.FUSED_MAX_TOKENS or any(b[f"{k}_w"].data_ptr() % 16 for b in banks
+                                                     for k in ("gate", "up", "down")):
             return 0
         return int(_lib.load().zmoe_layer_decode_mxfp4_workspace_bytes(ctypes.byref(self._desc), T))
 
