@@ -88,3 +88,25 @@ def test_head_shapes_without_a_kernel_are_left_to_torch():
         q = torch.zeros((1, hq, 1, hd), dtype=torch.bfloat16, device=DEV)
         c = torch.zeros((1, hk, 8, hd), dtype=torch.bfloat16, device=DEV)
         assert ops.decode_attention(q, c, c, npos=3) is None
+
+
+@pytest.mark.parametrize("hq,hk,hd", [(4, 2, 64), (8, 1, 128)])
+def test_decode_attention_with_infinite_keys(hq, hk, hd):
+    """Positions whose score is -inf weigh nothing, also where a whole block or slice of the cache holds only such; a row
+    without any other score, or with one of +inf, is NaN, as softmax has it."""
+    g = torch.Generator(device=DEV).manual_seed(5)
+    npos, n = 700, 64
+    q = _randn(g, 4, hq, 1, hd).abs() + 0.125
+    kc, vc = _randn(g, 4, hk, npos, hd), _randn(g, 4, hk, npos, hd)
+    dead = torch.zeros((4, npos), dtype=torch.bool, device=DEV)
+    dead[0, :3 * n], dead[1, n + 5:-1], dead[2] = True, True, True
+    kd, vd = (t.double().repeat_interleave(hq // hk, 1) for t in (kc, vc))
+    sc = ((q.double() @ kd.transpose(-1, -2)) / math.sqrt(hd))[:, :, 0].masked_fill(dead[:, None], -math.inf)
+    pr = torch.softmax(sc, dim=-1)[:, :, None]
+    ref, mass = (pr @ vd)[:, :, 0], (pr @ vd.abs())[:, :, 0]
+    kc[:, :, :, 7] = torch.where(dead[:, None], -math.inf, kc[:, :, :, 7].float()).to(torch.bfloat16)
+    kc[3, :, 100, 7] = math.inf
+    got = ops.decode_attention(q, kc, vc, npos=npos).view(4, hq, hd).double()
+    for b in (0, 1):
+        assert bool(((got[b] - ref[b]).abs() <= 2.0 ** -8 * ref[b].abs() + 2.0 ** -15 * mass[b]).all()), b
+    assert bool(got[2].isnan().all()) and bool(got[3].isnan().all())

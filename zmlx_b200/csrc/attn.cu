@@ -229,13 +229,14 @@ __global__ void __launch_bounds__(kAttThreads) decode_attn_kernel(const AttParam
     __syncthreads();
     if (wid < REP) {  // one warp per head: running maximum and sum
       const float s0 = sc[lane][wid], s1 = sc[lane + 32][wid];
-      const float m = fmaxf(run_m[wid], warp_max(fmaxf(s0, s1)));  // finite: the block has at least one position
-      const float e0 = expf(s0 - m), e1 = expf(s1 - m);
+      const float m = fmaxf(run_m[wid], warp_max(fmaxf(s0, s1)));
+      const float ref = m == -INFINITY ? 0.0f : m;  // every score so far is -inf: their weights are 0, not exp(-inf + inf)
+      const float e0 = expf(s0 - ref), e1 = expf(s1 - ref);
       const float sum = warp_sum(e0 + e1);
       sc[lane][wid] = e0;
       sc[lane + 32][wid] = e1;
       if (lane == 0) {
-        const float f = expf(run_m[wid] - m);
+        const float f = expf(run_m[wid] - ref);
         fac[wid] = f;
         run_s[wid] = run_s[wid] * f + sum;
         run_m[wid] = m;
