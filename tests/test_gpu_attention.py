@@ -110,3 +110,19 @@ def test_decode_attention_with_infinite_keys(hq, hk, hd):
     for b in (0, 1):
         assert bool(((got[b] - ref[b]).abs() <= 2.0 ** -8 * ref[b].abs() + 2.0 ** -15 * mass[b]).all()), b
     assert bool(got[2].isnan().all()) and bool(got[3].isnan().all())
+
+
+def test_tensors_the_kernels_cannot_read_are_refused():
+    """Another dtype, a transposed or a short tensor: an error, not other values read through the pointer."""
+    h, w = torch.zeros((4, 64), dtype=torch.bfloat16, device=DEV), torch.ones(64, dtype=torch.bfloat16, device=DEV)
+    for delta in (h.float(), torch.zeros((64, 4), dtype=torch.bfloat16, device=DEV).T, h[:2]):
+        with pytest.raises(ValueError):
+            ops.add_rms_norm(h, delta, w, 1e-6)
+    c = torch.zeros((2, 2, 8, 64), dtype=torch.bfloat16, device=DEV)
+    q = torch.zeros((2, 64, 1, 2), dtype=torch.bfloat16, device=DEV).transpose(1, 3)
+    with pytest.raises(ValueError):
+        ops.decode_attention(q, c, c, npos=3)
+    cos = torch.zeros((8, 32), device=DEV)
+    rows = torch.zeros((2, 128), dtype=torch.bfloat16, device=DEV)
+    with pytest.raises(ValueError):
+        ops.qkv_post(rows, rows.float(), rows, w, w, cos, cos, 1e-6, 2, 1, 0, c, c)

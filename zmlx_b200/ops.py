@@ -258,9 +258,20 @@ def router_logits(x: torch.Tensor, wr: torch.Tensor, *, out_dtype: torch.dtype =
 # ------------------------------------------------------------------ the attention side of the decoder
 
 
+def _dense_bf16(name: str, t: torch.Tensor, numel: int) -> None:
+    """The decoder's kernels take pointers only: what they assume about the tensors is checked here."""
+    if t.dtype != torch.bfloat16 or not t.is_contiguous() or t.numel() != numel:
+        raise ValueError(f"{name}: expected {numel} contiguous bfloat16 values, got {tuple(t.shape)} {t.dtype} with "
+                         f"strides {t.stride()}")
+
+
 def add_rms_norm(h: torch.Tensor, delta: torch.Tensor | None, w: torch.Tensor, eps: float) -> torch.Tensor:
     """``h += delta`` in place (when given), then the RMS norm of the rows of h (R, d) with weight w (d)."""
     dev = _need_cuda(h, delta, w)
+    _dense_bf16("h", h, h.numel())
+    if delta is not None:
+        _dense_bf16("delta", delta, h.numel())
+    _dense_bf16("w", w, h.shape[1])
     x = torch.empty_like(h)
     with torch.cuda.device(dev):
         _lib.check(_lib.load().zmoe_add_rms_norm(_ptr(h), _ptr(delta), _ptr(w), ctypes.c_float(eps), h.shape[0],
@@ -274,6 +285,8 @@ def qkv_post(q, k, v, q_norm, k_norm, cos, sin, eps: float, B: int, S: int, pos,
     dev = _need_cuda(q, k, v, k_cache, v_cache)
     hk, max_seq, hd = k_cache.shape[-3:]
     hq = q.shape[-1] // hd
+    for name, t, heads in (("q", q, hq), ("k", k, hk), ("v", v, hk)):
+        _dense_bf16(name, t, B * S * heads * hd)
     out = torch.empty((B, hq, S, hd), dtype=torch.bfloat16, device=dev)
     on_dev = isinstance(pos, torch.Tensor)
     with torch.cuda.device(dev):
@@ -290,6 +303,7 @@ def decode_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
     and including the int64 device scalar ``pos``): (B, Hq * hd) bfloat16, or None for head shapes without a kernel."""
     dev = _need_cuda(q, k_cache, v_cache, pos)
     B, hq, _, hd = q.shape
+    _dense_bf16("q", q, B * hq * hd)
     hk, max_seq = k_cache.shape[-3], k_cache.shape[-2]
     lib = _lib.load()
     n = int(lib.zmoe_decode_attention_workspace_bytes(B, hq, hk, hd, max_seq if npos is None else npos))
