@@ -163,3 +163,34 @@ def test_block_loaded_from_an_mlx_format_checkpoint_gives_the_same_bits(tmp_path
     a = MoELayer(cfg, params, max_tokens=8)(x).clone()
     b = MoELayer(cfg, loaded, max_tokens=8)(x).clone()
     assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("name,scaled,T", [("c1", {}, 9), ("c2", dict(n_experts=32), 64),
+                                           ("c3", dict(d_model=512, d_ff=256, n_experts=16), 40),
+                                           ("c5", dict(n_experts=32, d_model=512, d_ff=256, n_group=4, topk_group=2), 100)])
+def test_forward_allocates_nothing_and_can_be_captured(name, scaled, T):
+    """Once a layer is built for a token count, a pass takes nothing from the allocator: neither eagerly nor under a
+    capture, on another stream, whose replay gives the same bits."""
+    cfg = synthetic.CONFIGS[name].scaled(**scaled)
+    layer = MoELayer(cfg, synthetic.make_layer(cfg, device=DEV), max_tokens=T)
+    x = synthetic.make_tokens(cfg, T, device=DEV)
+    out = torch.empty_like(x)
+    want = layer(x, out).clone()
+
+    def allocations():
+        return torch.cuda.memory_stats()["allocation.all.allocated"]
+
+    before = allocations()
+    layer(x, out)
+    assert allocations() == before
+    stream = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        before = allocations()
+        layer(x, out)
+        assert allocations() == before
+    out.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
+    layer.check_status()

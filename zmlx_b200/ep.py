@@ -134,9 +134,10 @@ class EPMoELayer:
         st = ops._stream()
         _lib.check(lib.zmoe_build_plan(None, K, p(li), TA * K, 1, self.n_local, p(self.local_plan),
                                        self.local_plan.numel() * 4, st))
+        inner._gate_up(x_all, inner.p, self.n_local, cfg.d_ff, self.local_plan, TA * K, TA, inner.h, inner.swiglu, inner.work)
         y = inner.y[:TA * K]
-        y.zero_()
-        inner._mlp(x_all, inner.p, self.n_local, cfg.d_ff, self.local_plan, TA * K, TA, inner.h, y, inner.swiglu, 1)
+        y.zero_()  # only now: the gate/up matmul's workspace lies there
+        inner._down(inner.h, inner.p, self.n_local, cfg.d_ff, self.local_plan, TA * K, TA, 1, y, inner.work)
 
     def _run_segment(self, TA: int) -> None:
         if not self.segment_graphs:

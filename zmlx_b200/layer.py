@@ -3,9 +3,9 @@
 This is the order of the reference's patched block
 (src/zmlx/patch/patterns/moe_mlp.py:883-1063) with every step running in a
 libzmoe kernel.  ``MoELayer`` owns the packed tensors of one layer and
-preallocated work buffers for a fixed maximum token count, so that a forward
-pass can be captured in a CUDA graph; above eight rows the grouped matmuls take a
-workspace from torch's allocator for the length of the call.
+preallocated work buffers for a fixed maximum token count, the matmuls' workspace
+among them, so that a forward pass allocates nothing and can be captured in a CUDA
+graph.
 """
 
 from __future__ import annotations
@@ -240,13 +240,29 @@ class MoELayer:
         self.plan = torch.zeros(ops.plan_bytes(T * K, cfg.n_experts) // 4, dtype=i32, device=dev)  # no status yet
         self.counter = torch.zeros(1, dtype=i32, device=dev)
         self.h = torch.empty((T * K, cfg.d_ff), dtype=bf, device=dev)
-        self.y = torch.empty((T * K, cfg.d_model), dtype=bf, device=dev)
+        self.y, self.work = self._rows_and_work(T * K, cfg.n_experts, cfg.d_ff, T)
         self.out = torch.empty((T, cfg.d_model), dtype=bf, device=dev)
         if cfg.n_shared:
             self.zero_idx = torch.zeros((T,), dtype=i32, device=dev)
             self.shared_plan = torch.zeros(ops.plan_bytes(T, 1) // 4, dtype=i32, device=dev)
             self.sh_h = torch.empty((T, cfg.d_ff * cfg.n_shared), dtype=bf, device=dev)
-            self.sh_y = torch.empty((T, cfg.d_model), dtype=bf, device=dev)
+            self.sh_y, self.sh_work = self._rows_and_work(T, 1, cfg.d_ff * cfg.n_shared, T)
+
+    def _rows_and_work(self, rows: int, E: int, f: int, rows_hint: int):
+        """The projected rows (rows, d_model) of a bank with inner width f, and the workspaces of its two matmuls (or None):
+        the gate/up one lies where the projected rows come to lie afterwards, the down one behind them.  One allocation, a
+        third larger than the rows alone."""
+        cfg = self.cfg
+        gate_up, down = (ops.qmm_workspace_bytes(rows, E, K, rows_hint=rows_hint, mode=cfg.mode) for K in (cfg.d_model, f))
+        y_bytes = rows * cfg.d_model * 2
+        if gate_up or down:
+            behind = (y_bytes + 255) // 256 * 256
+            try:
+                buf = torch.empty(max(gate_up, behind + down), dtype=torch.uint8, device=self.device)
+                return buf[:y_bytes].view(torch.bfloat16).view(rows, cfg.d_model), (buf, buf[behind:])
+            except torch.OutOfMemoryError:
+                pass  # the kernels that need none still serve the block
+        return torch.empty((rows, cfg.d_model), dtype=torch.bfloat16, device=self.device), None
 
     # -- steps -------------------------------------------------------------
     def _route_args(self):
@@ -308,35 +324,30 @@ class MoELayer:
         cfg = self.cfg
         T = x.shape[0]
         K = cfg.top_k
-        self._mlp(x, self.p, cfg.n_experts, cfg.d_ff, self.plan, T * K, T, self.h, self.y, self.swiglu, 3)
+        self._gate_up(x, self.p, cfg.n_experts, cfg.d_ff, self.plan, T * K, T, self.h, self.swiglu, self.work)
+        self._down(self.h, self.p, cfg.n_experts, cfg.d_ff, self.plan, T * K, T, 3, self.y, self.work)
 
-    def _workspace(self, rows: int, E: int, f: int, rows_hint: int) -> torch.Tensor | None:
-        # one workspace serves both matmuls: the second prepares its rows after the first has read its own
-        return ops.qmm_workspace(rows, E, max(self.cfg.d_model, f), rows_hint=rows_hint, mode=self.cfg.mode,
-                                 device=self.device)
-
-    def _mlp(self, x, bank: dict, E: int, f: int, plan, rows: int, rows_hint: int, h, y, swiglu: int, down_flags: int,
-             ws: torch.Tensor | None = None):
-        """gate/up + SwiGLU of `rows` planned rows into h, and their down projection into y; ``ws``: their workspace, by
-        default one of this call's own."""
-        cfg = self.cfg
-        lib = _lib.load()
-        st = ops._stream()
+    def _gate_up(self, x, bank: dict, E: int, f: int, plan, rows: int, rows_hint: int, h, swiglu: int, work):
+        """gate/up + SwiGLU of `rows` planned rows into h; ``work`` as ``_rows_and_work`` returns it (its first part, the
+        memory of the projected rows, is overwritten)."""
         p = ops._ptr
-        qm = ops.qmode_code(cfg.mode)
-        ws = ops._ws_args(self._workspace(rows, E, f, rows_hint) if ws is None else ws)
-        _lib.check(lib.zmoe_gather_qmm_swiglu_ws(p(x), x.shape[0], x.stride(0), p(bank["gate_w"]), p(bank["gate_s"]),
-                                                 p(bank["gate_b"]), p(bank["up_w"]), p(bank["up_s"]), p(bank["up_b"]),
-                                                 E, f, cfg.d_model, self.gs, qm, p(plan), rows, rows_hint, p(h),
-                                                 swiglu, *ws, st))
-        _lib.check(lib.zmoe_gather_qmm_ws(p(h), rows, f, p(bank["down_w"]), p(bank["down_s"]), p(bank["down_b"]), E,
-                                          cfg.d_model, f, self.gs, qm, p(plan), rows, rows_hint, down_flags, p(y), *ws,
-                                          st))
+        _lib.check(_lib.load().zmoe_gather_qmm_swiglu_ws(
+            p(x), x.shape[0], x.stride(0), p(bank["gate_w"]), p(bank["gate_s"]), p(bank["gate_b"]), p(bank["up_w"]),
+            p(bank["up_s"]), p(bank["up_b"]), E, f, self.cfg.d_model, self.gs, ops.qmode_code(self.cfg.mode), p(plan), rows,
+            rows_hint, p(h), swiglu, *ops._ws_args(work and work[0]), ops._stream()))
+
+    def _down(self, h, bank: dict, E: int, f: int, plan, rows: int, rows_hint: int, flags: int, y, work):
+        """Down projection of the planned rows of h into y."""
+        p = ops._ptr
+        _lib.check(_lib.load().zmoe_gather_qmm_ws(
+            p(h), rows, f, p(bank["down_w"]), p(bank["down_s"]), p(bank["down_b"]), E, self.cfg.d_model, f, self.gs,
+            ops.qmode_code(self.cfg.mode), p(plan), rows, rows_hint, flags, p(y), *ops._ws_args(work and work[1]),
+            ops._stream()))
 
     def _new_shared_plan(self, T: int) -> torch.Tensor:
         return torch.zeros(ops.plan_bytes(T, 1) // 4, dtype=torch.int32, device=self.device)
 
-    def shared(self, x: torch.Tensor, ws: torch.Tensor | None = None, plan_buf: torch.Tensor | None = None):
+    def shared(self, x: torch.Tensor, plan_buf: torch.Tensor | None = None):
         """The always-on shared expert: the same kernels with a one-expert bank."""
         cfg = self.cfg
         T = x.shape[0]
@@ -351,8 +362,9 @@ class MoELayer:
                                                    ops._stream()))
             if not capturing:
                 self._shared_plans[T] = plan
-        self._mlp(x, self.p["shared"], 1, cfg.d_ff * cfg.n_shared, plan, T, T, self.sh_h, self.sh_y, _lib.SWIGLU_PER_OP, 1,
-                  ws)
+        f, bank = cfg.d_ff * cfg.n_shared, self.p["shared"]
+        self._gate_up(x, bank, 1, f, plan, T, T, self.sh_h, _lib.SWIGLU_PER_OP, self.sh_work)
+        self._down(self.sh_h, bank, 1, f, plan, T, T, 1, self.sh_y, self.sh_work)
 
     def forward(self, x: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
         """x (T, d_model) bfloat16 on this layer's device -> (T, d_model) bfloat16: ``out`` when given (contiguous,
@@ -397,20 +409,17 @@ class MoELayer:
             cur = torch.cuda.current_stream(self.device)
             if self._side is None:
                 self._side = torch.cuda.Stream(device=self.device)
-            # its workspace and plan are the current stream's memory (a side stream's pool starts empty, and what is
-            # taken there stays there); the workspace is held until that stream has joined the side stream below
-            shared_ws = self._workspace(T, 1, cfg.d_ff * cfg.n_shared, T)
+            # its plan is the current stream's memory (a side stream's pool starts empty, and what is taken there stays)
             first = T not in self._shared_plans and not torch.cuda.is_current_stream_capturing()
             plan_buf = self._new_shared_plan(T) if first else None
             self._side.wait_stream(cur)
             with torch.cuda.stream(self._side):
-                self.shared(x, shared_ws, plan_buf)
+                self.shared(x, plan_buf)
             residual = self.sh_y
         self.route(x)
         self.experts(x)
         if cfg.n_shared:
             cur.wait_stream(self._side)
-            del shared_ws
         dst = self.out if out is None else out
         _lib.check(_lib.load().zmoe_moe_combine(
             ops._ptr(self.y), _lib.BF16, ops._ptr(self.weights), _lib.F32, T, cfg.top_k, cfg.d_model,

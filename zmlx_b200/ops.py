@@ -93,10 +93,15 @@ def check_plan(plan: torch.Tensor) -> None:
         _lib.check(_lib.load().zmoe_plan_status(_ptr(plan), 1, _stream()))
 
 
+def qmm_workspace_bytes(rows: int, E: int, K: int, *, rows_hint: int, mode: str) -> int:
+    """Size of the workspace of one grouped matmul call; 0 where the call gains nothing from one."""
+    return int(_lib.load().zmoe_qmm_workspace_bytes(int(rows), int(E), int(K), int(rows_hint), qmode_code(mode)))
+
+
 def qmm_workspace(rows: int, E: int, K: int, *, rows_hint: int, mode: str, device) -> torch.Tensor | None:
     """Workspace of one grouped matmul call, from torch's allocator (so it belongs to the current stream and goes back
     to the pool when the call's reference is dropped), or None where the call gains nothing from one."""
-    n = int(_lib.load().zmoe_qmm_workspace_bytes(int(rows), int(E), int(K), int(rows_hint), qmode_code(mode)))
+    n = qmm_workspace_bytes(rows, E, K, rows_hint=rows_hint, mode=mode)
     if n == 0:
         return None
     try:
