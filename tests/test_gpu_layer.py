@@ -30,8 +30,9 @@ def _layer(name):
                                           ("c2", 1, True), ("c2", 2, True), ("c2", 3, True), ("c2", 4, True),
                                           ("c2", 7, True), ("c2", 8, True), ("c5", 1, True), ("c5", 2, True),
                                           ("c5", 4, True), ("c5", 8, True),
-                                          # more rows than one launch takes: consecutive passes of eight
-                                          ("c2", 16, True), ("c2", 29, True), ("c5", 20, True), ("c5", 24, True), ("c5", 64, True)])
+                                          # more rows than one launch takes: two passes for wide blocks of up to
+                                          # twelve rows, the separate kernels for the others
+                                          ("c5", 9, True), ("c5", 11, True), ("c5", 12, True), ("c2", 16, True), ("c2", 29, True), ("c5", 20, True), ("c5", 24, True), ("c5", 64, True)])
 def test_layer_matches_oracle(name, T, fused):
     cfg, params = _layer(name)
     layer = MoELayer(cfg, params, max_tokens=max(64, T), fused=fused)
@@ -39,6 +40,10 @@ def test_layer_matches_oracle(name, T, fused):
     x = synthetic.make_tokens(cfg, T, device="cpu").to(DEV)
     out = layer(x).clone()
     assert layer.fused_status(T) == 0
+    layer.check_status()
+    if fused:
+        passes = 1 if T <= 8 else (2 if name == "c5" and T <= 12 else 0)
+        assert len(layer.passes(T)) == passes and layer._fused_ok[T] == ("chunks" if passes > 1 else passes == 1)
     ref, w_ref = _oracle_layer(cfg, params, x, layer.router_logits(T), layer.indices[:T])
     w_gpu = t2n(layer.weights[:T])
     if cfg.family == "generic":  # the block casts the weights to T before combining (moe_mlp.py:288)
@@ -194,3 +199,22 @@ def test_forward_allocates_nothing_and_can_be_captured(name, scaled, T):
     torch.cuda.synchronize()
     assert torch.equal(out, want)
     layer.check_status()
+
+
+def test_a_block_whose_workspace_cannot_be_had_takes_the_kernels_without(monkeypatch):
+    cfg = synthetic.CONFIGS["c1"]
+    params = synthetic.make_layer(cfg, device=DEV)
+    x = synthetic.make_tokens(cfg, 40, device=DEV)
+    want = MoELayer(cfg, params, max_tokens=40)(x).clone()
+    real = torch.empty
+
+    def empty(*size, **kw):
+        if kw.get("dtype") is torch.uint8:
+            raise torch.OutOfMemoryError("no memory for a workspace")
+        return real(*size, **kw)
+
+    monkeypatch.setattr(torch, "empty", empty)
+    layer = MoELayer(cfg, params, max_tokens=40)
+    monkeypatch.undo()
+    assert layer.work is None
+    assert_close_rel(t2n(layer(x)), t2n(want), 2e-2, "without a workspace")

@@ -278,3 +278,39 @@ def test_the_operator_on_few_tokens(monkeypatch, mode, tokens, workspace):
     err = (h.reshape(want.shape).double() - want).abs()
     # gate and up may round to the neighbour (2^-7 of them), the result rounds once
     assert bool((err <= (3 * 2.0 ** -7) * (want.abs() + gv.abs() * uv.abs()) + 1e-6).all())
+
+
+@pytest.mark.parametrize("rows", [9, 60])
+@pytest.mark.parametrize("mode", ["affine", "mxfp4"])
+def test_a_row_that_is_not_finite_stays_alone(mode, rows):
+    """An infinity or a NaN makes its own row's results non-finite and leaves its neighbours' bits as they are."""
+    E, N, K = 2, 200, 512
+    g = torch.Generator(device=DEV).manual_seed(4)
+    a, _ = _bank(g, E, N, K, mode, False)
+    x = torch.randn((E * rows, K), generator=g, device=DEV).to(torch.bfloat16)
+    plan = ops.build_plan(torch.arange(E * rows, device=DEV) // rows, E)
+    ws = ops.qmm_workspace(E * rows, E, K, rows_hint=E * rows, mode=mode, device=DEV)
+    clean = _call(x, E * rows, K, [a], E, N, mode, plan, E * rows, E * rows, 1, ws)
+    x[3, 7], x[rows + 2, 300] = float("inf"), float("nan")
+    got = _call(x, E * rows, K, [a], E, N, mode, plan, E * rows, E * rows, 1, ws)
+    bad = torch.zeros(E * rows, dtype=torch.bool, device=DEV)
+    bad[3] = bad[rows + 2] = True
+    assert torch.equal(got[~bad], clean[~bad]) and not bool(got[bad].isfinite().any())
+
+
+def test_more_items_than_a_cta_keeps_in_its_list():
+    """400 experts x 128 row tiles over the SMs: 346 items per CTA on 148 of them, 256 of which are kept in shared memory."""
+    E, N, K = 400, 16384, 256
+    g = torch.Generator(device=DEV).manual_seed(6)
+    word = torch.randint(-2 ** 31, 2 ** 31, (E, N, K // 8), generator=g, device=DEV, dtype=torch.int64).to(torch.int32)
+    s = (torch.rand((E, N, K // 64), generator=g, device=DEV) + 0.5).to(torch.bfloat16)
+    b = (-8.0 * torch.rand((E, N, K // 64), generator=g, device=DEV)).to(torch.bfloat16)
+    rows = E + 20
+    ids = torch.cat([torch.arange(E, device=DEV), torch.full((20,), E - 1, device=DEV)])
+    x = torch.randn((rows, K), generator=g, device=DEV).to(torch.bfloat16)
+    ws = ops.qmm_workspace(rows, E, K, rows_hint=21, mode="affine", device=DEV)
+    got = _call(x, rows, K, [(word, s, b)], E, N, "affine", ops.build_plan(ids, E), rows, 21, 1, ws)
+    for e in range(E):
+        m = ids == e
+        A, xe = _weights(word[e], s[e], b[e]), x[m].double()
+        _within(got[m], xe @ A.T, xe.abs() @ A.abs().T, K)
