@@ -22,8 +22,8 @@
 // Arithmetic.  Affine: w = q s + b = (q - 8) s + (b + 8 s).  q - 8 has three bits and a sign, s eight: their product fits
 // fp16's eleven, so the scale goes into the operand and the accumulator runs over several groups.  The second term is two
 // more K = 16 steps on one operand, per group (b, b, -8 s, -8 s), against the group's float32 sum X as three fp16 pieces (33
-// bits): (X1, X2, -X1, -X2) and (X3, 0, -X3, 0).  The scales are first multiplied by a
-// power of two per (row, chunk), undone in fp32 by the finishers, so the range of fp16 is no limit on the checkpoint's.
+// bits): (X1, X2, -X1, -X2) and (X3, 0, -X3, 0).  The scales are first multiplied by a power of two per (row, chunk), undone
+// in fp32 by the finishers, so the range of fp16 is no limit on the checkpoint's.
 // (q - 8) s is exact while the four scales of a row's chunk lie within 12 binades of the largest; chunks with scales
 // further apart are expanded another way (tm_expand_far), exact over 28; below, a weight is off by at most 2^-39 of the
 // largest of its row's chunk.  mxfp4: e2m1 value x 2^(e - emax + 13), exact in fp16 over 36 binades, same row factor.
@@ -716,8 +716,8 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
 
 // ------------------------------------------------------------------ token rows in sorted order
 // One CTA per sorted row: |x|max, then fp16 values under 2^k with |x|max 2^k in [2^14, 2^15), or for affine banks in [2^9,
-// 2^10), whose group sums just fit fp16 (64 x 1020 = 65280), and the sums of its groups of 64 as (X1, X2, -X1, -X2) and (X3, 0, -X3, 0).  Affine rows take the order in which tm_expand_affine
-// leaves codes.
+// 2^10), whose group sums just fit fp16 (64 x 1020 = 65280), and the sums of its groups of 64 as (X1, X2, -X1, -X2) and
+// (X3, 0, -X3, 0).  Affine rows take the order in which tm_expand_affine leaves codes.
 constexpr int kPrepThreads = 128;
 
 template <bool MX>
