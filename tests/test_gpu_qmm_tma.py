@@ -255,31 +255,6 @@ def test_block_exponents_far_apart_in_one_chunk(rows):
     assert bool(((got.double() - ref).abs() <= bound).all())
 
 
-@pytest.mark.parametrize("mode,tokens,workspace", [("affine", 2, False), ("affine", 6, False), ("affine", 7, True),
-                                                   ("mxfp4", 2, True), ("affine", 19, True)])
-def test_the_operator_on_few_tokens(monkeypatch, mode, tokens, workspace):
-    """gather_qmm_swiglu takes the kernel that is the faster one for its size; either gives the same activations."""
-    from zmlx_b200.kernels import fused_moe
-
-    E, N, K, top = 32, 64, 256, 8
-    g = torch.Generator(device=DEV).manual_seed(tokens)
-    a, A = _bank(g, E, N, K, mode, False)
-    u, U = _bank(g, E, N, K, mode, False)
-    x = torch.randn((tokens, K), generator=g, device=DEV).to(torch.bfloat16)
-    idx = torch.rand((tokens, E), generator=g, device=DEV).topk(top, dim=-1).indices.to(torch.int32)
-    asked = []
-    real = ops.qmm_workspace
-    monkeypatch.setattr(ops, "qmm_workspace", lambda *args, **kw: asked.append(real(*args, **kw)) or asked[-1])
-    h = fused_moe.gather_qmm_swiglu(x[:, None, None, :], *a, *u, rhs_indices=idx, group_size=64, mode=mode)
-    assert any(w is not None for w in asked) == workspace
-    gv = torch.einsum("tk,tsnk->tsn", x.double(), A[idx.long()]).to(torch.bfloat16).double()
-    uv = torch.einsum("tk,tsnk->tsn", x.double(), U[idx.long()]).to(torch.bfloat16).double()
-    want = gv * torch.sigmoid(gv) * uv
-    err = (h.reshape(want.shape).double() - want).abs()
-    # gate and up may round to the neighbour (2^-7 of them), the result rounds once
-    assert bool((err <= (3 * 2.0 ** -7) * (want.abs() + gv.abs() * uv.abs()) + 1e-6).all())
-
-
 @pytest.mark.parametrize("rows", [9, 60])
 @pytest.mark.parametrize("mode", ["affine", "mxfp4"])
 def test_a_row_that_is_not_finite_stays_alone(mode, rows):

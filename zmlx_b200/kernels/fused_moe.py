@@ -136,13 +136,8 @@ def gather_qmm_swiglu(
         return torch.empty(out_batch + (M, N), dtype=torch.bfloat16, device=dev)
     plan = ops.build_plan(rhs.reshape(-1), E, M=M, lhs=lhs.reshape(-1))
     sw = _lib.SWIGLU_CPU if swiglu_contract == "cpu" else _lib.SWIGLU_PER_OP
-    # The pairs' experts are not known here, so an expert may own all P * M rows.  Affine calls of up to 48 rows, no more
-    # than two per expert on average, stay on the register-fed kernels all the same: 128 experts of 768 x 2048, top-8, 2 tokens 15
-    # against 24 us in the tensor-memory kernel, 6 tokens 36 against 38, 8 tokens 46 against 43; 32 experts of 768 x 1024,
-    # top-4, 12 tokens 17 against 21.  mxfp4 gains from nine rows on (64 experts, top-4, 3 tokens 31 against 23).
-    few = mode == "affine" and P * M <= 48 and P * M <= 2 * E
     out = ops.gather_qmm_swiglu_rows(x2, gw.contiguous(), gs_, gb_, uw.contiguous(), us_, ub_, plan, P * M,
-                                     rows_hint=P * M, group_size=gsz, mode=mode, swiglu=sw, workspace=not few)
+                                     rows_hint=P * M, group_size=gsz, mode=mode, swiglu=sw)
     return out.reshape(out_batch + (M, N))
 
 

@@ -123,9 +123,7 @@ def _check_packed(w: torch.Tensor, name: str) -> None:
 
 def gather_qmm_swiglu_rows(x2: torch.Tensor, gate_w, gate_s, gate_b, up_w, up_s, up_b, plan: torch.Tensor, rows: int,
                            *, rows_hint: int, group_size: int = 64, mode: str = "affine",
-                           swiglu: int = _lib.SWIGLU_CPU, out: torch.Tensor | None = None,
-                           workspace: bool = True) -> torch.Tensor:
-    """``workspace``: whether the call may take the kernels that need one."""
+                           swiglu: int = _lib.SWIGLU_CPU, out: torch.Tensor | None = None) -> torch.Tensor:
     dev = _need_cuda(x2, gate_w, gate_s, gate_b, up_w, up_s, up_b, plan)
     if x2.dtype != torch.bfloat16:
         raise TypeError(f"activations must be bfloat16, got {x2.dtype}")
@@ -138,7 +136,7 @@ def gather_qmm_swiglu_rows(x2: torch.Tensor, gate_w, gate_s, gate_b, up_w, up_s,
     if out is None:
         out = torch.empty((rows, N), dtype=torch.bfloat16, device=dev)
     with torch.cuda.device(dev):
-        ws = qmm_workspace(rows, E, K, rows_hint=rows_hint, mode=mode, device=dev) if workspace else None
+        ws = qmm_workspace(rows, E, K, rows_hint=rows_hint, mode=mode, device=dev)
         _lib.check(_lib.load().zmoe_gather_qmm_swiglu_ws(
             _ptr(x2), x2.shape[0], x2.stride(0), _ptr(gate_w), _ptr(gate_s), _ptr(gate_b), _ptr(up_w), _ptr(up_s),
             _ptr(up_b), E, N, K, int(group_size), qmode_code(mode), _ptr(plan), int(rows), int(rows_hint), _ptr(out),
