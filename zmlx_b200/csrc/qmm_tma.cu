@@ -12,21 +12,32 @@
 //              unbroken stream of chunks of 256 codes:
 //     weights   one thread keeps kTmRaw boxes of 128 rows x 128 packed bytes in flight;
 //     tokens    one thread keeps the ring of token tiles full;
-//     expanders two sets of 128 threads (one per weight row) turn every other chunk's codes into the fp16 A operand
-//               and store it straight into the set's stage in TENSOR MEMORY (tcgen05.st): no shared-memory round trip,
-//               no swizzle arithmetic; one set's waits and latencies lie under the other set's arithmetic;
+//     expanders two or three sets of 128 threads (one per weight row) take turns at the chunks, turn the codes into the fp16
+//               A operand and store it straight into the set's stage in TENSOR MEMORY (tcgen05.st): no shared-memory round
+//               trip, no swizzle arithmetic; one set's waits and latencies lie under the other sets' arithmetic;
 //     issuer    one thread issues tcgen05.mma (M 128 x N 16..96 x K 16, A in tensor memory, B in shared memory);
 //     finishers 256 threads fold the chunk's accumulator into fp32 registers and, at the end of an item, apply the
 //               SwiGLU contract and store bf16 rows through the plan.
+//
+// What bounds a chunk (clock stamps of one CTA, c5 with 64 rows, gate/up): not the tensor pipe (8 %) nor DRAM, but the
+// expanders.  A warp of theirs holds a chunk for 2000 cycles and more -- its instructions go one by one through a pipe that
+// takes two cycles each (shifts, masks, conversions), satisfied waits cost 100 cycles -- while the packed bytes need 830.  So:
+// five of those instructions per packed word instead of seven, scales converted once per group, the waits' looks taken
+// together, and up to 16 token rows (whose accumulators leave room for a third stage) three sets of expanders, and finishers
+// that take alternate ITEMS, one set's epilogue under the other's folds.  us, gate/up and down, before -> now: c2 T=32
+// 80.5/48.2 -> 63.5/38.5 (2990 GB/s), c5 T=64 1107/585 -> 836/427 (4300 GB/s), c5 T=512 1369/706 -> 1209/618, c2 T=4096
+// 442/294 -> 407/292, mxfp4 c3 T=300 89/49 -> 75/42.  (Alternate items above 16 rows: the finishers' registers do not
+// suffice; with setmaxnreg c5 T=512 took 1595/667, c2 T=4096 485/351.  Four stages of half a chunk: twice the waits, a fifth
+// slower.  Scales prepared by warps of their own: 974/468 for c5 T=64.)
 //
 // Arithmetic.  Affine: w = q s + b = (q - 8) s + (b + 8 s).  q - 8 has three bits and a sign, s eight: their product fits
 // fp16's eleven, so the scale goes into the operand and the accumulator runs over several groups.  The second term is two
 // more K = 16 steps on one operand, per group (b, b, -8 s, -8 s), against the group's float32 sum X as three fp16 pieces (33
 // bits): (X1, X2, -X1, -X2) and (X3, 0, -X3, 0).  The scales are first multiplied by a power of two per (row, chunk), undone
 // in fp32 by the finishers, so the range of fp16 is no limit on the checkpoint's.
-// (q - 8) s is exact while the four scales of a row's chunk lie within 12 binades of the largest; chunks with scales
-// further apart are expanded another way (tm_expand_far), exact over 28; below, a weight is off by at most 2^-39 of the
-// largest of its row's chunk.  mxfp4: e2m1 value x 2^(e - emax + 13), exact in fp16 over 36 binades, same row factor.
+// (q - 8) s and b are exact while the scales and offsets of a row's chunk (other than zero) lie within 8 binades below the
+// largest scale; chunks with values further apart are expanded another way (tm_expand_far), exact over 28; below, a weight is
+// off by at most 2^-39 of the largest of its row's chunk.  mxfp4: e2m1 value x 2^(e - emax + 13), exact in fp16 over 36 binades, same row factor.
 // Token rows carry a power of two per row: a bfloat16 of the row is exact down to 2^-26 (mxfp4: 2^-31) of its largest,
 // and off by at most 2^-34 (2^-39) of it below.  Chunks are
 // summed in fp32 registers rather than in the accumulator over all of K, so that no sum is longer than 160 products (mxfp4:
@@ -45,8 +56,6 @@
 
 namespace zmoe {
 
-constexpr int kTmExp = 256, kTmFin = 256;
-constexpr int kTmThreads = kTmExp + kTmFin + 96;  // + one warp each: issuer, weight copies, token copies
 constexpr int kTmRows = 128;                      // tensor-memory lanes = weight rows of an item
 constexpr int kTmChunk = 256;                     // codes per chunk
 constexpr int kTmRaw = 5;                         // chunks of packed bytes in flight
@@ -57,7 +66,6 @@ constexpr int kTmMaxX = 8;                        // token stages, at most
 constexpr int kTmMaxTasks = 1024;
 constexpr int kTmItems = 256;                     // work items of a CTA kept in shared memory
 constexpr int kTmCols = 512;
-constexpr int kTmColD = 128;                      // columns between the two accumulators
 constexpr int kTmSplitTok = 48;                   // up to so many token rows an accumulator is two, one per half chunk
 // How a chunk is summed.  The tensor core cuts products and sums off at a fixed distance below the largest of them, so
 // long sums lose.  Share of bfloat16 results that are not the float64 result's rounding, affine, K = 768 and 2048: whole
@@ -66,7 +74,8 @@ constexpr int kTmSplitTok = 48;                   // up to so many token rows an
 // after the other, which costs 6 % (c2 with 4096 rows: 828 -> 879 us a block; quarters: 1090).  Products of e2m1 codes and
 // powers of two hardly lose any bits: whole chunks, 0.1e-4 to 0.6e-4.
 enum TmSum { kTmWhole, kTmSplit, kTmTurns };
-constexpr int kTmColA = 224, kTmAStage = 136;     // two A stages: 128 columns of codes, 8 of scales and biases
+constexpr int kTmAStage = 136;                    // columns of an operand stage: 128 of codes, 8 of scales and biases
+constexpr int kTmInv = 8;                         // chunks whose row factors are kept
 
 struct TmArgs {
   CUtensorMap w[2];  // packed bytes (E*N, K/2): box 128 bytes x 128 (gate and up: 64) rows
@@ -99,6 +108,15 @@ __device__ __forceinline__ bool tm_try(uint32_t bar, uint32_t parity, uint32_t n
                : "memory");
   return ok != 0;
 }
+// The same look without a suspension: a phase that is already complete costs less this way.
+__device__ __forceinline__ bool tm_test(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{ .reg .pred p; mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+               : "=r"(ok)
+               : "r"(bar), "r"(parity)
+               : "memory");
+  return ok != 0;
+}
 __device__ __forceinline__ unsigned long long tm_now() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -107,7 +125,7 @@ __device__ __forceinline__ unsigned long long tm_now() {
 // Waits for the phase; false when a second passed or, unless `drain`, another thread of the CTA gave up.  Suspended
 // looks rather than a spin: polling warps would take the issue slots that the expanders live on.  The patient part is
 // out of line: the roles' loops share one instruction cache.
-__device__ __noinline__ bool tm_wait_long(uint32_t bar, uint32_t parity, volatile int* abort_flag, bool drain) {
+__device__ __forceinline__ bool tm_wait_long(uint32_t bar, uint32_t parity, volatile int* abort_flag, bool drain) {
   const unsigned long long t0 = tm_now();
   while (true) {
     if (tm_try(bar, parity, 20000u)) return true;
@@ -119,14 +137,24 @@ __device__ __noinline__ bool tm_wait_long(uint32_t bar, uint32_t parity, volatil
   }
 }
 __device__ __forceinline__ bool tm_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, bool drain = false) {
-#pragma unroll 1
-  for (int i = 0; i < 8; ++i)
-    if (tm_try(bar, parity, 20000u)) return true;
+  if (tm_test(bar, parity)) return true;
   return tm_wait_long(bar, parity, abort_flag, drain);
 }
 // The same for a whole warp: all lanes leave together, as the tcgen05.ld and .st that follow need them to.
 __device__ __forceinline__ bool tm_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   return __all_sync(0xffffffffu, tm_wait(bar, parity, abort_flag));
+}
+// Two or three phases: both looks at once where all are complete.
+__device__ __forceinline__ bool tm_wait_both(uint32_t b0, uint32_t p0, uint32_t b1, uint32_t p1, volatile int* abort_flag) {
+  const bool t0 = tm_test(b0, p0), t1 = tm_test(b1, p1);
+  if (__all_sync(0xffffffffu, t0 && t1)) return true;
+  return tm_wait_warp(b0, p0, abort_flag) && tm_wait_warp(b1, p1, abort_flag);
+}
+__device__ __forceinline__ bool tm_wait_three(uint32_t b0, uint32_t p0, uint32_t b1, uint32_t p1, uint32_t b2, uint32_t p2,
+                                              volatile int* abort_flag) {
+  const bool t0 = tm_test(b0, p0), t1 = tm_test(b1, p1), t2 = tm_test(b2, p2);
+  if (__all_sync(0xffffffffu, t0 && t1 && t2)) return true;
+  return tm_wait_warp(b0, p0, abort_flag) && tm_wait_warp(b1, p1, abort_flag) && tm_wait_warp(b2, p2, abort_flag);
 }
 __device__ __forceinline__ void tm_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
   asm volatile(
@@ -174,6 +202,29 @@ __device__ __forceinline__ void tm_st16(uint32_t taddr, const uint32_t (&r)[16])
 __device__ __forceinline__ void tm_st2(uint32_t taddr, uint32_t r0, uint32_t r1) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1,%2};" ::"r"(taddr), "r"(r0), "r"(r1) : "memory");
 }
+__device__ __forceinline__ void tm_st8(uint32_t taddr, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3, uint32_t r4,
+                                       uint32_t r5, uint32_t r6, uint32_t r7) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r0), "r"(r1), "r"(r2),
+               "r"(r3), "r"(r4), "r"(r5), "r"(r6), "r"(r7)
+               : "memory");
+}
+__device__ __forceinline__ void tm_st32(uint32_t taddr, const uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,"
+      "%32};" ::"r"(taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]),
+      "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]),
+      "r"(r[30]), "r"(r[31])
+      : "memory");
+}
+// What the warp loaded from an accumulator is in registers: its owner may write the accumulator again.
+__device__ __forceinline__ void tm_release(uint32_t bar, int lane) {
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncwarp();
+  if (lane == 0) tm_arrive(bar);
+}
 // One lane of a converged warp.  The compiler knows an elected thread to be alone; behind `lane == 0` it would wrap
 // every tcgen05.mma and TMA instruction in a loop over the lanes that might be active (measured: 190 cycles per MMA
 // whatever its shape, 17 of them per chunk).
@@ -182,25 +233,27 @@ __device__ __forceinline__ bool tm_elect() {
   asm volatile("{ .reg .pred p; elect.sync _|p, 0xffffffff; selp.u32 %0, 1, 0, p; }" : "=r"(one));
   return one != 0;
 }
+// Halves that are zero become the largest number.
+__device__ __forceinline__ uint32_t tm_zero_as_max(uint32_t v) { return v | __vcmpeq2(v, 0u); }
 __device__ __forceinline__ uint32_t tm_bits(__half2 h) { return *reinterpret_cast<const uint32_t*>(&h); }
 __device__ __forceinline__ __half2 tm_half2(uint32_t u) { return *reinterpret_cast<const __half2*>(&u); }
 
 // Eight codes of a packed word times the group's scale, as four half2 in the order (0,4) (1,5) (2,6) (3,7) that the
-// token rows are written in.  A nibble at bits 4-7 of a half IS the fp16 number q 2^-20 (subnormal or not), so one
-// fused multiply-add gives q 2^-20 (s 2^20) - 8 s = (q - 8) s, exact: three shifts, four masks, four half2 operations
-// per eight codes.
-__device__ __forceinline__ void tm_expand_affine(uint32_t w, __half2 s20, __half2 m8s, uint32_t* out) {
-  const uint32_t m = 0x00F000F0u;
-  out[0] = tm_bits(__hfma2(tm_half2((w << 4) & m), s20, m8s));
-  out[1] = tm_bits(__hfma2(tm_half2(w & m), s20, m8s));
-  out[2] = tm_bits(__hfma2(tm_half2((w >> 4) & m), s20, m8s));
-  out[3] = tm_bits(__hfma2(tm_half2((w >> 8) & m), s20, m8s));
+// token rows are written in.  A nibble at bits 0-3 (4-7) of a half IS the fp16 number q 2^-24 (q 2^-20), subnormal or not, so
+// one fused multiply-add gives q 2^-24 (s 2^24) - 8 s = (q - 8) s, exact: one shift, four masks, four half2 operations per
+// eight codes.
+__device__ __forceinline__ void tm_expand_affine(uint32_t w, __half2 s24, __half2 s20, __half2 m8s, uint32_t* out) {
+  const uint32_t m = 0x000F000Fu, m4 = 0x00F000F0u, w8 = w >> 8;
+  out[0] = tm_bits(__hfma2(tm_half2(w & m), s24, m8s));
+  out[1] = tm_bits(__hfma2(tm_half2(w & m4), s20, m8s));
+  out[2] = tm_bits(__hfma2(tm_half2(w8 & m), s24, m8s));
+  out[3] = tm_bits(__hfma2(tm_half2(w8 & m4), s20, m8s));
 }
 // A chunk whose scales lie further apart than tm_expand_affine takes: a nibble at bits 6-9 of a half under the exponent of
 // 16 is 16 + q, and (16 + q) s - 24 s = (q - 8) s is exact for s from 2^-17 to 2^11 (24 s has ten bits).  One more shift and
 // four more masks per word: every chunk done this way cost 9 to 13 % (c2 with 32 rows 600 -> 657 us, c5 with 64 rows 1790
-// -> 2038), so it is a call for the warps that meet such a chunk.
-__device__ __noinline__ void tm_expand_far(const unsigned char* src, uint32_t swz, uint4 sc, float P, uint32_t taddr) {
+// -> 2038), so it is a loop of its own, for the warps that meet such a chunk.
+__device__ __forceinline__ void tm_expand_far(const unsigned char* src, uint32_t swz, uint4 sc, float P, uint32_t taddr) {
   const uint32_t m = 0x03C003C0u, sixteen = 0x4C004C00u;
 #pragma unroll 1
   for (int i = 0; i < 8; ++i) {  // 16 bytes: half a group
@@ -250,7 +303,7 @@ struct TmItem {
 };
 // Items are numbered task-major; inside a task the token blocks of one row tile are neighbours, so that they run at
 // the same time on different SMs and share the weights through L2.  prefix[a] = token blocks of the tasks before a.
-__device__ __noinline__ TmItem tm_item(const PlanView& pv, const int* prefix, int ntasks, int ntiles, int tile_rows,
+__device__ __forceinline__ TmItem tm_item(const PlanView& pv, const int* prefix, int ntasks, int ntiles, int tile_rows,
                                           int w) {
   int lo = 0, hi = ntasks - 1;
   while (lo < hi) {
@@ -270,38 +323,9 @@ __device__ __noinline__ TmItem tm_item(const PlanView& pv, const int* prefix, in
   return it;
 }
 
-// EPI: the SwiGLU contract of gate and up (QmmParams::epilogue).
-template <bool MX, int NMAT, int EPI, TmSum SUM>
-__global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_constant__ TmArgs a) {
-  extern __shared__ __align__(1024) unsigned char tm_dyn[];
-  __shared__ uint32_t tmem_base_s;
-  // raw full / empty, token full / empty, A full, MMAs done, accumulator free, accumulator full (kTmTurns)
-  __shared__ __align__(8) unsigned long long bars_s[2 * kTmRaw + 2 * kTmMaxX + 8];
-  __shared__ float inv_s[4][kTmRows];
-  __shared__ volatile int abort_s;
-  __shared__ int prefix_s[kTmMaxTasks + 1];
-  __shared__ int4 items_s[kTmItems];
-
-  constexpr int kTile = kTmRows / NMAT;  // output rows of an item
-  const QmmParams& p = a.q;
-  const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
-  const int N = p.N, nch = a.nch, tn = a.tn, rx = a.rx;
-  const PlanView pv = plan_view(const_cast<int*>(p.plan), p.rows, p.E);
-  unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tm_dyn) + 1023) & ~(uintptr_t)1023);
-  unsigned char* raw = base;
-  unsigned char* tok = raw + kTmRaw * kTmRawBytes;
-  unsigned char* scr = tok + rx * a.xstage;  // [slot][expander thread][16 bytes]
-  const uint32_t bars = tm_smem(bars_s);
-  const uint32_t b_rawf = bars, b_rawe = bars + 8 * kTmRaw, b_tokf = bars + 16 * kTmRaw;
-  const uint32_t b_toke = b_tokf + 8 * kTmMaxX, b_af = b_toke + 8 * kTmMaxX, b_done = b_af + 16, b_dfree = b_done + 16;
-  const uint32_t b_acc = b_dfree + 16;
-
-  // The plan, the prepared rows and their factors may be the work of the kernel before, still running when this one
-  // starts: they are read with plain loads after the wait, never through the read-only path.
-  pdl_wait();
-  pdl_trigger();
-  const int ntasks = min(pv.hdr[0], kTmMaxTasks);
-  if (wid == 0) {  // token blocks per task, prefix-summed (lane = a contiguous run of tasks)
+// Token blocks of at most tn rows before every task (the first warp computes them, the CTA waits).
+__device__ __forceinline__ void tm_block_prefix(const PlanView& pv, int ntasks, int tn, int wid, int lane, int* prefix) {
+  if (wid == 0) {  // lane = a contiguous run of tasks
     const int per = (ntasks + 31) >> 5;
     int sum = 0;
     for (int i = lane * per; i < min(ntasks, (lane + 1) * per); ++i) sum += (pv.tasks[4 * i + 2] + tn - 1) / tn;
@@ -313,20 +337,107 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
     }
     int run = incl - sum;
     for (int i = lane * per; i < min(ntasks, (lane + 1) * per); ++i) {
-      prefix_s[i] = run;
+      prefix[i] = run;
       run += (pv.tasks[4 * i + 2] + tn - 1) / tn;
     }
-    if (lane == 31) prefix_s[ntasks] = incl;
+    if (lane == 31) prefix[ntasks] = incl;
   }
   __syncthreads();
+}
+
+// The sums of weight row (q4, lane) and token rows t0 .. t0 + 15 of the item, times the rows' factors, through the
+// SwiGLU contract to the output.  xin, dst: row factor and output row of token t0 + lane % 16.
+// No branch between the values, so that their exponentials and divisions overlap: one after the other they held
+// both accumulators for 14,000 cycles per item of 96 rows, half of its time.
+template <int NMAT, int EPI>
+__device__ __forceinline__ void tm_store_block(const QmmParams& p, const TmItem& it, int q4, int lane, int t0,
+                                               const float (&acc)[16], float xin, int dst, int N) {
+  if (NMAT == 2) {
+    const int n = it.n0 + q4 * 16 + (lane & 15);
+    const bool hi = lane >= 16;  // the lower lanes finish the even tokens, the upper lanes the odd ones
+    __nv_bfloat16* out = p.out + n;
+    float gv[8], uv[8];
+    int row[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float other = __shfl_xor_sync(0xffffffffu, hi ? acc[2 * i] : acc[2 * i + 1], 16);
+      const float xs = __shfl_sync(0xffffffffu, xin, 2 * i + (hi ? 1 : 0));
+      row[i] = __shfl_sync(0xffffffffu, dst, 2 * i + (hi ? 1 : 0));
+      gv[i] = (hi ? other : acc[2 * i]) * xs;
+      uv[i] = (hi ? acc[2 * i + 1] : other) * xs;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) gv[i] = swiglu_epilogue(EPI, gv[i], uv[i]);
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (t0 + 2 * i + (hi ? 1 : 0) < it.nt && n < N) out[(size_t)row[i] * p.ldo] = __float2bfloat16_rn(gv[i]);
+  } else {
+    const int n = it.n0 + q4 * 32 + lane;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const float xs = __shfl_sync(0xffffffffu, xin, i);
+      const int row = __shfl_sync(0xffffffffu, dst, i);
+      if (t0 + i < it.nt && n < N) p.out[(size_t)row * p.ldo + n] = __float2bfloat16_rn(acc[i] * xs);
+    }
+  }
+}
+
+// Shapes of an instance.  NB: blocks of 16 token rows an item may have.  SUM: see above.  The accumulators are a ring of nD, a
+// chunk takes one of them or (kTmTurns) two; kTmSplit puts a chunk's two halves side by side into one.
+template <int NB, TmSum SUM>
+struct TmShape {
+  static constexpr int nE = NB == 1 ? 3 : 2;                               // sets of expanders, operand stages
+  static constexpr bool alt = NB == 1;                                     // finisher sets take every other item, or block of it
+  static constexpr int threads = 128 * nE + 256 + 128;                     // expanders, finishers, issuer and copiers
+  static constexpr int parts = SUM == kTmTurns ? 2 : 1;                    // hand-overs of accumulators per chunk
+  static constexpr int colD = (SUM == kTmSplit ? 2 : 1) * 16 * NB;        // columns of an accumulator
+  static constexpr int colA = kTmCols - nE * kTmAStage;                    // first operand column
+  static constexpr int nD = colA / colD > 4 ? 4 : colA / colD;
+  static constexpr int nJ = alt ? NB : (NB + 1) / 2;                       // blocks of a finisher
+  static_assert(nD >= 2 && nE + nD < kTmInv, "tensor memory, row factors in flight");
+};
+
+// EPI: the SwiGLU contract of gate and up (QmmParams::epilogue).
+template <bool MX, int NMAT, int EPI, int NB, TmSum SUM>
+__global__ void __launch_bounds__((TmShape<NB, SUM>::threads), 1) qmm_tma_kernel(const __grid_constant__ TmArgs a) {
+  using S = TmShape<NB, SUM>;
+  extern __shared__ __align__(1024) unsigned char tm_dyn[];
+  __shared__ uint32_t tmem_base_s;
+  // raw full / empty, token full / empty, A full, MMAs done, accumulator full (one per finisher set) / free
+  __shared__ __align__(8) unsigned long long bars_s[2 * kTmRaw + 2 * kTmMaxX + 2 * S::nE + 3 * S::nD];
+  __shared__ float inv_s[kTmInv][kTmRows];
+  __shared__ volatile int abort_s;
+  __shared__ int prefix_s[kTmMaxTasks + 1];
+  __shared__ int4 items_s[kTmItems];
+
+  constexpr int kTile = kTmRows / NMAT;  // output rows of an item
+  const QmmParams& p = a.q;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int wid = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const int N = p.N, nch = a.nch, tn = a.tn, rx = a.rx;
+  const PlanView pv = plan_view(const_cast<int*>(p.plan), p.rows, p.E);
+  unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tm_dyn) + 1023) & ~(uintptr_t)1023);
+  unsigned char* raw = base;
+  unsigned char* tok = raw + kTmRaw * kTmRawBytes;
+  unsigned char* scr = tok + rx * a.xstage;  // [slot][expander thread][16 bytes]
+  const uint32_t b_rawf = tm_smem(bars_s), b_rawe = b_rawf + 8 * kTmRaw, b_tokf = b_rawe + 8 * kTmRaw;
+  const uint32_t b_toke = b_tokf + 8 * kTmMaxX, b_af = b_toke + 8 * kTmMaxX, b_done = b_af + 8 * S::nE;
+  const uint32_t b_dfull = b_done + 8 * S::nE, b_dfree = b_dfull + 16 * S::nD;
+
+  // The plan, the prepared rows and their factors may be the work of the kernel before, still running when this one
+  // starts: they are read with plain loads after the wait, never through the read-only path.
+  pdl_wait();
+  pdl_trigger();
+  const int ntasks = min(pv.hdr[0], kTmMaxTasks);
+  tm_block_prefix(pv, ntasks, tn, wid, lane, prefix_s);
   const int ntiles = (N + kTile - 1) / kTile;
   const int total = ntiles * prefix_s[ntasks];
   if ((int)blockIdx.x >= total) return;  // before any tensor memory is taken
-  const int n_items = (total - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int n_items = __shfl_sync(0xffffffffu, (total - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x, 0);
   const int n_chunks = n_items * nch;
   // Every role walks the CTA's items: they are looked up once, by all threads (a search, two divisions and a load of
   // the task record took each role some 1500 cycles per item); a CTA with more of them looks the rest up as it goes.
-  for (int i = tid; i < min(n_items, kTmItems); i += kTmThreads) {
+  for (int i = tid; i < min(n_items, kTmItems); i += S::threads) {
     const TmItem it = tm_item(pv, prefix_s, ntasks, ntiles, kTile, (int)blockIdx.x + i * (int)gridDim.x);
     items_s[i] = make_int4(it.e, it.p0, it.nt, it.n0);
   }
@@ -335,22 +446,21 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
     const int4 v = items_s[i];
     return TmItem{v.x, v.y, v.z, v.w};
   };
-
   if (tid == 0) {
     for (int i = 0; i < kTmRaw; ++i) {
       tm_bar_init(b_rawf + 8 * i, 1);
-      tm_bar_init(b_rawe + 8 * i, kTmExp / 64);
+      tm_bar_init(b_rawe + 8 * i, 4);
     }
     for (int i = 0; i < kTmMaxX; ++i) {
       tm_bar_init(b_tokf + 8 * i, 1);
       tm_bar_init(b_toke + 8 * i, 1);
     }
-    for (int i = 0; i < 2; ++i) {
-      tm_bar_init(b_af + 8 * i, kTmExp / 64);
+    for (int i = 0; i < S::nE; ++i) {
+      tm_bar_init(b_af + 8 * i, 4);
       tm_bar_init(b_done + 8 * i, 1);
-      tm_bar_init(b_dfree + 8 * i, kTmFin / 32);
-      tm_bar_init(b_acc + 8 * i, 1);
     }
+    for (int i = 0; i < 2 * S::nD; ++i) tm_bar_init(b_dfull + 8 * i, 1);
+    for (int i = 0; i < S::nD; ++i) tm_bar_init(b_dfree + 8 * i, S::alt ? 4 : 8);
     abort_s = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -365,58 +475,56 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = tmem_base_s;
-  constexpr int kParts = SUM == kTmTurns ? 2 : 1;  // hand-overs per chunk
+  const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base_s, 0);
   volatile int* ab = &abort_s;
   bool ok = true;
 
-  if (wid < kTmExp / 32) {
+  const int q4 = wid & 3;
+  const int r = q4 * 32 + lane;  // tensor-memory lane
+  if (wid < 4 * S::nE) {
     // ================================================================== expanders: a weight row of every other chunk
-    const int q4 = wid & 3, set = wid >> 2;
-    const int r = q4 * 32 + lane;  // tensor-memory lane
+    const int set = wid >> 2;
     const int mat = NMAT == 2 ? (lane >> 4) : 0;
     const int rb = NMAT == 2 ? q4 * 16 + (lane & 15) : r;  // row inside the matrix's box
-    const uint32_t at = tmem + ((uint32_t)(q4 * 32) << 16) + kTmColA + set * kTmAStage;
+    const int swz = rb & 7;
+    const uint32_t at = tmem + ((uint32_t)(q4 * 32) << 16) + S::colA + set * kTmAStage;
     const unsigned char* my_raw = raw + mat * (kTile * 128) + rb * 128;
     unsigned char* my_sc = scr + tid * 16;
     // the cursor of the scale copies runs kTmScAhead of the thread's chunks ahead
     int f_item = 0, f_c = set, f_slot = 0;
-    bool f_new = true;
     const unsigned char *f_s = nullptr, *f_b = nullptr;
     auto fetch = [&] {
       while (f_c >= nch) {
         f_c -= nch;
         ++f_item;
-        f_new = true;
+        f_s = nullptr;
       }
       if (f_item < n_items) {
-        if (f_new) {
-          f_new = false;
+        if (f_s == nullptr) {
           const TmItem it = item_at(f_item);
           const size_t row = (size_t)it.e * N + min(it.n0 + rb, N - 1);  // clamped rows are computed, not stored
           // 8 bytes per chunk: four bfloat16 scales (biases) or eight e8m0 bytes
           f_s = reinterpret_cast<const unsigned char*>(p.s[mat]) + row * nch * 8;
           if (!MX) f_b = reinterpret_cast<const unsigned char*>(p.b[mat]) + row * nch * 8;
         }
-        unsigned char* dst = my_sc + f_slot * (kTmExp * 16);
+        unsigned char* dst = my_sc + f_slot * (128 * S::nE * 16);
         cp_async_8(dst, f_s + f_c * 8);
         if (!MX) cp_async_8(dst + 8, f_b + f_c * 8);
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
-      f_c += 2;
+      f_c += S::nE;
       f_slot = (f_slot + 1) % kTmScRing;
     };
 #pragma unroll 1
     for (int i = 0; i < kTmScAhead; ++i) fetch();
-    int rs = set, rph = 0, slot = 0;  // raw slot and its phase, scale slot
+    int rs = set, rph = 0, slot = 0, aph = 1;  // raw slot and its phase, scale slot, phase of the operand stage
 #pragma unroll 1
-    for (int c = set; c < n_chunks; c += 2) {
+    for (int c = set; c < n_chunks; c += S::nE) {
       fetch();
       asm volatile("cp.async.wait_group %0;" ::"n"(kTmScAhead) : "memory");
-      const uint4 sc = *reinterpret_cast<const uint4*>(my_sc + slot * (kTmExp * 16));
+      const uint4 sc = *reinterpret_cast<const uint4*>(my_sc + slot * (128 * S::nE * 16));
       slot = (slot + 1) % kTmScRing;
       // ---- the chunk's power of two
-      uint32_t s_lo = sc.x, s_hi = sc.y, b_lo = sc.z, b_hi = sc.w;  // shifted through, one group at a time
       float inv, P = 0.0f;
       int emax = 0;
       bool far = false;
@@ -427,61 +535,68 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
         inv = emax >= 255 ? __uint_as_float(0x7f800000u) : exp2f((float)(emax - 127 - 13));
       } else {
         // largest |s| and |b| (bits order like magnitudes), as bfloat16 bits
-        uint32_t ms = __vmaxu2(sc.x & 0x7fff7fffu, sc.y & 0x7fff7fffu);
-        uint32_t mb = __vmaxu2(sc.z & 0x7fff7fffu, sc.w & 0x7fff7fffu);
+        const uint32_t m15 = 0x7fff7fffu;
+        uint32_t ms = __vmaxu2(sc.x & m15, sc.y & m15);
+        uint32_t mb = __vmaxu2(sc.z & m15, sc.w & m15);
         ms = max(ms & 0xffffu, ms >> 16);
         mb = max(mb & 0xffffu, mb >> 16);
-        // 2^(140 - e) brings |s| below 2^-4 (so that s 2^20 stays below 2^16) and |b| below 2^14; a scale that this
-        // leaves below 2^-17 asks for the wider form, where |s| may reach 2^11
+        // 2^(140 - e) brings |s| below 2^-8 (so that s 2^24 stays below 2^16) and |b| below 2^14; a scale or an offset, other
+        // than zero, that this leaves below 2^-17 asks for the wider form, where |s| may reach 2^11 (so do scales at float's
+        // upper end)
         const int es = (int)(ms >> 7), eb = (int)(mb >> 7);
-        int e = max(es + 18, eb);
-        const uint32_t least = __vminu2(sc.x & 0x7fff7fffu, sc.y & 0x7fff7fffu);
-        far = __any_sync(0xffffffffu, (int)(min(least & 0xffffu, least >> 16) >> 7) + 30 < e);
+        int e = max(es + 22, eb);
+        const uint32_t least = __vminu2(__vminu2(tm_zero_as_max(sc.x & m15), tm_zero_as_max(sc.y & m15)),
+                                        __vminu2(tm_zero_as_max(sc.z & m15), tm_zero_as_max(sc.w & m15)));
+        far = __any_sync(0xffffffffu, (int)(min(least & 0xffffu, least >> 16) >> 7) + 30 < e || e > 253);
         if (far) e = max(es + 3, eb);
-        e = min(max(e, far ? 14 : 34), 253);
+        e = min(max(e, far ? 14 : 38), 253);
         P = __uint_as_float((uint32_t)(267 - e) << 23);
         inv = __uint_as_float((uint32_t)(e - 13) << 23);
       }
-      // ---- the stage is free once the MMAs of the thread's previous chunk are done
-      ok = tm_wait_warp(b_rawf + 8 * rs, rph, ab);
-      if (ok && c >= 2) ok = tm_wait_warp(b_done + 8 * set, ((c >> 1) - 1) & 1, ab);
+      // ---- the chunk is there, and the stage is free: the MMAs of the thread's previous chunk are done (at once the first time)
+      ok = tm_wait_both(b_rawf + 8 * rs, rph, b_done + 8 * set, aph, ab);
       if (!ok) break;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const unsigned char* src = my_raw + rs * kTmRawBytes;
-      uint4 wa = *reinterpret_cast<const uint4*>(src + ((rb & 7) << 4));
-      uint4 wb = *reinterpret_cast<const uint4*>(src + ((1 ^ (rb & 7)) << 4));
-      if (!MX && far) tm_expand_far(src, rb & 7, sc, P, at);
-#pragma unroll 1
-      for (int i = !MX && far ? 4 : 0; i < 4; ++i) {  // 64 codes each: a group, or two mxfp4 blocks.  Rolled: see tm_wait_long
-        const int nx = 2 * min(i + 1, 3);
-        const uint4 na = *reinterpret_cast<const uint4*>(src + ((nx ^ (rb & 7)) << 4));
-        const uint4 nb = *reinterpret_cast<const uint4*>(src + (((nx + 1) ^ (rb & 7)) << 4));
-        const uint32_t ws[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
-        uint32_t o[2][16];
-        if (MX) {
-          // fp16 2^(e - emax + 13) in both halves, subnormal ones included
-          const __half2 s0 = __float2half2_rn(__uint_as_float((uint32_t)max((int)(s_lo & 0xffu) - emax + 140, 0) << 23));
-          const __half2 s1 = __float2half2_rn(__uint_as_float((uint32_t)max((int)((s_lo >> 8) & 0xffu) - emax + 140, 0) << 23));
+      uint4 w[2];
+      w[0] = *reinterpret_cast<const uint4*>(src + (swz << 4));
+      w[1] = *reinterpret_cast<const uint4*>(src + ((1 ^ swz) << 4));
+      aph ^= 1;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (!MX && far) {
+        tm_expand_far(src, swz, sc, P, at);
+      } else {
+        const float P24 = P * 16777216.0f;
+        uint32_t bias[8];
 #pragma unroll
-          for (int k = 0; k < 8; ++k) tm_expand_mx(ws[k], k < 4 ? s0 : s1, o[k >> 2] + 4 * (k & 3));
-        } else {
-          const float s = __uint_as_float(s_lo << 16);
-          const __half2 s_op = __float2half2_rn(s * (P * 1048576.0f)), s_off = __float2half2_rn(s * (-8.0f * P));
+        for (int i = 0; i < 4; ++i) {  // 64 codes each: a group, or two mxfp4 blocks
+          uint32_t o[32];
+          const uint32_t ws[8] = {w[0].x, w[0].y, w[0].z, w[0].w, w[1].x, w[1].y, w[1].z, w[1].w};
+          if (i < 3) {
+            w[0] = *reinterpret_cast<const uint4*>(src + (((2 * i + 2) ^ swz) << 4));
+            w[1] = *reinterpret_cast<const uint4*>(src + (((2 * i + 3) ^ swz) << 4));
+          }
+          const uint32_t s2 = i < 2 ? sc.x : sc.y, b2 = i < 2 ? sc.z : sc.w;
+          if (MX) {
+            // fp16 2^(e - emax + 13) in both halves, subnormal ones included
+            const uint32_t ee = (i & 1) ? s2 >> 16 : s2;
+            const __half2 s0 = __float2half2_rn(__uint_as_float((uint32_t)max((int)(ee & 0xffu) - emax + 140, 0) << 23));
+            const __half2 s1 = __float2half2_rn(__uint_as_float((uint32_t)max((int)((ee >> 8) & 0xffu) - emax + 140, 0) << 23));
 #pragma unroll
-          for (int k = 0; k < 8; ++k) tm_expand_affine(ws[k], s_op, s_off, o[k >> 2] + 4 * (k & 3));
-          const __half2 b_op = __float2half2_rn(__uint_as_float(b_lo << 16) * P);
-          tm_st2(at + 128 + 2 * i, tm_bits(b_op), tm_bits(s_off));
-          b_lo = __funnelshift_r(b_lo, b_hi, 16);
-          b_hi >>= 16;
+            for (int k = 0; k < 8; ++k) tm_expand_mx(ws[k], k < 4 ? s0 : s1, o + 4 * k);
+          } else {
+            const __half2 s24 = __float2half2_rn(__uint_as_float((i & 1) ? s2 & 0xffff0000u : s2 << 16) * P24);
+            const __half2 s20 = __hmul2(s24, __float2half2_rn(0x1p-4f)), s_off = __hmul2(s24, __float2half2_rn(-0x1p-21f));
+#pragma unroll
+            for (int k = 0; k < 8; ++k) tm_expand_affine(ws[k], s24, s20, s_off, o + 4 * k);
+            const __half2 b_op = __float2half2_rn(__uint_as_float((i & 1) ? b2 & 0xffff0000u : b2 << 16) * P);
+            bias[2 * i] = tm_bits(b_op);
+            bias[2 * i + 1] = tm_bits(s_off);
+          }
+          tm_st32(at + i * 32, o);
         }
-        tm_st16(at + i * 32, o[0]);
-        tm_st16(at + i * 32 + 16, o[1]);
-        s_lo = __funnelshift_r(s_lo, s_hi, 16);
-        s_hi >>= 16;
-        wa = na;
-        wb = nb;
+        if (!MX) tm_st8(at + 128, bias[0], bias[1], bias[2], bias[3], bias[4], bias[5], bias[6], bias[7]);
       }
-      inv_s[c & 3][r] = inv;
+      inv_s[c & (kTmInv - 1)][r] = inv;  // the finishers are at most nE + nD chunks behind: the MMAs wait for them
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
@@ -490,210 +605,198 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
         tm_arrive(b_rawe + 8 * rs);
       }
       __syncwarp();
-      rs += 2;
+      rs += S::nE;
       if (rs >= kTmRaw) {
         rs -= kTmRaw;
         rph ^= 1;
       }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
-  } else if (wid < (kTmExp + kTmFin) / 32) {
-    // ================================================================== finishers: weight row x every other 16 tokens
-    const int q4 = wid & 3, ch = (wid - kTmExp / 32) >> 2;
-    const int r = q4 * 32 + lane;
-    const uint32_t lane_base = tmem + ((uint32_t)(q4 * 32) << 16);
-    float acc[3][16];
-    int c = 0;
+  } else if (wid < 4 * S::nE + 8) {
+    // ================================================================== finishers: a weight row of every other item (or block)
+    const int set = (wid >> 2) - S::nE;
+    const uint32_t lane_base = tmem + ((uint32_t)(q4 * 32) << 16), b_full = b_dfull + (S::alt ? 8 * S::nD * set : 0);
+    uint32_t phases = 0;  // of the set's barriers, one bit each
 #pragma unroll 1
-    for (int item = 0; item < n_items && ok; ++item) {
+    for (int item = S::alt ? set : 0; item < n_items && ok; item += S::alt ? 2 : 1) {
       const TmItem it = item_at(item);
-      int dst[3];     // output row and row factor of token 16 (ch + 2 j) + lane % 16
-      float xin[3];
+      float acc[S::nJ][16];  // of token block j, or set + 2 j
 #pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        const int t = 16 * (ch + 2 * j) + (lane & 15);
-        dst[j] = t < it.nt ? pv.row_dst[it.p0 + t] : 0;
-        xin[j] = t < it.nt ? a.xinv[it.p0 + t] : 0.0f;
+      for (int j = 0; j < S::nJ; ++j)
 #pragma unroll
         for (int i = 0; i < 16; ++i) acc[j][i] = 0.0f;
-      }
+      auto t0_of = [&](int j) { return 16 * (S::alt ? j : set + 2 * j); };
+      int c = item * nch;
+      int buf = (c * S::parts) % S::nD;
 #pragma unroll 1
-      for (int cc = 0; cc < nch * kParts; ++cc, ++c) {
-        const int buf = c & 1;
-        ok = tm_wait_warp((SUM == kTmTurns ? b_acc : b_done) + 8 * buf, (c >> 1) & 1, ab);
+      for (int cc = 0; cc < nch * S::parts; ++cc) {
+        ok = tm_wait_warp(b_full + 8 * buf, (phases >> buf) & 1, ab);
         if (!ok) break;
+        phases ^= 1u << buf;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const float inv = inv_s[(c / kParts) & 3][r];
-        const uint32_t at = lane_base + buf * kTmColD;
+        const float inv = inv_s[c & (kTmInv - 1)][r];
+        if (S::parts == 1 || (cc & 1)) ++c;
+        const uint32_t at = lane_base + buf * S::colD;
+        if (NB == 1) {  // both halves at once
+          float d[2][16];
+          tm_ld16(at, d[0]);
+          if (SUM == kTmSplit) tm_ld16(at + 16, d[1]);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          tm_release(b_dfree + 8 * buf, lane);
 #pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          if (16 * (ch + 2 * j) < it.nt) {
-            float d[16];
-            tm_ld16(at + 16 * (ch + 2 * j), d);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          for (int h = 0; h < (SUM == kTmSplit ? 2 : 1); ++h)
 #pragma unroll
-            for (int i = 0; i < 16; ++i) acc[j][i] = fmaf(d[i], inv, acc[j][i]);
-            if (SUM == kTmSplit) {
-              tm_ld16(at + kTmSplitTok + 16 * (ch + 2 * j), d);
-              asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            for (int i = 0; i < 16; ++i) acc[0][i] = fmaf(d[h][i], inv, acc[0][i]);
+        } else {
 #pragma unroll
-              for (int i = 0; i < 16; ++i) acc[j][i] = fmaf(d[i], inv, acc[j][i]);
+          for (int j = 0; j < S::nJ; ++j)
+            if (t0_of(j) < it.nt) {
+#pragma unroll
+              for (int h = 0; h < (SUM == kTmSplit ? 2 : 1); ++h) {
+                float d[16];
+                tm_ld16(at + h * 16 * NB + t0_of(j), d);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (int i = 0; i < 16; ++i) acc[j][i] = fmaf(d[i], inv, acc[j][i]);
+              }
             }
-          }
+          tm_release(b_dfree + 8 * buf, lane);
         }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) tm_arrive(b_dfree + 8 * buf);
+        if (++buf == S::nD) buf = 0;
       }
       if (!ok) break;
 #pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        const int t0 = 16 * (ch + 2 * j);
-        if (t0 >= it.nt) break;
-        // no branch between the values, so that their exponentials and divisions overlap: one after the other they held
-        // both accumulators for 14,000 cycles per item of 96 rows, half of its time
-        if (NMAT == 2) {
-          const int n = it.n0 + q4 * 16 + (lane & 15);
-          const bool hi = lane >= 16;  // the lower lanes finish the even tokens, the upper lanes the odd ones
-          __nv_bfloat16* out = p.out + n;
-          float gv[8], uv[8];
-          int row[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const float other = __shfl_xor_sync(0xffffffffu, hi ? acc[j][2 * i] : acc[j][2 * i + 1], 16);
-            const float xs = __shfl_sync(0xffffffffu, xin[j], 2 * i + (hi ? 1 : 0));
-            row[i] = __shfl_sync(0xffffffffu, dst[j], 2 * i + (hi ? 1 : 0));
-            gv[i] = (hi ? other : acc[j][2 * i]) * xs;
-            uv[i] = (hi ? acc[j][2 * i + 1] : other) * xs;
-          }
-#pragma unroll
-          for (int i = 0; i < 8; ++i) gv[i] = swiglu_epilogue(EPI, gv[i], uv[i]);
-#pragma unroll
-          for (int i = 0; i < 8; ++i)
-            if (t0 + 2 * i + (hi ? 1 : 0) < it.nt && n < N) out[(size_t)row[i] * p.ldo] = __float2bfloat16_rn(gv[i]);
-        } else {
-          const int n = it.n0 + r;
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const float xs = __shfl_sync(0xffffffffu, xin[j], i);
-            const int row = __shfl_sync(0xffffffffu, dst[j], i);
-            if (t0 + i < it.nt && n < N) p.out[(size_t)row * p.ldo + n] = __float2bfloat16_rn(acc[j][i] * xs);
-          }
+      for (int j = 0; j < S::nJ; ++j)
+        if (t0_of(j) < it.nt) {
+          const int t = it.p0 + min(t0_of(j) + (lane & 15), it.nt - 1);
+          tm_store_block<NMAT, EPI>(p, it, q4, lane, t0_of(j), acc[j], a.xinv[t], pv.row_dst[t], N);
         }
-      }
     }
-  } else if (wid == (kTmExp + kTmFin) / 32) {
-    // ================================================================== the warp that issues the MMAs (one lane does)
-    int c = 0, xs = 0, xph = 0, n_first = 0;  // n_first: first halves committed (kTmTurns)
+  } else {
+    if (wid == 4 * S::nE + 8) {
+      // ================================================================ the warp that issues the MMAs (one lane does)
+      int c = 0, xs = 0, xph = 0, as = 0, aph = 0, ds = 0, dph = 1;
+      uint32_t used = 0, last = 0;  // accumulator-full barriers committed to, and the parity of each one's latest phase
 #pragma unroll 1
-    for (int item = 0; item < n_items && ok; ++item) {
-      const TmItem it = item_at(item);
-      const uint32_t idesc = tm_idesc((it.nt + 15) & ~15);
+      for (int item = 0; item < n_items && ok; ++item) {
+        const int nt = __shfl_sync(0xffffffffu, item_at(item).nt, 0);
+        const uint32_t idesc = tm_idesc((nt + 15) & ~15);
+        const int first_full = S::alt ? (item & 1) * S::nD : 0;
 #pragma unroll 1
-      for (int cc = 0; cc < nch; ++cc, ++c) {
-        const int buf = c & 1;
-        ok = tm_wait_warp(b_tokf + 8 * xs, xph, ab);
-        if (ok && SUM != kTmTurns && c >= 2) ok = tm_wait_warp(b_dfree + 8 * buf, ((c >> 1) - 1) & 1, ab);
-        if (ok) ok = tm_wait_warp(b_af + 8 * buf, (c >> 1) & 1, ab);
-        if (ok && SUM == kTmTurns && c >= 1) ok = tm_wait_warp(b_dfree, (c - 1) & 1, ab);
-        if (!ok) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t d = tmem + (SUM == kTmTurns ? 0 : buf * kTmColD), at = tmem + kTmColA + buf * kTmAStage;
-        const uint32_t d2 = SUM == kTmWhole ? d : d + (SUM == kTmSplit ? kTmSplitTok : kTmColD);  // the chunk's second half
-        const uint32_t bt = tm_smem(tok + xs * a.xstage);
-        auto half = [&](int h) {
+        for (int cc = 0; cc < nch; ++cc, ++c) {
+          const uint32_t at = tmem + S::colA + as * kTmAStage;
+          ok = tm_wait_three(b_tokf + 8 * xs, xph, b_dfree + 8 * ds, dph, b_af + 8 * as, aph, ab);  // an accumulator is free at
+          if (!ok) break;                                                                          // once the first time round
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t bt = tm_smem(tok) + xs * a.xstage;
+          auto half = [&](uint32_t d, int h) {
 #pragma unroll
-          for (int g = 2 * h; g < 2 * h + 2; ++g) {
-            const uint64_t bd = tm_desc128(bt + g * tn * 128);
+            for (int g = 2 * h; g < 2 * h + 2; ++g) {
+              const uint64_t bd = tm_desc128(bt + g * tn * 128);
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
-              tm_mma(h ? d2 : d, at + g * 32 + k * 8, bd + 2 * k, idesc, k != 0 || (g & 1) != 0 || (h == 1 && SUM == kTmWhole));
+              for (int k = 0; k < 4; ++k)
+                tm_mma(d, at + g * 32 + k * 8, bd + 2 * k, idesc, k != 0 || (g & 1) != 0 || (h == 1 && SUM == kTmWhole));
+            }
+          };
+          auto next = [&] {  // the ring's next accumulator
+            const int full = first_full + ds;
+            last = ((last ^ (used & (1u << full))) & (1u << full)) | (last & ~(1u << full));
+            used |= 1u << full;
+            if (++ds == S::nD) {
+              ds = 0;
+              dph ^= 1;
+            }
+          };
+          if (SUM == kTmTurns) {
+            if (tm_elect()) {
+              half(tmem + ds * S::colD, 0);
+              tm_commit(b_dfull + 8 * (first_full + ds));
+            }
+            __syncwarp();
+            next();
+            ok = tm_wait_warp(b_dfree + 8 * ds, dph, ab);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           }
-        };
-        if (SUM == kTmTurns) {
+          const uint32_t d = tmem + ds * S::colD, d2 = SUM == kTmSplit ? d + 16 * NB : d;
           if (tm_elect()) {
-            half(0);
-            tm_commit(b_acc);
+            if (SUM != kTmTurns) half(d, 0);
+            half(d2, 1);
+            if (!MX) {  // the sums' first two pieces, and their third
+              const uint64_t bx = tm_desc64(bt + tn * 512);
+              tm_mma(d2, at + 128, bx, idesc, true);
+              tm_mma(d2, at + 128, bx + 2, idesc, true);
+            }
+            tm_commit(b_dfull + 8 * (first_full + ds));
+            tm_commit(b_done + 8 * as);
+            tm_commit(b_toke + 8 * xs);
           }
           __syncwarp();
-          ++n_first;
-          if (c >= 1) ok = tm_wait_warp(b_dfree + 8, (c - 1) & 1, ab);
+          next();
+          if (++as == S::nE) {
+            as = 0;
+            aph ^= 1;
+          }
+          if (++xs == rx) {
+            xs = 0;
+            xph ^= 1;
+          }
+        }
+      }
+      // MMAs in flight, and the arrivals they still owe
+      for (int i = 0; i < 2 * S::nD; ++i)
+        if ((used >> i) & 1) tm_wait(b_dfull + 8 * i, (last >> i) & 1, ab, true);
+      for (int i = max(c - S::nE, 0); i < c; ++i) tm_wait(b_done + 8 * (i % S::nE), (i / S::nE) & 1, ab, true);
+      for (int i = max(c - rx, 0); i < c; ++i) tm_wait(b_toke + 8 * (i % rx), (i / rx) & 1, ab, true);
+    } else if (wid == 4 * S::nE + 9) {
+      // ================================================================ the warp that copies packed weights
+      int c = 0;
+#pragma unroll 1
+      for (int item = 0; item < n_items && ok; ++item) {
+        const TmItem it = item_at(item);
+        const int y = it.e * N + it.n0;  // a tile's rows beyond N are the next expert's: computed, not stored
+#pragma unroll 1
+        for (int cc = 0; cc < nch; ++cc, ++c) {
+          const int rs = c % kTmRaw;
+          if (c >= kTmRaw) ok = tm_wait_warp(b_rawe + 8 * rs, (c / kTmRaw - 1) & 1, ab);
           if (!ok) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        }
-        if (tm_elect()) {
-          if (SUM != kTmTurns) half(0);
-          half(1);
-          if (!MX) {  // the sums' first two pieces, and their third
-            tm_mma(d2, at + 128, tm_desc64(bt + tn * 512), idesc, true);
-            tm_mma(d2, at + 128, tm_desc64(bt + tn * 512) + 2, idesc, true);
-          }
-          if (SUM == kTmTurns) tm_commit(b_acc + 8);
-          tm_commit(b_done + 8 * buf);
-          tm_commit(b_toke + 8 * xs);
-        }
-        __syncwarp();
-        if (++xs == rx) {
-          xs = 0;
-          xph ^= 1;
-        }
-      }
-    }
-    // MMAs in flight, and the arrivals they still owe
-    if (SUM == kTmTurns) {
-      if (n_first > 0) tm_wait(b_acc, (n_first - 1) & 1, ab, true);
-      if (c > 0) tm_wait(b_acc + 8, (c - 1) & 1, ab, true);
-    }
-    for (int i = max(c - 2, 0); i < c; ++i) tm_wait(b_done + 8 * (i & 1), (i >> 1) & 1, ab, true);
-    for (int i = max(c - rx, 0); i < c; ++i) tm_wait(b_toke + 8 * (i % rx), (i / rx) & 1, ab, true);
-  } else if (wid == (kTmExp + kTmFin) / 32 + 1) {
-    // ================================================================== the warp that copies packed weights
-    int c = 0;
-#pragma unroll 1
-    for (int item = 0; item < n_items && ok; ++item) {
-      const TmItem it = item_at(item);
-      const int y = it.e * N + it.n0;  // a tile's rows beyond N are the next expert's: computed, not stored
-#pragma unroll 1
-      for (int cc = 0; cc < nch; ++cc, ++c) {
-        const int rs = c % kTmRaw;
-        if (c >= kTmRaw) ok = tm_wait_warp(b_rawe + 8 * rs, (c / kTmRaw - 1) & 1, ab);
-        if (!ok) break;
-        const uint32_t bar = b_rawf + 8 * rs, dst = tm_smem(raw + rs * kTmRawBytes);
-        if (tm_elect()) {
-          tm_expect(bar, kTmRawBytes);
+          const uint32_t bar = b_rawf + 8 * rs, to = tm_smem(raw + rs * kTmRawBytes);
+          if (tm_elect()) {
+            tm_expect(bar, kTmRawBytes);
 #pragma unroll
-          for (int m = 0; m < NMAT; ++m) tm_load_2d(dst + m * (kTile * 128), &a.w[m], cc * 128, y, bar);
-        }
-        __syncwarp();
-      }
-    }
-    for (int i = max(c - kTmRaw, 0); i < c; ++i) tm_wait(b_rawf + 8 * (i % kTmRaw), (i / kTmRaw) & 1, ab, true);
-  } else {
-    // ================================================================== the warp that copies token tiles
-    int c = 0;
-#pragma unroll 1
-    for (int item = 0; item < n_items && ok && !p.withhold; ++item) {
-      const TmItem it = item_at(item);
-      const int nb = (it.nt + 15) >> 4;
-#pragma unroll 1
-      for (int cc = 0; cc < nch; ++cc, ++c) {
-        const int xs = c % rx;
-        if (c >= rx) ok = tm_wait_warp(b_toke + 8 * xs, (c / rx - 1) & 1, ab);
-        if (!ok) break;
-        const uint32_t bar = b_tokf + 8 * xs, dst = tm_smem(tok + xs * a.xstage);
-        if (tm_elect()) {
-          tm_expect(bar, nb * (MX ? 8192 : 8192 + 1024));
-          for (int b = 0; b < nb; ++b) {
-#pragma unroll
-            for (int g = 0; g < 4; ++g)
-              tm_load_2d(dst + g * tn * 128 + b * 2048, &a.x, cc * kTmChunk + g * 64, it.p0 + 16 * b, bar);
-            if (!MX) tm_load_2d(dst + tn * 512 + b * 1024, &a.xb, cc * 32, it.p0 + 16 * b, bar);
+            for (int m = 0; m < NMAT; ++m) tm_load_2d(to + m * (kTile * 128), &a.w[m], cc * 128, y, bar);
           }
+          __syncwarp();
         }
-        __syncwarp();
       }
+      for (int i = max(c - kTmRaw, 0); i < c; ++i) tm_wait(b_rawf + 8 * (i % kTmRaw), (i / kTmRaw) & 1, ab, true);
+    } else if (wid == 4 * S::nE + 10) {
+      // ================================================================ the warp that copies token tiles
+      int c = 0;
+#pragma unroll 1
+      for (int item = 0; item < n_items && ok && !p.withhold; ++item) {
+        const TmItem it = item_at(item);
+        const int nb = (it.nt + 15) >> 4;
+#pragma unroll 1
+        for (int cc = 0; cc < nch; ++cc, ++c) {
+          const int xs = c % rx;
+          if (c >= rx) ok = tm_wait_warp(b_toke + 8 * xs, (c / rx - 1) & 1, ab);
+          if (!ok) break;
+          const uint32_t bar = b_tokf + 8 * xs, to = tm_smem(tok + xs * a.xstage);
+          if (tm_elect()) {
+            tm_expect(bar, nb * (MX ? 8192 : 8192 + 1024));
+            for (int b = 0; b < nb; ++b) {
+#pragma unroll
+              for (int g = 0; g < 4; ++g)
+                tm_load_2d(to + g * tn * 128 + b * 2048, &a.x, cc * kTmChunk + g * 64, it.p0 + 16 * b, bar);
+              if (!MX) tm_load_2d(to + tn * 512 + b * 1024, &a.xb, cc * 32, it.p0 + 16 * b, bar);
+            }
+          }
+          __syncwarp();
+        }
+      }
+      for (int i = max(c - rx, 0); i < c; ++i) tm_wait(b_tokf + 8 * (i % rx), (i / rx) & 1, ab, true);
     }
-    for (int i = max(c - rx, 0); i < c; ++i) tm_wait(b_tokf + 8 * (i % rx), (i / rx) & 1, ab, true);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -702,7 +805,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) qmm_tma_kernel(const __grid_con
     if (tid == 0) atomicExch(pv.hdr + 2, kPlanTimeout);
     for (int i = 0; i < n_items; ++i) {
       const TmItem it = item_at(i);
-      for (int j = tid; j < it.nt * kTile; j += kTmThreads) {
+      for (int j = tid; j < it.nt * kTile; j += S::threads) {
         const int n = it.n0 + j % kTile;
         if (n < N) p.out[(size_t)pv.row_dst[it.p0 + j / kTile] * p.ldo + n] = __float2bfloat16_rn(__int_as_float(0x7fc00000));
       }
@@ -839,10 +942,12 @@ static bool map_2d(CUtensorMap* m, CUtensorMapDataType dt, const void* ptr, size
 
 template <bool MX, int NMAT, int EPI>
 static int launch_tma(const TmArgs& a, int grid, size_t smem, cudaStream_t st, const char* who) {
-  auto kern = a.tn <= kTmSplitTok ? qmm_tma_kernel<MX, NMAT, EPI, kTmSplit>
-                                  : qmm_tma_kernel<MX, NMAT, EPI, MX ? kTmWhole : kTmTurns>;
+  auto kern = a.tn <= 16            ? qmm_tma_kernel<MX, NMAT, EPI, 1, kTmSplit>
+              : a.tn <= kTmSplitTok ? qmm_tma_kernel<MX, NMAT, EPI, 3, kTmSplit>
+                                    : qmm_tma_kernel<MX, NMAT, EPI, 6, MX ? kTmWhole : kTmTurns>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess) e = launch_pdl(kern, dim3(grid), dim3(kTmThreads), smem, st, a);
+  const int threads = a.tn <= 16 ? TmShape<1, kTmSplit>::threads : TmShape<3, kTmSplit>::threads;
+  if (e == cudaSuccess) e = launch_pdl(kern, dim3(grid), dim3(threads), smem, st, a);
   if (e != cudaSuccess) return fail(ZMOE_ERR_CUDA, "%s: launch failed: %s", who, cudaGetErrorString(e));
   return check_launch("qmm_tma_kernel");
 }
@@ -877,8 +982,8 @@ int qmm_tma_launch(const QmmParams& q, int nmat, bool mx, int rows_hint, int max
   tn = (tn + 15) / 16 * 16;
   a.tn = tn > kTmMaxTok ? kTmMaxTok : (int)tn;
   a.xstage = (a.tn * (mx ? 512 : 576) + 1023) & ~1023;
-  const int fixed = 1024 + kTmRaw * kTmRawBytes + kTmScRing * kTmExp * 16;
-  const int room = 227 * 1024 - 12 * 1024 - fixed;  // 12 KB: the static part (prefix sums, items, barriers, row factors)
+  const int fixed = 1024 + kTmRaw * kTmRawBytes + kTmScRing * 128 * (a.tn <= 16 ? 3 : 2) * 16;
+  const int room = 227 * 1024 - 14 * 1024 - fixed;  // 14 KB: the static part (prefix sums, items, barriers, row factors)
   a.rx = room / a.xstage > kTmMaxX ? kTmMaxX : room / a.xstage;
   const size_t smem = (size_t)fixed + (size_t)a.rx * a.xstage;
   int sms = 0, dev = 0;
