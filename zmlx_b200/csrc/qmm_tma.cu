@@ -823,7 +823,7 @@ __global__ void __launch_bounds__((TmShape<NB, SUM>::threads), 1) qmm_tma_kernel
 // (X3, 0, -X3, 0).  Affine rows take the order in which tm_expand_affine leaves codes.
 constexpr int kPrepThreads = 128;
 
-template <bool MX>
+template <bool MX, int R>
 __global__ void __launch_bounds__(kPrepThreads) prep_rows_kernel(const __nv_bfloat16* x, int ldx, const int* plan,
                                                                  int rows, int E, int x_by_dst, int K, __half* xs,
                                                                  float* xinv) {
@@ -836,13 +836,18 @@ __global__ void __launch_bounds__(kPrepThreads) prep_rows_kernel(const __nv_bflo
   const int src = x_by_dst ? pv.row_dst[pos] : pv.row_src[pos];
   const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)src * ldx);
   const int nv = K >> 3;
+  uint4 keep[R];  // the thread's first R pieces; more are read twice
   uint32_t mx = 0;
-  for (int i = tid; i < nv; i += kPrepThreads) {
-    const uint4 v = xr[i];
+  auto look = [&](const uint4& v) {
     const uint32_t q[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
     for (int k = 0; k < 4; ++k) mx = max(mx, max(q[k] & 0x7fffu, (q[k] >> 16) & 0x7fffu));
-  }
+  };
+#pragma unroll
+  for (int j = 0; j < R; ++j) keep[j] = tid + j * kPrepThreads < nv ? xr[tid + j * kPrepThreads] : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+  for (int j = 0; j < R; ++j) look(keep[j]);
+  for (int i = tid + R * kPrepThreads; i < nv; i += kPrepThreads) look(xr[i]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   if ((tid & 31) == 0) warp_max[tid >> 5] = mx;
@@ -855,8 +860,7 @@ __global__ void __launch_bounds__(kPrepThreads) prep_rows_kernel(const __nv_bflo
   if (tid == 0) xinv[pos] = __uint_as_float((uint32_t)(254 - ef) << 23);
   const size_t stride = MX ? (size_t)K : (size_t)K + K / 8;
   __half* row = xs + (size_t)pos * stride;
-  for (int i = tid; i < nv; i += kPrepThreads) {  // nv is a multiple of 32: a warp is whole or absent
-    const uint4 v = xr[i];
+  auto write = [&](int i, const uint4& v) {
     const uint32_t q[4] = {v.x, v.y, v.z, v.w};
     float f[8];
 #pragma unroll
@@ -889,7 +893,12 @@ __global__ void __launch_bounds__(kPrepThreads) prep_rows_kernel(const __nv_bflo
         to[4] = make_uint2(x3, x3 ^ 0x80008000u);
       }
     }
-  }
+  };
+  // nv is a multiple of 32: a warp is whole or absent
+#pragma unroll
+  for (int j = 0; j < R; ++j)
+    if (tid + j * kPrepThreads < nv) write(tid + j * kPrepThreads, keep[j]);
+  for (int i = tid + R * kPrepThreads; i < nv; i += kPrepThreads) write(i, xr[i]);
 }
 
 // ------------------------------------------------------------------ host side
@@ -990,11 +999,11 @@ int qmm_tma_launch(const QmmParams& q, int nmat, bool mx, int rows_hint, int max
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
     return fail(ZMOE_ERR_CUDA, "%s: SM count query failed", who);
-  cudaError_t e =
-      mx ? launch_pdl(prep_rows_kernel<true>, dim3(q.rows), dim3(kPrepThreads), 0, st, q.x, q.ldx, q.plan, q.rows, q.E,
-                      q.x_by_dst, q.K, (__half*)xs, xinv)
-         : launch_pdl(prep_rows_kernel<false>, dim3(q.rows), dim3(kPrepThreads), 0, st, q.x, q.ldx, q.plan, q.rows, q.E,
-                      q.x_by_dst, q.K, (__half*)xs, xinv);
+  // rows of up to 2048 (8192) values stay in registers between their largest value and their conversion
+  auto prep = q.K <= 2048 ? (mx ? prep_rows_kernel<true, 2> : prep_rows_kernel<false, 2>)
+                          : (mx ? prep_rows_kernel<true, 8> : prep_rows_kernel<false, 8>);
+  cudaError_t e = launch_pdl(prep, dim3(q.rows), dim3(kPrepThreads), 0, st, q.x, q.ldx, q.plan, q.rows, q.E, q.x_by_dst, q.K,
+                             (__half*)xs, xinv);
   if (e != cudaSuccess) return fail(ZMOE_ERR_CUDA, "%s: launch failed: %s", who, cudaGetErrorString(e));
   // one CTA per SM, fewer when the work list is shorter
   const long long ntiles = (q.N * (long long)nmat + kTmRows - 1) / kTmRows;

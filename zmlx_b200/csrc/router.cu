@@ -25,7 +25,7 @@ __global__ void __launch_bounds__(128) softmax_topk_kernel(const void* __restric
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= T) return;
   softmax_topk_row<VPL>(logits, dtype, row, E, K, flavour, bias, renorm, weights, indices, lane,
-                        topk_sm + (size_t)(threadIdx.x >> 5) * (E + 2 * kMaxK));
+                        topk_sm + (size_t)(threadIdx.x >> 5) * E);
 }
 
 
@@ -42,7 +42,7 @@ __global__ void __launch_bounds__(128) sigmoid_topk_kernel(const void* __restric
   const int row = blockIdx.x * (blockDim.x >> 5) + wid;
   if (row >= T) return;
   sigmoid_topk_row<VPL>(logits, dtype, row, E, K, bias, n_group, topk_group, scale, weights, indices, lane,
-                        sm + (size_t)wid * (2 * E + 64 + 2 * kMaxK));
+                        sm + (size_t)wid * (E + 64));
 }
 
 // Router linear.  One warp per (expert, token tile of 8): 16-byte loads of the expert's weight row, the
@@ -77,54 +77,68 @@ __global__ void __launch_bounds__(128) router_logits_kernel(const __nv_bfloat16*
   }
 }
 
-// Router linear for many rows, on the tensor cores: a CTA owns 16 tokens x 32 experts, its eight warps take every
-// eighth block of 32 along d and their fp32 sums are added in warp order.  Both operands are read straight into
+// Router linear for many rows, on the tensor cores: a CTA owns 16 MT tokens x 8 NT experts, its eight warps take every
+// eighth block of 32 along d and their fp32 sums are added in warp order, the same order for every tile.  Both operands are
+// read straight into
 // mma fragments, 16 bytes per lane: a lane's eight consecutive values serve as the K pairs of two mma steps, the
 // same permutation of K on both sides.  Products of bfloat16 are exact in fp32, so this is the same sum as the warp
 // form above in another order.  The warp form spends three instructions per product on widening and adding, and one
 // warp walks all of d: bound by latency at tens of rows and by issue from hundreds on (c2, cold: 16 us for 16 rows, 31
 // us for 300).  Up to eight rows keep it: the one-launch block has the same order, and both give the same bits.
-constexpr int kRtTok = 16, kRtExp = 32, kRtWarps = 8;
+// Tiles: what bounds few rows is one CTA's walk along d (one round trip per turn of the loop), so tiles of 16 x 8 spread them
+// over the SMs and four turns' loads are in flight; what bounds many rows is the way of both operands from L2, so tiles
+// of 32 x 32 halve the router rows' share.  us, one tile of 16 x 32 with two turns in flight -> now: d 7168, 256 experts, 64
+// rows 13.9 -> 8.0; d 2048, 128 experts, 32 rows 5.2 -> 3.4, 1500 rows 8.1 -> 8.2, 4096 rows 19.6 -> 14.7.
+constexpr int kRtWarps = 8;
 
+template <int MT, int NT>
 __global__ void __launch_bounds__(32 * kRtWarps) router_logits_mma_kernel(const __nv_bfloat16* x,
                                                                           const __nv_bfloat16* __restrict__ wr, int T,
                                                                           int E, int d, void* __restrict__ logits,
                                                                           int out_dtype) {
-  __shared__ float part[kRtWarps][kRtTok][kRtExp + 1];
+  __shared__ float part[kRtWarps][16 * MT][8 * NT + 1];
   pdl_wait();
   pdl_trigger();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, g = lane >> 2, tig = lane & 3;
-  const int t0 = blockIdx.y * kRtTok, e0 = blockIdx.x * kRtExp;
-  const uint4* xa = reinterpret_cast<const uint4*>(x + (size_t)min(t0 + g, T - 1) * d) + tig;
-  const uint4* xb = reinterpret_cast<const uint4*>(x + (size_t)min(t0 + g + 8, T - 1) * d) + tig;
-  const uint4* wp[4];
+  const int t0 = blockIdx.y * 16 * MT, e0 = blockIdx.x * 8 * NT;
+  const uint4* xp[2 * MT];
 #pragma unroll
-  for (int n = 0; n < 4; ++n) wp[n] = reinterpret_cast<const uint4*>(wr + (size_t)min(e0 + 8 * n + g, E - 1) * d) + tig;
-  float acc[4][4];
+  for (int m = 0; m < 2 * MT; ++m) xp[m] = reinterpret_cast<const uint4*>(x + (size_t)min(t0 + g + 8 * m, T - 1) * d) + tig;
+  const uint4* wp[NT];
 #pragma unroll
-  for (int n = 0; n < 4; ++n)
+  for (int n = 0; n < NT; ++n) wp[n] = reinterpret_cast<const uint4*>(wr + (size_t)min(e0 + 8 * n + g, E - 1) * d) + tig;
+  float acc[MT][NT][4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[n][j] = 0.0f;
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[m][n][j] = 0.0f;
   const int nblk = d >> 5;
-#pragma unroll 2
+#pragma unroll(MT == 1 ? 4 : 2)
   for (int b = wid; b < nblk; b += kRtWarps) {
-    const uint4 va = xa[b * 4], vb = xb[b * 4];
-    uint4 vw[4];
+    uint4 vx[2 * MT], vw[NT];
 #pragma unroll
-    for (int n = 0; n < 4; ++n) vw[n] = __ldg(wp[n] + b * 4);
+    for (int m = 0; m < 2 * MT; ++m) vx[m] = xp[m][b * 4];
 #pragma unroll
-    for (int n = 0; n < 4; ++n) {
-      mma_bf16_m16n8k16(acc[n], va.x, vb.x, va.y, vb.y, vw[n].x, vw[n].y);
-      mma_bf16_m16n8k16(acc[n], va.z, vb.z, va.w, vb.w, vw[n].z, vw[n].w);
-    }
+    for (int n = 0; n < NT; ++n) vw[n] = __ldg(wp[n] + b * 4);
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+        mma_bf16_m16n8k16(acc[m][n], vx[2 * m].x, vx[2 * m + 1].x, vx[2 * m].y, vx[2 * m + 1].y, vw[n].x, vw[n].y);
+        mma_bf16_m16n8k16(acc[m][n], vx[2 * m].z, vx[2 * m + 1].z, vx[2 * m].w, vx[2 * m + 1].w, vw[n].z, vw[n].w);
+      }
   }
 #pragma unroll
-  for (int n = 0; n < 4; ++n)
+  for (int m = 0; m < MT; ++m)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) part[wid][g + 8 * (j >> 1)][8 * n + 2 * tig + (j & 1)] = acc[n][j];
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) part[wid][16 * m + g + 8 * (j >> 1)][8 * n + 2 * tig + (j & 1)] = acc[m][n][j];
   __syncthreads();
-  for (int i = threadIdx.x; i < kRtTok * kRtExp; i += 32 * kRtWarps) {
-    const int t = i / kRtExp, e = i - t * kRtExp;
+  for (int i = threadIdx.x; i < 128 * MT * NT; i += 32 * kRtWarps) {
+    const int t = i / (8 * NT), e = i - t * (8 * NT);
     if (t0 + t < T && e0 + e < E) {
       float v = part[0][t][e];
 #pragma unroll
@@ -188,11 +202,11 @@ __global__ void __launch_bounds__(128) route_fused_kernel(const RouteParams p) {
   for (int row = wid; row < T; row += 4) {
     if (p.family == 2)
       sigmoid_topk_row<VPL>(p.logits, ZMOE_BF16, row, E, p.K, p.bias, p.n_group, p.topk_group, p.scale, p.weights,
-                            p.indices, lane, scratch + (size_t)wid * (2 * E + 64 + 2 * kMaxK));
+                            p.indices, lane, scratch + (size_t)wid * (E + 64));
     else
       softmax_topk_row<VPL>(p.logits, ZMOE_BF16, row, E, p.K,
                             p.family == 0 ? ZMOE_ROUTER_TOPK_THEN_SOFTMAX : ZMOE_ROUTER_SOFTMAX_THEN_TOPK, p.bias,
-                            p.renorm, p.weights, p.indices, lane, scratch + (size_t)wid * (2 * E + 64 + 2 * kMaxK));
+                            p.renorm, p.weights, p.indices, lane, scratch + (size_t)wid * (E + 64));
   }
   __syncthreads();
   // ---- phase 3: plan over the (token, slot) pairs; pair p reads token row p / K
@@ -233,7 +247,7 @@ int zmoe_router_softmax_topk(const void* logits, int logits_dtype, int T, int E,
   dim3 grid((T + 3) / 4), block(128);
   cudaStream_t st = (cudaStream_t)stream;
   dispatch_vpl(E, [&](auto vpl) {
-    launch_pdl(softmax_topk_kernel<decltype(vpl)::value>, grid, block, 4 * (size_t)(E + 2 * kMaxK) * sizeof(float), st, logits, logits_dtype, T, E, K, flavour,
+    launch_pdl(softmax_topk_kernel<decltype(vpl)::value>, grid, block, 4 * (size_t)E * sizeof(float), st, logits, logits_dtype, T, E, K, flavour,
                bias, renorm, weights, indices);
     return 0;
   });
@@ -258,7 +272,7 @@ int zmoe_router_sigmoid_bias_topk(const void* logits, int logits_dtype, int T, i
                "zmoe_router_sigmoid_bias_topk: logits dtype %d", logits_dtype);
   if (T == 0) return ZMOE_OK;
   dim3 grid((T + 3) / 4), block(128);
-  size_t smem = 4 * (size_t)(2 * E + 64 + 2 * kMaxK) * sizeof(float);
+  size_t smem = 4 * (size_t)(E + 64) * sizeof(float);
   cudaStream_t st = (cudaStream_t)stream;
   dispatch_vpl(E, [&](auto vpl) {
     launch_pdl(sigmoid_topk_kernel<decltype(vpl)::value>, grid, block, smem, st, logits, logits_dtype, T, E, K, bias,
@@ -278,10 +292,19 @@ int zmoe_router_logits(const void* x, const void* wr, int T, int E, int d, void*
   ZMOE_REQUIRE(out_dtype == ZMOE_F32 || out_dtype == ZMOE_BF16, ZMOE_ERR_DTYPE, "zmoe_router_logits: out dtype %d",
                out_dtype);
   if (T == 0) return ZMOE_OK;
-  if (T > 8 && d % 32 == 0 && (T + kRtTok - 1) / kRtTok <= 65535) {
-    launch_pdl(router_logits_mma_kernel, dim3((E + kRtExp - 1) / kRtExp, (T + kRtTok - 1) / kRtTok),
-               dim3(32 * kRtWarps), 0, (cudaStream_t)stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)wr, T, E, d,
-               logits, out_dtype);
+  if (T > 8 && d % 32 == 0 && (T + 15) / 16 <= 65535) {
+    // large tiles as long as they still give each of some 150 SMs two CTAs, the smallest where 16 x 32 would leave SMs idle
+    const long long tiles = (long long)((E + 31) / 32) * ((T + 15) / 16);
+    auto launch = [&](auto kern, int mt, int nt) {
+      launch_pdl(kern, dim3((E + 8 * nt - 1) / (8 * nt), (T + 16 * mt - 1) / (16 * mt)), dim3(32 * kRtWarps), 0,
+                 (cudaStream_t)stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)wr, T, E, d, logits, out_dtype);
+    };
+    if (tiles >= 600)
+      launch(router_logits_mma_kernel<2, 4>, 2, 4);
+    else if (tiles >= 150)
+      launch(router_logits_mma_kernel<1, 4>, 1, 4);
+    else
+      launch(router_logits_mma_kernel<1, 1>, 1, 1);
     return check_launch("zmoe_router_logits");
   }
   dim3 grid((E + 3) / 4, (T + 7) / 8), block(128);
@@ -330,7 +353,7 @@ int zmoe_route(const void* x, const void* wr, int T, int E, int d, int K, int fa
   p.plan = (int*)plan;
   p.counter = counter;
   size_t smem_plan = (size_t)(2 * E + 2 * 128 + 2) * sizeof(int);
-  size_t smem_sig = 4 * (size_t)(2 * E + 64 + 2 * kMaxK) * sizeof(float);
+  size_t smem_sig = 4 * (size_t)(E + 64) * sizeof(float);
   size_t smem = smem_plan > smem_sig ? smem_plan : smem_sig;
   dim3 grid((E + 3) / 4), block(128);
   cudaStream_t st = (cudaStream_t)stream;

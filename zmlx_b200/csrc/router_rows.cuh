@@ -18,53 +18,44 @@ __device__ __forceinline__ float load_logit(const void* p, int dtype, size_t i) 
   return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p)[i]);
 }
 
-// Top-k of the lane-strided values v[j] (expert id = lane + 32*j) by ranking: every value
-// counts how many others beat it under the canonical order (value descending, id ascending);
-// the ranks are a permutation, so the entries ranked below K write themselves straight into
-// slot order.  `scratch` is E + 2 * kMaxK floats owned by the warp.  All lanes end with the
-// winners in sel_val/sel_idx.
+// Top-k of the lane-strided values v[j] (expert id = lane + 32*j) in K rounds of a warp arg-max under the canonical order
+// (value descending, id ascending): one redux for the largest key, one for the lowest id that holds it; the winner leaves the
+// race.  Lane r < K returns the expert of slot r.  The values are left in `vals` (E floats owned by the warp) for the caller to
+// look winners up.  (Ranking every value against every other one took E * VPL comparisons a lane and left the slots' arithmetic
+// to one lane.  us, before -> now: top-8 of 128, 1500 rows 9.5 -> 3.1, 4096 rows 18.8 -> 4.8; of 256 in groups, 512 rows 16.9 ->
+// 8.5.)
 template <int VPL>
-__device__ __forceinline__ void warp_topk_masked(float (&v)[VPL], int E, int K, int lane, float* sel_val,
-                                                 int* sel_idx, float* scratch) {
-  // ranking runs on order-preserving integer keys (ld_order_key): a total order even when a row holds NaN
-  // (NaN ranks below every number), so the ranks are always a permutation and every slot gets written
-  uint32_t* keys = reinterpret_cast<uint32_t*>(scratch);
-  float* out_v = scratch + E;
-  int* out_i = reinterpret_cast<int*>(scratch + E + kMaxK);
-  __syncwarp();
+__device__ __forceinline__ int warp_topk(const float (&v)[VPL], int E, int K, int lane, float* vals) {
+  // order-preserving integer keys (ld_order_key): a total order even when a row holds NaN (NaN ranks below every number)
   uint32_t kv[VPL];
+  uint32_t live = 0u;
 #pragma unroll
   for (int j = 0; j < VPL; ++j) {
     const int idx = lane + 32 * j;
     kv[j] = ld_order_key(v[j] + 0.0f);
-    if (idx < E) keys[idx] = kv[j];
-  }
-  if (lane < K) out_i[lane] = 0;
-  __syncwarp();
-  int rank[VPL];
-#pragma unroll
-  for (int j = 0; j < VPL; ++j) rank[j] = 0;
-  for (int o = 0; o < E; ++o) {
-    const uint32_t ok = keys[o];  // broadcast read
-#pragma unroll
-    for (int j = 0; j < VPL; ++j) {
-      const int idx = lane + 32 * j;
-      rank[j] += (ok > kv[j]) || (ok == kv[j] && o < idx);
+    if (idx < E) {
+      vals[idx] = v[j];
+      live |= 1u << j;
     }
   }
-#pragma unroll
-  for (int j = 0; j < VPL; ++j) {
-    const int idx = lane + 32 * j;
-    if (idx < E && rank[j] < K) {
-      out_v[rank[j]] = v[j];
-      out_i[rank[j]] = idx;
-    }
-  }
-  __syncwarp();
+  int mine = 0;
+#pragma unroll 1
   for (int r = 0; r < K; ++r) {
-    sel_val[r] = out_v[r];
-    sel_idx[r] = min(max(out_i[r], 0), E - 1);
+    uint32_t bk = 0u;
+    int bj = -1;
+#pragma unroll
+    for (int j = 0; j < VPL; ++j)
+      if (((live >> j) & 1u) && (bj < 0 || kv[j] > bk)) {
+        bk = kv[j];
+        bj = j;
+      }
+    const uint32_t mx = __reduce_max_sync(0xffffffffu, bk);
+    const uint32_t win = __reduce_min_sync(0xffffffffu, bj >= 0 && bk == mx ? (uint32_t)(lane + 32 * bj) : 0xffffffffu);
+    if ((int)(win & 31u) == lane) live &= ~(1u << (win >> 5));  // K <= E: there always is a winner
+    if (r == lane) mine = (int)win;
   }
+  __syncwarp();
+  return mine;
 }
 
 // One warp routes one token row (softmax family); see zmoe_router_softmax_topk.
@@ -81,18 +72,16 @@ __device__ __forceinline__ void softmax_topk_row(const void* __restrict__ logits
     v[j] = (idx < E) ? load_logit(logits, dtype, (size_t)row * E + idx) : -CUDART_INF_F;
     mx = fmaxf(mx, v[j]);
   }
-  float sel_val[kMaxK];
-  int sel_idx[kMaxK];
+  // lane i < K owns slot i; sums run over the slots in order 0..K-1 (every lane repeats them)
   if (flavour == ZMOE_ROUTER_TOPK_THEN_SOFTMAX) {
-    warp_topk_masked<VPL>(v, E, K, lane, sel_val, sel_idx, scratch);
-    if (lane == 0) {
-      float m = sel_val[0];
-      float s = 0.0f;
-      for (int i = 0; i < K; ++i) s += expf(sel_val[i] - m);
-      for (int i = 0; i < K; ++i) {
-        weights[(size_t)row * K + i] = expf(sel_val[i] - m) / s;
-        indices[(size_t)row * K + i] = (uint32_t)sel_idx[i];
-      }
+    const int si = warp_topk<VPL>(v, E, K, lane, scratch);
+    const float sv = scratch[si];
+    const float term = expf(sv - __shfl_sync(0xffffffffu, sv, 0));
+    float s = 0.0f;
+    for (int i = 0; i < K; ++i) s += __shfl_sync(0xffffffffu, term, i);
+    if (lane < K) {
+      weights[(size_t)row * K + lane] = term / s;
+      indices[(size_t)row * K + lane] = (uint32_t)si;
     }
     return;
   }
@@ -114,24 +103,23 @@ __device__ __forceinline__ void softmax_topk_row(const void* __restrict__ logits
       if (bias) v[j] += bias[idx];
     }
   }
-  warp_topk_masked<VPL>(v, E, K, lane, sel_val, sel_idx, scratch);
-  if (lane == 0) {
-    float denom = 1.0f;
-    if (renorm) {
-      float sk = 0.0f;
-      for (int i = 0; i < K; ++i) sk += sel_val[i];
-      denom = (renorm == 1) ? sk + 1e-20f : sk;
-    }
-    for (int i = 0; i < K; ++i) {
-      weights[(size_t)row * K + i] = renorm ? sel_val[i] / denom : sel_val[i];
-      indices[(size_t)row * K + i] = (uint32_t)sel_idx[i];
-    }
+  const int si = warp_topk<VPL>(v, E, K, lane, scratch);
+  const float sv = scratch[si];
+  float denom = 1.0f;
+  if (renorm) {
+    float sk = 0.0f;
+    for (int i = 0; i < K; ++i) sk += __shfl_sync(0xffffffffu, sv, i);
+    denom = (renorm == 1) ? sk + 1e-20f : sk;
+  }
+  if (lane < K) {
+    weights[(size_t)row * K + lane] = renorm ? sv / denom : sv;
+    indices[(size_t)row * K + lane] = (uint32_t)si;
   }
 }
 
 // sigmoid + selection bias, optional group-limited selection.  One warp routes one token row;
-// `sc` is 2 * E + 64 + 2 * kMaxK floats of scratch owned by the warp (scores, group scores and
-// keep flags, then the top-k scratch).
+// `sc` is E + 64 floats of scratch owned by the warp (scores, then group scores and keep flags).
+// Groups of whole 32s are scored in registers: expert lane + 32 j belongs to group j / (per / 32).
 template <int VPL>
 __device__ __forceinline__ void sigmoid_topk_row(const void* __restrict__ logits, int dtype, int row, int E, int K,
                                                  const float* __restrict__ bias, int n_group, int topk_group,
@@ -154,22 +142,42 @@ __device__ __forceinline__ void sigmoid_topk_row(const void* __restrict__ logits
   if (n_group > 1) {
     __syncwarp();
     const int per = E / n_group;
-    for (int g0 = 0; g0 < n_group; g0 += 32) {
-      // this build keeps n_group <= 32 (validated on the host); loop kept for clarity
-      int g = g0 + lane;
-      if (g < n_group) {
-        float t1 = -CUDART_INF_F, t2 = -CUDART_INF_F;
-        for (int j = 0; j < per; ++j) {
-          float x = sc[g * per + j];
-          if (x > t1) {
+    if (per % 32 == 0) {
+      float t1 = -CUDART_INF_F, t2 = -CUDART_INF_F;
+#pragma unroll
+      for (int j = 0; j < VPL; ++j) {
+        if (32 * j < E) {
+          if (v[j] > t1) {  // the same comparisons as below: a NaN is nobody's best
             t2 = t1;
-            t1 = x;
-          } else if (x > t2) {
-            t2 = x;
+            t1 = v[j];
+          } else if (v[j] > t2) {
+            t2 = v[j];
+          }
+          if ((j + 1) % (per >> 5) == 0) {  // the group is complete: merge the lanes' (largest, second largest) pairs
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+              const float o1 = __shfl_xor_sync(0xffffffffu, t1, o);
+              const float o2 = __shfl_xor_sync(0xffffffffu, t2, o);
+              t2 = fmaxf(fminf(t1, o1), fmaxf(t2, o2));
+              t1 = fmaxf(t1, o1);
+            }
+            if (lane == 0) gsc[j / (per >> 5)] = t1 + t2;
+            t1 = t2 = -CUDART_INF_F;
           }
         }
-        gsc[g] = t1 + t2;
       }
+    } else if (lane < n_group) {
+      float t1 = -CUDART_INF_F, t2 = -CUDART_INF_F;
+      for (int j = 0; j < per; ++j) {
+        const float x = sc[lane * per + j];
+        if (x > t1) {
+          t2 = t1;
+          t1 = x;
+        } else if (x > t2) {
+          t2 = x;
+        }
+      }
+      gsc[lane] = t1 + t2;
     }
     __syncwarp();
     if (lane < n_group) {
@@ -188,23 +196,17 @@ __device__ __forceinline__ void sigmoid_topk_row(const void* __restrict__ logits
       if (idx < E && gkeep[idx / per] == 0.0f) v[j] = 0.0f;
     }
   }
-  float sel_val[kMaxK];
-  int sel_idx[kMaxK];
-  warp_topk_masked<VPL>(v, E, K, lane, sel_val, sel_idx, sc + E + 64);
-  if (lane == 0) {
-    float aff[kMaxK];
-    float sum = 0.0f;
-    for (int i = 0; i < K; ++i) {
-      aff[i] = sigmoid_stable(load_logit(logits, dtype, (size_t)row * E + sel_idx[i]));
-      sum += aff[i];
-    }
-    float inv = 1.0f / sum;
-    for (int i = 0; i < K; ++i) {
-      float w = aff[i] * inv;
-      if (scale != 1.0f) w = w * scale;
-      weights[(size_t)row * K + i] = w;
-      indices[(size_t)row * K + i] = (uint32_t)sel_idx[i];
-    }
+  __syncwarp();
+  const int si = warp_topk<VPL>(v, E, K, lane, sc);
+  const float aff = sigmoid_stable(load_logit(logits, dtype, (size_t)row * E + si));
+  float sum = 0.0f;
+  for (int i = 0; i < K; ++i) sum += __shfl_sync(0xffffffffu, aff, i);
+  const float inv = 1.0f / sum;
+  float w = aff * inv;
+  if (scale != 1.0f) w = w * scale;
+  if (lane < K) {
+    weights[(size_t)row * K + lane] = w;
+    indices[(size_t)row * K + lane] = (uint32_t)si;
   }
 }
 
