@@ -126,3 +126,17 @@ def test_tensors_the_kernels_cannot_read_are_refused():
     rows = torch.zeros((2, 128), dtype=torch.bfloat16, device=DEV)
     with pytest.raises(ValueError):
         ops.qkv_post(rows, rows.float(), rows, w, w, cos, cos, 1e-6, 2, 1, 0, c, c)
+
+
+@pytest.mark.parametrize("pairs,npos", [(32, 200), (33, 200), (64, 70), (65, 300), (128, 130), (129, 130),  # 8, 4, 2, 1 CTAs
+                                        (2, 8192), (40, 4096), (40, 4097), (130, 1024), (130, 1025), (3, 18000)])
+def test_decode_attention_work_sharing(pairs, npos):
+    """Either side of every cluster size, and of the lengths that several clusters share."""
+    g = torch.Generator(device=DEV).manual_seed(npos)
+    q, kc, vc = _randn(g, pairs, 2, 1, 64, std=2.0), _randn(g, pairs, 1, npos, 64, std=2.0), _randn(g, pairs, 1, npos, 64)
+    kd, vd = kc.double().expand(-1, 2, -1, -1), vc.double().expand(-1, 2, -1, -1)
+    pr = torch.softmax((q.double() @ kd.transpose(-1, -2)) / math.sqrt(64), dim=-1)
+    ref, mass = (pr @ vd)[:, :, 0].reshape(pairs, -1), (pr @ vd.abs())[:, :, 0].reshape(pairs, -1)
+    for _ in range(3):
+        got = ops.decode_attention(q, kc, vc, npos=npos).double()
+        assert bool(((got - ref).abs() <= 2.0 ** -8 * ref.abs() + 2.0 ** -15 * mass).all())

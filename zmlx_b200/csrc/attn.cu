@@ -128,154 +128,221 @@ __global__ void __launch_bounds__(256) qkv_post_kernel(const QkvParams p) {
 
 // ------------------------------------------------------------------ one-token attention over the cache
 // A CTA owns one (sequence, KV head) and a slice of the positions, for all REP query heads that share the KV head: the
-// cache is read once, where the op-by-op form first wrote float32 copies of it.  Per block of 64 positions: scores (a row of keys is split over HD/8 lanes, the REP sums are
-// folded by halving exchanges), a running maximum, probabilities in shared memory, values (a thread owns two
-// dimensions and every fourth position).  Bound by the cache's way from HBM (2 * hd * 2 bytes per position and KV
-// head); slices are as many as fill the chip.  With the norm and q/k kernels above, a decode step of four sequences at
-// position 3000 through four layers went from 3.31 to 0.71 ms (0.62 of it the projections, blocks and the head).
-constexpr int kAttThreads = 256, kAttBlock = 64;
+// cache is read once.  Its eight warps take tiles of 16 positions and never wait for one another: scores by mma.sync (products of
+// bfloat16, exact in fp32, fp32 sums; the heads are the eight columns), a running maximum and sum per warp, probabilities in
+// float32 through the warp's own corner of shared memory, values by float32 multiply-adds (a lane owns HD / 32 dimensions of all
+// heads).  A tile's values and the next tile's keys are on their way while a tile is worked out.
+// The slices of a (sequence, KV head) are the CTAs of a cluster, which joins their results through distributed shared memory and
+// writes the output; only where eight CTAs would be too few for the positions do several clusters share them, and a second
+// kernel joins theirs.  Bound by latency at a few sequences: keys and values of four sequences at position 3000 (25 MB a layer)
+// take 4 us from HBM.  us in a graph, 32 query and 4 KV heads of 128, the form with barriers between scores, probabilities and
+// values and always a second kernel -> now: one sequence at 3000 18.4 -> 11.7, four at 512 8.7 -> 7.5, four at 3000 30.6 -> 17.3,
+// eight at 4200 63.4 -> 23.6.
+constexpr int kAttThreads = 256, kAttTile = 16, kAttWarps = kAttThreads / 32;
 
 struct AttParams {
   const __nv_bfloat16 *q, *kc, *vc;  // (B, Hq, hd), caches (B, Hk, max_seq, hd)
   const long long* pos_dev;          // last valid position, or NULL: npos - 1
-  int npos, hk, max_seq, nsplit;
+  int npos, hk, max_seq, nsplit;  // nsplit: clusters per (sequence, KV head)
   float scale;
-  float* part;  // (B*Hk, nsplit, REP, hd + 2): accumulator, maximum, sum
+  float* part;  // (B*Hk, nsplit, REP, hd + 2): accumulator, maximum, sum; unused with one cluster
   __nv_bfloat16* out;  // (B, Hq, hd)
 };
 
-template <int HD, int REP>
-__global__ void __launch_bounds__(kAttThreads) decode_attn_kernel(const AttParams p) {
-  constexpr int LPR = HD / 8;            // lanes per key row
-  constexpr int RPW = 32 / LPR;          // rows a warp takes at once
-  constexpr int PAIRS = HD / 2;          // value threads across the dimensions
-  constexpr int GRP = kAttThreads / PAIRS;
-  __shared__ float sc[kAttBlock][REP];   // scores, then probabilities
-  __shared__ float red[GRP][REP][HD];
-  __shared__ float run_m[REP], run_s[REP], fac[REP];
+__device__ __forceinline__ void att_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                        uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+template <int HD, int REP, int C>
+__global__ void __launch_bounds__(kAttThreads, 2) decode_attn_kernel(const AttParams p) {
+  constexpr int KJ = HD / 32;  // 16-byte pieces of a key row per lane
+  constexpr int VD = HD / 32;  // dimensions of a lane
+  __shared__ __align__(16) float prob[kAttWarps][kAttTile][8];
+  __shared__ __align__(16) float fac[kAttWarps][8];
+  __shared__ float red[kAttWarps][REP][HD];
+  __shared__ float warp_m[kAttWarps][8], warp_s[kAttWarps][8];
+  __shared__ float mine[REP][HD + 2];  // the CTA's result: accumulator, maximum, sum (read by the cluster)
   pdl_wait();  // from here on plain loads: the non-coherent path must not run ahead of the wait
   pdl_trigger();
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, g = lane >> 2, tig = lane & 3;
   const int pair = blockIdx.y, b = pair / p.hk, kh = pair - b * p.hk;
   const int P = p.pos_dev != nullptr ? min((int)*p.pos_dev + 1, p.max_seq) : p.npos;
-  const int per = ((P + p.nsplit - 1) / p.nsplit + kAttBlock - 1) / kAttBlock * kAttBlock;
+  const int slices = p.nsplit * C, per = ((P + slices - 1) / slices + kAttTile - 1) / kAttTile * kAttTile;
   const int lo = min((int)blockIdx.x * per, P), hi = min(lo + per, P);
   const __nv_bfloat16* kc = p.kc + ((size_t)b * p.hk + kh) * p.max_seq * HD;
   const __nv_bfloat16* vc = p.vc + ((size_t)b * p.hk + kh) * p.max_seq * HD;
-  // this lane's eight dimensions of the REP queries, scaled
-  float q[REP][8];
+  // head g's values as column g of the second operand, in the order in which a lane's 16 bytes serve two mma steps
+  uint4 q[KJ];
 #pragma unroll
-  for (int r = 0; r < REP; ++r) {
-    const uint4 v = *(reinterpret_cast<const uint4*>(p.q + (((size_t)b * p.hk + kh) * REP + r) * HD) + lane % LPR);
-    const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+  for (int j = 0; j < KJ; ++j)
+    q[j] = g < REP ? *(reinterpret_cast<const uint4*>(p.q + (((size_t)b * p.hk + kh) * REP + min(g, REP - 1)) * HD) + tig + 4 * j)
+                   : make_uint4(0u, 0u, 0u, 0u);
+  float m[2] = {-INFINITY, -INFINITY}, sum[2] = {0.0f, 0.0f};  // of heads 2 tig and 2 tig + 1; sums: this lane's share
+  float acc[REP][VD];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      q[r][2 * k] = bf16_bits_to_float(u[k] & 0xffffu);
-      q[r][2 * k + 1] = bf16_bits_to_float(u[k] >> 16);
+  for (int r = 0; r < REP; ++r)
+#pragma unroll
+    for (int k = 0; k < VD; ++k) acc[r][k] = 0.0f;
+  uint4 ka[KJ], kb[KJ];
+  auto keys = [&](int p0) {
+#pragma unroll
+    for (int j = 0; j < KJ; ++j) {
+      const int i0 = p0 + g, i1 = p0 + g + 8;
+      ka[j] = i0 < hi ? *(reinterpret_cast<const uint4*>(kc + (size_t)i0 * HD) + tig + 4 * j) : make_uint4(0u, 0u, 0u, 0u);
+      kb[j] = i1 < hi ? *(reinterpret_cast<const uint4*>(kc + (size_t)i1 * HD) + tig + 4 * j) : make_uint4(0u, 0u, 0u, 0u);
+    }
+  };
+  int p0 = lo + wid * kAttTile;
+  keys(p0);
+#pragma unroll 1
+  for (; p0 < hi; p0 += kAttWarps * kAttTile) {
+    uint32_t v[kAttTile][VD / 2];
+#pragma unroll
+    for (int i = 0; i < kAttTile; ++i) {
+      const __nv_bfloat16* at = vc + (size_t)(p0 + i) * HD + lane * VD;
+      const bool in = p0 + i < hi;
+      if constexpr (VD == 4) {
+        const uint2 two = in ? *reinterpret_cast<const uint2*>(at) : make_uint2(0u, 0u);
+        v[i][0] = two.x;
+        v[i][1] = two.y;
+      } else {
+        v[i][0] = in ? *reinterpret_cast<const uint32_t*>(at) : 0u;
+      }
+    }
+    float c[2][4];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) c[h][k] = 0.0f;
+#pragma unroll
+    for (int j = 0; j < KJ; ++j) {
+      att_mma(c[0], ka[j].x, kb[j].x, ka[j].y, kb[j].y, q[j].x, q[j].y);
+      att_mma(c[1], ka[j].z, kb[j].z, ka[j].w, kb[j].w, q[j].z, q[j].w);
+    }
+    // ---- scores of positions g and g + 8 for heads 2 tig and 2 tig + 1
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const float s0 = p0 + g < hi ? (c[0][h] + c[1][h]) * p.scale : -INFINITY;
+      const float s1 = p0 + g + 8 < hi ? (c[0][h + 2] + c[1][h + 2]) * p.scale : -INFINITY;
+      float top = fmaxf(s0, s1);
+#pragma unroll
+      for (int o = 4; o < 32; o <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+      top = fmaxf(m[h], top);
+      const float ref = top == -INFINITY ? 0.0f : top;  // every score so far is -inf: their weights are 0, not exp(-inf + inf)
+      const float e0 = expf(s0 - ref), e1 = expf(s1 - ref), f = expf(m[h] - ref);
+      m[h] = top;
+      sum[h] = sum[h] * f + (e0 + e1);
+      prob[wid][g][2 * tig + h] = e0;
+      prob[wid][g + 8][2 * tig + h] = e1;
+      if (g == 0) fac[wid][2 * tig + h] = f;
+    }
+    __syncwarp();
+    float fr[8];
+    *reinterpret_cast<float4*>(fr) = *reinterpret_cast<const float4*>(&fac[wid][0]);
+    *reinterpret_cast<float4*>(fr + 4) = *reinterpret_cast<const float4*>(&fac[wid][4]);
+#pragma unroll
+    for (int r = 0; r < REP; ++r)
+#pragma unroll
+      for (int k = 0; k < VD; ++k) acc[r][k] *= fr[r];
+#pragma unroll
+    for (int i = 0; i < kAttTile; ++i) {
+      // the next tile's keys, once half of the values' registers are free
+      if (i == kAttTile / 2 && p0 + kAttWarps * kAttTile < hi) keys(p0 + kAttWarps * kAttTile);
+      float w[8];
+      *reinterpret_cast<float4*>(w) = *reinterpret_cast<const float4*>(&prob[wid][i][0]);
+      if (REP > 4) *reinterpret_cast<float4*>(w + 4) = *reinterpret_cast<const float4*>(&prob[wid][i][4]);
+      float x[VD];
+#pragma unroll
+      for (int k = 0; k < VD; ++k) x[k] = bf16_bits_to_float((k & 1) ? v[i][k >> 1] >> 16 : v[i][k >> 1] & 0xffffu);
+#pragma unroll
+      for (int r = 0; r < REP; ++r)
+#pragma unroll
+        for (int k = 0; k < VD; ++k) acc[r][k] = fmaf(w[r], x[k], acc[r][k]);
+    }
+    __syncwarp();  // the probabilities are used up
+  }
+  // ---- the warps' results under their common maximum
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) sum[h] += __shfl_xor_sync(0xffffffffu, sum[h], o);
+    if (g == 0) {
+      warp_m[wid][2 * tig + h] = m[h];
+      warp_s[wid][2 * tig + h] = sum[h];
     }
   }
-  if (tid < REP) {
-    run_m[tid] = -INFINITY;
-    run_s[tid] = 0.0f;
-  }
-  float acc[REP][2];
 #pragma unroll
-  for (int r = 0; r < REP; ++r) acc[r][0] = acc[r][1] = 0.0f;
-  const int dp = tid % PAIRS, grp = tid / PAIRS;
-
-  for (int p0 = lo; p0 < hi; p0 += kAttBlock) {
-    const int n = min(kAttBlock, hi - p0);
-    // the block's values are requested before the scores are worked out
-    uint32_t vv[kAttBlock / GRP];
+  for (int r = 0; r < REP; ++r)
 #pragma unroll
-    for (int j = 0; j < kAttBlock / GRP; ++j) {
-      const int i = grp + j * GRP;
-      vv[j] = i < n ? *(reinterpret_cast<const uint32_t*>(vc + (size_t)(p0 + i) * HD) + dp) : 0u;
-    }
-    __syncthreads();  // the previous block's probabilities are used up
-#pragma unroll
-    for (int j = 0; j < kAttBlock / (8 * RPW); ++j) {
-      const int i = (j * 8 + wid) * RPW + lane / LPR;
-      float s[REP];
-#pragma unroll
-      for (int r = 0; r < REP; ++r) s[r] = 0.0f;
-      if (i < n) {
-        const uint4 v = *(reinterpret_cast<const uint4*>(kc + (size_t)(p0 + i) * HD) + lane % LPR);
-        const uint32_t u[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const float a0 = bf16_bits_to_float(u[k] & 0xffffu), a1 = bf16_bits_to_float(u[k] >> 16);
-#pragma unroll
-          for (int r = 0; r < REP; ++r) s[r] = fmaf(a1, q[r][2 * k + 1], fmaf(a0, q[r][2 * k], s[r]));
-        }
-      }
-      // fold over the row's lanes: every exchange halves the heads a lane still carries, then plain butterflies
-      int head = 0;
-      int o = LPR >> 1;
-#pragma unroll
-      for (int cnt = REP; cnt > 1 && o > 0; cnt >>= 1, o >>= 1) {
-        const bool up = (lane & o) != 0;
-#pragma unroll
-        for (int r = 0; r < cnt / 2; ++r) {
-          const float give = up ? s[r] : s[r + cnt / 2], keep = up ? s[r + cnt / 2] : s[r];
-          s[r] = keep + __shfl_xor_sync(0xffffffffu, give, o);
-        }
-        if (up) head += cnt / 2;
-      }
-      for (; o > 0; o >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], o);
-      // lanes whose low bits are zero hold one head each
-      if ((lane % LPR) % (LPR / REP) == 0) sc[i][head] = i < n ? s[0] * p.scale : -INFINITY;
-    }
-    __syncthreads();
-    if (wid < REP) {  // one warp per head: running maximum and sum
-      const float s0 = sc[lane][wid], s1 = sc[lane + 32][wid];
-      const float m = fmaxf(run_m[wid], warp_max(fmaxf(s0, s1)));
-      const float ref = m == -INFINITY ? 0.0f : m;  // every score so far is -inf: their weights are 0, not exp(-inf + inf)
-      const float e0 = expf(s0 - ref), e1 = expf(s1 - ref);
-      const float sum = warp_sum(e0 + e1);
-      sc[lane][wid] = e0;
-      sc[lane + 32][wid] = e1;
-      if (lane == 0) {
-        const float f = expf(run_m[wid] - ref);
-        fac[wid] = f;
-        run_s[wid] = run_s[wid] * f + sum;
-        run_m[wid] = m;
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < REP; ++r) {
-      acc[r][0] *= fac[r];
-      acc[r][1] *= fac[r];
-    }
-#pragma unroll
-    for (int j = 0; j < kAttBlock / GRP; ++j) {
-      const int i = grp + j * GRP;
-      if (i < n) {
-        const float v0 = bf16_bits_to_float(vv[j] & 0xffffu), v1 = bf16_bits_to_float(vv[j] >> 16);
-#pragma unroll
-        for (int r = 0; r < REP; ++r) {
-          const float pr = sc[i][r];
-          acc[r][0] = fmaf(pr, v0, acc[r][0]);
-          acc[r][1] = fmaf(pr, v1, acc[r][1]);
-        }
-      }
-    }
-  }
-#pragma unroll
-  for (int r = 0; r < REP; ++r) *reinterpret_cast<float2*>(&red[grp][r][2 * dp]) = make_float2(acc[r][0], acc[r][1]);
+    for (int k = 0; k < VD; ++k) red[wid][r][lane * VD + k] = acc[r][k];
   __syncthreads();
-  float* part = p.part + ((size_t)pair * p.nsplit + blockIdx.x) * REP * (HD + 2);
   for (int i = tid; i < REP * HD; i += kAttThreads) {
-    const int r = i / HD, c = i - r * HD;
-    float t = 0.0f;
+    const int r = i / HD, d = i - r * HD;
+    float top = -INFINITY;
 #pragma unroll
-    for (int k = 0; k < GRP; ++k) t += red[k][r][c];
-    part[r * (HD + 2) + c] = t;
+    for (int w = 0; w < kAttWarps; ++w) top = fmaxf(top, warp_m[w][r]);
+    float num = 0.0f, den = 0.0f;
+#pragma unroll
+    for (int w = 0; w < kAttWarps; ++w) {
+      const float f = warp_m[w][r] == -INFINITY ? 0.0f : expf(warp_m[w][r] - top);  // a warp without a position
+      num = fmaf(f, red[w][r][d], num);
+      den = fmaf(f, warp_s[w][r], den);
+    }
+    mine[r][d] = num;
+    if (d == 0) {
+      mine[r][HD] = top;
+      mine[r][HD + 1] = den;
+    }
   }
-  if (tid < REP) {
-    part[tid * (HD + 2) + HD] = run_m[tid];
-    part[tid * (HD + 2) + HD + 1] = run_s[tid];
+  // ---- the cluster's slices under their common maximum: CTA c takes every C-th run of kAttThreads values
+  if (C > 1) {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  } else {
+    __syncthreads();
+  }
+  auto peer = [&](const float* at, int c) -> float {
+    if (C == 1) return *at;
+    uint32_t addr;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"((uint32_t)__cvta_generic_to_shared(at)), "r"(c));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+    return v;
+  };
+  const int rank = (int)blockIdx.x % C;
+  for (int i = rank * kAttThreads + tid; i < REP * HD; i += C * kAttThreads) {
+    const int r = i / HD, d = i - r * HD;
+    float ms[C], top = -INFINITY;
+#pragma unroll
+    for (int k = 0; k < C; ++k) {
+      ms[k] = peer(&mine[r][HD], k);
+      top = fmaxf(top, ms[k]);
+    }
+    float num = 0.0f, den = 0.0f;
+#pragma unroll
+    for (int k = 0; k < C; ++k) {
+      const float f = ms[k] == -INFINITY ? 0.0f : expf(ms[k] - top);  // an empty slice
+      num = fmaf(f, peer(&mine[r][d], k), num);
+      den = fmaf(f, peer(&mine[r][HD + 1], k), den);
+    }
+    if (p.nsplit == 1) {
+      p.out[((size_t)pair * REP + r) * HD + d] = __float2bfloat16_rn(num / den);
+    } else {
+      float* part = p.part + (((size_t)pair * p.nsplit + blockIdx.x / C) * REP + r) * (HD + 2);
+      part[d] = num;
+      if (d == 0) {
+        part[HD] = top;
+        part[HD + 1] = den;
+      }
+    }
+  }
+  if (C > 1) {  // nobody reads this CTA's results any more
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   }
 }
 
@@ -299,20 +366,51 @@ __global__ void decode_attn_join_kernel(const float* part, int nsplit, int rep, 
   out[(size_t)head * hd + c] = __float2bfloat16_rn(num / den);
 }
 
+// CTAs of a cluster: as many as give every (sequence, KV head) a cluster at two CTAs per SM.
+static int attn_cluster(int B, int hk) {
+  const int pairs = B * hk;
+  return pairs <= 32 ? 8 : pairs <= 64 ? 4 : pairs <= 128 ? 2 : 1;
+}
+// Clusters per (sequence, KV head): one up to 1024 positions a CTA, since a second launch costs more than it gains (four
+// sequences at 4200: three clusters 28 us, one 22); above, about two CTAs per SM in all.
 static int attn_splits(int B, int hk, int max_pos) {
-  const int want = (2 * 148 + B * hk - 1) / (B * hk);  // about two CTAs per SM
-  const int most = (max_pos + kAttBlock - 1) / kAttBlock;
-  return want < most ? want : (most > 0 ? most : 1);
+  const int c = attn_cluster(B, hk), tile = kAttWarps * kAttTile;
+  if (max_pos <= 1024 * c) return 1;
+  const int want = (2 * 148 + B * hk * c - 1) / (B * hk * c);
+  const int most = (max_pos + tile * c - 1) / (tile * c);
+  return want < most ? want : most;
+}
+
+template <int HD, int REP>
+static cudaError_t launch_attn_rep(const AttParams& p, int pairs, int cluster, cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(p.nsplit * cluster, pairs);
+  cfg.blockDim = dim3(kAttThreads);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  switch (cluster) {
+    case 8: return cudaLaunchKernelEx(&cfg, decode_attn_kernel<HD, REP, 8>, p);
+    case 4: return cudaLaunchKernelEx(&cfg, decode_attn_kernel<HD, REP, 4>, p);
+    case 2: return cudaLaunchKernelEx(&cfg, decode_attn_kernel<HD, REP, 2>, p);
+    default: return cudaLaunchKernelEx(&cfg, decode_attn_kernel<HD, REP, 1>, p);
+  }
 }
 
 template <int HD>
-static int launch_attn(const AttParams& p, int rep, dim3 grid, cudaStream_t st) {
+static int launch_attn(const AttParams& p, int rep, int pairs, int cluster, cudaStream_t st) {
   cudaError_t e;
   switch (rep) {
-    case 1: e = launch_pdl(decode_attn_kernel<HD, 1>, grid, dim3(kAttThreads), 0, st, p); break;
-    case 2: e = launch_pdl(decode_attn_kernel<HD, 2>, grid, dim3(kAttThreads), 0, st, p); break;
-    case 4: e = launch_pdl(decode_attn_kernel<HD, 4>, grid, dim3(kAttThreads), 0, st, p); break;
-    default: e = launch_pdl(decode_attn_kernel<HD, 8>, grid, dim3(kAttThreads), 0, st, p); break;
+    case 1: e = launch_attn_rep<HD, 1>(p, pairs, cluster, st); break;
+    case 2: e = launch_attn_rep<HD, 2>(p, pairs, cluster, st); break;
+    case 4: e = launch_attn_rep<HD, 4>(p, pairs, cluster, st); break;
+    default: e = launch_attn_rep<HD, 8>(p, pairs, cluster, st); break;
   }
   if (e != cudaSuccess) return fail(ZMOE_ERR_CUDA, "zmoe_decode_attention: %s", cudaGetErrorString(e));
   return check_launch("decode_attn_kernel");
@@ -411,9 +509,9 @@ int zmoe_decode_attention(const void* q, const void* k_cache, const void* v_cach
   p.out = (__nv_bfloat16*)out;
   cudaStream_t st = (cudaStream_t)stream;
   const int rep = hq / hk;
-  const dim3 grid(p.nsplit, B * hk);
-  const int rc = hd == 128 ? launch_attn<128>(p, rep, grid, st) : launch_attn<64>(p, rep, grid, st);
-  if (rc != ZMOE_OK) return rc;
+  const int cluster = attn_cluster(B, hk);
+  const int rc = hd == 128 ? launch_attn<128>(p, rep, B * hk, cluster, st) : launch_attn<64>(p, rep, B * hk, cluster, st);
+  if (rc != ZMOE_OK || p.nsplit == 1) return rc;
   launch_pdl(decode_attn_join_kernel, dim3(B * hq), dim3(hd), 0, st, (const float*)workspace, p.nsplit, rep, hd,
              (__nv_bfloat16*)out);
   return check_launch("decode_attn_join_kernel");
