@@ -40,6 +40,16 @@ def _indices_or_default(idx, batch_shape, device):
     return idx
 
 
+def _pairs_per_row(rows, batch) -> int:
+    """How many consecutive pairs of the broadcast batch read the same row, when the rows 0, 1, ... of shape ``rows`` are
+    broadcast along trailing dimensions only; 0 otherwise."""
+    rows = (1,) * (len(batch) - len(rows)) + tuple(rows)
+    lead = 0
+    while lead < len(batch) and rows[lead] == batch[lead]:
+        lead += 1
+    return _batch_numel(batch[lead:]) if _batch_numel(rows[lead:]) == 1 else 0
+
+
 def gather_qmm_swiglu(
     x: Any,
     gate_w: Any,
@@ -113,10 +123,18 @@ def gather_qmm_swiglu(
         raise ValueError("[gather_qmm_swiglu] affine mode needs biases.")
 
     dev = x.device
-    lhs = _indices_or_default(lhs_indices, x.shape[:-2], dev)
     rhs = _indices_or_default(rhs_indices, gate_w.shape[:-2], dev)
-    lhs, rhs = torch.broadcast_tensors(lhs, rhs)
-    out_batch = tuple(lhs.shape)
+    # The default rows are 0, 1, ... in the shape of x.  Broadcast along trailing dimensions only, as in a block whose experts
+    # all read the token's row, they need no index tensor: the plan divides.
+    lhs, lhs_div = None, 0
+    if lhs_indices is None:
+        out_batch = tuple(torch.broadcast_shapes(x.shape[:-2], rhs.shape))
+        lhs_div = _pairs_per_row(tuple(x.shape[:-2]), out_batch)
+    if lhs_div == 0:
+        lhs, rhs = torch.broadcast_tensors(_indices_or_default(lhs_indices, x.shape[:-2], dev), rhs)
+        out_batch, lhs_div = tuple(lhs.shape), 1
+    else:
+        rhs = rhs.expand(out_batch)
     E = _batch_numel(gate_w.shape[:-2])
 
     x2 = x.reshape(-1, K)
@@ -131,10 +149,10 @@ def gather_qmm_swiglu(
     gb_ = None if gate_biases is None else gate_biases.reshape(E, N, -1).contiguous()
     ub_ = None if up_biases is None else up_biases.reshape(E, N, -1).contiguous()
 
-    P = lhs.numel()
+    P = rhs.numel()
     if P * M == 0:
         return torch.empty(out_batch + (M, N), dtype=torch.bfloat16, device=dev)
-    plan = ops.build_plan(rhs.reshape(-1), E, M=M, lhs=lhs.reshape(-1))
+    plan = ops.build_plan(rhs, E, M=M, lhs=lhs, lhs_div=lhs_div)
     sw = _lib.SWIGLU_CPU if swiglu_contract == "cpu" else _lib.SWIGLU_PER_OP
     out = ops.gather_qmm_swiglu_rows(x2, gw.contiguous(), gs_, gb_, uw.contiguous(), us_, ub_, plan, P * M,
                                      rows_hint=P * M, group_size=gsz, mode=mode, swiglu=sw)

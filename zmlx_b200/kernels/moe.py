@@ -179,7 +179,7 @@ def moe_dispatch(x: Any, indices: Any) -> Any:
     return x.unsqueeze(-2).expand(*x.shape[:-1], K, x.shape[-1]).contiguous()
 
 
-def _combine(expert_outputs: torch.Tensor, weights: torch.Tensor, mode: int) -> torch.Tensor:
+def _combine(expert_outputs: torch.Tensor, weights: torch.Tensor, mode: int, *, out_t: bool = False) -> torch.Tensor:
     lead = tuple(weights.shape[:-1])
     K = int(weights.shape[-1])
     D = int(expert_outputs.shape[-1])
@@ -189,7 +189,7 @@ def _combine(expert_outputs: torch.Tensor, weights: torch.Tensor, mode: int) -> 
     w = weights.reshape(-1, K)
     if w.dtype not in (torch.bfloat16, torch.float32):
         w = w.to(torch.float32)
-    out = ops.combine(y, w, mode)
+    out = ops.combine(y, w, mode, out_t=out_t)
     return out.reshape(lead + (D,))
 
 
@@ -296,7 +296,7 @@ def _finish_combine(proj: torch.Tensor, gate: torch.Tensor, B: int, streaming: b
         return _cast(out, out_dtype)
     # non-streaming: sum(proj * gate[..., None]) in the promoted dtype (moe.py:2120-2125)
     if gate.dtype == torch.float32 or proj.dtype == torch.float32:
-        out = _combine(proj, _cast(gate, torch.float32), _lib.COMBINE_FP32_NO_FMA)
+        out = _combine(proj, _cast(gate, torch.float32), _lib.COMBINE_FP32_NO_FMA, out_t=out_dtype == torch.bfloat16)
     else:
         out = _combine(proj, gate, _lib.COMBINE_EXACT)
     return _cast(out, out_dtype)

@@ -7,6 +7,7 @@ there is no CPU path.
 
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import math
 
@@ -28,6 +29,14 @@ _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
 
 def _stream():
     return _raw_stream(torch.cuda.current_device())
+
+
+_HERE = contextlib.nullcontext()
+
+
+def _on(dev: torch.device):
+    """``dev`` as the current device; nothing to switch where it is that already (some microseconds a call)."""
+    return _HERE if torch.cuda.current_device() == dev.index else torch.cuda.device(dev)
 
 
 def _need_cuda(*tensors: torch.Tensor | None) -> torch.device:
@@ -67,20 +76,26 @@ def plan_bytes(rows: int, E: int) -> int:
     return int(_lib.load().zmoe_plan_bytes(int(rows), int(E)))
 
 
+def _int32(idx: torch.Tensor) -> torch.Tensor:
+    """Flat int32 indices; the uint32 ones that the routers return are taken as they are."""
+    idx = idx.reshape(-1).contiguous()
+    return idx.view(torch.int32) if idx.dtype == torch.uint32 else idx.to(torch.int32)
+
+
 def build_plan(rhs: torch.Tensor, E: int, *, M: int = 1, lhs: torch.Tensor | None = None, lhs_div: int = 1,
                out: torch.Tensor | None = None) -> torch.Tensor:
     """Group (lhs, rhs) gather pairs by expert; returns the int32 plan buffer."""
     dev = _need_cuda(rhs, lhs)
-    rhs = rhs.reshape(-1).to(torch.int32).contiguous()
+    rhs = _int32(rhs)
     if lhs is not None:
-        lhs = lhs.reshape(-1).to(torch.int32).contiguous()
+        lhs = _int32(lhs)
         if lhs.numel() != rhs.numel():
             raise ValueError("lhs and rhs index counts differ")
     P = rhs.numel()
     nbytes = plan_bytes(P * M, E)
     if out is None:
         out = torch.empty(nbytes // 4, dtype=torch.int32, device=dev)
-    with torch.cuda.device(dev):
+    with _on(dev):
         _lib.check(_lib.load().zmoe_build_plan(_ptr(lhs), int(lhs_div), _ptr(rhs), P, int(M), int(E), _ptr(out),
                                                out.numel() * 4, _stream()))
     return out
@@ -135,7 +150,7 @@ def gather_qmm_swiglu_rows(x2: torch.Tensor, gate_w, gate_s, gate_b, up_w, up_s,
         raise ValueError(f"x has inner dimension {x2.shape[-1]}, weights expect {K}")
     if out is None:
         out = torch.empty((rows, N), dtype=torch.bfloat16, device=dev)
-    with torch.cuda.device(dev):
+    with _on(dev):
         ws = qmm_workspace(rows, E, K, rows_hint=rows_hint, mode=mode, device=dev)
         _lib.check(_lib.load().zmoe_gather_qmm_swiglu_ws(
             _ptr(x2), x2.shape[0], x2.stride(0), _ptr(gate_w), _ptr(gate_s), _ptr(gate_b), _ptr(up_w), _ptr(up_s),
@@ -157,7 +172,7 @@ def gather_qmm_rows(x2: torch.Tensor, w, s, b, plan: torch.Tensor, rows: int, *,
         raise ValueError(f"x has inner dimension {x2.shape[-1]}, weights expect {K}")
     if out is None:
         out = torch.empty((rows, N), dtype=torch.bfloat16, device=dev)
-    with torch.cuda.device(dev):
+    with _on(dev):
         ws = qmm_workspace(rows, E, K, rows_hint=rows_hint, mode=mode, device=dev)
         _lib.check(_lib.load().zmoe_gather_qmm_ws(
             _ptr(x2), x2.shape[0], x2.stride(0), _ptr(w), _ptr(s), _ptr(b), E, N, K, int(group_size),
@@ -182,7 +197,7 @@ def combine(y: torch.Tensor, w: torch.Tensor, mode: int, *, out_t: bool = False,
             raise ValueError("residual must be bfloat16 of shape (T, D)")
     if T == 0:
         return out
-    with torch.cuda.device(dev):
+    with _on(dev):
         for t0 in range(0, T, 65535):
             n = min(T - t0, 65535)
             _lib.check(_lib.load().zmoe_moe_combine(
@@ -202,7 +217,7 @@ def swiglu(gate: torch.Tensor, up: torch.Tensor, *, mode: int = _lib.SWIGLU_PER_
     out = torch.empty_like(g)
     if g.numel() == 0:
         return out
-    with torch.cuda.device(dev):
+    with _on(dev):
         _lib.check(_lib.load().zmoe_swiglu(_ptr(g), _ptr(u), g.numel(), int(mode), _ptr(out), _stream()))
     return out
 
@@ -217,7 +232,7 @@ def router_softmax_topk(logits: torch.Tensor, k: int, *, flavour: int, bias: tor
         bias = bias.reshape(-1).to(torch.float32).contiguous()
     w = torch.empty((T, k), dtype=torch.float32, device=dev)
     idx = torch.empty((T, k), dtype=torch.int32, device=dev)
-    with torch.cuda.device(dev):
+    with _on(dev):
         if T > 0:
             _lib.check(_lib.load().zmoe_router_softmax_topk(_ptr(l2), _dtype_code(l2), T, E, int(k), int(flavour),
                                                             _ptr(bias), int(renorm), _ptr(w), _ptr(idx), _stream()))
@@ -234,7 +249,7 @@ def router_sigmoid_topk(logits: torch.Tensor, bias: torch.Tensor, k: int, *, n_g
     bias = bias.reshape(-1).to(torch.float32).contiguous()
     w = torch.empty((T, k), dtype=torch.float32, device=dev)
     idx = torch.empty((T, k), dtype=torch.int32, device=dev)
-    with torch.cuda.device(dev):
+    with _on(dev):
         if T > 0:
             _lib.check(_lib.load().zmoe_router_sigmoid_bias_topk(_ptr(l2), _dtype_code(l2), T, E, int(k), _ptr(bias),
                                                                  int(n_group), int(topk_group),
@@ -253,7 +268,7 @@ def router_logits(x: torch.Tensor, wr: torch.Tensor, *, out_dtype: torch.dtype =
     wr = wr.contiguous()
     T, E = x2.shape[0], wr.shape[0]
     out = torch.empty((T, E), dtype=out_dtype, device=dev)
-    with torch.cuda.device(dev):
+    with _on(dev):
         if T > 0:
             _lib.check(_lib.load().zmoe_router_logits(_ptr(x2), _ptr(wr), T, E, d, _ptr(out), _dtype_code(out),
                                                       _stream()))
@@ -278,7 +293,7 @@ def add_rms_norm(h: torch.Tensor, delta: torch.Tensor | None, w: torch.Tensor, e
         _dense_bf16("delta", delta, h.numel())
     _dense_bf16("w", w, h.shape[1])
     x = torch.empty_like(h)
-    with torch.cuda.device(dev):
+    with _on(dev):
         _lib.check(_lib.load().zmoe_add_rms_norm(_ptr(h), _ptr(delta), _ptr(w), ctypes.c_float(eps), h.shape[0],
                                                  h.shape[1], _ptr(x), _stream()))
     return x
@@ -294,7 +309,7 @@ def qkv_post(q, k, v, q_norm, k_norm, cos, sin, eps: float, B: int, S: int, pos,
         _dense_bf16(name, t, B * S * heads * hd)
     out = torch.empty((B, hq, S, hd), dtype=torch.bfloat16, device=dev)
     on_dev = isinstance(pos, torch.Tensor)
-    with torch.cuda.device(dev):
+    with _on(dev):
         _lib.check(_lib.load().zmoe_qkv_post(
             _ptr(q), _ptr(k), _ptr(v), _ptr(q_norm), _ptr(k_norm), _ptr(cos), _ptr(sin), ctypes.c_float(eps), B, S, hq,
             hk, hd, _ptr(pos) if on_dev else None, 0 if on_dev else int(pos), max_seq, _ptr(out), _ptr(k_cache),
@@ -316,7 +331,7 @@ def decode_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
         return None
     ws = torch.empty(n, dtype=torch.uint8, device=dev)
     out = torch.empty((B, hq * hd), dtype=torch.bfloat16, device=dev)
-    with torch.cuda.device(dev):
+    with _on(dev):
         _lib.check(lib.zmoe_decode_attention(_ptr(q), _ptr(k_cache), _ptr(v_cache), B, hq, hk, hd, _ptr(pos),
                                              0 if npos is None else int(npos), max_seq,
                                              ctypes.c_float(1.0 / math.sqrt(hd)), _ptr(ws), n, _ptr(out), _stream()))
