@@ -58,3 +58,21 @@ def test_values_around_the_narrow_expansions_reach(of, down, rows):
     plan = ops.build_plan(torch.zeros(rows, dtype=torch.int32, device=DEV), E)
     got = _call(x, rows, K, [(word, s, b)], E, N, "affine", plan, rows, rows, 1, ws)
     _within(got, x.double() @ A.T, x.double().abs() @ A.abs().T, K)
+
+
+@pytest.mark.parametrize("mode", ["affine", "mxfp4"])
+@pytest.mark.parametrize("counts", [[9] * 24, [10] * 24, [1, 40, 3, 17, 16, 0, 33, 8] * 3, [2] * 23 + [170]])
+def test_items_of_16_rows_with_larger_tasks(counts, mode):
+    """Averages of 7 to 10 rows: items of 16 up to 9.6, which larger tasks are cut into."""
+    E, N, K = len(counts), 160, 768
+    g = torch.Generator(device=DEV).manual_seed(len(set(counts)))
+    a, A = _bank(g, E, N, K, mode, False)
+    ids = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))
+    ids = ids[torch.randperm(len(ids), generator=torch.Generator().manual_seed(1))].to(DEV)
+    rows = len(ids)
+    x = torch.randn((rows, K), generator=g, device=DEV).to(torch.bfloat16)
+    ws = ops.qmm_workspace(rows, E, K, rows_hint=rows, mode=mode, device=DEV)
+    got = _call(x, rows, K, [a], E, N, mode, ops.build_plan(ids, E), rows, rows, 1, ws)
+    for e in range(E):
+        m = ids == e
+        _within(got[m], x[m].double() @ A[e].T, x[m].double().abs() @ A[e].abs().T, K)

@@ -986,7 +986,12 @@ int qmm_tma_launch(const QmmParams& q, int nmat, bool mx, int rows_hint, int max
   if (!fine) return fail(ZMOE_ERR_CUDA, "%s: a tensor map was refused", who);
   // Token rows per item: up to twice the average task in whole 16s (a larger task takes several equal blocks); the
   // fewer rows a stage must hold, the more stages are in flight.
+  // While nearly all tasks fit 16 rows -- the average and two standard deviations of evenly routed rows -- the items do: the third
+  // set of expanders is worth more than a weight tile read twice for the few larger ones (gate/up and down, us, blocks of 48 ->
+  // 16: c5 T=150 1157/527 -> 941/497, c2 T=100 74/45 -> 71/42, mxfp4 c3 T=100 70/38 -> 62/36; an average of 12 to 14 is even).
   long long tn = 2ll * q.rows / max_groups + 8;
+  const double avg = (double)q.rows / max_groups;
+  if (avg < 16.0 && (16.0 - avg) * (16.0 - avg) >= 4.0 * avg) tn = 16;
   if (tn > rows_hint) tn = rows_hint;
   tn = (tn + 15) / 16 * 16;
   a.tn = tn > kTmMaxTok ? kTmMaxTok : (int)tn;
