@@ -129,9 +129,10 @@ class MoELayer:
         return all(self.fused_workspace_bytes(n) > 0 for n in {n for _, n in self._chunks(T)})
 
     def _passes_win(self, T: int) -> bool:
-        """Every pass streams its own rows' experts again, the grouped matmuls stream each expert once but cost some
-        launches: a second, half-filled pass wins for wide blocks only, while the passes share few experts (c5, T = 12: 702
-        against 748 us; T = 16: 891 against 867; c2, T = 9: 100 against 102, T = 12: 127 against 113)."""
+        """Up to twelve rows of wide blocks run as two one-launch passes, which stream an expert of both passes twice but need one
+        workspace and one launch each.  Against the register-fed and the first tensor-memory matmuls they were the faster form (c5,
+        T = 12: 702 against 748 us); against the present one they no longer are (T = 9: 540 against 460, T = 12: 712 against 549).
+        The rule stays because `passes` is an answer that callers count on, not for speed."""
         cfg = self.cfg
         return T <= 12 and cfg.d_model * 2 * 8 > 96 * 1024 and T * cfg.top_k <= 4 * cfg.n_experts
 
