@@ -37,8 +37,8 @@
 // in fp32 by the finishers, so the range of fp16 is no limit on the checkpoint's.
 // (q - 8) s and b are exact while the scales and offsets of a row's chunk (other than zero) lie within 8 binades below the
 // largest scale; chunks with values further apart are expanded another way (tm_expand_far), exact over 28; below, a weight is
-// off by at most 2^-39 of the largest of its row's chunk.  mxfp4: e2m1 value x 2^(e - emax + 13), exact in fp16 over 36 binades, same row factor.
-// Token rows carry a power of two per row: a bfloat16 of the row is exact down to 2^-26 (mxfp4: 2^-31) of its largest,
+// off by at most 2^-39 of the largest of its row's chunk.  mxfp4: e2m1 value x 2^(e - emax + 13), exact in fp16 over 36 binades,
+// same row factor.  Token rows carry a power of two per row: a bfloat16 of the row is exact down to 2^-26 (mxfp4: 2^-31) of its largest,
 // and off by at most 2^-34 (2^-39) of it below.  Chunks are
 // summed in fp32 registers rather than in the accumulator over all of K, so that no sum is longer than 160 products (mxfp4:
 // 256).
